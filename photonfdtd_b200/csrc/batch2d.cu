@@ -911,12 +911,11 @@ int pfb_finalize(pf_batch* b, int checkpoint_every, int tile_rows) {
     if ((rc = bup(b, &w, b->h_wave.data(), b->h_wave.size() * 8))) return rc;
     b->src.wave = (const double*)w;
   }
-  if (b->rb == 4) {
-    for (int ax = 0; ax < 2; ++ax) {
-      const float d = (float)(ax == 0 ? b->dx : b->dy);
-      b->rd[ax] = (double)(1.0f / d);
-      b->fd[ax] = !getenv("PFB200_IEEE_DIV") && host_recip_division_exact(d);
-    }
+  for (int ax = 0; ax < 2; ++ax) {
+    const double d = ax == 0 ? b->dx : b->dy;
+    b->rd[ax] = b->rb == 4 ? (double)(1.0f / (float)d) : 1.0 / d;
+    b->fd[ax] = !getenv("PFB200_IEEE_DIV") &&
+                (b->rb == 4 ? host_recip_division_exact((float)d) : host_recip_division_exact(d));
   }
   B_CUDA(b, cudaStreamSynchronize(b->stream));
   b->finalized = true;

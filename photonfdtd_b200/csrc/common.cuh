@@ -24,40 +24,62 @@ __device__ __forceinline__ double fma_rn(double a, double b, double c) { return 
 __device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(a, b); }
 
-// Correctly rounded a / d given r = RN(1/d), by Markstein's correction:
-// q0 = RN(a * r), rem = a - q0 * d (exact with one FMA), q = RN(q0 + rem * r).
-// The host enables it for a divisor d only after checking that it reproduces
-// IEEE a / d for every float significand of a; the identity is invariant
-// under scaling a by powers of two while a stays in [2^-100, 2^90) and the
-// residual cannot underflow. qdiv_fast first scales a by 2^64 (exact), so
-// every |a| < 2^26 - zero and subnormals included - lands in that window,
-// and scales the quotient back by 2^-64, which is exact while the quotient
-// is normal: guaranteed for d <= 2^-23 (the host requires d in
-// [2^-30, 2^-23]). copysign keeps the sign of a zero quotient. The caller
-// guarantees |a| < 2^26 (qdiv_ok); qdiv checks it itself.
-constexpr float kQdivLimit = 0x1p26f;
-__device__ __forceinline__ float qdiv_fast(float a, float d, float r) {
-  const float as = __fmul_rn(a, 0x1p64f);
-  const float q0 = __fmul_rn(as, r);
-  const float rem = __fmaf_rn(-q0, d, as);
-  return copysignf(__fmul_rn(__fmaf_rn(rem, r, q0), 0x1p-64f), a);
-}
-__device__ __forceinline__ float qdiv(float a, float d, float r, bool fast) {
-  if (fast && fabsf(a) < kQdivLimit) return qdiv_fast(a, d, r);
-  return __fdiv_rn(a, d);
-}
-__device__ __forceinline__ double qdiv_fast(double a, double d, double) { return __ddiv_rn(a, d); }
-__device__ __forceinline__ double qdiv(double a, double d, double, bool) { return __ddiv_rn(a, d); }
-// Two exact quotients sharing one range check and one branch: both by the
-// reciprocal path when it applies to both, else each by qdiv.
+// Correctly rounded a / d given r = RN(1/d), by Markstein's correction (P.
+// Markstein, IBM J. Res. Dev. 34(1), 1990): q0 = RN(a r), rem = a - q0 d
+// (exact in one FMA), q = RN(q0 + rem r). Everything runs on numerators
+// prescaled by a power of two (exact), so that rem cannot underflow for any
+// a down to the smallest subnormal, and the quotient is scaled back at the
+// end; rem is formed as q0 d - a, which keeps the sign of a zero quotient.
+//  float: prescale 2^64. The host enables it for a divisor d in [2^-30,
+//    2^-23] only after checking all 2^23 significands of a against IEEE
+//    division. |a| < 2^26 keeps every intermediate below 2^121, and a
+//    quotient is 0 or at least 2^-126, so scaling it back is exact.
+//  double: prescale 2^200, and one more correction: q0 can be two units off,
+//    q1 = RN(q0 - rem r) is one of the two neighbours of a / d, and from such
+//    a q1 Markstein's theorem makes the second correction the rounded
+//    quotient for every d whose significand is not all ones and r = RN(1/d)
+//    (the host checks that, and d in [2^-30, 2^-23]). |a| < 2^700. Quotients
+//    below 2^-1022, where scaling back rounds, may differ from IEEE division
+//    by one unit of 2^-1074.
+// Four FP32 (six FP64) operations per quotient and one to scale it back;
+// sums and differences of scaled quotients are the scaled sums and
+// differences, so a curl scales back once (kUnscale) instead of per term.
 template <typename T>
-__device__ __forceinline__ void qdiv2(T a0, T d0, T r0, bool f0, T a1, T d1, T r1, bool f1,
-                                      T& q0, T& q1);
-// Whether every numerator of a cell may take qdiv_fast.
-__device__ __forceinline__ bool qdiv_ok(float m) { return m < kQdivLimit; }
-__device__ __forceinline__ bool qdiv_ok(double) { return false; }
+struct QScale;
+template <>
+struct QScale<float> {
+  static constexpr float up = 0x1p64f, down = 0x1p-64f, limit = 0x1p26f;
+};
+template <>
+struct QScale<double> {
+  static constexpr double up = 0x1p200, down = 0x1p-200, limit = 0x1p700;
+};
+// Quotient of a prescaled numerator, still scaled.
+__device__ __forceinline__ float qscaled(float as, float d, float r) {
+  const float q0 = __fmul_rn(as, r);
+  return __fmaf_rn(-__fmaf_rn(q0, d, -as), r, q0);
+}
+__device__ __forceinline__ double qscaled(double as, double d, double r) {
+  const double q0 = __dmul_rn(as, r);
+  const double q1 = __fma_rn(-__fma_rn(q0, d, -as), r, q0);
+  return __fma_rn(-__fma_rn(q1, d, -as), r, q1);
+}
+template <typename T>
+__device__ __forceinline__ T qdiv_fast(T a, T d, T r) {
+  return mul_rn(qscaled(mul_rn(a, QScale<T>::up), d, r), QScale<T>::down);
+}
 __device__ __forceinline__ float absmax(float a, float b) { return fmaxf(fabsf(a), fabsf(b)); }
 __device__ __forceinline__ double absmax(double a, double b) { return fmax(fabs(a), fabs(b)); }
+// Whether every numerator of a cell may take qdiv_fast.
+template <typename T>
+__device__ __forceinline__ bool qdiv_ok(T m) { return m < QScale<T>::limit; }
+template <typename T>
+__device__ __forceinline__ T qdiv(T a, T d, T r, bool fast) {
+  if (fast && qdiv_ok(absmax(a, a))) return qdiv_fast(a, d, r);
+  return div_rn(a, d);
+}
+// Two exact quotients sharing one range check and one branch: both by the
+// reciprocal path when it applies to both, else each by qdiv.
 template <typename T>
 __device__ __forceinline__ void qdiv2(T a0, T d0, T r0, bool f0, T a1, T d1, T r1, bool f1,
                                       T& q0, T& q1) {
@@ -136,6 +158,7 @@ struct StepArgs {
   T dx, dy, dz;  // derivative divisors (1 on a collapsed axis)
   T rdx, rdy, rdz;      // RN(1/d) per axis
   bool fdx, fdy, fdz;   // reciprocal division verified exact for that axis
+  bool fdall;           // and for all three
   T ch;          // dt / mu0 rounded to T; the H coefficient is -ch
   const T* Ein[3];
   const T* Hin[3];
@@ -200,8 +223,10 @@ struct EpiParam<T, false> {
 
 enum CeMode { kCeCell1 = 0, kCeCell3 = 1, kCeTable = 2 };
 
-// Host: whether the float reciprocal division of qdiv is exact for divisor d
-// (exhaustive check over all significands; defined in engine.cu).
+// Host: whether the reciprocal division of qdiv is exact for divisor d (float:
+// exhaustive check over all significands; double: the theorem's conditions;
+// defined in engine.cu).
 bool host_recip_division_exact(float d);
+bool host_recip_division_exact(double d);
 
 }  // namespace pfb

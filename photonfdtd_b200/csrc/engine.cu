@@ -266,6 +266,16 @@ bool recip_division_exact_scan(float d) {
   return true;
 }
 
+// The double reciprocal division of qdiv (two corrections): r = 1 / d is
+// correctly rounded here, so Markstein's theorem needs only a divisor whose
+// significand is not all ones, and a range where nothing over- or underflows.
+bool recip_division_exact(double d) {
+  uint64_t bits;
+  memcpy(&bits, &d, 8);
+  const uint64_t frac = (1ull << 52) - 1;
+  return d >= 0x1p-30 && d <= 0x1p-23 && (bits & frac) != frac;
+}
+
 // Bracket one launch of `kind` (0 step, 1 sources, 2 sampling, 3 flush).
 struct LaunchScope {
   pf_engine* e;
@@ -516,6 +526,7 @@ StepArgs<T> step_args(pf_engine* e) {
   a.fdx = e->fdiv[0];
   a.fdy = e->fdiv[1];
   a.fdz = e->fdiv[2];
+  a.fdall = a.fdx && a.fdy && a.fdz;
   a.ch = (T)e->ch;
   for (int ax = 0; ax < 3; ++ax) {
     a.hb0[ax] = e->hb0[ax];
@@ -825,6 +836,7 @@ bool valid_comp(int c) { return c >= 0 && c < 6; }
 
 namespace pfb {
 bool host_recip_division_exact(float d) { return recip_division_exact(d); }
+bool host_recip_division_exact(double d) { return recip_division_exact(d); }
 }  // namespace pfb
 
 // ===========================================================================
@@ -1124,18 +1136,13 @@ int pf_finalize(pf_engine* e) {
     if (const char* v = getenv("PFB200_XCHUNKS")) nch = std::max(1, atoi(v));
     e->fused_chunks = nch;
   }
-  if (e->rb == 4) {
+  {
     const int dims[3] = {e->nx, e->ny, e->nz};
     for (int ax = 0; ax < 3; ++ax) {
-      const float d = (float)e->dl[ax];
-      e->rdl[ax] = (double)(1.0f / d);
-      bool same = false;
-      for (int q = 0; q < ax; ++q)
-        if (dims[q] > 1 && (float)e->dl[q] == d) {
-          e->fdiv[ax] = e->fdiv[q];
-          same = true;
-        }
-      if (!same && dims[ax] > 1 && !getenv("PFB200_IEEE_DIV")) e->fdiv[ax] = recip_division_exact(d);
+      const double d = e->rb == 4 ? (double)(float)e->dl[ax] : e->dl[ax];
+      e->rdl[ax] = e->rb == 4 ? (double)(1.0f / (float)d) : 1.0 / d;
+      if (dims[ax] > 1 && !getenv("PFB200_IEEE_DIV"))
+        e->fdiv[ax] = e->rb == 4 ? recip_division_exact((float)d) : recip_division_exact(d);
     }
   }
   int rc = e->rb == 4 ? finalize_typed<float>(e) : finalize_typed<double>(e);

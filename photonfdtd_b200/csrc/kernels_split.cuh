@@ -19,15 +19,22 @@
 #include "cell3d.cuh"
 
 // Minimum resident 256-thread blocks per SM the split passes are compiled
-// for (register budget 65536 / (256 * n)). Measured on config 3 (384^3 ADE):
-// H at 8 (32 registers, a 12-byte spill) and E at 5 (48 registers) give
-// 1.52 ms of step kernels against 1.77 ms at the compiler's choice (48 / 59
-// registers); E at 6 spills 28 bytes and is slower.
+// for (register budget 65536 / (256 * n)). float: measured on 384^3 cells
+// with ADE, H at 8 (32 registers) and E at 5 (48 registers) give 1.52 ms of
+// step kernels against 1.77 ms at the compiler's choice (48 / 59 registers);
+// E at 6 spills and is slower. double values take two registers each: at the
+// float budgets both passes spill (H 212, E with ADE 404 bytes per thread).
 #ifndef PFB_MINB_H
 #define PFB_MINB_H 8
 #endif
 #ifndef PFB_MINB_E
 #define PFB_MINB_E 5
+#endif
+#ifndef PFB_MINB_H64
+#define PFB_MINB_H64 4
+#endif
+#ifndef PFB_MINB_E64
+#define PFB_MINB_E64 3
 #endif
 
 namespace pfb {
@@ -38,27 +45,49 @@ __device__ __forceinline__ T ld_if(const T* f, long long id, long long off, bool
   return cond ? f[id + off] : T(0);
 }
 
-// Three curl updates sharing one magnitude check of their six numerators:
-// out[c] = f[c] + K[c] * (n[2c]/d[2c] - n[2c+1]/d[2c+1]), the divisors in
-// axis order ax[0..5]. The fast exact division applies when every numerator
-// is within its range, otherwise each division is IEEE.
-template <typename T>
+// Three curl updates of a bulk cell, out[c] = f[c] + K[c] * (d[2c] - d[2c+1])
+// with d the exactly rounded quotients of the differences hi - lo along axes
+// ax[0..5]. `own` holds the cell's three source-field values, `nb` the six
+// neighbours and c[t] the own component each is paired with; sgn = 1: d =
+// (nb - own) / dl (forward, H), -1: d = (own - nb) / dl (backward, E). The
+// own values are prescaled once and each prescaled difference is one FMA
+// (the scaled rounded difference: scaling by a power of two commutes with
+// rounding here), which makes 7 operations per term and component of what
+// took 11 with a difference, a prescale, a quotient and a sign fix per term.
+// One magnitude check covers the six numerators; cells beyond it divide.
+template <typename T, int SGN>
 __device__ __forceinline__ void bulk3(const StepArgs<T>& a, const T f[3], const T K[3],
-                                      const T n[6], const int ax[6], T out[3]) {
+                                      const T own[3], const T nb[6], T out[3]) {
+  constexpr int ax[6] = {1, 2, 2, 0, 0, 1};
+  constexpr int oc[6] = {2, 1, 0, 2, 1, 0};
   const T dl[3] = {a.dx, a.dy, a.dz};
   const T rl[3] = {a.rdx, a.rdy, a.rdz};
-  const bool fl[3] = {a.fdx, a.fdy, a.fdz};
+  const T up = QScale<T>::up;
+  T os[3], n[6];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) os[c] = mul_rn(own[c], up);
+#pragma unroll
+  for (int t = 0; t < 6; ++t)
+    n[t] = SGN > 0 ? fma_rn(nb[t], up, -os[oc[t]]) : fma_rn(-nb[t], up, os[oc[t]]);
   const T m = absmax(absmax(n[0], n[1]), absmax(absmax(n[2], n[3]), absmax(n[4], n[5])));
-  T q[6];
-  if (a.fdx && a.fdy && a.fdz && qdiv_ok(m)) {
+  if (a.fdall && m < QScale<T>::limit * up) {
 #pragma unroll
-    for (int t = 0; t < 6; ++t) q[t] = qdiv_fast(n[t], dl[ax[t]], rl[ax[t]]);
+    for (int c = 0; c < 3; ++c) {
+      const T dA = qscaled(n[2 * c], dl[ax[2 * c]], rl[ax[2 * c]]);
+      const T dB = qscaled(n[2 * c + 1], dl[ax[2 * c + 1]], rl[ax[2 * c + 1]]);
+      out[c] = add_rn(f[c], mul_rn(mul_rn(sub_rn(dA, dB), QScale<T>::down), K[c]));
+    }
   } else {
+    const bool fl[3] = {a.fdx, a.fdy, a.fdz};
+    T q[6];
 #pragma unroll
-    for (int t = 0; t < 6; ++t) q[t] = qdiv(n[t], dl[ax[t]], rl[ax[t]], fl[ax[t]]);
+    for (int t = 0; t < 6; ++t) {
+      const T d = SGN > 0 ? sub_rn(nb[t], own[oc[t]]) : sub_rn(own[oc[t]], nb[t]);
+      q[t] = qdiv(d, dl[ax[t]], rl[ax[t]], fl[ax[t]]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) out[c] = bulk(f[c], K[c], q[2 * c], q[2 * c + 1]);
   }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) out[c] = bulk(f[c], K[c], q[2 * c], q[2 * c + 1]);
 }
 
 __device__ __forceinline__ bool in_box(int i, int j0, int j1, int k0, int k1, const int* b0,
@@ -78,12 +107,11 @@ __device__ __forceinline__ void h_cell(const StepArgs<T>& a, int i, int j, int k
     const T mch = -a.ch;
     const T K[3] = {mch, mch, mch};
     // Hx: +dEz/dy - dEy/dz; Hy: +dEx/dz - dEz/dx; Hz: +dEy/dx - dEx/dy
-    const T n[6] = {sub_rn(a.Ein[2][id + sy], ez), sub_rn(a.Ein[1][id + 1], ey),
-                    sub_rn(a.Ein[0][id + 1], ex), sub_rn(a.Ein[2][id + sx], ez),
-                    sub_rn(a.Ein[1][id + sx], ey), sub_rn(a.Ein[0][id + sy], ex)};
-    const int ax[6] = {1, 2, 2, 0, 0, 1};
+    const T own[3] = {ex, ey, ez};
+    const T nb[6] = {a.Ein[2][id + sy], a.Ein[1][id + 1], a.Ein[0][id + 1],
+                     a.Ein[2][id + sx], a.Ein[1][id + sx], a.Ein[0][id + sy]};
     T h[3];
-    bulk3<T>(a, f, K, n, ax, h);
+    bulk3<T, 1>(a, f, K, own, nb, h);
     a.Hout[0][id] = h[0];
     a.Hout[1][id] = h[1];
     a.Hout[2][id] = h[2];
@@ -111,7 +139,7 @@ __device__ __forceinline__ void h_cell(const StepArgs<T>& a, int i, int j, int k
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256, PFB_MINB_H) k_h_split(const __grid_constant__ StepArgs<T> a) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? PFB_MINB_H : PFB_MINB_H64) k_h_split(const __grid_constant__ StepArgs<T> a) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int i = blockIdx.z;
@@ -202,7 +230,7 @@ __device__ __forceinline__ bool epilogue_block(const EpiArgs<T>& a) {
 // epilogue above (a separate instantiation: the plain pass carries none of
 // its code).
 template <typename T, int CE, bool ADE, bool EPI>
-__global__ void __launch_bounds__(256, PFB_MINB_E)
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? PFB_MINB_E : PFB_MINB_E64)
     k_e_split(const __grid_constant__ StepArgs<T> a,
               const __grid_constant__ typename EpiParam<T, EPI>::type ep) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -246,16 +274,14 @@ __global__ void __launch_bounds__(256, PFB_MINB_E)
   AdeRec<T> rec;
   if (ADE && w) ade_load<T>(a, media, w, rec);
   T e[3];
-  if (box || d3) {
+  if (box) {
     // Ex: +dHz/dy - dHy/dz; Ey: +dHx/dz - dHz/dx; Ez: +dHy/dx - dHx/dy
+    const T own[3] = {hx, hy, hz};
+    bulk3<T, -1>(a, en, K, own, hn, e);
+  } else if (d3) {
     const T n[6] = {sub_rn(hz, hn[0]), sub_rn(hy, hn[1]), sub_rn(hx, hn[2]),
                     sub_rn(hz, hn[3]), sub_rn(hy, hn[4]), sub_rn(hx, hn[5])};
-    if (box) {
-      const int ax[6] = {1, 2, 2, 0, 0, 1};
-      bulk3<T>(a, en, K, n, ax, e);
-    } else {
-      e3<T>(a, i, j, k, en, K, n, e);
-    }
+    e3<T>(a, i, j, k, en, K, n, e);
   } else {
     const bool lx = i > 0, ly = j > 0, lz = k > 0;
     e[0] = upd_ex<T>(a, i, j, k, en[0], K[0], hz, ld_if(a.Hin[2], id, -sy, ly), hy,
