@@ -32,28 +32,28 @@ __device__ __forceinline__ void divide6(const StepArgs<T>& a, const T n[6], cons
 
 // psi element of a term on axis AX at (i, j, k) whose axis index maps to m.
 template <int AX>
-__device__ __forceinline__ int psi_at(int m, int i, int j, int k, int ny, int nz, int np) {
-  if (AX == 0) return (m * ny + j) * nz + k;
-  if (AX == 1) return (i * np + m) * nz + k;
+__device__ __forceinline__ int psi_at(int m, int i, int j, int k, int ny, int pz, int np) {
+  if (AX == 0) return (m * ny + j) * pz + k;
+  if (AX == 1) return (i * np + m) * pz + k;
   return (i * ny + j) * np + m;
 }
 
 // f + k*(dA - dB), then psiA (+k) and psiB (-k) corrections where present.
 template <typename T, int AXA, int AXB>
 __device__ __forceinline__ T curl3(T f, T k, T dA, T dB, int mA, int mB, int i, int j, int k_,
-                                   int ny, int nz, const int* np, const T* bA, const T* cA,
+                                   int ny, int pz, const int* np, const T* bA, const T* cA,
                                    const T* bB, const T* cB, const T* psiAin, T* psiAout,
                                    const T* psiBin, T* psiBout, bool write_psi) {
   f = add_rn(f, mul_rn(sub_rn(dA, dB), k));
   const int pos[3] = {i, j, k_};
   if (mA >= 0) {
-    const int q = psi_at<AXA>(mA, i, j, k_, ny, nz, np[AXA]);
+    const int q = psi_at<AXA>(mA, i, j, k_, ny, pz, np[AXA]);
     const T psi = add_rn(mul_rn(bA[pos[AXA]], psiAin[q]), mul_rn(cA[pos[AXA]], dA));
     if (write_psi) psiAout[q] = psi;
     f = add_rn(f, mul_rn(k, psi));
   }
   if (mB >= 0) {
-    const int q = psi_at<AXB>(mB, i, j, k_, ny, nz, np[AXB]);
+    const int q = psi_at<AXB>(mB, i, j, k_, ny, pz, np[AXB]);
     const T psi = add_rn(mul_rn(bB[pos[AXB]], psiBin[q]), mul_rn(cB[pos[AXB]], dB));
     if (write_psi) psiBout[q] = psi;
     f = add_rn(f, mul_rn(-k, psi));
@@ -74,15 +74,15 @@ __device__ __forceinline__ void h3(const StepArgs<T>& a, int i, int j, int k, co
   const bool fx = i < a.nx - 1, fy = j < a.ny - 1, fz = k < a.nz - 1;
   const int mx = a.maph[0][i], my = a.maph[1][j], mz = a.maph[2][k];
   const T mch = -a.ch;
-  h[0] = (fy && fz) ? curl3<T, 1, 2>(hold[0], mch, d[0], d[1], my, mz, i, j, k, a.ny, a.nz, a.nph,
+  h[0] = (fy && fz) ? curl3<T, 1, 2>(hold[0], mch, d[0], d[1], my, mz, i, j, k, a.ny, a.pz, a.nph,
                                      a.bh[1], a.cph[1], a.bh[2], a.cph[2], a.psiHin[0],
                                      a.psiHout[0], a.psiHin[1], a.psiHout[1], write_psi)
                     : hold[0];
-  h[1] = (fz && fx) ? curl3<T, 2, 0>(hold[1], mch, d[2], d[3], mz, mx, i, j, k, a.ny, a.nz, a.nph,
+  h[1] = (fz && fx) ? curl3<T, 2, 0>(hold[1], mch, d[2], d[3], mz, mx, i, j, k, a.ny, a.pz, a.nph,
                                      a.bh[2], a.cph[2], a.bh[0], a.cph[0], a.psiHin[2],
                                      a.psiHout[2], a.psiHin[3], a.psiHout[3], write_psi)
                     : hold[1];
-  h[2] = (fx && fy) ? curl3<T, 0, 1>(hold[2], mch, d[4], d[5], mx, my, i, j, k, a.ny, a.nz, a.nph,
+  h[2] = (fx && fy) ? curl3<T, 0, 1>(hold[2], mch, d[4], d[5], mx, my, i, j, k, a.ny, a.pz, a.nph,
                                      a.bh[0], a.cph[0], a.bh[1], a.cph[1], a.psiHin[4],
                                      a.psiHout[4], a.psiHin[5], a.psiHout[5], write_psi)
                     : hold[2];
@@ -99,15 +99,15 @@ __device__ __forceinline__ void e3(const StepArgs<T>& a, int i, int j, int k, co
   divide6<T>(a, n, ax, d);
   const bool bx = i >= 1, by = j >= 1, bz = k >= 1;
   const int mx = a.mape[0][i], my = a.mape[1][j], mz = a.mape[2][k];
-  e[0] = (by && bz) ? curl3<T, 1, 2>(eold[0], K[0], d[0], d[1], my, mz, i, j, k, a.ny, a.nz, a.npe,
+  e[0] = (by && bz) ? curl3<T, 1, 2>(eold[0], K[0], d[0], d[1], my, mz, i, j, k, a.ny, a.pz, a.npe,
                                      a.be[1], a.cpe[1], a.be[2], a.cpe[2], a.psiE[0], a.psiE[0],
                                      a.psiE[1], a.psiE[1], true)
                     : eold[0];
-  e[1] = (bz && bx) ? curl3<T, 2, 0>(eold[1], K[1], d[2], d[3], mz, mx, i, j, k, a.ny, a.nz, a.npe,
+  e[1] = (bz && bx) ? curl3<T, 2, 0>(eold[1], K[1], d[2], d[3], mz, mx, i, j, k, a.ny, a.pz, a.npe,
                                      a.be[2], a.cpe[2], a.be[0], a.cpe[0], a.psiE[2], a.psiE[2],
                                      a.psiE[3], a.psiE[3], true)
                     : eold[1];
-  e[2] = (bx && by) ? curl3<T, 0, 1>(eold[2], K[2], d[4], d[5], mx, my, i, j, k, a.ny, a.nz, a.npe,
+  e[2] = (bx && by) ? curl3<T, 0, 1>(eold[2], K[2], d[4], d[5], mx, my, i, j, k, a.ny, a.pz, a.npe,
                                      a.be[0], a.cpe[0], a.be[1], a.cpe[1], a.psiE[4], a.psiE[4],
                                      a.psiE[5], a.psiE[5], true)
                     : eold[2];

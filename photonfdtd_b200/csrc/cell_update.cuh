@@ -43,14 +43,14 @@ __device__ __forceinline__ T bulk(T f, T k, T dA, T dB) {
 // Compact psi index of a term on axis `ax` at (i, j, k), or -1 (bulk).
 template <typename T>
 __device__ __forceinline__ long long psi_index(const int* map, const int* np, int ax, int i, int j,
-                                               int k, int ny, int nz) {
+                                               int k, int ny, int pz) {
   if (ax == 0) {
     const int m = map[i];
-    return m < 0 ? -1 : ((long long)m * ny + j) * nz + k;
+    return m < 0 ? -1 : ((long long)m * ny + j) * pz + k;
   }
   if (ax == 1) {
     const int m = map[j];
-    return m < 0 ? -1 : ((long long)i * np[1] + m) * nz + k;
+    return m < 0 ? -1 : ((long long)i * np[1] + m) * pz + k;
   }
   const int m = map[k];
   return m < 0 ? -1 : ((long long)i * ny + j) * np[2] + m;
@@ -67,11 +67,11 @@ __device__ __forceinline__ T upd_hx(const StepArgs<T>& a, int i, int j, int k, T
   long long qA = -1, qB = -1;
   if (ry) {
     dA = qdiv(sub_rn(ez_jp, ez), a.dy, a.rdy, a.fdy);
-    qA = psi_index<T>(a.maph[1], a.nph, 1, i, j, k, a.ny, a.nz);
+    qA = psi_index<T>(a.maph[1], a.nph, 1, i, j, k, a.ny, a.pz);
   }
   if (rz) {
     dB = qdiv(sub_rn(ey_kp, ey), a.dz, a.rdz, a.fdz);
-    qB = psi_index<T>(a.maph[2], a.nph, 2, i, j, k, a.ny, a.nz);
+    qB = psi_index<T>(a.maph[2], a.nph, 2, i, j, k, a.ny, a.pz);
   }
   return curl_term<T>(h, -a.ch, ry, dA, rz, dB, qA, ry ? a.bh[1][j] : T(0), ry ? a.cph[1][j] : T(0),
                       a.psiHin[0], a.psiHout[0], qB, rz ? a.bh[2][k] : T(0),
@@ -88,11 +88,11 @@ __device__ __forceinline__ T upd_hy(const StepArgs<T>& a, int i, int j, int k, T
   long long qA = -1, qB = -1;
   if (rz) {
     dA = qdiv(sub_rn(ex_kp, ex), a.dz, a.rdz, a.fdz);
-    qA = psi_index<T>(a.maph[2], a.nph, 2, i, j, k, a.ny, a.nz);
+    qA = psi_index<T>(a.maph[2], a.nph, 2, i, j, k, a.ny, a.pz);
   }
   if (rx) {
     dB = qdiv(sub_rn(ez_ip, ez), a.dx, a.rdx, a.fdx);
-    qB = psi_index<T>(a.maph[0], a.nph, 0, i, j, k, a.ny, a.nz);
+    qB = psi_index<T>(a.maph[0], a.nph, 0, i, j, k, a.ny, a.pz);
   }
   return curl_term<T>(h, -a.ch, rz, dA, rx, dB, qA, rz ? a.bh[2][k] : T(0), rz ? a.cph[2][k] : T(0),
                       a.psiHin[2], a.psiHout[2], qB, rx ? a.bh[0][i] : T(0),
@@ -109,11 +109,11 @@ __device__ __forceinline__ T upd_hz(const StepArgs<T>& a, int i, int j, int k, T
   long long qA = -1, qB = -1;
   if (rx) {
     dA = qdiv(sub_rn(ey_ip, ey), a.dx, a.rdx, a.fdx);
-    qA = psi_index<T>(a.maph[0], a.nph, 0, i, j, k, a.ny, a.nz);
+    qA = psi_index<T>(a.maph[0], a.nph, 0, i, j, k, a.ny, a.pz);
   }
   if (ry) {
     dB = qdiv(sub_rn(ex_jp, ex), a.dy, a.rdy, a.fdy);
-    qB = psi_index<T>(a.maph[1], a.nph, 1, i, j, k, a.ny, a.nz);
+    qB = psi_index<T>(a.maph[1], a.nph, 1, i, j, k, a.ny, a.pz);
   }
   return curl_term<T>(h, -a.ch, rx, dA, ry, dB, qA, rx ? a.bh[0][i] : T(0), rx ? a.cph[0][i] : T(0),
                       a.psiHin[4], a.psiHout[4], qB, ry ? a.bh[1][j] : T(0),
@@ -131,11 +131,11 @@ __device__ __forceinline__ T upd_ex(const StepArgs<T>& a, int i, int j, int k, T
   long long qA = -1, qB = -1;
   if (ry) {
     dA = qdiv(sub_rn(hz, hz_jm), a.dy, a.rdy, a.fdy);
-    qA = psi_index<T>(a.mape[1], a.npe, 1, i, j, k, a.ny, a.nz);
+    qA = psi_index<T>(a.mape[1], a.npe, 1, i, j, k, a.ny, a.pz);
   }
   if (rz) {
     dB = qdiv(sub_rn(hy, hy_km), a.dz, a.rdz, a.fdz);
-    qB = psi_index<T>(a.mape[2], a.npe, 2, i, j, k, a.ny, a.nz);
+    qB = psi_index<T>(a.mape[2], a.npe, 2, i, j, k, a.ny, a.pz);
   }
   return curl_term<T>(e, K, ry, dA, rz, dB, qA, ry ? a.be[1][j] : T(0), ry ? a.cpe[1][j] : T(0),
                       a.psiE[0], a.psiE[0], qB, rz ? a.be[2][k] : T(0), rz ? a.cpe[2][k] : T(0),
@@ -152,11 +152,11 @@ __device__ __forceinline__ T upd_ey(const StepArgs<T>& a, int i, int j, int k, T
   long long qA = -1, qB = -1;
   if (rz) {
     dA = qdiv(sub_rn(hx, hx_km), a.dz, a.rdz, a.fdz);
-    qA = psi_index<T>(a.mape[2], a.npe, 2, i, j, k, a.ny, a.nz);
+    qA = psi_index<T>(a.mape[2], a.npe, 2, i, j, k, a.ny, a.pz);
   }
   if (rx) {
     dB = qdiv(sub_rn(hz, hz_im), a.dx, a.rdx, a.fdx);
-    qB = psi_index<T>(a.mape[0], a.npe, 0, i, j, k, a.ny, a.nz);
+    qB = psi_index<T>(a.mape[0], a.npe, 0, i, j, k, a.ny, a.pz);
   }
   return curl_term<T>(e, K, rz, dA, rx, dB, qA, rz ? a.be[2][k] : T(0), rz ? a.cpe[2][k] : T(0),
                       a.psiE[2], a.psiE[2], qB, rx ? a.be[0][i] : T(0), rx ? a.cpe[0][i] : T(0),
@@ -173,11 +173,11 @@ __device__ __forceinline__ T upd_ez(const StepArgs<T>& a, int i, int j, int k, T
   long long qA = -1, qB = -1;
   if (rx) {
     dA = qdiv(sub_rn(hy, hy_im), a.dx, a.rdx, a.fdx);
-    qA = psi_index<T>(a.mape[0], a.npe, 0, i, j, k, a.ny, a.nz);
+    qA = psi_index<T>(a.mape[0], a.npe, 0, i, j, k, a.ny, a.pz);
   }
   if (ry) {
     dB = qdiv(sub_rn(hx, hx_jm), a.dy, a.rdy, a.fdy);
-    qB = psi_index<T>(a.mape[1], a.npe, 1, i, j, k, a.ny, a.nz);
+    qB = psi_index<T>(a.mape[1], a.npe, 1, i, j, k, a.ny, a.pz);
   }
   return curl_term<T>(e, K, rx, dA, ry, dB, qA, rx ? a.be[0][i] : T(0), rx ? a.cpe[0][i] : T(0),
                       a.psiE[4], a.psiE[4], qB, ry ? a.be[1][j] : T(0), ry ? a.cpe[1][j] : T(0),

@@ -147,14 +147,11 @@ struct DftRegion {
   int comps[6];
 };
 
-// Source groups and DFT monitors the split E pass handles itself.
-constexpr int kInlineSrc = 8;
-constexpr int kInlineDft = 4;
-
 // Arguments of one H + E step (split or fused kernels).
 template <typename T>
 struct StepArgs {
   int nx, ny, nz;
+  int pz;  // reals from one row to the next: nz padded to 32 bytes (1 when nz = 1)
   T dx, dy, dz;  // derivative divisors (1 on a collapsed axis)
   T rdx, rdy, rdz;      // RN(1/d) per axis
   bool fdx, fdy, fdz;   // reciprocal division verified exact for that axis
@@ -192,33 +189,6 @@ struct StepArgs {
   long long plev;  // reals per polarisation level
   int lvl;         // polarisation level holding P^n (n & 1)
   int wait_test;   // test hook of the TMA-staged step (pf_set_wait_test)
-};
-
-// Arguments of the split E pass's epilogue (the opt-in in-kernel sources
-// and DFT sampling): the E-family soft sources of this step (group g at
-// block isrc_blk[g], thread isrc_tid[g]) and the samples of the DFT monitors
-// sampled at this step (ring slot idft_slot[m], -1: none). A separate kernel
-// parameter, so the plain E pass does not carry it.
-template <typename T>
-struct EpiArgs {
-  long long step;
-  int n_isrc;
-  int isrc_blk[kInlineSrc], isrc_tid[kInlineSrc];
-  SourceGroups isrc;
-  int n_idft;
-  DftRegion idft[kInlineDft];
-  T* idft_ring[kInlineDft];
-  int idft_slot[kInlineDft];
-};
-// The epilogue parameter of k_e_split<..., EPI>: EpiArgs, or nothing.
-struct NoEpi {};
-template <typename T, bool EPI>
-struct EpiParam {
-  using type = EpiArgs<T>;
-};
-template <typename T>
-struct EpiParam<T, false> {
-  using type = NoEpi;
 };
 
 enum CeMode { kCeCell1 = 0, kCeCell3 = 1, kCeTable = 2 };

@@ -1,12 +1,13 @@
 // engine.cu - the C ABI of libpfb200.so (declared in include/pfb200.h).
 //
 // Device state of one engine (all in HBM for the whole run):
-//   fields   2 time levels x 6 components, C-order (nx, ny, nz); a step reads
-//            level `cur` and writes level `cur ^ 1` (the fused kernel
-//            recomputes H on tile halos, so reads and writes must not alias)
+//   fields   6 components, C-order (nx, ny, nz) with rows padded to 32 bytes
+//            (pz reals, the padding zero). The split and vector passes update
+//            in place (level 0); the fused kernels recompute H on tile halos,
+//            so they read level `cur` and write level `cur ^ 1`
 //   ce       one or three per-cell arrays, or a uint32 word per cell + table
 //   CPML     b/c per axis and stagger, compact maps (-1 = no psi), psi
-//            compacted along its derivative axis; H psi double-buffered
+//            compacted along its derivative axis
 //   ADE      compact polarisation state [level][pole][comp][cells] per medium
 //   monitors sample rings + complex128 accumulators (DFT), block partials +
 //            float64 accumulators (flux)
@@ -29,6 +30,7 @@
 #include "kernels_fused.cuh"
 #include "kernels_split.cuh"
 #include "kernels_tma.cuh"
+#include "kernels_vec3d.cuh"
 
 using namespace pfb;
 
@@ -82,6 +84,9 @@ struct pf_engine {
   double ch = 0;
   long long n_steps = 0;
   long long ncell = 0;
+  int pz = 1;            // row pitch of fields, coefficients, words and psi rows
+  long long ncellp = 0;  // nx * ny * pz
+  bool vec = false;      // 3D with aligned rows: the vector passes
   int kernel = PF_KERNEL_AUTO;
   bool finalized = false;
   long long step = 0;
@@ -125,7 +130,8 @@ struct pf_engine {
   int hb0[3] = {}, hb1[3] = {}, eb0[3] = {}, eb1[3] = {};
   void* psiE[6] = {};
   void* psiH[2][6] = {};
-  long long npsiE[6] = {}, npsiH[6] = {};  // reals per psi array
+  long long npsiE[6] = {}, npsiH[6] = {};  // reals per psi array (padded rows)
+  long long rpsiE[6] = {}, rpsiH[6] = {};  // its rows of nz reals (0: contiguous)
   void* P = nullptr;
   long long plev = 0;  // reals per polarisation level
   void* media = nullptr;
@@ -140,13 +146,6 @@ struct pf_engine {
   TmaMaps maps;
   int* tma_err = nullptr;
   int wait_test = 0;     // pf_set_wait_test: one TMA stage wait runs out
-  // With env PFB200_INLINE=1 the split E pass adds the E-family sources and
-  // writes the DFT samples itself (at most kInlineSrc groups, kInlineDft
-  // monitors). Off by default: on config 3 (384^3) the epilogue instantiation
-  // of the E pass runs 0.08 ms slower per step than the plain one, more than
-  // the 0.024 ms of injection and sampling launches it replaces.
-  bool inline_epi = false;
-  int isrc_blk[kInlineSrc] = {}, isrc_tid[kInlineSrc] = {};
   long long check_every = 0;  // pf_set_check_every: non-finite scan period
   int fused_ty = 8;      // fused tile height (8 or 16), env PFB200_FUSED_TY
   int fused_chunks = 0;  // x chunks per column (0 = auto), env PFB200_XCHUNKS
@@ -225,6 +224,62 @@ int upload(pf_engine* e, void** p, const void* src, size_t bytes) {
   if (rc) return rc;
   if (bytes) PF_CUDA(e, cudaMemcpyAsync(*p, src, bytes, cudaMemcpyHostToDevice, e->stream));
   return PF_OK;
+}
+
+// The compact staging buffer, grown on demand (pf_read_region and copies
+// between compact host arrays and padded rows).
+int stage(pf_engine* e, size_t bytes) {
+  if (bytes <= e->region_bytes) return PF_OK;
+  if (e->region) {
+    PF_CUDA(e, cudaStreamSynchronize(e->stream));
+    cudaFree(e->region);
+    e->dev_bytes -= e->region_bytes;
+    e->region = nullptr;
+    e->region_bytes = 0;
+  }
+  const cudaError_t rc = cudaMalloc(&e->region, bytes);
+  if (rc != cudaSuccess)
+    return fail(e, PF_ERR_OOM, "CUDA error: cudaMalloc of %zu bytes failed", bytes);
+  e->region_bytes = bytes;
+  e->dev_bytes += bytes;
+  return PF_OK;
+}
+
+// Copies `rows` rows of nz elements between a compact array and a device
+// array with the engine's row pitch. `kind` says where the compact side lies;
+// host arrays go through the staging buffer in one contiguous copy.
+int copy_rows(pf_engine* e, void* padded, void* compact, size_t rows, size_t elem,
+              cudaMemcpyKind kind, bool to_padded) {
+  const size_t w = (size_t)e->nz * elem, p = (size_t)e->pz * elem, bytes = rows * w;
+  if (bytes == 0) return PF_OK;
+  if (w == p) {
+    PF_CUDA(e, cudaMemcpyAsync(to_padded ? padded : compact, to_padded ? compact : padded, bytes,
+                               kind, e->stream));
+    return PF_OK;
+  }
+  void* dense = compact;
+  if (kind != cudaMemcpyDeviceToDevice) {
+    int rc = stage(e, bytes);
+    if (rc) return rc;
+    dense = e->region;
+    if (to_padded) PF_CUDA(e, cudaMemcpyAsync(dense, compact, bytes, kind, e->stream));
+  }
+  if (to_padded) {
+    PF_CUDA(e, cudaMemcpy2DAsync(padded, p, dense, w, w, rows, cudaMemcpyDeviceToDevice, e->stream));
+    // the staging buffer is free for the next copy only in stream order
+  } else {
+    PF_CUDA(e, cudaMemcpy2DAsync(dense, w, padded, p, w, rows, cudaMemcpyDeviceToDevice, e->stream));
+    if (dense != compact) PF_CUDA(e, cudaMemcpyAsync(compact, dense, bytes, kind, e->stream));
+  }
+  return PF_OK;
+}
+
+// A cell array of the grid from the host, into new padded device memory.
+int upload_cells(pf_engine* e, void** p, const void* src, size_t elem) {
+  int rc = dalloc(e, p, (size_t)e->ncellp * elem);
+  if (rc) return rc;
+  return copy_rows(e, *p, const_cast<void*>(src), (size_t)e->nx * e->ny, elem,
+                   cudaMemcpyHostToDevice, true);
 }
 
 // Whether qdiv's reciprocal division (q0 = a*r, rem = fma(-q0, d, a),
@@ -330,11 +385,11 @@ EncodeTiledFn encode_fn() {
 // Tiled map over a C-order (nx, ny, nz) array, box (bw along z) x (bh along y)
 // x 1 plane. Zero fill outside the array.
 bool make_map(CUtensorMap* m, void* ptr, CUtensorMapDataType dt, int elem, int nx, int ny, int nz,
-              int bw, int bh) {
+              int pz, int bw, int bh) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return false;
   const cuuint64_t dims[3] = {(cuuint64_t)nz, (cuuint64_t)ny, (cuuint64_t)nx};
-  const cuuint64_t strides[2] = {(cuuint64_t)nz * elem, (cuuint64_t)ny * nz * elem};
+  const cuuint64_t strides[2] = {(cuuint64_t)pz * elem, (cuuint64_t)ny * pz * elem};
   const cuuint32_t box[3] = {(cuuint32_t)bw, (cuuint32_t)bh, 1};
   const cuuint32_t es[3] = {1, 1, 1};
   return enc(m, dt, 3, ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -352,37 +407,40 @@ bool build_maps(pf_engine* e) {
   bool ok = true;
   for (int l = 0; l < 2; ++l)
     for (int c = 0; c < 3; ++c) {
-      ok = ok && make_map(&e->maps.e[l][c], e->E[l][c], dt, S, e->nx, e->ny, e->nz, kBoxW, TY + 2);
-      ok = ok && make_map(&e->maps.h[l][c], e->H[l][c], dt, S, e->nx, e->ny, e->nz, kBoxW, TY + 1);
+      ok = ok && make_map(&e->maps.e[l][c], e->E[l][c], dt, S, e->nx, e->ny, e->nz, e->pz, kBoxW,
+                         TY + 2);
+      ok = ok && make_map(&e->maps.h[l][c], e->H[l][c], dt, S, e->nx, e->ny, e->nz, e->pz, kBoxW,
+                         TY + 1);
     }
   void* wptr = e->ce_mode == PF_CE_TABLE ? (void*)e->word : (void*)e->adeword;
   if (wptr)
     ok = ok && make_map(&e->maps.word, wptr, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, e->nx, e->ny,
-                        e->nz, 32, TY);
+                        e->nz, e->pz, 32, TY);
   if (e->ce_mode != PF_CE_TABLE)
     for (int c = 0; c < 3; ++c)
-      ok = ok && make_map(&e->maps.ce[c], e->ce[c], dt, S, e->nx, e->ny, e->nz, 32, TY);
+      ok = ok && make_map(&e->maps.ce[c], e->ce[c], dt, S, e->nx, e->ny, e->nz, e->pz, 32, TY);
   return ok;
 }
 
 template <typename T>
 int finalize_typed(pf_engine* e) {
   const size_t S = sizeof(T);
-  const long long n = e->ncell;
+  const long long n = e->ncellp;
   const int dims[3] = {e->nx, e->ny, e->nz};
   int rc;
-  for (int lvl = 0; lvl < 2; ++lvl)
+  const int levels = e->fused ? 2 : 1;
+  for (int lvl = 0; lvl < levels; ++lvl)
     for (int c = 0; c < 3; ++c) {
       if ((rc = dalloc(e, &e->E[lvl][c], n * S))) return rc;
       if ((rc = dalloc(e, &e->H[lvl][c], n * S))) return rc;
     }
   // E coefficients
   if (e->ce_mode == PF_CE_CELL1) {
-    if ((rc = upload(e, &e->ce[0], e->h_ce[0].data(), n * S))) return rc;
+    if ((rc = upload_cells(e, &e->ce[0], e->h_ce[0].data(), S))) return rc;
     e->ce[1] = e->ce[2] = e->ce[0];
   } else if (e->ce_mode == PF_CE_CELL3) {
     for (int c = 0; c < 3; ++c)
-      if ((rc = upload(e, &e->ce[c], e->h_ce[c].data(), n * S))) return rc;
+      if ((rc = upload_cells(e, &e->ce[c], e->h_ce[c].data(), S))) return rc;
   } else {
     std::vector<T> tab(e->h_table.size());
     for (size_t q = 0; q < tab.size(); ++q) tab[q] = (T)e->h_table[q];
@@ -426,19 +484,24 @@ int finalize_typed(pf_engine* e) {
     if ((rc = upload(e, (void**)&e->map_e[ax], me.data(), na * 4))) return rc;
     if ((rc = upload(e, (void**)&e->map_h[ax], mh.data(), na * 4))) return rc;
   }
-  const long long nx = e->nx, ny = e->ny, nz = e->nz;
-  // psi extents: the term's derivative axis replaced by its PML cell count
-  const long long eE[6] = {nx * e->npe[1] * nz, nx * ny * e->npe[2], nx * ny * e->npe[2],
-                           (long long)e->npe[0] * ny * nz, (long long)e->npe[0] * ny * nz,
-                           nx * e->npe[1] * nz};
-  const long long eH[6] = {nx * e->nph[1] * nz, nx * ny * e->nph[2], nx * ny * e->nph[2],
-                           (long long)e->nph[0] * ny * nz, (long long)e->nph[0] * ny * nz,
-                           nx * e->nph[1] * nz};
+  const long long nx = e->nx, ny = e->ny, pz = e->pz;
+  // psi extents: the term's derivative axis replaced by its PML cell count;
+  // the x and y layers keep rows along z with the fields' pitch
+  const long long rE[6] = {nx * e->npe[1], 0, 0, e->npe[0] * ny, e->npe[0] * ny, nx * e->npe[1]};
+  const long long rH[6] = {nx * e->nph[1], 0, 0, e->nph[0] * ny, e->nph[0] * ny, nx * e->nph[1]};
+  long long eE[6], eH[6];
+  for (int q = 0; q < 6; ++q) {
+    const bool z = q == 1 || q == 2;
+    e->rpsiE[q] = rE[q];
+    e->rpsiH[q] = rH[q];
+    eE[q] = z ? nx * ny * e->npe[2] : rE[q] * pz;
+    eH[q] = z ? nx * ny * e->nph[2] : rH[q] * pz;
+  }
   for (int q = 0; q < 6; ++q) {
     e->npsiE[q] = eE[q];
     e->npsiH[q] = eH[q];
     if ((rc = dalloc(e, &e->psiE[q], eE[q] * S))) return rc;
-    for (int lvl = 0; lvl < 2; ++lvl)
+    for (int lvl = 0; lvl < levels; ++lvl)
       if ((rc = dalloc(e, &e->psiH[lvl][q], eH[q] * S))) return rc;
   }
   // ADE: two levels of per-medium cell records [pole][component]; each
@@ -467,7 +530,7 @@ int finalize_typed(pf_engine* e) {
     if ((rc = dalloc(e, &e->P, 2 * e->plev * S))) return rc;
     if ((rc = upload(e, &e->media, md.data(), md.size() * sizeof(MediumT<T>)))) return rc;
     if (e->ce_mode == PF_CE_CELL1)
-      if ((rc = upload(e, (void**)&e->adeword, e->h_adeword.data(), n * 4))) return rc;
+      if ((rc = upload_cells(e, (void**)&e->adeword, e->h_adeword.data(), 4))) return rc;
     if (e->ce_mode == PF_CE_TABLE && e->m_ce.size() != (size_t)e->n_media)
       return fail(e, PF_ERR_INVALID, "table mode needs each medium's coefficient");
   }
@@ -481,7 +544,9 @@ int finalize_typed(pf_engine* e) {
     d.n_steps = e->n_steps;
     d.wave = e->wave;
     if (d.n_groups == 0) continue;
-    if ((rc = upload(e, (void**)&d.cell, s.cell.data(), s.cell.size() * 8))) return rc;
+    std::vector<long long> cell(s.cell);
+    for (long long& c : cell) c = c / e->nz * e->pz + c % e->nz;
+    if ((rc = upload(e, (void**)&d.cell, cell.data(), cell.size() * 8))) return rc;
     if ((rc = upload(e, (void**)&d.comp, s.comp.data(), s.comp.size() * 4))) return rc;
     if ((rc = upload(e, (void**)&d.start, s.start.data(), s.start.size() * 4))) return rc;
     if ((rc = upload(e, (void**)&d.wave_row, s.wave_row.data(), s.wave_row.size() * 4))) return rc;
@@ -517,6 +582,7 @@ StepArgs<T> step_args(pf_engine* e) {
   a.nx = e->nx;
   a.ny = e->ny;
   a.nz = e->nz;
+  a.pz = e->pz;
   a.dx = (T)e->dl[0];
   a.dy = (T)e->dl[1];
   a.dz = (T)e->dl[2];
@@ -534,7 +600,7 @@ StepArgs<T> step_args(pf_engine* e) {
     a.eb0[ax] = e->eb0[ax];
     a.eb1[ax] = e->eb1[ax];
   }
-  const int c0 = e->cur, c1 = e->cur ^ 1;
+  const int c0 = e->cur, c1 = e->fused ? e->cur ^ 1 : e->cur;
   for (int c = 0; c < 3; ++c) {
     a.Ein[c] = (const T*)e->E[c0][c];
     a.Hin[c] = (const T*)e->H[c0][c];
@@ -576,9 +642,9 @@ int scan_finite(pf_engine* e) {
   for (int c = 0; c < 6; ++c) {
     const void* f = c < 3 ? e->E[e->cur][c] : e->H[e->cur][c - 3];
     if (e->rb == 4)
-      k_nonfinite<float><<<592, 256, 0, e->stream>>>((const float*)f, e->ncell, flag);
+      k_nonfinite<float><<<592, 256, 0, e->stream>>>((const float*)f, e->ncellp, flag);
     else
-      k_nonfinite<double><<<592, 256, 0, e->stream>>>((const double*)f, e->ncell, flag);
+      k_nonfinite<double><<<592, 256, 0, e->stream>>>((const double*)f, e->ncellp, flag);
   }
   int h = 0;
   PF_CUDA(e, cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
@@ -586,33 +652,61 @@ int scan_finite(pf_engine* e) {
   return h ? fail(e, PF_ERR_NONFINITE, "non-finite field value at step %lld", e->step) : PF_OK;
 }
 
-template <typename T>
-void launch_h_split(pf_engine* e, const StepArgs<T>& a, dim3 g, dim3 b) {
-  k_h_split<T><<<g, b, 0, e->stream>>>(a);
+// Vectors along z per block of the vector passes: 8 (128 bytes of a row) or,
+// where that wastes more of the last block, 4; fewer on short rows. 256^3
+// without CPML: 243 us at 8, 255 at 4; at 32 a warp that touches a layer at
+// the end of a row drags 128 cells along the general path (with CPML 314 us
+// at 8, 461 at 32).
+int vec_lanes(int nzv) {
+  if (nzv <= 2) return nzv;
+  if (nzv <= 4) return 4;
+  return (nzv + 7) / 8 * 8 > (nzv + 3) / 4 * 4 ? 4 : 8;
 }
 
-template <typename T, bool EPI>
-void launch_e_split_epi(pf_engine* e, const StepArgs<T>& a,
-                        const typename EpiParam<T, EPI>::type& ep, dim3 g, dim3 b) {
+// H and E passes over planes [i0, i1).
+template <typename T>
+void launch_h(pf_engine* e, const StepArgs<T>& a, int i0, int i1) {
+  if (e->vec) {
+    const int nzv = (e->nz + kVec<T> - 1) / kVec<T>;
+    const dim3 b(vec_lanes(nzv), kVecThreads / vec_lanes(nzv));
+    k_h_vec<T><<<dim3((nzv + b.x - 1) / b.x, (e->ny + b.y - 1) / b.y, i1 - i0), b, 0, e->stream>>>(
+        a, i0);
+    return;
+  }
+  const dim3 b = e->nz > 1 ? dim3(32, 8) : dim3(1, 256);
+  k_h_split<T><<<dim3((e->nz + b.x - 1) / b.x, (e->ny + b.y - 1) / b.y, e->nx), b, 0, e->stream>>>(
+      a);
+}
+
+template <typename T, int CE, bool ADE>
+void launch_e_mode(pf_engine* e, const StepArgs<T>& a, int i0, int i1) {
+  if (e->vec) {
+    const int nzv = (e->nz + kVec<T> - 1) / kVec<T>;
+    const dim3 b(vec_lanes(nzv), kVecThreads / vec_lanes(nzv));
+    k_e_vec<T, CE, ADE>
+        <<<dim3((nzv + b.x - 1) / b.x, (e->ny + b.y - 1) / b.y, i1 - i0), b, 0, e->stream>>>(a, i0);
+    return;
+  }
+  const dim3 b = e->nz > 1 ? dim3(32, 8) : dim3(1, 256);
+  k_e_split<T, CE, ADE>
+      <<<dim3((e->nz + b.x - 1) / b.x, (e->ny + b.y - 1) / b.y, e->nx), b, 0, e->stream>>>(a);
+}
+
+template <typename T>
+void launch_e(pf_engine* e, const StepArgs<T>& a, int i0, int i1) {
   const bool ade = e->n_media > 0;
   switch (e->ce_mode) {
     case PF_CE_CELL1:
-      if (ade) k_e_split<T, kCeCell1, true, EPI><<<g, b, 0, e->stream>>>(a, ep);
-      else k_e_split<T, kCeCell1, false, EPI><<<g, b, 0, e->stream>>>(a, ep);
+      if (ade) launch_e_mode<T, kCeCell1, true>(e, a, i0, i1);
+      else launch_e_mode<T, kCeCell1, false>(e, a, i0, i1);
       break;
     case PF_CE_CELL3:
-      k_e_split<T, kCeCell3, false, EPI><<<g, b, 0, e->stream>>>(a, ep);
+      launch_e_mode<T, kCeCell3, false>(e, a, i0, i1);
       break;
     default:
-      if (ade) k_e_split<T, kCeTable, true, EPI><<<g, b, 0, e->stream>>>(a, ep);
-      else k_e_split<T, kCeTable, false, EPI><<<g, b, 0, e->stream>>>(a, ep);
+      if (ade) launch_e_mode<T, kCeTable, true>(e, a, i0, i1);
+      else launch_e_mode<T, kCeTable, false>(e, a, i0, i1);
   }
-}
-
-template <typename T>
-void launch_e_split(pf_engine* e, const StepArgs<T>& a, const EpiArgs<T>& ep, dim3 g, dim3 b) {
-  if (e->inline_epi) launch_e_split_epi<T, true>(e, a, ep, g, b);
-  else launch_e_split_epi<T, false>(e, a, NoEpi{}, g, b);
 }
 
 template <typename T>
@@ -649,11 +743,10 @@ int flush_monitors(pf_engine* e) {
 
 // Monitors of step s read the level just written (E at t_e, H at t_h).
 template <typename T>
-int sample_monitors(pf_engine* e, long long s, int lvl, bool dft = true) {
+int sample_monitors(pf_engine* e, long long s, int lvl) {
   if (e->dfts.empty() && e->fluxes.empty()) return PF_OK;
   const Fields6<T> f = level_fields<T>(e, lvl);
   for (DftMon& m : e->dfts) {
-    if (!dft) break;  // the E pass sampled them
     if (s % m.interval) continue;
     if (m.pending == m.ring_cap) {
       int rc = flush_monitors<T>(e);
@@ -662,7 +755,7 @@ int sample_monitors(pf_engine* e, long long s, int lvl, bool dft = true) {
     const int B = 256;
     LaunchScope ls(e, 2);
     k_dft_sample<T><<<(unsigned)((m.r.ncell + B - 1) / B), B, 0, e->stream>>>(
-        m.r, (T*)m.ring, m.pending, f, e->ny, e->nz);
+        m.r, (T*)m.ring, m.pending, f, e->ny, e->pz);
     m.pending++;
   }
   // every flux plane samples every step: up to kFluxBatch planes per launch
@@ -686,7 +779,7 @@ int sample_monitors(pf_engine* e, long long s, int lvl, bool dft = true) {
     }
     LaunchScope ls(e, 2);
     k_flux_sample_batch<T><<<dim3(maxblk, (unsigned)(q1 - q0)), 256, 0, e->stream>>>(fb, f, e->ny,
-                                                                                     e->nz);
+                                                                                     e->pz);
     for (size_t q = q0; q < q1; ++q) e->fluxes[q].pending++;
   }
   return PF_OK;
@@ -708,7 +801,7 @@ template <typename T>
 int record_step(pf_engine* e, long long t) {
   if (t < 0 || t >= e->ring_steps) return fail(e, PF_ERR_STATE, "record slot out of range");
   char* base = e->rec + (size_t)t * e->rec_slot;
-  const size_t S = sizeof(T), n = (size_t)e->ncell * S;
+  const size_t S = sizeof(T), n = (size_t)e->ncellp * S;
   size_t off = 0;
   for (int c = 0; c < 3; ++c, off += n)
     PF_CUDA(e, cudaMemcpyAsync(base + off, e->H[e->cur][c], n, cudaMemcpyDeviceToDevice,
@@ -724,7 +817,7 @@ int record_step(pf_engine* e, long long t) {
     const long long np = (long long)f.p.n0 * f.p.n1;
     k_flux_plane_record<T><<<(unsigned)((np + 255) / 256), 256, 0, e->stream>>>(
         f.p, (const T*)e->E[e->cur][0], (const T*)e->E[e->cur][1], (const T*)e->E[e->cur][2],
-        (T*)f.rec + (size_t)t * 2 * np, e->ny, e->nz);
+        (T*)f.rec + (size_t)t * 2 * np, e->ny, e->pz);
   }
   PF_CUDA(e, cudaGetLastError());
   return PF_OK;
@@ -732,12 +825,11 @@ int record_step(pf_engine* e, long long t) {
 
 template <typename T>
 int advance_typed(pf_engine* e, long long n_sub) {
-  const int nz = e->nz, ny = e->ny, nx = e->nx;
-  const dim3 blk = nz > 1 ? dim3(32, 8) : dim3(1, 256);
-  const dim3 grd((nz + blk.x - 1) / blk.x, (ny + blk.y - 1) / blk.y, nx);
   for (long long t = 0; t < n_sub; ++t) {
     const long long s = e->step;
-    const int nxt = e->cur ^ 1;
+    // the split passes update in place: a cell's pass reads only its own old
+    // value and the other family's fields
+    const int nxt = e->fused ? e->cur ^ 1 : e->cur;
     StepArgs<T> a = step_args<T>(e);
     if (e->fused) {
       int rc;
@@ -758,54 +850,19 @@ int advance_typed(pf_engine* e, long long n_sub) {
     } else {
       {
         LaunchScope ls(e, 0);
-        launch_h_split<T>(e, a, grd, blk);
+        launch_h<T>(e, a, 0, e->nx);
       }
       inject<T>(e, 1, nxt, s);
       a.Hin[0] = a.Hout[0];
       a.Hin[1] = a.Hout[1];
       a.Hin[2] = a.Hout[2];
-      EpiArgs<T> ep;
-      memset(&ep, 0, sizeof ep);
-      if (e->inline_epi) {
-        ep.step = s;
-        ep.n_isrc = (int)e->src[0].cell.size();
-        for (int g = 0; g < ep.n_isrc; ++g) {
-          ep.isrc_blk[g] = e->isrc_blk[g];
-          ep.isrc_tid[g] = e->isrc_tid[g];
-        }
-        ep.isrc = e->src[0].dev;
-        // an adjoint replay (recording) samples no monitor
-        ep.n_idft = e->recording ? 0 : (int)e->dfts.size();
-        // a full ring flushes every monitor, so flush before handing out slots
-        for (const DftMon& dm : e->dfts) {
-          if (!ep.n_idft) break;
-          if (s % dm.interval == 0 && dm.pending == dm.ring_cap) {
-            const int frc = flush_monitors<T>(e);
-            if (frc) return frc;
-            break;
-          }
-        }
-        for (int m = 0; m < ep.n_idft; ++m) {
-          DftMon& dm = e->dfts[m];
-          ep.idft_slot[m] = -1;
-          if (s % dm.interval) continue;
-          ep.idft[m] = dm.r;
-          ep.idft_ring[m] = (T*)dm.ring;
-          ep.idft_slot[m] = dm.pending;
-        }
-      }
       {
         LaunchScope ls(e, 0);
-        launch_e_split<T>(e, a, ep, grd, blk);
+        launch_e<T>(e, a, 0, e->nx);
       }
-      if (e->inline_epi) {
-        for (int m = 0; m < ep.n_idft; ++m)
-          if (ep.idft_slot[m] >= 0) e->dfts[m].pending++;
-      } else {
-        inject<T>(e, 0, nxt, s);
-      }
+      inject<T>(e, 0, nxt, s);
     }
-    int rc = e->recording ? PF_OK : sample_monitors<T>(e, s, nxt, !(e->inline_epi && !e->fused));
+    int rc = e->recording ? PF_OK : sample_monitors<T>(e, s, nxt);
     if (rc) return rc;
     e->cur = nxt;
     e->step++;
@@ -873,6 +930,12 @@ int pf_create(int nx, int ny, int nz, int real_bytes, double dx, double dy, doub
   e->ch = ch;
   e->n_steps = n_steps;
   e->ncell = (long long)nx * ny * nz;
+  // rows padded to 32 bytes, unless that takes a grid past 2^31 cells
+  const int unit = 32 / real_bytes;
+  e->pz = nz > 1 ? (nz + unit - 1) / unit * unit : 1;
+  if ((long long)nx * ny * e->pz > 0x7fffffffLL) e->pz = nz;
+  e->ncellp = (long long)nx * ny * e->pz;
+  e->vec = nx > 1 && ny > 1 && nz > 1 && e->pz % (16 / real_bytes) == 0;
   cudaError_t rc = cudaGetDevice(&e->device);
   if (rc == cudaSuccess) rc = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
   if (rc != cudaSuccess) {
@@ -914,13 +977,12 @@ int pf_set_ce(pf_engine* e, int mode, const void* ce0, const void* ce1, const vo
         return fail(e, PF_ERR_INVALID, "ce word %u at cell %lld exceeds table size %d", w, q, n_table);
       }
     }
-    const size_t wb = (size_t)e->ncell * 4;
     PF_CUDA(e, cudaSetDevice(e->device));
-    if (!e->word) {
-      int rc = dalloc(e, (void**)&e->word, wb);
-      if (rc) return rc;
-    }
-    PF_CUDA(e, cudaMemcpyAsync(e->word, word, wb, cudaMemcpyHostToDevice, e->stream));
+    int rc;
+    if (!e->word && (rc = dalloc(e, (void**)&e->word, (size_t)e->ncellp * 4))) return rc;
+    if ((rc = copy_rows(e, e->word, const_cast<uint32_t*>(word), (size_t)e->nx * e->ny, 4,
+                        cudaMemcpyHostToDevice, true)))
+      return rc;
     PF_CUDA(e, cudaStreamSynchronize(e->stream));
     memcpy(e->word_need, need, sizeof need);
     e->h_table.assign(table, table + n_table);
@@ -1147,20 +1209,6 @@ int pf_finalize(pf_engine* e) {
   }
   int rc = e->rb == 4 ? finalize_typed<float>(e) : finalize_typed<double>(e);
   if (rc) return rc;
-  e->inline_epi = !e->fused && getenv("PFB200_INLINE") &&
-                  e->src[0].cell.size() <= (size_t)kInlineSrc &&
-                  e->dfts.size() <= (size_t)kInlineDft;
-  if (e->inline_epi) {
-    // each E source group's block and thread in the E pass's grid
-    const int bx = e->nz > 1 ? 32 : 1, by = e->nz > 1 ? 8 : 256;
-    const long long gx = (e->nz + bx - 1) / bx, gy = (e->ny + by - 1) / by;
-    for (size_t g = 0; g < e->src[0].cell.size(); ++g) {
-      const long long c = e->src[0].cell[g];
-      const long long i = c / ((long long)e->ny * e->nz), j = (c / e->nz) % e->ny, k = c % e->nz;
-      e->isrc_blk[g] = (int)((i * gy + j / by) * gx + k / bx);
-      e->isrc_tid[g] = (int)((j % by) * bx + k % bx);
-    }
-  }
   // host staging no longer needed
   for (int c = 0; c < 3; ++c) std::vector<char>().swap(e->h_ce[c]);
   std::vector<uint32_t>().swap(e->h_adeword);
@@ -1185,7 +1233,8 @@ int pf_read_field(pf_engine* e, int comp, void* dst) {
   if (!e->finalized) return fail(e, PF_ERR_STATE, "pf_read_field before pf_finalize");
   if (!valid_comp(comp)) return fail(e, PF_ERR_INVALID, "bad component %d", comp);
   void* src = comp < 3 ? e->E[e->cur][comp] : e->H[e->cur][comp - 3];
-  PF_CUDA(e, cudaMemcpyAsync(dst, src, (size_t)e->ncell * e->rb, cudaMemcpyDeviceToHost, e->stream));
+  int rc = copy_rows(e, src, dst, (size_t)e->nx * e->ny, e->rb, cudaMemcpyDeviceToHost, false);
+  if (rc) return rc;
   PF_CUDA(e, cudaStreamSynchronize(e->stream));
   return PF_OK;
 }
@@ -1234,34 +1283,24 @@ int pf_read_region(pf_engine* e, int comp, const int32_t start[3], const int32_t
   const size_t bytes = (size_t)n * e->rb;
   PF_CUDA(e, cudaSetDevice(e->device));
   const void* src = comp < 3 ? e->E[e->cur][comp] : e->H[e->cur][comp - 3];
+  int rc;
   if (n == e->ncell) {  // the whole field: no gather
-    PF_CUDA(e, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, e->stream));
+    if ((rc = copy_rows(e, const_cast<void*>(src), dst, (size_t)e->nx * e->ny, e->rb,
+                        cudaMemcpyDeviceToHost, false)))
+      return rc;
     PF_CUDA(e, cudaStreamSynchronize(e->stream));
     return PF_OK;
   }
-  if (bytes > e->region_bytes) {
-    if (e->region) {
-      PF_CUDA(e, cudaStreamSynchronize(e->stream));
-      cudaFree(e->region);
-      e->dev_bytes -= e->region_bytes;
-      e->region = nullptr;
-      e->region_bytes = 0;
-    }
-    const cudaError_t rc = cudaMalloc(&e->region, bytes);
-    if (rc != cudaSuccess)
-      return fail(e, PF_ERR_OOM, "CUDA error: cudaMalloc of %zu bytes failed", bytes);
-    e->region_bytes = bytes;
-    e->dev_bytes += bytes;
-  }
+  if ((rc = stage(e, bytes))) return rc;
   const int3 st = make_int3(start[0], start[1], start[2]);
   const int3 sd = make_int3(stride[0], stride[1], stride[2]);
   const int3 ct = make_int3(cnt[0], cnt[1], cnt[2]);
   const unsigned g = (unsigned)std::min<long long>((n + 255) / 256, 148LL * 16);
   if (e->rb == 4)
-    k_gather_region<float><<<g, 256, 0, e->stream>>>((const float*)src, e->ny, e->nz, st, sd, ct,
+    k_gather_region<float><<<g, 256, 0, e->stream>>>((const float*)src, e->ny, e->pz, st, sd, ct,
                                                      (float*)e->region);
   else
-    k_gather_region<double><<<g, 256, 0, e->stream>>>((const double*)src, e->ny, e->nz, st, sd,
+    k_gather_region<double><<<g, 256, 0, e->stream>>>((const double*)src, e->ny, e->pz, st, sd,
                                                       ct, (double*)e->region);
   PF_CUDA(e, cudaGetLastError());
   PF_CUDA(e, cudaMemcpyAsync(dst, e->region, bytes, cudaMemcpyDeviceToHost, e->stream));
@@ -1275,28 +1314,38 @@ int pf_write_field(pf_engine* e, int comp, const void* src) {
   if (!valid_comp(comp)) return fail(e, PF_ERR_INVALID, "bad component %d", comp);
   PF_CUDA(e, cudaSetDevice(e->device));
   void* dst = comp < 3 ? e->E[e->cur][comp] : e->H[e->cur][comp - 3];
-  PF_CUDA(e, cudaMemcpyAsync(dst, src, (size_t)e->ncell * e->rb, cudaMemcpyHostToDevice, e->stream));
+  int rc = copy_rows(e, dst, const_cast<void*>(src), (size_t)e->nx * e->ny, e->rb,
+                     cudaMemcpyHostToDevice, true);
+  if (rc) return rc;
   PF_CUDA(e, cudaStreamSynchronize(e->stream));
   return PF_OK;
 }
 
 namespace {
-// The stepping state as a list of (device pointer, bytes) pieces in the
-// order of the state blob: the six current field components, the six E psi
-// arrays, the six current H psi arrays, then the polarisation level holding
-// P^n followed by the one holding P^(n-1) for `step` n.
-std::vector<std::pair<char*, size_t>> state_pieces(pf_engine* e, long long step) {
-  std::vector<std::pair<char*, size_t>> v;
-  const size_t S = e->rb, n = (size_t)e->ncell * S;
-  for (int c = 0; c < 3; ++c) v.push_back({(char*)e->E[e->cur][c], n});
-  for (int c = 0; c < 3; ++c) v.push_back({(char*)e->H[e->cur][c], n});
-  for (int q = 0; q < 6; ++q) v.push_back({(char*)e->psiE[q], (size_t)e->npsiE[q] * S});
-  for (int q = 0; q < 6; ++q) v.push_back({(char*)e->psiH[e->cur][q], (size_t)e->npsiH[q] * S});
+// The stepping state as a list of pieces in the order of the state blob: the
+// six current field components, the six E psi arrays, the six current H psi
+// arrays, then the polarisation level holding P^n followed by the one holding
+// P^(n-1) for `step` n. The blob is compact: pieces with rows along z (rows
+// > 0) lose their padding.
+struct StatePiece {
+  char* p;
+  size_t rows, bytes;  // bytes in the blob
+};
+std::vector<StatePiece> state_pieces(pf_engine* e, long long step) {
+  std::vector<StatePiece> v;
+  const size_t S = e->rb, rows = (size_t)e->nx * e->ny, w = (size_t)e->nz * S;
+  auto psi = [&](void* p, long long r, long long n) {
+    v.push_back({(char*)p, (size_t)r, r ? (size_t)r * w : (size_t)n * S});
+  };
+  for (int c = 0; c < 3; ++c) v.push_back({(char*)e->E[e->cur][c], rows, rows * w});
+  for (int c = 0; c < 3; ++c) v.push_back({(char*)e->H[e->cur][c], rows, rows * w});
+  for (int q = 0; q < 6; ++q) psi(e->psiE[q], e->rpsiE[q], e->npsiE[q]);
+  for (int q = 0; q < 6; ++q) psi(e->psiH[e->cur][q], e->rpsiH[q], e->npsiH[q]);
   if (e->n_media > 0) {
     const size_t lev = (size_t)e->plev * S;
     const int ln = (int)(step & 1);
-    v.push_back({(char*)e->P + ln * lev, lev});
-    v.push_back({(char*)e->P + (ln ^ 1) * lev, lev});
+    v.push_back({(char*)e->P + ln * lev, 0, lev});
+    v.push_back({(char*)e->P + (ln ^ 1) * lev, 0, lev});
   }
   return v;
 }
@@ -1306,7 +1355,7 @@ int copy_state(pf_engine* e, long long step, void* buf, int64_t bytes, int on_de
   if (!e->finalized) return fail(e, PF_ERR_STATE, "state access before pf_finalize");
   const auto pieces = state_pieces(e, step);
   size_t total = 0;
-  for (const auto& p : pieces) total += p.second;
+  for (const auto& p : pieces) total += p.bytes;
   if ((int64_t)total != bytes)
     return fail(e, PF_ERR_INVALID, "state buffer holds %lld bytes, the state is %zu",
                 (long long)bytes, total);
@@ -1315,12 +1364,14 @@ int copy_state(pf_engine* e, long long step, void* buf, int64_t bytes, int on_de
                                         : (get ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice);
   size_t off = 0;
   for (const auto& p : pieces) {
-    if (p.second) {
-      char* b = (char*)buf + off;
-      if (get) PF_CUDA(e, cudaMemcpyAsync(b, p.first, p.second, kind, e->stream));
-      else PF_CUDA(e, cudaMemcpyAsync(p.first, b, p.second, kind, e->stream));
+    char* b = (char*)buf + off;
+    off += p.bytes;
+    if (p.rows) {
+      int rc = copy_rows(e, p.p, b, p.rows, e->rb, kind, !get);
+      if (rc) return rc;
+    } else if (p.bytes) {
+      PF_CUDA(e, cudaMemcpyAsync(get ? b : p.p, get ? p.p : b, p.bytes, kind, e->stream));
     }
-    off += p.second;
   }
   PF_CUDA(e, cudaStreamSynchronize(e->stream));
   return PF_OK;
@@ -1331,7 +1382,7 @@ int pf_state_bytes(const pf_engine* e, int64_t* bytes) {
   if (!e || !bytes) return PF_ERR_INVALID;
   if (!e->finalized) return PF_ERR_STATE;
   size_t total = 0;
-  for (const auto& p : state_pieces(const_cast<pf_engine*>(e), e->step)) total += p.second;
+  for (const auto& p : state_pieces(const_cast<pf_engine*>(e), e->step)) total += p.bytes;
   *bytes = (int64_t)total;
   return PF_OK;
 }
@@ -1456,7 +1507,7 @@ AdjState<T> adj_state(pf_engine* e, long long slot) {
   AdjState<T> s;
   memset(&s, 0, sizeof s);
   const char* base = e->rec + (size_t)slot * e->rec_slot;
-  const size_t S = sizeof(T), n = (size_t)e->ncell * S;
+  const size_t S = sizeof(T), n = (size_t)e->ncellp * S;
   size_t off = 0;
   for (int c = 0; c < 3; ++c, off += n) s.Hrec[c] = (const T*)(base + off);
   for (int q = 0; q < 6; ++q) {
@@ -1474,11 +1525,10 @@ AdjState<T> adj_state(pf_engine* e, long long slot) {
     s.lpH[q] = (T*)e->lpH[q];
   }
   s.grad = e->grad;
-  s.ncell = e->ncell;
   // per-component coefficients are differentiated per component; one
   // coefficient per cell needs only the sum (16 instead of 48 bytes of
   // gradient traffic per cell and reverse step)
-  s.gstride = e->ce_mode == PF_CE_CELL3 ? e->ncell : 0;
+  s.gstride = e->ce_mode == PF_CE_CELL3 ? e->ncellp : 0;
   for (int a = 0; a < 3; ++a) s.idl[a] = (T)(1.0 / e->dl[a]);
   return s;
 }
@@ -1497,19 +1547,19 @@ int adj_sources(pf_engine* e, long long m, int fam, const AdjState<T>& st, long 
     const double* ph = (fam == 0 ? dm.ph_e : dm.ph_h) + q * dm.n_freq * 2;
     const long long nt = dm.r.ncell * dm.r.ncomp;
     k_adj_dft_src<T><<<(unsigned)((nt + B - 1) / B), B, 0, e->stream>>>(
-        dm.r, e->dft_cot[k], ph, dm.n_freq, dm.dt, fam, l[0], l[1], l[2], e->ny, e->nz);
+        dm.r, e->dft_cot[k], ph, dm.n_freq, dm.dt, fam, l[0], l[1], l[2], e->ny, e->pz);
   }
   for (const FluxMon& f : e->fluxes) {
     if (f.cot == 0.0) continue;
     const long long np = (long long)f.p.n0 * f.p.n1;
     k_adj_flux_src<T><<<(unsigned)((np + B - 1) / B), B, 0, e->stream>>>(
         f.p, f.cot * f.dA * f.dt, fam, st.Hrec[0], st.Hrec[1], st.Hrec[2],
-        (const T*)f.rec + (size_t)slot * 2 * np, l[0], l[1], l[2], e->ny, e->nz);
+        (const T*)f.rec + (size_t)slot * 2 * np, l[0], l[1], l[2], e->ny, e->pz);
   }
   for (const auto& rs : e->rsrc) {
     if (rs.step != m || (rs.comp >= 3) != (fam == 1)) continue;
     k_adj_region_src<T><<<(unsigned)((rs.r.ncell + B - 1) / B), B, 0, e->stream>>>(
-        rs.r, rs.vals, l[rs.comp % 3], e->ny, e->nz);
+        rs.r, rs.vals, l[rs.comp % 3], e->ny, e->pz);
   }
   PF_CUDA(e, cudaGetLastError());
   return PF_OK;
@@ -1545,7 +1595,7 @@ int adj_segment_typed(pf_engine* e, long long step0, long long n) {
 }
 
 int adj_zero(pf_engine* e) {
-  const size_t S = e->rb, n = (size_t)e->ncell * S;
+  const size_t S = e->rb, n = (size_t)e->ncellp * S;
   for (int c = 0; c < 3; ++c) {
     PF_CUDA(e, cudaMemsetAsync(e->lamE[c], 0, n, e->stream));
     PF_CUDA(e, cudaMemsetAsync(e->lamH[c], 0, n, e->stream));
@@ -1556,7 +1606,7 @@ int adj_zero(pf_engine* e) {
     if (e->npsiE[q]) PF_CUDA(e, cudaMemsetAsync(e->lpE[q], 0, e->npsiE[q] * S, e->stream));
     if (e->npsiH[q]) PF_CUDA(e, cudaMemsetAsync(e->lpH[q], 0, e->npsiH[q] * S, e->stream));
   }
-  PF_CUDA(e, cudaMemsetAsync(e->grad, 0, (size_t)e->ncell * 24, e->stream));
+  PF_CUDA(e, cudaMemsetAsync(e->grad, 0, (size_t)e->ncellp * 24, e->stream));
   PF_CUDA(e, cudaStreamSynchronize(e->stream));
   e->adj_next = e->n_steps;
   return PF_OK;
@@ -1590,7 +1640,7 @@ int pf_adj_init(pf_engine* e, int64_t ring_steps) {
     return fail(e, PF_ERR_INVALID, "ring_steps %lld outside [1, n_steps]", (long long)ring_steps);
   PF_CUDA(e, cudaSetDevice(e->device));
   int rc;
-  const size_t S = e->rb, n = (size_t)e->ncell * S;
+  const size_t S = e->rb, n = (size_t)e->ncellp * S;
   if (!e->adj) {
     for (int c = 0; c < 3; ++c) {
       if ((rc = dalloc(e, &e->lamE[c], n))) return rc;
@@ -1602,7 +1652,7 @@ int pf_adj_init(pf_engine* e, int64_t ring_steps) {
       if ((rc = dalloc(e, &e->lpE[q], e->npsiE[q] * S))) return rc;
       if ((rc = dalloc(e, &e->lpH[q], e->npsiH[q] * S))) return rc;
     }
-    if ((rc = dalloc(e, (void**)&e->grad, (size_t)e->ncell * 24))) return rc;
+    if ((rc = dalloc(e, (void**)&e->grad, (size_t)e->ncellp * 24))) return rc;
     e->dft_cot.assign(e->dfts.size(), nullptr);
     e->adj = true;
   }
@@ -1690,7 +1740,9 @@ int pf_adj_read_grad_components(pf_engine* e, double* dst) {
                 "per-component gradient kept only for per-component coefficients "
                 "(PF_CE_CELL3); use pf_adj_read_grad");
   PF_CUDA(e, cudaSetDevice(e->device));
-  PF_CUDA(e, cudaMemcpy(dst, e->grad, (size_t)e->ncell * 24, cudaMemcpyDeviceToHost));
+  int rc = copy_rows(e, e->grad, dst, (size_t)e->nx * e->ny * 3, 8, cudaMemcpyDeviceToHost, false);
+  if (rc) return rc;
+  PF_CUDA(e, cudaStreamSynchronize(e->stream));
   return PF_OK;
 }
 
@@ -1700,7 +1752,9 @@ int pf_adj_read_grad(pf_engine* e, double* dst) {
   const size_t n = (size_t)e->ncell;
   if (e->ce_mode != PF_CE_CELL3) {  // accumulated summed over the components
     PF_CUDA(e, cudaSetDevice(e->device));
-    PF_CUDA(e, cudaMemcpy(dst, e->grad, n * 8, cudaMemcpyDeviceToHost));
+    int rc = copy_rows(e, e->grad, dst, (size_t)e->nx * e->ny, 8, cudaMemcpyDeviceToHost, false);
+    if (rc) return rc;
+    PF_CUDA(e, cudaStreamSynchronize(e->stream));
     return PF_OK;
   }
   std::vector<double> g(n * 3);

@@ -40,8 +40,7 @@ struct AdjState {
   T* lpE[6];  // psi adjoints (compact, like psiE / psiH)
   T* lpH[6];
   double* grad;  // dJ/dK: per component (Ex cells, then Ey, then Ez) or summed
-  long long ncell;
-  long long gstride;  // ncell: one gradient per component; 0: the three summed
+  long long gstride;  // cells of a padded grid: one gradient per component; 0: the three summed
   T idl[3];      // 1 / dl per axis
 };
 
@@ -83,7 +82,7 @@ __global__ void __launch_bounds__(256) k_adj_e(const __grid_constant__ StepArgs<
   if (k >= a.nz || j >= a.ny) return;
   const int n[3] = {a.nx, a.ny, a.nz};
   const int pos[3] = {i, j, k};
-  const long long st[3] = {(long long)a.ny * a.nz, a.nz, 1};
+  const long long st[3] = {(long long)a.ny * a.pz, a.pz, 1};
   const long long id = i * st[0] + j * st[1] + k;
   const T dl[3] = {a.dx, a.dy, a.dz};
   T K[3];
@@ -117,8 +116,8 @@ __global__ void __launch_bounds__(256) k_adj_e(const __grid_constant__ StepArgs<
       const T dA = rA ? div_rn(sub_rn(HA[id], HA[id - st[axA]]), dl[axA]) : T(0);
       const T dB = rB ? div_rn(sub_rn(HB[id], HB[id - st[axB]]), dl[axB]) : T(0);
       T g = sub_rn(dA, dB);
-      const long long qA = rA ? psi_index<T>(a.mape[axA], a.npe, axA, i, j, k, a.ny, a.nz) : -1;
-      const long long qB = rB ? psi_index<T>(a.mape[axB], a.npe, axB, i, j, k, a.ny, a.nz) : -1;
+      const long long qA = rA ? psi_index<T>(a.mape[axA], a.npe, axA, i, j, k, a.ny, a.pz) : -1;
+      const long long qB = rB ? psi_index<T>(a.mape[axB], a.npe, axB, i, j, k, a.ny, a.pz) : -1;
       if (qA >= 0) g = add_rn(g, s.psiErec[2 * c][qA]);
       if (qB >= 0) g = sub_rn(g, s.psiErec[2 * c + 1][qB]);
       const double gc = __dmul_rn((double)x, (double)g);
@@ -143,7 +142,7 @@ __global__ void __launch_bounds__(256) k_adj_h(const __grid_constant__ StepArgs<
   if (k >= a.nz || j >= a.ny) return;
   const int n[3] = {a.nx, a.ny, a.nz};
   const int pos[3] = {i, j, k};
-  const long long st[3] = {(long long)a.ny * a.nz, a.nz, 1};
+  const long long st[3] = {(long long)a.ny * a.pz, a.pz, 1};
   const long long id = i * st[0] + j * st[1] + k;
   const T K = -a.ch;
 #pragma unroll
@@ -168,8 +167,8 @@ __global__ void __launch_bounds__(256) k_adj_h(const __grid_constant__ StepArgs<
     const bool upd = (!rA || pos[axA] < n[axA] - 1) && (!rB || pos[axB] < n[axB] - 1) && (rA || rB);
     T qa = T(0), qb = T(0);
     if (upd) {
-      const long long qA = rA ? psi_index<T>(a.maph[axA], a.nph, axA, i, j, k, a.ny, a.nz) : -1;
-      const long long qB = rB ? psi_index<T>(a.maph[axB], a.nph, axB, i, j, k, a.ny, a.nz) : -1;
+      const long long qA = rA ? psi_index<T>(a.maph[axA], a.nph, axA, i, j, k, a.ny, a.pz) : -1;
+      const long long qB = rB ? psi_index<T>(a.maph[axB], a.nph, axB, i, j, k, a.ny, a.pz) : -1;
       curl_transpose<T>(y, K, rA, rB, qA, qB, rA ? a.bh[axA][pos[axA]] : T(0),
                         rA ? a.cph[axA][pos[axA]] : T(0), rB ? a.bh[axB][pos[axB]] : T(0),
                         rB ? a.cph[axB][pos[axB]] : T(0), s.lpH[2 * c], s.lpH[2 * c + 1], qa,
@@ -187,7 +186,7 @@ __global__ void __launch_bounds__(256) k_adj_h(const __grid_constant__ StepArgs<
 // the adjoint of every sampled component of family fam (0: E, 1: H).
 template <typename T>
 __global__ void k_adj_dft_src(DftRegion r, const double* cot, const double* ph, int n_freq,
-                              double dt, int fam, T* l0, T* l1, T* l2, int ny, int nz) {
+                              double dt, int fam, T* l0, T* l1, T* l2, int ny, int pz) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= r.ncell * r.ncomp) return;
   const long long cell = t % r.ncell;
@@ -205,7 +204,7 @@ __global__ void k_adj_dft_src(DftRegion r, const double* cot, const double* ph, 
   const long long cj = rest % r.count[1];
   const long long ci = rest / r.count[1];
   const long long id = ((long long)(r.start[0] + ci * r.stride[0]) * ny +
-                        (r.start[1] + cj * r.stride[1])) * nz +
+                        (r.start[1] + cj * r.stride[1])) * pz +
                        (r.start[2] + ck * r.stride[2]);
   T* l = (c % 3) == 0 ? l0 : ((c % 3) == 1 ? l1 : l2);
   l[id] = to_real(__dadd_rn((double)l[id], v), T());
@@ -214,7 +213,7 @@ __global__ void k_adj_dft_src(DftRegion r, const double* cot, const double* ph, 
 // The loss's source on one recorded field snapshot (a FieldMonitor frame):
 // vals[cell] = dJ / d f(cell) over the region, added to the adjoint field.
 template <typename T>
-__global__ void k_adj_region_src(DftRegion r, const double* vals, T* l, int ny, int nz) {
+__global__ void k_adj_region_src(DftRegion r, const double* vals, T* l, int ny, int pz) {
   const long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (cell >= r.ncell) return;
   const long long ck = cell % r.count[2];
@@ -222,7 +221,7 @@ __global__ void k_adj_region_src(DftRegion r, const double* vals, T* l, int ny, 
   const long long cj = rest % r.count[1];
   const long long ci = rest / r.count[1];
   const long long id = ((long long)(r.start[0] + ci * r.stride[0]) * ny +
-                        (r.start[1] + cj * r.stride[1])) * nz +
+                        (r.start[1] + cj * r.stride[1])) * pz +
                        (r.start[2] + ck * r.stride[2]);
   l[id] = to_real(__dadd_rn((double)l[id], vals[cell]), T());
 }
@@ -233,21 +232,21 @@ __global__ void k_adj_region_src(DftRegion r, const double* vals, T* l, int ny, 
 // order, as k_flux_sample_batch). With c = dJ/dflux * dA * dt its sources on
 // the adjoint are dS/dE_t1 = H_t2, dS/dE_t2 = -H_t1, dS/dH_t2 = E_t1,
 // dS/dH_t1 = -E_t2 at every plane cell.
-__device__ __forceinline__ long long flux_cell(const FluxPlane& p, long long t, int ny, int nz) {
+__device__ __forceinline__ long long flux_cell(const FluxPlane& p, long long t, int ny, int pz) {
   const int u = (int)(t / p.n1), w = (int)(t % p.n1);
-  if (p.axis == 0) return ((long long)p.idx * ny + u) * nz + w;
-  if (p.axis == 1) return ((long long)u * ny + p.idx) * nz + w;
-  return ((long long)u * ny + w) * nz + p.idx;
+  if (p.axis == 0) return ((long long)p.idx * ny + u) * pz + w;
+  if (p.axis == 1) return ((long long)u * ny + p.idx) * pz + w;
+  return ((long long)u * ny + w) * pz + p.idx;
 }
 
 // E_t1, E_t2 of the plane after a step, into a record of 2 * n0 * n1 reals.
 template <typename T>
 __global__ void k_flux_plane_record(FluxPlane p, const T* E0, const T* E1, const T* E2, T* dst,
-                                    int ny, int nz) {
+                                    int ny, int pz) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long np = (long long)p.n0 * p.n1;
   if (t >= np) return;
-  const long long id = flux_cell(p, t, ny, nz);
+  const long long id = flux_cell(p, t, ny, pz);
   const T* E[3] = {E0, E1, E2};
   dst[t] = E[(p.axis + 1) % 3][id];
   dst[np + t] = E[(p.axis + 2) % 3][id];
@@ -257,11 +256,11 @@ __global__ void k_flux_plane_record(FluxPlane p, const T* E0, const T* E1, const
 // fields); fam 1: lamH_t2 += c E_t1, lamH_t1 -= c E_t2 from the plane record.
 template <typename T>
 __global__ void k_adj_flux_src(FluxPlane p, double c, int fam, const T* H0, const T* H1,
-                               const T* H2, const T* erec, T* l0, T* l1, T* l2, int ny, int nz) {
+                               const T* H2, const T* erec, T* l0, T* l1, T* l2, int ny, int pz) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long np = (long long)p.n0 * p.n1;
   if (t >= np) return;
-  const long long id = flux_cell(p, t, ny, nz);
+  const long long id = flux_cell(p, t, ny, pz);
   const int t1 = (p.axis + 1) % 3, t2 = (p.axis + 2) % 3;
   T* l[3] = {l0, l1, l2};
   double a, b;  // sources on component t1, t2

@@ -40,7 +40,7 @@ struct Fields6 {
 
 template <typename T>
 __global__ void k_dft_sample(DftRegion r, T* ring, int slot, Fields6<T> fields, int ny,
-                             int nz) {
+                             int pz) {
   const long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (cell >= r.ncell) return;
   const long long ck = cell % r.count[2];
@@ -48,7 +48,7 @@ __global__ void k_dft_sample(DftRegion r, T* ring, int slot, Fields6<T> fields, 
   const long long cj = rest % r.count[1];
   const long long ci = rest / r.count[1];
   const long long id = ((long long)(r.start[0] + ci * r.stride[0]) * ny +
-                        (r.start[1] + cj * r.stride[1])) * nz +
+                        (r.start[1] + cj * r.stride[1])) * pz +
                        (r.start[2] + ck * r.stride[2]);
   for (int q = 0; q < r.ncomp; ++q)
     ring[((long long)slot * r.ncomp + q) * r.ncell + cell] = fields.f[r.comps[q]][id];
@@ -139,7 +139,7 @@ struct FluxBatch {
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_flux_sample_batch(FluxBatch b, Fields6<T> fields, int ny,
-                                                           int nz) {
+                                                           int pz) {
   __shared__ double sh[8];
   const FluxPlane& p = b.p[blockIdx.y];
   if ((int)blockIdx.x >= p.nblk) return;  // uniform over the block
@@ -150,13 +150,13 @@ __global__ void __launch_bounds__(256) k_flux_sample_batch(FluxBatch b, Fields6<
     long long id;
     int e1, h2, e2, h1;
     if (p.axis == 0) {  // S = Ey*Hz - Ez*Hy
-      id = ((long long)p.idx * ny + u) * nz + w;
+      id = ((long long)p.idx * ny + u) * pz + w;
       e1 = 1; h2 = 5; e2 = 2; h1 = 4;
     } else if (p.axis == 1) {  // S = Ez*Hx - Ex*Hz
-      id = ((long long)u * ny + p.idx) * nz + w;
+      id = ((long long)u * ny + p.idx) * pz + w;
       e1 = 2; h2 = 3; e2 = 0; h1 = 5;
     } else {  // S = Ex*Hy - Ey*Hx
-      id = ((long long)u * ny + w) * nz + p.idx;
+      id = ((long long)u * ny + w) * pz + p.idx;
       e1 = 0; h2 = 4; e2 = 1; h1 = 3;
     }
     const T s = sub_rn(mul_rn(fields.f[e1][id], fields.f[h2][id]),
@@ -189,14 +189,14 @@ __global__ void __launch_bounds__(256) k_flux_flush(const double* partial, int n
 // Strided sub-block of one field into a compact C-order buffer (the
 // FieldMonitor snapshot: every stride-th cell per axis, or one z plane).
 template <typename T>
-__global__ void k_gather_region(const T* f, int ny, int nz, int3 start, int3 stride,
+__global__ void k_gather_region(const T* f, int ny, int pz, int3 start, int3 stride,
                                 int3 count, T* out) {
   const long long n = (long long)count.x * count.y * count.z;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
     const long long ck = t % count.z, rest = t / count.z;
     const long long cj = rest % count.y, ci = rest / count.y;
-    out[t] = f[((long long)(start.x + ci * stride.x) * ny + (start.y + cj * stride.y)) * nz +
+    out[t] = f[((long long)(start.x + ci * stride.x) * ny + (start.y + cj * stride.y)) * pz +
                (start.z + ck * stride.z)];
   }
 }

@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(32 * TY, 1024 / (32 * TY)) k_fused(
   const int k0 = blockIdx.x * TZ, j0 = blockIdx.y * TY;
   const int k = k0 + tz, j = j0 + ty;
   const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const int sy = nz, sx = ny * nz;  // cell count < 2^31 (checked at pf_create)
+  const int sy = a.pz, sx = ny * a.pz;  // cell count < 2^31 (checked at pf_create)
   const int ib = blockIdx.z * xchunk;
   if (ib >= nx) return;  // whole block: no barrier is skipped by a subset
   const int ie = min(nx, ib + xchunk);

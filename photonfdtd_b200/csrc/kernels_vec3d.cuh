@@ -1,0 +1,519 @@
+// kernels_vec3d.cuh - H and E passes of 3D grids, one 16-byte vector of z cells per thread.
+//
+// The per-component arithmetic and its order are the scalar passes'
+// (cell_update.cuh; src/photonfdtd/simulation.py:1252-1309), so the bits are
+// too. What bounds a step here is memory latency and issue slots, not FLOPs:
+// with one cell per thread the passes ran 222 (H) and 414 (E with ADE)
+// instructions per cell at 4.2 TB/s, most of them addresses, bounds and CPML
+// tests that V cells of one row share. Rows are padded to 32 bytes
+// (StepArgs::pz), so every row's vectors are aligned. At 256^3 without CPML
+// the H pass now runs 88 instructions per cell at 5.5 TB/s of DRAM traffic
+// (84% of a plain copy), the E pass with ADE 181 at 5.05 TB/s. Step kernels
+// before and after, in us: 384^3 with ADE 1453, 1354; 301x287x263 with three
+// coefficients 517, 473; 160x152x144 double 165, 145.
+//
+// A warp covers a patch of rows (blockDim.x vectors along z); when every cell
+// of it lies in the bulk box (both differences, no CPML state) the warp takes
+// the straight-line path, else curl_general.
+#pragma once
+
+#include "cell_update.cuh"
+
+// Minimum resident 128-thread blocks per SM the passes are compiled for
+// (float H, float E, float E with ADE, double H, double E). Measured step
+// kernels in us at 4/4/3/4/3, 5/5/4/5/4, 6/6/4/8/6 and 8/6/5/6/5: 384^3 with
+// ADE 1526, 1354, 1375, 1457; 301x287x263 tensor 507, 473, 504, 505;
+// 160x152x144 double 155, 152, 153, 145.
+#ifndef PFB_MINB_HV
+#define PFB_MINB_HV 5
+#endif
+#ifndef PFB_MINB_EV
+#define PFB_MINB_EV 5
+#endif
+#ifndef PFB_MINB_EVA
+#define PFB_MINB_EVA 4
+#endif
+#ifndef PFB_MINB_HV64
+#define PFB_MINB_HV64 6
+#endif
+#ifndef PFB_MINB_EV64
+#define PFB_MINB_EV64 5
+#endif
+
+namespace pfb {
+
+constexpr int kVecThreads = 128;
+
+template <typename T>
+constexpr int kVec = 16 / (int)sizeof(T);
+
+__device__ __forceinline__ void vld(const float* p, float (&o)[4]) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+}
+__device__ __forceinline__ void vld(const double* p, double (&o)[2]) {
+  const double2 v = *reinterpret_cast<const double2*>(p);
+  o[0] = v.x; o[1] = v.y;
+}
+__device__ __forceinline__ void vst(float* p, const float* o) {
+  *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
+}
+__device__ __forceinline__ void vst(double* p, const double* o) {
+  *reinterpret_cast<double2*>(p) = make_double2(o[0], o[1]);
+}
+__device__ __forceinline__ void wld(const uint32_t* p, uint32_t (&o)[4]) {
+  const uint4 v = *reinterpret_cast<const uint4*>(p);
+  o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+}
+__device__ __forceinline__ void wld(const uint32_t* p, uint32_t (&o)[2]) {
+  const uint2 v = *reinterpret_cast<const uint2*>(p);
+  o[0] = v.x; o[1] = v.y;
+}
+// The vector at p when ok, else zeros.
+template <typename T>
+__device__ __forceinline__ void vld_if(const T* p, bool ok, T (&o)[kVec<T>]) {
+  if (ok) {
+    vld(p, o);
+  } else {
+#pragma unroll
+    for (int q = 0; q < kVec<T>; ++q) o[q] = T(0);
+  }
+}
+
+// Difference term t of a curl: components of the source field and axes in
+// the order x A, x B, y A, y B, z A, z B (A enters with +, B with -).
+__device__ __forceinline__ constexpr int term_comp(int t) {
+  return t == 0 || t == 3 ? 2 : (t == 1 || t == 4 ? 1 : 0);
+}
+__device__ __forceinline__ constexpr int term_axis(int t) {
+  return t == 0 || t == 5 ? 1 : (t == 1 || t == 2 ? 2 : 0);
+}
+
+// The six exact quotients of one cell, IEEE division where a numerator is
+// out of the reciprocal path's range.
+template <typename T, int SGN>
+__device__ __forceinline__ void quotients_ieee(const StepArgs<T>& a, const T own[3], const T nb[6],
+                                               T d[6]) {
+  const T dl[3] = {a.dx, a.dy, a.dz};
+#pragma unroll
+  for (int t = 0; t < 6; ++t) {
+    const T o = own[term_comp(t)];
+    d[t] = div_rn(SGN > 0 ? sub_rn(nb[t], o) : sub_rn(o, nb[t]), dl[term_axis(t)]);
+  }
+}
+
+// out[c] = f[c] + K[c] (d_A - d_B) for V bulk cells. SGN 1: forward
+// differences d = (nb - own) / dl (H), -1: backward d = (own - nb) / dl (E).
+// Own values are prescaled once; a prescaled difference is then one FMA, and
+// the curl is scaled back once per component (QScale in common.cuh): 6.5
+// operations per term instead of 11. One range check covers the V cells.
+template <typename T, int SGN, int NC>
+__device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][kVec<T>],
+                                          const T (&K)[NC][kVec<T>], const T (&own)[3][kVec<T>],
+                                          const T (&nb)[6][kVec<T>], T (&out)[3][kVec<T>]) {
+  constexpr int V = kVec<T>;
+  const T dl[3] = {a.dx, a.dy, a.dz};
+  const T rl[3] = {a.rdx, a.rdy, a.rdz};
+  const T up = QScale<T>::up;
+  T m = T(0);
+#pragma unroll
+  for (int q = 0; q < V; ++q) {
+    T os[3], n[6];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) os[c] = mul_rn(own[c][q], up);
+#pragma unroll
+    for (int t = 0; t < 6; ++t) {
+      n[t] = SGN > 0 ? fma_rn(nb[t][q], up, -os[term_comp(t)])
+                     : fma_rn(-nb[t][q], up, os[term_comp(t)]);
+      m = absmax(m, n[t]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const T dA = qscaled(n[2 * c], dl[term_axis(2 * c)], rl[term_axis(2 * c)]);
+      const T dB = qscaled(n[2 * c + 1], dl[term_axis(2 * c + 1)], rl[term_axis(2 * c + 1)]);
+      out[c][q] = add_rn(f[c][q], mul_rn(mul_rn(sub_rn(dA, dB), QScale<T>::down), K[c % NC][q]));
+    }
+  }
+  if (!(a.fdall && m < QScale<T>::limit * up)) {
+#pragma unroll
+    for (int q = 0; q < V; ++q) {
+      T o[3], n[6], d[6];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) o[c] = own[c][q];
+#pragma unroll
+      for (int t = 0; t < 6; ++t) n[t] = nb[t][q];
+      quotients_ieee<T, SGN>(a, o, n, d);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) out[c][q] = bulk(f[c][q], K[c % NC][q], d[2 * c], d[2 * c + 1]);
+    }
+  }
+}
+
+// CPML tables of one field family as curl_general reads them.
+template <typename T>
+struct Cpml {
+  const int* map[3];
+  const int* np;
+  const T* b[3];
+  const T* c[3];
+  const T* in[6];
+  T* out[6];
+};
+
+// One CPML term of one cell: psi' = b psi + c d, and its share of the update.
+template <typename T>
+__device__ __forceinline__ T cpml_term(T f, T k, T d, T b, T c, T& psi) {
+  psi = add_rn(mul_rn(b, psi), mul_rn(c, d));
+  return add_rn(f, mul_rn(k, psi));
+}
+
+// The curl update of V cells anywhere in a 3D grid: components outside the
+// reference's loop extents keep their value (and row padding stays zero),
+// psi state is touched only where the compact map of its axis is >= 0. The x
+// and y layers' psi rows have the fields' pitch, so they are vectors too.
+template <typename T, int SGN, int NC>
+__device__ __forceinline__ void curl_general(const StepArgs<T>& a, const Cpml<T>& p, int i, int j,
+                                             int k, const T (&f)[3][kVec<T>],
+                                             const T (&K)[NC][kVec<T>],
+                                             const T (&own)[3][kVec<T>],
+                                             const T (&nb)[6][kVec<T>], T (&out)[3][kVec<T>]) {
+  constexpr int V = kVec<T>;
+  const bool okx = SGN > 0 ? i < a.nx - 1 : i >= 1;
+  const bool oky = SGN > 0 ? j < a.ny - 1 : j >= 1;
+  const int mx = p.map[0][i], my = p.map[1][j];
+  T y0[V], y5[V], x3[V], x4[V];
+  T by = T(0), cy = T(0), bx = T(0), cx = T(0);
+  const long long qy = ((long long)i * p.np[1] + my) * a.pz + k;
+  const long long qx = ((long long)mx * a.ny + j) * a.pz + k;
+  if (my >= 0) {
+    by = p.b[1][j];
+    cy = p.c[1][j];
+    vld(p.in[0] + qy, y0);
+    vld(p.in[5] + qy, y5);
+  }
+  if (mx >= 0) {
+    bx = p.b[0][i];
+    cx = p.c[0][i];
+    vld(p.in[3] + qx, x3);
+    vld(p.in[4] + qx, x4);
+  }
+  const T dl[3] = {a.dx, a.dy, a.dz};
+  const T rl[3] = {a.rdx, a.rdy, a.rdz};
+#pragma unroll
+  for (int q = 0; q < V; ++q) {
+    const int kk = k + q;
+    const bool okz = SGN > 0 ? kk < a.nz - 1 : (kk >= 1 && kk < a.nz);
+    T o[3], n[6], d[6];
+    T m = T(0);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) o[c] = own[c][q];
+#pragma unroll
+    for (int t = 0; t < 6; ++t) {
+      n[t] = nb[t][q];
+      d[t] = SGN > 0 ? sub_rn(n[t], o[term_comp(t)]) : sub_rn(o[term_comp(t)], n[t]);
+      m = absmax(m, d[t]);
+    }
+    if (a.fdall && qdiv_ok(m)) {
+#pragma unroll
+      for (int t = 0; t < 6; ++t) d[t] = qdiv_fast(d[t], dl[term_axis(t)], rl[term_axis(t)]);
+    } else {
+      quotients_ieee<T, SGN>(a, o, n, d);
+    }
+    const int mz = kk < a.nz ? p.map[2][kk] : -1;
+    T bz = T(0), cz = T(0), z1 = T(0), z2 = T(0);
+    const long long qz = ((long long)i * a.ny + j) * p.np[2] + mz;
+    if (mz >= 0) {
+      bz = p.b[2][kk];
+      cz = p.c[2][kk];
+      z1 = p.in[1][qz];
+      z2 = p.in[2][qz];
+    }
+    const T k0 = K[0][q], k1 = K[1 % NC][q], k2 = K[2 % NC][q];
+    T r0 = f[0][q], r1 = f[1][q], r2 = f[2][q];
+    if (oky && okz) {
+      r0 = bulk(r0, k0, d[0], d[1]);
+      if (my >= 0) r0 = cpml_term(r0, k0, d[0], by, cy, y0[q]);
+      if (mz >= 0) {
+        r0 = cpml_term(r0, -k0, d[1], bz, cz, z1);
+        p.out[1][qz] = z1;
+      }
+    }
+    if (okz && okx) {
+      r1 = bulk(r1, k1, d[2], d[3]);
+      if (mz >= 0) {
+        r1 = cpml_term(r1, k1, d[2], bz, cz, z2);
+        p.out[2][qz] = z2;
+      }
+      if (mx >= 0) r1 = cpml_term(r1, -k1, d[3], bx, cx, x3[q]);
+    }
+    if (okx && oky) {
+      r2 = bulk(r2, k2, d[4], d[5]);
+      if (mx >= 0) r2 = cpml_term(r2, k2, d[4], bx, cx, x4[q]);
+      if (my >= 0) r2 = cpml_term(r2, -k2, d[5], by, cy, y5[q]);
+    }
+    out[0][q] = r0;
+    out[1][q] = r1;
+    out[2][q] = r2;
+  }
+  if (my >= 0) {
+    vst(p.out[0] + qy, y0);
+    vst(p.out[5] + qy, y5);
+  }
+  if (mx >= 0) {
+    vst(p.out[3] + qx, x3);
+    vst(p.out[4] + qx, x4);
+  }
+}
+
+// Whether every cell of the warp's patch lies in the bulk box [b0, b1).
+template <int V>
+__device__ __forceinline__ bool warp_bulk(bool live, int i, int j, int k, const int* b0,
+                                          const int* b1) {
+  const bool in = live && i >= b0[0] && i < b1[0] && j >= b0[1] && j < b1[1] && k >= b0[2] &&
+                  k + V <= b1[2];
+  return __all_sync(0xffffffffu, in);
+}
+
+// H pass: H^{n+1/2} = H^{n-1/2} - ch (curl E^n + psi), planes i0 + blockIdx.z.
+template <typename T>
+__global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? PFB_MINB_HV : PFB_MINB_HV64)
+    k_h_vec(const __grid_constant__ StepArgs<T> a, int i0) {
+  constexpr int V = kVec<T>;
+  const int k = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int i = i0 + blockIdx.z;
+  const bool live = k < a.nz && j < a.ny;
+  const bool box = warp_bulk<V>(live, i, j, k, a.hb0, a.hb1);
+  if (!live) return;
+  const long long sx = (long long)a.ny * a.pz;
+  const long long id = i * sx + (unsigned)(j * a.pz + k);
+  T own[3][V], nb[6][V], f[3][V], out[3][V];
+  const bool hx = i + 1 < a.nx, hy = j + 1 < a.ny, hz = k + V < a.nz;
+  vld(a.Ein[0] + id, own[0]);
+  vld(a.Ein[1] + id, own[1]);
+  vld(a.Ein[2] + id, own[2]);
+  const T e1 = hz ? a.Ein[1][id + V] : T(0), e0 = hz ? a.Ein[0][id + V] : T(0);
+  vld_if(a.Ein[2] + id + a.pz, hy, nb[0]);
+  vld_if(a.Ein[0] + id + a.pz, hy, nb[5]);
+  vld_if(a.Ein[2] + id + sx, hx, nb[3]);
+  vld_if(a.Ein[1] + id + sx, hx, nb[4]);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) vld(a.Hin[c] + id, f[c]);
+#pragma unroll
+  for (int q = 0; q < V; ++q) {
+    nb[1][q] = q + 1 < V ? own[1][q + 1 < V ? q + 1 : 0] : e1;
+    nb[2][q] = q + 1 < V ? own[0][q + 1 < V ? q + 1 : 0] : e0;
+  }
+  T K[1][V];
+#pragma unroll
+  for (int q = 0; q < V; ++q) K[0][q] = -a.ch;
+  if (box) {
+    curl_bulk<T, 1, 1>(a, f, K, own, nb, out);
+  } else {
+    Cpml<T> p;
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+      p.map[x] = a.maph[x];
+      p.b[x] = a.bh[x];
+      p.c[x] = a.cph[x];
+    }
+    p.np = a.nph;
+#pragma unroll
+    for (int t = 0; t < 6; ++t) {
+      p.in[t] = a.psiHin[t];
+      p.out[t] = a.psiHout[t];
+    }
+    curl_general<T, 1, 1>(a, p, i, j, k, f, K, own, nb, out);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) vst(a.Hout[c] + id, out[c]);
+}
+
+// ---- dispersive cells (simulation.py:645-669), V at a time -------------------
+// V cells of one medium with consecutive ranks own 3 V NP consecutive reals
+// per level ([cell][pole][component]): NP chunks of three vectors, of V / NP
+// cells each. The first chunk of both levels is loaded ahead (c0: P^n, p0:
+// P^{n-1}). The operations of each cell are ade_np's.
+template <typename T, int NP>
+__device__ __forceinline__ void ade_vec(const MediumT<T>& M, const T* Rc, T* Rp,
+                                        const T (&en)[3][kVec<T>], T (&e)[3][kVec<T>],
+                                        T (&c0)[3][kVec<T>], T (&p0)[3][kVec<T>]) {
+  constexpr int V = kVec<T>;
+#pragma unroll
+  for (int ch = 0; ch < NP; ++ch) {
+    if (ch > 0) {
+#pragma unroll
+      for (int u = 0; u < 3; ++u) {
+        vld(Rc + (ch * 3 + u) * V, c0[u]);
+        vld(Rp + (ch * 3 + u) * V, p0[u]);
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < V / NP; ++s) {
+      const int q = ch * (V / NP) + s;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        T delta = T(0);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          const int x = (s * NP + p) * 3 + c;
+          const T pc = c0[x / V][x % V];
+          const T pn = add_rn(add_rn(mul_rn(M.a[p], pc), mul_rn(M.b[p], p0[x / V][x % V])),
+                              mul_rn(M.c[p], en[c][q]));
+          p0[x / V][x % V] = pn;
+          const T inc = sub_rn(pn, pc);
+          delta = p == 0 ? inc : add_rn(delta, inc);
+        }
+        e[c][q] = sub_rn(e[c][q], mul_rn(M.inv, delta));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 3; ++u) vst(Rp + (ch * 3 + u) * V, p0[u]);
+  }
+}
+
+// One dispersive cell, any pole count, state read and written in place.
+template <typename T>
+__device__ __forceinline__ void ade_cell(const StepArgs<T>& a, uint32_t w, T en0, T en1, T en2,
+                                         T& e0, T& e1, T& e2) {
+  const MediumT<T>& M = a.media[(w >> kMediumShift) & 15u];
+  const int np = M.npole;
+  if (np == 0) return;
+  const T* Rc = a.P + M.poff + (long long)(w & kLocMask) * (3 * np) + a.lvl * a.plev;
+  T* Rp = a.P + M.poff + (long long)(w & kLocMask) * (3 * np) + (a.lvl ^ 1) * a.plev;
+  T d0 = T(0), d1 = T(0), d2 = T(0);
+  for (int p = 0; p < np; ++p) {
+    const T A = M.a[p], B = M.b[p], C = M.c[p];
+    const T c0 = Rc[3 * p], c1 = Rc[3 * p + 1], c2 = Rc[3 * p + 2];
+    const T n0 = add_rn(add_rn(mul_rn(A, c0), mul_rn(B, Rp[3 * p])), mul_rn(C, en0));
+    const T n1 = add_rn(add_rn(mul_rn(A, c1), mul_rn(B, Rp[3 * p + 1])), mul_rn(C, en1));
+    const T n2 = add_rn(add_rn(mul_rn(A, c2), mul_rn(B, Rp[3 * p + 2])), mul_rn(C, en2));
+    Rp[3 * p] = n0;
+    Rp[3 * p + 1] = n1;
+    Rp[3 * p + 2] = n2;
+    const T i0 = sub_rn(n0, c0), i1 = sub_rn(n1, c1), i2 = sub_rn(n2, c2);
+    d0 = p == 0 ? i0 : add_rn(d0, i0);
+    d1 = p == 0 ? i1 : add_rn(d1, i1);
+    d2 = p == 0 ? i2 : add_rn(d2, i2);
+  }
+  e0 = sub_rn(e0, mul_rn(M.inv, d0));
+  e1 = sub_rn(e1, mul_rn(M.inv, d1));
+  e2 = sub_rn(e2, mul_rn(M.inv, d2));
+}
+
+// E pass: E^{n+1} = E^n + ce (curl H^{n+1/2} + psi), then ADE. Loads are
+// issued in dependency order: the words, every field vector, then what the
+// words select (coefficients, ADE records of a run).
+template <typename T, int CE, bool ADE>
+__global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? (ADE ? PFB_MINB_EVA : PFB_MINB_EV)
+                                                              : PFB_MINB_EV64)
+    k_e_vec(const __grid_constant__ StepArgs<T> a, int i0) {
+  constexpr int V = kVec<T>;
+  constexpr int NC = CE == kCeCell3 ? 3 : 1;
+  const int k = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int i = i0 + blockIdx.z;
+  const bool live = k < a.nz && j < a.ny;
+  const bool box = warp_bulk<V>(live, i, j, k, a.eb0, a.eb1);
+  if (!live) return;
+  const long long sx = (long long)a.ny * a.pz;
+  const long long id = i * sx + (unsigned)(j * a.pz + k);
+  uint32_t t[V];
+  T K[NC][V];
+  if (CE == kCeTable) wld(a.word + id, t);
+  else if (ADE) wld(a.adeword + id, t);
+  if (CE != kCeTable) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) vld(a.ce[c] + id, K[c]);
+  }
+  T own[3][V], nb[6][V], en[3][V], e[3][V];
+  const bool lx = i > 0, ly = j > 0, lz = k > 0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) vld(a.Hin[c] + id, own[c]);
+  const T h1 = lz ? a.Hin[1][id - 1] : T(0), h0 = lz ? a.Hin[0][id - 1] : T(0);
+  vld_if(a.Hin[2] + id - a.pz, ly, nb[0]);
+  vld_if(a.Hin[0] + id - a.pz, ly, nb[5]);
+  vld_if(a.Hin[2] + id - sx, lx, nb[3]);
+  vld_if(a.Hin[1] + id - sx, lx, nb[4]);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) vld(a.Ein[c] + id, en[c]);
+  // a run: V plain cells of one table entry, or V cells of one dispersive
+  // medium with consecutive ranks
+  bool vec = false;
+  T c0[3][V], p0[3][V];
+  const T* Rc = nullptr;
+  T* Rp = nullptr;
+  int np = 0;
+  if (CE == kCeTable || ADE) {
+    const bool disp = ADE && (t[0] & kDispersiveBit);
+    bool run = (t[V - 1] >> kMediumShift) == (t[0] >> kMediumShift);
+#pragma unroll
+    for (int q = 1; q < V; ++q) run = run && t[q] == t[0] + (disp ? (uint32_t)q : 0u);
+    if (ADE && disp && run) {
+      const MediumT<T>& M = a.media[(t[0] >> kMediumShift) & 15u];
+      np = M.npole;
+      const long long rec = M.poff + (long long)(t[0] & kLocMask) * (3 * np);
+      vec = (np == 1 || np == 2) && rec % V == 0;
+      if (vec) {
+        Rc = a.P + rec + a.lvl * a.plev;
+        Rp = a.P + rec + (a.lvl ^ 1) * a.plev;
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+          vld(Rc + u * V, c0[u]);
+          vld(Rp + u * V, p0[u]);
+        }
+      }
+    }
+    if (CE == kCeTable) {
+      if (run) {
+        const T K0 = disp ? a.media[(t[0] >> kMediumShift) & 15u].ce : a.table[t[0]];
+#pragma unroll
+        for (int q = 0; q < V; ++q) K[0][q] = K0;
+      } else {
+#pragma unroll
+        for (int q = 0; q < V; ++q)
+          K[0][q] = ADE && (t[q] & kDispersiveBit) ? a.media[(t[q] >> kMediumShift) & 15u].ce
+                                                   : a.table[t[q]];
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < V; ++q) {
+    nb[1][q] = q > 0 ? own[1][q > 0 ? q - 1 : 0] : h1;
+    nb[2][q] = q > 0 ? own[0][q > 0 ? q - 1 : 0] : h0;
+  }
+  if (box) {
+    curl_bulk<T, -1, NC>(a, en, K, own, nb, e);
+  } else {
+    Cpml<T> p;
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+      p.map[x] = a.mape[x];
+      p.b[x] = a.be[x];
+      p.c[x] = a.cpe[x];
+    }
+    p.np = a.npe;
+#pragma unroll
+    for (int s = 0; s < 6; ++s) {
+      p.in[s] = a.psiE[s];
+      p.out[s] = a.psiE[s];
+    }
+    curl_general<T, -1, NC>(a, p, i, j, k, en, K, own, nb, e);
+  }
+  if (ADE) {
+    if (vec) {
+      const MediumT<T>& M = a.media[(t[0] >> kMediumShift) & 15u];
+      if (np == 1) ade_vec<T, 1>(M, Rc, Rp, en, e, c0, p0);
+      else ade_vec<T, 2>(M, Rc, Rp, en, e, c0, p0);
+    } else {
+#pragma unroll
+      for (int q = 0; q < V; ++q)
+        if (t[q] & kDispersiveBit)
+          ade_cell<T>(a, t[q], en[0][q], en[1][q], en[2][q], e[0][q], e[1][q], e[2][q]);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) vst(a.Eout[c] + id, e[c]);
+}
+
+}  // namespace pfb
