@@ -251,7 +251,7 @@ __device__ __forceinline__ void ade_load(const StepArgs<T>& a, const MediumT<T>*
 // (simulation.py:645-669): P^{n+1} = a P^n + b P^{n-1} + c E^n per pole and
 // component, E -= inv * sum_p (P^{n+1} - P^n), with the Python-float
 // coefficients rounded to the field type as numpy's weak scalars are.
-// P^{n+1} overwrites P^{n-1} (level a.lvl holds P^n). Records with more than
+// P^{n+1} overwrites P^{n-1} (level lvl holds P^n). Records with more than
 // two poles are read and written in place.
 // NP-pole update from a loaded record; out[] receives P^{n+1} per
 // [pole][component]. The level of P^n (lc) selects between compile-time
@@ -277,11 +277,11 @@ __device__ __forceinline__ void ade_np(const MediumT<T>& M, const T* v, int lc, 
 
 template <typename T>
 __device__ __forceinline__ void ade_update(const StepArgs<T>& a, const MediumT<T>* media,
-                                           const AdeRec<T>& r, const T en[3], T e[3]) {
+                                           const AdeRec<T>& r, int lvl, const T en[3], T e[3]) {
   const MediumT<T>& M = media[r.m];
   const int np = M.npole;
   T* R = a.P + M.poff + (long long)r.loc * (3 * np);  // level 0 record
-  const int lc = a.lvl, lp = a.lvl ^ 1;
+  const int lc = lvl, lp = lvl ^ 1;
   T* Rc = R + lc * a.plev;
   T* Rp = R + lp * a.plev;
   if (np == 2) {

@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kNoAllocThreads) k_flux_partials_static(FluxPl
     }
     v = (double)sub_rn(mul_rn(f.f[e1][id], f.f[h2][id]), mul_rn(f.f[e2][id], f.f[h1][id]));
   }
-  v = block_sum<T>(v, sh);
+  v = block_sum256<T>(v, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = v;
 }
 
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kNoAllocThreads) k_flux_total_static(const dou
   __shared__ double sh[8];
   double v = 0.0;
   for (int b = threadIdx.x; b < nblk; b += blockDim.x) v += part[b];
-  v = block_sum<T>(v, sh);
+  v = block_sum256<T>(v, sh);
   if (threadIdx.x == 0) {
     const T s = to_real(v, T());
     *out = __dmul_rn((double)mul_rn(s, (T)dA), dt);

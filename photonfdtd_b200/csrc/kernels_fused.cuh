@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(32 * TY, 1024 / (32 * TY)) k_fused(
         e[1] = upd_ey<T>(a, i, j, k, en[1], K[1], hx, sm.h[0][jj][kk - 1], hz, hz_prev);
         e[2] = upd_ez<T>(a, i, j, k, en[2], K[2], hy, hy_prev, hx, sm.h[0][jj - 1][kk]);
       }
-      if (ADE && w) ade_update<T>(a, media, rec, en, e);
+      if (ADE && w) ade_update<T>(a, media, rec, a.lvl, en, e);
       a.Eout[0][id] = e[0];
       a.Eout[1][id] = e[1];
       a.Eout[2][id] = e[2];

@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(256) k_e_split(const __grid_constant__ StepArg
                    ld_if(a.Hin[2], id, -sx, lx));
   e[2] = upd_ez<T>(a, i, j, k, en[2], K[2], hy, ld_if(a.Hin[1], id, -sx, lx), hx,
                    ld_if(a.Hin[0], id, -sy, ly));
-  if (ADE && w) ade_update<T>(a, media, rec, en, e);
+  if (ADE && w) ade_update<T>(a, media, rec, a.lvl, en, e);
   a.Eout[0][id] = e[0];
   a.Eout[1][id] = e[1];
   a.Eout[2][id] = e[2];

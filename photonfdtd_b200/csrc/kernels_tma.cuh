@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(32 * TY, 1024 / (32 * TY))
                         sub_rn(hy, hy_prev), sub_rn(hx, sh[0][jj - 1][kk])};
         e3<T>(a, i, j, k, en, K, n, e);
       }
-      if (ADE && w) ade_update<T>(a, media, rec, en, e);
+      if (ADE && w) ade_update<T>(a, media, rec, a.lvl, en, e);
       a.Eout[0][id] = e[0];
       a.Eout[1][id] = e[1];
       a.Eout[2][id] = e[2];
