@@ -1,0 +1,24 @@
+// devmem.cuh - device memory of engines and batches from a per-device pool.
+//
+// Building an engine takes some 60 allocations, and cudaMalloc / cudaFree of
+// them took 3 to 30 ms per run (each cudaFree waits for the device and unmaps),
+// as long as a small scene's stepping. A stream-ordered pool keeps up to
+// kPoolKeep bytes of freed memory mapped for the next engine; what is above
+// that goes back to the driver at the next synchronisation, and everything
+// when an allocation fails (pool_trim). The pool belongs to no engine and is
+// never handed pointers of another allocator. Its calls are thread safe, and
+// its ordering is per stream: memory freed on one engine's stream reaches
+// another only behind the work queued before the free.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace pfb {
+
+constexpr unsigned long long kPoolKeep = 2ull << 30;
+
+// bytes of device memory in `st`'s order (a stream of device `dev`).
+cudaError_t pool_alloc(void** p, size_t bytes, int dev, cudaStream_t st);
+void pool_free(void* p, cudaStream_t st);
+
+}  // namespace pfb

@@ -26,6 +26,7 @@
 
 #include "../../include/pfb200.h"
 #include "common.cuh"
+#include "devmem.cuh"
 #include "kernels_adj.cuh"
 #include "kernels_aux.cuh"
 #include "kernels_fused.cuh"
@@ -216,9 +217,9 @@ int fail(pf_engine* e, int code, const char* fmt, ...) {
 
 int dalloc(pf_engine* e, void** p, size_t bytes) {
   if (bytes == 0) bytes = 16;
-  cudaError_t rc = cudaMalloc(p, bytes);
+  cudaError_t rc = pool_alloc(p, bytes, e->device, e->stream);
   if (rc != cudaSuccess)
-    return fail(e, PF_ERR_OOM, "CUDA error: cudaMalloc of %zu bytes failed: %s", bytes,
+    return fail(e, PF_ERR_OOM, "CUDA error: allocation of %zu bytes failed: %s", bytes,
                 cudaGetErrorString(rc));
   e->allocs.push_back(*p);
   e->dev_bytes += bytes;
@@ -239,15 +240,14 @@ int upload(pf_engine* e, void** p, const void* src, size_t bytes) {
 int stage(pf_engine* e, size_t bytes) {
   if (bytes <= e->region_bytes) return PF_OK;
   if (e->region) {
-    PF_CUDA(e, cudaStreamSynchronize(e->stream));
-    cudaFree(e->region);
+    pool_free(e->region, e->stream);
     e->dev_bytes -= e->region_bytes;
     e->region = nullptr;
     e->region_bytes = 0;
   }
-  const cudaError_t rc = cudaMalloc(&e->region, bytes);
+  const cudaError_t rc = pool_alloc(&e->region, bytes, e->device, e->stream);
   if (rc != cudaSuccess)
-    return fail(e, PF_ERR_OOM, "CUDA error: cudaMalloc of %zu bytes failed", bytes);
+    return fail(e, PF_ERR_OOM, "CUDA error: allocation of %zu bytes failed", bytes);
   e->region_bytes = bytes;
   e->dev_bytes += bytes;
   return PF_OK;
@@ -1149,6 +1149,60 @@ bool valid_comp(int c) { return c >= 0 && c < 6; }
 }  // namespace
 
 namespace pfb {
+namespace {
+std::mutex g_pool_mu;
+std::map<int, cudaMemPool_t> g_pools;  // per device, kept for the process
+}  // namespace
+
+namespace {
+// The pool of a device, made on first use; fresh: replace the one there (a
+// device reset took it).
+cudaMemPool_t device_pool(int dev, bool fresh) {
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  auto it = g_pools.find(dev);
+  if (it != g_pools.end() && !fresh) return it->second;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  unsigned long long keep = kPoolKeep;
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  g_pools[dev] = pool;
+  return pool;
+}
+}  // namespace
+
+cudaError_t pool_alloc(void** p, size_t bytes, int dev, cudaStream_t st) {
+  *p = nullptr;
+  cudaMemPool_t pool = device_pool(dev, false);
+  cudaError_t rc = pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaErrorMemoryAllocation;
+  if (rc == cudaErrorMemoryAllocation && pool) {
+    cudaGetLastError();
+    // freed blocks that the pool still holds may be what is missing
+    cudaStreamSynchronize(st);
+    cudaMemPoolTrimTo(pool, 0);
+    rc = cudaMallocFromPoolAsync(p, bytes, pool, st);
+  } else if (rc == cudaErrorInvalidValue) {
+    cudaGetLastError();
+    pool = device_pool(dev, true);
+    rc = pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaErrorMemoryAllocation;
+  }
+  if (rc != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+  }
+  return rc;
+}
+
+void pool_free(void* p, cudaStream_t st) {
+  if (p) cudaFreeAsync(p, st);
+}
+
 bool host_recip_division_exact(float d) { return recip_division_exact(d); }
 bool host_recip_division_exact(double d) { return recip_division_exact(d); }
 }  // namespace pfb
@@ -1739,9 +1793,9 @@ int pf_device_bytes(const pf_engine* e, int64_t* bytes) {
 
 void pf_destroy(pf_engine* e) {
   if (!e) return;
+  for (void* p : e->allocs) pool_free(p, e->stream);
+  if (e->region) pool_free(e->region, e->stream);
   if (e->stream) cudaStreamSynchronize(e->stream);
-  for (void* p : e->allocs) cudaFree(p);
-  if (e->region) cudaFree(e->region);
   if (e->res_err) err_word_release(e->res_err);
   for (cudaEvent_t ev : e->ev_pool) cudaEventDestroy(ev);
   if (e->stream) cudaStreamDestroy(e->stream);
