@@ -30,6 +30,8 @@
 // ceil(N / K) - 1 states + K window rings; K >= N keeps no state and needs no
 // replay.
 #include <algorithm>
+#include <array>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -73,10 +75,7 @@ struct pf_batch {
   std::vector<void*> allocs;
   Inst* d_inst = nullptr;
   TileRec* d_tiles = nullptr;
-  SegRec* d_segs = nullptr;   // marching segments (forward step)
-  int nsegs = 0;
-  size_t seg_cap = 0;         // SegRec slots of d_segs (the shortest segments)
-  bool march = true;          // forward step: marching warps (else kb_step tiles)
+  bool vec = true;            // fused steps: one vector per thread (else kb_step tiles)
   int ntiles = 0;
   int tile_rows = 32;
   size_t tile_cap = 0;  // TileRec slots of d_tiles (the 8-row list, the longest)
@@ -90,6 +89,7 @@ struct pf_batch {
   void* alvl1[5] = {};
   void* coef[8] = {};
   void* psi[4] = {};
+  int* groups[2] = {};        // psi groups per 4 pooled columns: E, H
   int* maps[4] = {};  // mex mhx mey mhy
   void* aE[3] = {};
   void* apsi[4] = {};
@@ -105,7 +105,14 @@ struct pf_batch {
   double* phase = nullptr;
   long long* base = nullptr;  // first step of the running chunk
   void* dring = nullptr;      // DFT line samples, kDftRing x line cells
+  cudaStream_t side = nullptr;  // captured with the main stream: the edge tiles
+  cudaEvent_t fork = nullptr, join = nullptr;
+  int nedge = 0;
   BSources src{};
+  int* srow = nullptr;  // StepPost's tables: per pooled x row, per column
+  int* scol = nullptr;
+  std::vector<std::array<int, 4>> inner;  // per instance: [x0, x1), [y0, y1) free of CPML state
+  std::vector<char> src_rows;             // pooled x rows with an E source
   // instantiated graphs and their kernel counts, keyed by (chunk kind, steps)
   std::map<std::pair<int, long long>, std::pair<cudaGraphExec_t, long long>> graphs;
   int64_t launches = 0;
@@ -157,9 +164,8 @@ BArgs<T> bargs(pf_batch* b) {
   memset(&a, 0, sizeof a);
   a.inst = b->d_inst;
   a.tiles = b->d_tiles;
-  a.segs = b->d_segs;
-  a.nsegs = b->nsegs;
   a.ntiles = b->ntiles;
+  a.nedge = b->nedge;
   a.Ex = (T*)b->Ex;
   a.Ey = (T*)b->Ey;
   a.Hz = (T*)b->Hz;
@@ -170,6 +176,8 @@ BArgs<T> bargs(pf_batch* b) {
   a.mhx = b->maps[1];
   a.mey = b->maps[2];
   a.mhy = b->maps[3];
+  a.gey = b->groups[0];
+  a.ghy = b->groups[1];
   a.pHzx = (T*)b->psi[0];
   a.pHzy = (T*)b->psi[1];
   a.pExy = (T*)b->psi[2];
@@ -181,6 +189,7 @@ BArgs<T> bargs(pf_batch* b) {
   a.fdx = b->fd[0];
   a.fdy = b->fd[1];
   a.ch = (T)b->ch;
+  a.fast = a.fdx && a.fdy && std::fabs(b->ch) >= 0x1p-60 && std::fabs(b->ch) < 0x1p60;
   a.idx = (T)(1.0 / b->dx);
   a.idy = (T)(1.0 / b->dy);
   a.base = b->base;
@@ -242,6 +251,29 @@ AArgs<T> aargs(pf_batch* b) {
 // One tile per block (the kernels also accept a smaller grid).
 int grid_blocks(const pf_batch* b) { return std::max(1, b->ntiles); }
 
+// One step's edge and bulk kernels side by side: the edge tiles' on a second
+// captured stream, both behind everything before and before everything after.
+template <typename T, typename Arg>
+void vec_launch(pf_batch* b, int rows, void (*edge)(const BArgs<T>, const Arg, int),
+                void (*bulk)(const BArgs<T>, const Arg, int), const BArgs<T>& a, const Arg& arg,
+                int t) {
+  const int nbulk = b->ntiles - b->nedge;
+  const bool both = b->nedge > 0 && nbulk > 0;
+  cudaStream_t es = b->stream;
+  if (both) {
+    es = b->side;
+    cudaEventRecord(b->fork, b->stream);
+    cudaStreamWaitEvent(es, b->fork, 0);
+  }
+  if (b->nedge) edge<<<b->nedge, dim3(tile_x<T>(true), 2 * rows), 0, es>>>(a, arg, t);
+  if (nbulk) bulk<<<nbulk, dim3(tile_x<T>(false), rows), 0, b->stream>>>(a, arg, t);
+  if (both) {
+    cudaEventRecord(b->join, es);
+    cudaStreamWaitEvent(b->stream, b->join, 0);
+  }
+  b->capture_launches += (b->nedge > 0) + (nbulk > 0);
+}
+
 template <typename T, int R>
 void fwd_kernels(pf_batch* b, long long len, bool dft) {
   const BArgs<T> a = bargs<T>(b);
@@ -251,10 +283,19 @@ void fwd_kernels(pf_batch* b, long long len, bool dft) {
   const long long ng = b->src.n_groups;
   int pend = 0;
   for (long long t = 0; t < len; ++t) {
-    if (b->fused && b->march) {
-      kb_march<T><<<(unsigned)((b->nsegs + kMarchWarps - 1) / kMarchWarps), dim3(32, kMarchWarps),
-                    0, b->stream>>>(a, (int)t);
-      b->capture_launches += 1;
+    if (b->vec) {
+      StepPost<T> post;
+      post.srow = b->srow;
+      post.scol = b->scol;
+      post.start = b->src.start;
+      post.wave_row = b->src.wave_row;
+      post.amp = b->src.amp;
+      post.wave = b->src.wave;
+      post.n_steps = b->src.n_steps;
+      post.dring = dft ? (T*)b->dring : nullptr;
+      post.nline = b->nline;
+      vec_launch(b, kWarps * R, kb_tile<T, true>, kb_tile<T, false>, a, post,
+                 (int)t);
     } else if (b->fused) {
       kb_step<T, R><<<G, blk, 0, b->stream>>>(a, (int)t);
       b->capture_launches += 1;
@@ -269,7 +310,9 @@ void fwd_kernels(pf_batch* b, long long len, bool dft) {
       b->capture_launches += 2;
     }
     T* dring = dft ? (T*)b->dring : nullptr;
-    if (b->merge_post || !dft) {
+    if (b->vec) {
+      // the step itself injects and samples
+    } else if (b->merge_post || !dft) {
       const long long n = ng + (dft ? b->nline : 0);
       if (n) {
         kb_post<T><<<(unsigned)((n + 127) / 128), 128, 0, b->stream>>>(
@@ -313,16 +356,18 @@ void adj_kernels(pf_batch* b, long long len) {
   const AArgs<T> d = aargs<T>(b);
   const dim3 blk(32, kWarps);
   const int G = grid_blocks(b);
-  if (b->fused && b->march) {
-    const dim3 mg((unsigned)((b->nsegs + kMarchWarps - 1) / kMarchWarps)), mb(32, kMarchWarps);
-    kb_adj_march<T, false, true><<<mg, mb, 0, b->stream>>>(a, d, (int)(len - 1));
+  if (b->vec) {
+    const int tb = kWarps * R;
+    vec_launch(b, tb, kb_adj_tile<T, false, true, true>, kb_adj_tile<T, false, true, false>, a, d,
+               (int)(len - 1));
     for (long long t = len - 1; t >= 0; --t) {
       if (t > 0)
-        kb_adj_march<T, true, true><<<mg, mb, 0, b->stream>>>(a, d, (int)t);
+        vec_launch(b, tb, kb_adj_tile<T, true, true, true>, kb_adj_tile<T, true, true, false>, a, d,
+                   (int)t);
       else
-        kb_adj_march<T, true, false><<<mg, mb, 0, b->stream>>>(a, d, 0);
+        vec_launch(b, tb, kb_adj_tile<T, true, false, true>, kb_adj_tile<T, true, false, false>, a,
+                   d, 0);
     }
-    b->capture_launches += 1 + len;
     return;
   }
   if (b->fused) {
@@ -522,8 +567,11 @@ int pfb_create(int n_inst, int real_bytes, double dx, double dy, double ch, doub
   for (Inst& I : b->inst) memset(&I, 0, sizeof I);
   b->h_ce.resize(n_inst);
   for (int q = 0; q < 8; ++q) b->h_coef[q].resize(n_inst);
-  if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
-    delete b;
+  if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming) != cudaSuccess) {
+    pfb_destroy(b);
     return PF_ERR_CUDA;
   }
   *out = b;
@@ -613,51 +661,88 @@ int pfb_set_dft(pf_batch* b, int n_freq, const double* phase) {
 
 namespace {
 
-// The work list at a tile height of tile_rows rows (x) by 32 cells (y),
-// every instance's tiles in order.
-std::vector<TileRec> make_tiles(const pf_batch* b, int tile_rows) {
-  std::vector<TileRec> tiles;
-  for (int k = 0; k < b->n_inst; ++k) {
-    const Inst& I = b->inst[k];
-    for (int i0 = 0; i0 < I.nx; i0 += tile_rows)
-      for (int j0 = 0; j0 < I.ny; j0 += 32) {
-        TileRec tr;
-        tr.base = I.off + (long long)i0 * I.pitch + j0;
-        tr.nx = I.nx;
-        tr.ny = I.ny;
-        tr.pitch = I.pitch;
-        tr.i0 = i0;
-        tr.j0 = j0;
-        tr.ox = I.ox + i0;
-        tr.oy = I.oy + j0;
-        tr.k = k;
-        tr.wdi = I.di0 - i0;
-        tr.wdj = I.dj0 - j0;
-        tr.wdn = I.dn;
-        tr.pad[0] = 0;
-        tiles.push_back(tr);
-      }
-  }
-  return tiles;
+TileRec tile_at(const pf_batch* b, int k, int i0, int j0, int rows, int cols) {
+  const Inst& I = b->inst[k];
+  TileRec tr;
+  memset(&tr, 0, sizeof tr);
+  tr.base = I.off + (long long)i0 * I.pitch + j0;
+  tr.nx = I.nx;
+  tr.ny = I.ny;
+  tr.pitch = I.pitch;
+  tr.i0 = i0;
+  tr.j0 = j0;
+  tr.ox = I.ox + i0;
+  tr.oy = I.oy + j0;
+  tr.k = k;
+  tr.wdi = I.di0 - i0;
+  tr.wdj = I.dj0 - j0;
+  tr.wdn = I.dn;
+  tr.p_hzx = I.p_hzx;
+  tr.p_hzy = I.p_hzy;
+  tr.p_exy = I.p_exy;
+  tr.p_eyx = I.p_eyx;
+  tr.nphy = I.nphy;
+  tr.npey = I.npey;
+  const int i1 = i0 + rows, j1 = j0 + cols;
+  if (i0 < I.di0 + I.dn && i1 > I.di0 && j0 < I.dj0 + I.dn && j1 > I.dj0) tr.flags |= kTileWindow;
+  bool post = I.line_i >= i0 && I.line_i < i1;
+  for (int i = i0; i < std::min(i1, I.nx) && !post; ++i)
+    post = !b->src_rows.empty() && b->src_rows[I.ox + i];
+  if (post) tr.flags |= kTilePost;
+  return tr;
 }
 
-// The marching segments at a height of seg_rows rows: every instance's
-// strips of 31 owned columns, each cut into row ranges.
-std::vector<SegRec> make_segs(const pf_batch* b, int seg_rows) {
-  std::vector<SegRec> segs;
+// The work list at a tile height of tile_rows rows (x): tiles of 32 columns
+// (y), every instance's in order; for the vector steps the bulk region of
+// every instance in such tiles, and first the frame around it (CPML layers,
+// grid edges, what the bulk tiles leave over) in tiles of 16 columns and 2 x
+// tile_rows rows, which the edge kernels take.
+std::vector<TileRec> make_tiles(const pf_batch* b, int tile_rows) {
+  std::vector<TileRec> edge, bulk;
   for (int k = 0; k < b->n_inst; ++k) {
     const Inst& I = b->inst[k];
-    for (int j0 = 0; j0 < I.ny; j0 += kMarchCols)
-      for (int i0 = 0; i0 < I.nx; i0 += seg_rows) {
-        SegRec sg;
-        sg.k = k;
-        sg.i0 = i0;
-        sg.i1 = std::min(I.nx, i0 + seg_rows);
-        sg.j0 = j0;
-        segs.push_back(sg);
+    if (!b->vec) {
+      for (int i0 = 0; i0 < I.nx; i0 += tile_rows)
+        for (int j0 = 0; j0 < I.ny; j0 += 32) bulk.push_back(tile_at(b, k, i0, j0, tile_rows, 32));
+      continue;
+    }
+    const auto& in = b->inner[k];
+    int A = std::max(1, in[0]) + 1, B = std::min(I.nx - 1, in[1]);
+    int C = (std::max(1, in[2]) + 1 + 15) / 16 * 16, D = std::min(I.ny - 1, in[3]);
+    B = A + std::max(0, B - A) / tile_rows * tile_rows;
+    D = C + std::max(0, D - C) / 32 * 32;
+    if (B <= A || D <= C) A = B = C = D = 0;
+    auto frame = [&](int i0, int i1, int j0, int j1) {
+      for (int i = i0; i < i1; i += 2 * tile_rows)
+        for (int j = j0; j < j1; j += 16) {
+          TileRec t = tile_at(b, k, i, j, 2 * tile_rows, 16);
+          t.nx_end = std::min(i1, i + 2 * tile_rows);
+          edge.push_back(t);
+        }
+    };
+    if (A == B) {
+      frame(0, I.nx, 0, I.ny);
+      continue;
+    }
+    frame(0, I.nx, 0, C);
+    frame(0, I.nx, D, I.ny);
+    frame(0, A, C, D);
+    frame(B, I.nx, C, D);
+    for (int i0 = A; i0 < B; i0 += tile_rows)
+      for (int j0 = C; j0 < D; j0 += 32) {
+        TileRec t = tile_at(b, k, i0, j0, tile_rows, 32);
+        t.flags |= kTileBulk;
+        bulk.push_back(t);
       }
   }
-  return segs;
+  edge.insert(edge.end(), bulk.begin(), bulk.end());
+  return edge;
+}
+
+int count_edge(const std::vector<TileRec>& tiles) {
+  int n = 0;
+  for (const TileRec& t : tiles) n += (t.flags & kTileBulk) ? 0 : 1;  // they come first
+  return n;
 }
 
 int set_tile_rows(pf_batch* b, int tile_rows) {
@@ -665,15 +750,10 @@ int set_tile_rows(pf_batch* b, int tile_rows) {
   if (tiles.size() > b->tile_cap) return bfail(b, PF_ERR_INVALID, "tile list exceeds its buffer");
   B_CUDA(b, cudaMemcpyAsync(b->d_tiles, tiles.data(), tiles.size() * sizeof(TileRec),
                             cudaMemcpyHostToDevice, b->stream));
-  // the marching steps' segments are 2 x tile_rows rows high
-  const std::vector<SegRec> segs = make_segs(b, 2 * tile_rows);
-  if (segs.size() > b->seg_cap) return bfail(b, PF_ERR_INVALID, "segment list exceeds its buffer");
-  B_CUDA(b, cudaMemcpyAsync(b->d_segs, segs.data(), segs.size() * sizeof(SegRec),
-                            cudaMemcpyHostToDevice, b->stream));
-  b->nsegs = (int)segs.size();
-  B_CUDA(b, cudaStreamSynchronize(b->stream));  // before `tiles` and `segs` go
+  B_CUDA(b, cudaStreamSynchronize(b->stream));  // before `tiles` goes
   destroy_graphs(b);  // captured with the old grid and row count
   b->ntiles = (int)tiles.size();
+  b->nedge = count_edge(tiles);
   b->rows = tile_rows / kWarps;
   b->tile_rows = tile_rows;
   return PF_OK;
@@ -761,7 +841,7 @@ int pfb_finalize(pf_batch* b, int checkpoint_every, int tile_rows) {
   b->ckpt = (int)std::min<long long>(b->fwd_only ? 512 : checkpoint_every, b->n_steps);
   b->rows = tile_rows / kWarps;
   const size_t S = b->rb;
-  std::vector<int> mp[4];
+  std::vector<int> mp[4], grp[2];
   std::vector<char> coefp[8], cep;
   std::vector<long long> lcell;
   std::vector<TileRec> tiles;
@@ -784,69 +864,104 @@ int pfb_finalize(pf_batch* b, int checkpoint_every, int tile_rows) {
     };
     I.npex = build(b->h_coef[1][k], I.nx, mp[0]);
     I.nphx = build(b->h_coef[3][k], I.nx, mp[1]);
-    I.npey = build(b->h_coef[5][k], I.ny, mp[2]);
-    I.nphy = build(b->h_coef[7][k], I.ny, mp[3]);
+    // y: whole groups of four columns, so that psi rows are vectors; the
+    // pooled columns of an instance start on a group
+    const int ny4 = (I.ny + 3) / 4 * 4;
+    auto build4 = [&](const std::vector<char>& c, std::vector<int>& pool, std::vector<int>& groups) {
+      int cnt = 0;
+      for (int t = 0; t < ny4; t += 4) {
+        bool any = false;
+        for (int u = t; u < t + 4; ++u) {
+          const double v = u >= I.ny ? 0.0
+                           : S == 4  ? (double)((const float*)c.data())[u]
+                                     : ((const double*)c.data())[u];
+          pool.push_back(v != 0.0 ? 4 * cnt + (u - t) : -1);
+          any = any || v != 0.0;
+        }
+        groups.push_back(any ? cnt++ : -1);
+      }
+      return 4 * cnt;
+    };
+    I.npey = build4(b->h_coef[5][k], mp[2], grp[0]);
+    I.nphy = build4(b->h_coef[7][k], mp[3], grp[1]);
     I.p_hzx = b->npsi[0];
     I.p_hzy = b->npsi[1];
     I.p_exy = b->npsi[2];
     I.p_eyx = b->npsi[3];
-    b->npsi[0] += (long long)I.nphx * I.ny;
+    b->npsi[0] += (long long)I.nphx * I.pitch;
     b->npsi[1] += (long long)I.nx * I.nphy;
     b->npsi[2] += (long long)I.nx * I.npey;
-    b->npsi[3] += (long long)I.npex * I.ny;
+    b->npsi[3] += (long long)I.npex * I.pitch;
     {
       const size_t row = (size_t)I.ny * S, prow = (size_t)I.pitch * S, o = cep.size();
       cep.resize(o + (size_t)I.nx * prow, 0);
       for (int i = 0; i < I.nx; ++i)
         memcpy(cep.data() + o + i * prow, b->h_ce[k].data() + i * row, row);
     }
-    for (int q = 0; q < 8; ++q)
+    for (int q = 0; q < 8; ++q) {
       coefp[q].insert(coefp[q].end(), b->h_coef[q][k].begin(), b->h_coef[q][k].end());
+      if (q >= 4) coefp[q].resize(coefp[q].size() + (size_t)(ny4 - I.ny) * S, 0);
+    }
     for (int j = 0; j < I.ny; ++j) lcell.push_back(I.off + (long long)I.line_i * I.pitch + j);
     b->ncell += (long long)I.nx * I.pitch;
     b->ncell_real += (long long)I.nx * I.ny;
     b->nx_tot += I.nx;
-    b->ny_tot += I.ny;
+    b->ny_tot += ny4;
     b->n_design += (long long)I.dn * I.dn;
     b->nline += I.ny;
     std::vector<char>().swap(b->h_ce[k]);
   }
-  tiles = make_tiles(b, tile_rows);
-  b->tile_cap = make_tiles(b, 8).size();
-  if ((long long)b->tile_cap >= (1LL << 31)) return bfail(b, PF_ERR_INVALID, "too many tiles");
-  b->ntiles = (int)tiles.size();
-  b->tile_rows = tile_rows;
-  int rc;
-  if ((rc = bup(b, (void**)&b->d_inst, b->inst.data(), b->inst.size() * sizeof(Inst)))) return rc;
-  if ((rc = balloc(b, (void**)&b->d_tiles, b->tile_cap * sizeof(TileRec)))) return rc;
-  B_CUDA(b, cudaMemcpyAsync(b->d_tiles, tiles.data(), tiles.size() * sizeof(TileRec),
-                            cudaMemcpyHostToDevice, b->stream));
-  {
-    const std::vector<SegRec> segs = make_segs(b, 2 * tile_rows);
-    b->seg_cap = make_segs(b, 16).size();
-    if ((long long)b->seg_cap >= (1LL << 31)) return bfail(b, PF_ERR_INVALID, "too many segments");
-    b->nsegs = (int)segs.size();
-    if ((rc = balloc(b, (void**)&b->d_segs, b->seg_cap * sizeof(SegRec)))) return rc;
-    B_CUDA(b, cudaMemcpyAsync(b->d_segs, segs.data(), segs.size() * sizeof(SegRec),
-                              cudaMemcpyHostToDevice, b->stream));
-    B_CUDA(b, cudaStreamSynchronize(b->stream));
-    b->march = !getenv("PFB200_BATCH_TILESTEP");
-  }
-  if ((rc = bup(b, &b->ce, cep.data(), cep.size()))) return rc;
-  for (int q = 0; q < 8; ++q)
-    if ((rc = bup(b, &b->coef[q], coefp[q].data(), coefp[q].size()))) return rc;
-  for (int q = 0; q < 4; ++q)
-    if ((rc = bup(b, (void**)&b->maps[q], mp[q].data(), mp[q].size() * 4))) return rc;
-  for (void** p : {&b->Ex, &b->Ey, &b->Hz})
-    if ((rc = balloc(b, p, b->ncell * S))) return rc;
-  for (int q = 0; q < 4; ++q)
-    if ((rc = balloc(b, &b->psi[q], b->npsi[q] * S))) return rc;
   // the fused steps need no H-family source (an Hz source would have to
   // reach the halo recomputation); PFB200_BATCH_SPLIT=1 keeps the split
   // passes
   bool any_h = false;
   for (size_t q = 0; q < b->s_comp.size(); ++q) any_h = any_h || b->s_comp[q] == 2;
   b->fused = !any_h && !getenv("PFB200_BATCH_SPLIT");
+  b->vec = b->fused && !getenv("PFB200_BATCH_TILESTEP");
+  // interior stretches and source rows, before the tiles that are marked by them
+  b->inner.resize(b->n_inst);
+  for (int k = 0; k < b->n_inst; ++k) {
+    const Inst& I = b->inst[k];
+    auto stretch = [](const std::vector<int>& e, const std::vector<int>& h, size_t o, int n,
+                      int& b0, int& b1) {
+      b0 = b1 = 0;
+      for (int t = 0, s0 = 0; t <= n; ++t)
+        if (t == n || e[o + t] >= 0 || h[o + t] >= 0) {
+          if (t - s0 > b1 - b0) { b0 = s0; b1 = t; }
+          s0 = t + 1;
+        }
+    };
+    stretch(mp[0], mp[1], I.ox, I.nx, b->inner[k][0], b->inner[k][1]);
+    stretch(mp[2], mp[3], I.oy, I.ny, b->inner[k][2], b->inner[k][3]);
+  }
+  b->src_rows.assign((size_t)b->nx_tot, 0);
+  for (size_t q = 0; q < b->s_cell.size(); ++q) {
+    const Inst& I = b->inst[(int)(b->s_cell[q] >> 32)];
+    b->src_rows[I.ox + (b->s_cell[q] & 0xffffffffLL) / I.ny] = 1;
+  }
+  tiles = make_tiles(b, tile_rows);
+  b->tile_cap = make_tiles(b, 8).size();
+  if ((long long)b->tile_cap >= (1LL << 31)) return bfail(b, PF_ERR_INVALID, "too many tiles");
+  b->ntiles = (int)tiles.size();
+  b->nedge = count_edge(tiles);
+  b->tile_rows = tile_rows;
+  int rc;
+  if ((rc = bup(b, (void**)&b->d_inst, b->inst.data(), b->inst.size() * sizeof(Inst)))) return rc;
+  if ((rc = balloc(b, (void**)&b->d_tiles, b->tile_cap * sizeof(TileRec)))) return rc;
+  B_CUDA(b, cudaMemcpyAsync(b->d_tiles, tiles.data(), tiles.size() * sizeof(TileRec),
+                            cudaMemcpyHostToDevice, b->stream));
+  B_CUDA(b, cudaStreamSynchronize(b->stream));
+  if ((rc = bup(b, &b->ce, cep.data(), cep.size()))) return rc;
+  for (int q = 0; q < 8; ++q)
+    if ((rc = bup(b, &b->coef[q], coefp[q].data(), coefp[q].size()))) return rc;
+  for (int q = 0; q < 4; ++q)
+    if ((rc = bup(b, (void**)&b->maps[q], mp[q].data(), mp[q].size() * 4))) return rc;
+  for (int q = 0; q < 2; ++q)
+    if ((rc = bup(b, (void**)&b->groups[q], grp[q].data(), grp[q].size() * 4))) return rc;
+  for (void** p : {&b->Ex, &b->Ey, &b->Hz})
+    if ((rc = balloc(b, p, b->ncell * S))) return rc;
+  for (int q = 0; q < 4; ++q)
+    if ((rc = balloc(b, &b->psi[q], b->npsi[q] * S))) return rc;
   if (b->fused) {
     for (int q = 0; q < 3; ++q)
       if ((rc = balloc(b, &b->lvl1[q], b->ncell * S))) return rc;
@@ -901,6 +1016,26 @@ int pfb_finalize(pf_batch* b, int checkpoint_every, int tile_rows) {
   }
   b->src.n_groups = (int)b->s_cell.size();
   b->src.n_steps = b->n_steps;
+  if (b->src.n_groups && b->vec) {
+    // rows with E sources: each column's Ex and Ey source group, or -1
+    std::vector<int> srow((size_t)b->nx_tot, -1), scol;
+    for (size_t g = 0; g < b->s_cell.size(); ++g) {
+      const long long c = b->s_cell[g];
+      const auto it = std::upper_bound(b->inst.begin(), b->inst.end(), c,
+                                       [](long long v, const Inst& I) { return v < I.off; });
+      const Inst& I = *(it - 1);
+      const int i = (int)((c - I.off) / I.pitch), j = (int)((c - I.off) % I.pitch);
+      int& row = srow[I.ox + i];
+      if (row < 0) {
+        row = (int)scol.size();
+        scol.resize(scol.size() + 2 * (size_t)I.ny, -1);
+      }
+      scol[row + b->s_comp[g] * I.ny + j] = (int)g;
+    }
+    if ((rc = bup(b, (void**)&b->srow, srow.data(), srow.size() * 4))) return rc;
+    if ((rc = bup(b, (void**)&b->scol, scol.data(), scol.size() * 4))) return rc;
+    B_CUDA(b, cudaStreamSynchronize(b->stream));
+  }
   if (b->src.n_groups) {
     if ((rc = bup(b, (void**)&b->src.cell, b->s_cell.data(), b->s_cell.size() * 8))) return rc;
     if ((rc = bup(b, (void**)&b->src.comp, b->s_comp.data(), b->s_comp.size() * 4))) return rc;
@@ -1015,6 +1150,9 @@ void pfb_destroy(pf_batch* b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   destroy_graphs(b);
   for (void* p : b->allocs) cudaFree(p);
+  if (b->fork) cudaEventDestroy(b->fork);
+  if (b->join) cudaEventDestroy(b->join);
+  if (b->side) cudaStreamDestroy(b->side);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
 }

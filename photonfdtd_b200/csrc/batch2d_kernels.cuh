@@ -29,14 +29,18 @@ constexpr int kWarps = 8;     // warps per block
 #ifndef PFB_MINB_ASTEP
 #define PFB_MINB_ASTEP 4
 #endif
-// Minimum resident 128-thread blocks per SM of the marching forward and
-// reverse steps (forward at 12: 40 registers, measured 5% faster than at 10;
-// the reverse step needs 46-48 registers and slows down at 12).
-#ifndef PFB_MINB_MARCH
-#define PFB_MINB_MARCH 12
+// Minimum resident 256-thread blocks per SM of the vector steps (float).
+#ifndef PFB_MINB_TILE
+#define PFB_MINB_TILE 4
 #endif
-#ifndef PFB_MINB_AMARCH
-#define PFB_MINB_AMARCH 10
+#ifndef PFB_MINB_ATILE
+#define PFB_MINB_ATILE 4
+#endif
+#ifndef PFB_MINB_EDGE
+#define PFB_MINB_EDGE 2
+#endif
+#ifndef PFB_MINB_AEDGE
+#define PFB_MINB_AEDGE 3
 #endif
 constexpr int kDftRing = 32;  // line samples kept before a DFT flush
 
@@ -46,7 +50,7 @@ struct Inst {
   long long off;                         // first cell in the pooled field arrays (32-aligned)
   int ox, oy;                            // first entry in the pooled x / y coefficients
   long long p_hzx, p_hzy, p_exy, p_eyx;  // first element of each psi array
-  int nphx, nphy, npex, npey;            // compact psi extents along their axes
+  int nphx, nphy, npex, npey;            // psi extents along their axes (y: whole groups of 4)
   int di0, dj0, dn;                      // design window
   long long goff;                        // first design cell (dn * dn per instance)
   int line_i;                            // x index of the output line
@@ -60,32 +64,44 @@ struct __align__(16) TileRec {
   int ox, oy;          // pooled coefficient index of row i0 / column j0
   int k;               // instance
   int wdi, wdj, wdn;   // design window relative to the tile origin, its size
-  int pad[1];
+  int flags;           // kTile* below
+  long long p_hzx, p_hzy, p_exy, p_eyx;  // the instance's psi arrays
+  int nphy, npey;
+  int nx_end;          // edge tiles: rows from here on belong to another tile
+  int pad;
 };
+// A tile of the vector steps whose cells and the row above and column left of
+// them lie in the interior (every difference exists) and hold no CPML state.
+constexpr int kTileBulk = 1;
+constexpr int kTileWindow = 2;  // some cells of the design window
+constexpr int kTilePost = 4;    // the output line or a row with sources
 
-// A marching segment: instance k, rows [i0, i1), owned columns [j0, j0 + 31).
-// Its warp's lane l holds column j0 - 1 + l: lane 0 is the halo column.
-struct SegRec {
-  int k, i0, i1, j0;
-};
-constexpr int kMarchCols = 31;  // owned columns per warp
-constexpr int kMarchWarps = 4;  // warps (segments) per block
+// Columns per thread of the vector steps (16 bytes), and threads per tile row:
+// bulk tiles are 32 columns wide, edge tiles 16 (the CPML layers at the ends
+// of a row are about that wide) and twice as high.
+template <typename T>
+constexpr int kTileV = 16 / (int)sizeof(T);
+template <typename T>
+__host__ __device__ constexpr int tile_x(bool edge) {
+  return (edge ? 16 : 32) / kTileV<T>;
+}
 
 template <typename T>
 struct BArgs {
   const Inst* inst;
   const TileRec* tiles;
   int ntiles;
-  const SegRec* segs;
-  int nsegs;
+  int nedge;  // the first nedge tiles are not kTileBulk
   T *Ex, *Ey, *Hz;
   const T* ce;
   const T *bex, *cex, *bhx, *chx, *bey, *cey, *bhy, *chy;
   const int *mex, *mhx, *mey, *mhy;
+  const int *gey, *ghy;  // per 4 pooled columns: psi group (4 entries), or -1
   T *pHzx, *pHzy, *pExy, *pEyx;
   T dx, dy, rdx, rdy, ch;
   T idx, idy;  // 1/dx, 1/dy rounded once (adjoint kernels only)
   bool fdx, fdy;
+  bool fast;   // fdx, fdy, and ch scaled down by QScale is exact
   const long long* base;  // first step of the running chunk
   T* ring;                // design-window curls, slot = n mod ring_len
   long long n_design;
@@ -131,7 +147,7 @@ __global__ void __launch_bounds__(32 * kWarps) kb_h(const __grid_constant__ BArg
       if (mx[r] >= 0 || my >= 0) {
         const Inst& I = a.inst[tr.k];
         if (mx[r] >= 0) {
-          const long long q = I.p_hzx + (long long)mx[r] * tr.ny + j;
+          const long long q = I.p_hzx + (long long)mx[r] * tr.pitch + j;
           const int c = tr.ox + r0 + r;
           const T psi = add_rn(mul_rn(a.bhx[c], a.pHzx[q]), mul_rn(a.chx[c], dA));
           a.pHzx[q] = psi;
@@ -203,7 +219,7 @@ __global__ void __launch_bounds__(32 * kWarps) kb_e(const __grid_constant__ BArg
         cy = -dB;
         if (mx[r] >= 0) {
           const Inst& I = a.inst[tr.k];
-          const long long q = I.p_eyx + (long long)mx[r] * tr.ny + j;
+          const long long q = I.p_eyx + (long long)mx[r] * tr.pitch + j;
           const int c = tr.ox + r0 + r;
           const T psi = add_rn(mul_rn(a.bex[c], a.pEyx[q]), mul_rn(a.cex[c], dB));
           a.pEyx[q] = psi;
@@ -249,7 +265,7 @@ __device__ __forceinline__ T hz_value(const BArgs<T>& a, const Inst& I, int i, i
   qdiv2(sub_rn(eyp, ey), a.dx, a.rdx, a.fdx, sub_rn(exp_, ex), a.dy, a.rdy, a.fdy, dA, dB);
   T h = add_rn(hz, mul_rn(sub_rn(dA, dB), mch));
   if (mx >= 0) {
-    const long long q = I.p_hzx + (long long)mx * ny + j;
+    const long long q = I.p_hzx + (long long)mx * I.pitch + j;
     const T psi = add_rn(mul_rn(a.bhx[crow], pzx[q]), mul_rn(a.chx[crow], dA));
     if (pzxo) pzxo[q] = psi;
     h = add_rn(h, mul_rn(mch, psi));
@@ -391,7 +407,7 @@ __global__ void __launch_bounds__(32 * kWarps, PFB_MINB_STEP) kb_step(
         e = add_rn(ey[r], mul_rn(-dB, K[r]));
         cy = -dB;
         if (mxe[r] >= 0) {
-          const long long q = I.p_eyx + (long long)mxe[r] * tr.ny + j;
+          const long long q = I.p_eyx + (long long)mxe[r] * tr.pitch + j;
           const int c = tr.ox + r0 + r;
           const T psi = add_rn(mul_rn(a.bex[c], a.pEyx[q]), mul_rn(a.cex[c], dB));
           a.pEyx[q] = psi;
@@ -412,143 +428,355 @@ __global__ void __launch_bounds__(32 * kWarps, PFB_MINB_STEP) kb_step(
   }
 }
 
-// ---- marching forward step ---------------------------------------------------
-// One warp per segment marches down its rows: lane l holds column
-// j0 - 1 + l, so the left neighbour of every owned column (lanes 1..31) sits
-// in the lane below and the right neighbour in the lane above (shuffles);
-// lane 0 is a halo column whose Hz it recomputes without storing, and lane 31
-// loads the one Ex beyond the strip. The Hz of the previous row stays in a
-// register; a segment that starts below row 0 first recomputes its row
-// i0 - 1 (Hz only). The next row's loads are issued before the current row is
-// computed. As in kb_step, level n & 1 is read and level (n & 1) ^ 1
-// written, so segments never race, and every cell's arithmetic is kb_h's and
-// kb_e's (hz_value and the E update below), bit for bit. No shared memory,
-// no barriers, about four cell loads and three stores per cell and step.
+// ---- vector forward step -------------------------------------------------------
+// What the vector step does after its E update: the E sources and the
+// output-line samples (kb_post's work; a separate launch per step cost 3 us).
+// srow[x row]: -1, or where the row's source groups per column start in scol
+// (Ex for ny columns, then Ey); dring: null in replays.
 template <typename T>
-__global__ void __launch_bounds__(32 * kMarchWarps, PFB_MINB_MARCH) kb_march(
-    const __grid_constant__ BArgs<T> a, int step_t) {
-  const int w = blockIdx.x * kMarchWarps + threadIdx.y;
-  if (w >= a.nsegs) return;  // uniform over the warp
-  const SegRec sg = a.segs[w];
-  const Inst& I = a.inst[sg.k];
-  const long long n = *a.base + step_t;
+struct StepPost {
+  const int* srow;
+  const int* scol;
+  const int* start;
+  const int* wave_row;
+  const double* amp;
+  const double* wave;
+  long long n_steps;
+  T* dring;
+  long long nline;
+};
+
+__device__ __forceinline__ void tld(const float* p, float (&o)[4]) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+}
+__device__ __forceinline__ void tld(const double* p, double (&o)[2]) {
+  const double2 v = *reinterpret_cast<const double2*>(p);
+  o[0] = v.x; o[1] = v.y;
+}
+// The vector at p when ok, else zeros.
+template <typename T>
+__device__ __forceinline__ void tld_if(const T* p, bool ok, T (&o)[kTileV<T>]) {
+  if (ok) {
+    tld(p, o);
+  } else {
+#pragma unroll
+    for (int v = 0; v < kTileV<T>; ++v) o[v] = T(0);
+  }
+}
+// Stores the vector's first n columns (n >= 1).
+__device__ __forceinline__ void tst(float* p, const float (&o)[4], int n) {
+  if (n >= 4) {
+    *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
+  } else {
+    p[0] = o[0];
+    if (n > 1) p[1] = o[1];
+    if (n > 2) p[2] = o[2];
+  }
+}
+__device__ __forceinline__ void tst(double* p, const double (&o)[2], int n) {
+  if (n >= 2) *reinterpret_cast<double2*>(p) = make_double2(o[0], o[1]);
+  else p[0] = o[0];
+}
+
+// CPML of a thread's columns (y axis) and row (x axis) of one field family.
+// The y layers' psi rows hold whole groups of four columns, the x layers' rows
+// have the fields' pitch, so psi and column coefficients are vectors like the
+// fields; a column has CPML state exactly where its coefficient c is not 0.
+// An edge thread loads everything in two rounds before its first use (fields
+// and indices, then coefficients and psi): loaded where they are used, between
+// the psi stores, they made one serial chain of memory latencies.
+template <typename T, int NV>
+struct ColPml {
+  T b[NV], c[NV];
+};
+template <typename T>
+__device__ __forceinline__ void load_cols(const T* b, const T* c, int at, bool ok,
+                                          ColPml<T, kTileV<T>>& p) {
+  tld_if<T>(b + at, ok, p.b);
+  tld_if<T>(c + at, ok, p.c);
+}
+template <typename T>
+struct RowPml {
+  int m;
+  T b, c;
+};
+template <typename T>
+__device__ __forceinline__ RowPml<T> load_row(const int* map, const T* b, const T* c, int at,
+                                              bool ok) {
+  RowPml<T> p;
+  p.m = ok ? __ldg(map + at) : -1;
+  p.b = ok ? __ldg(b + at) : T(0);
+  p.c = ok ? __ldg(c + at) : T(0);
+  return p;
+}
+
+// Hz^{n+1/2} of NV interior columns without CPML state.
+template <typename T, int NV>
+__device__ __forceinline__ void h_cols(const BArgs<T>& a, const T (&ey)[NV], const T (&eyn)[NV],
+                                       const T (&ex)[NV], T exr, const T (&hz)[NV], T (&h)[NV]) {
+  const T up = QScale<T>::up;
+  const T mch = -a.ch, mchs = mul_rn(mch, QScale<T>::down);
+  T nA[NV], nB[NV], m = T(0);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    nA[v] = fma_rn(eyn[v], up, -mul_rn(ey[v], up));
+    nB[v] = fma_rn(v + 1 < NV ? ex[v + 1 < NV ? v + 1 : 0] : exr, up, -mul_rn(ex[v], up));
+    m = absmax(m, absmax(nA[v], nB[v]));
+  }
+  if (a.fast && m < QScale<T>::limit * up) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+      h[v] = add_rn(hz[v], mul_rn(sub_rn(qscaled(nA[v], a.dx, a.rdx), qscaled(nB[v], a.dy, a.rdy)),
+                                  mchs));
+    return;
+  }
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const T dA = div_cold(sub_rn(eyn[v], ey[v]), a.dx);
+    const T dB = div_cold(sub_rn(v + 1 < NV ? ex[v + 1 < NV ? v + 1 : 0] : exr, ex[v]), a.dy);
+    h[v] = add_rn(hz[v], mul_rn(sub_rn(dA, dB), mch));
+  }
+}
+// The same anywhere: kb_h's tests, and psi (vx, vy: before and after).
+template <typename T, int NV>
+__device__ __forceinline__ void h_cols_pml(const BArgs<T>& a, int j, int ny, bool row,
+                                           const RowPml<T>& rp, const ColPml<T, NV>& cp,
+                                           const T (&ey)[NV], const T (&eyn)[NV],
+                                           const T (&ex)[NV], T exr, const T (&hz)[NV],
+                                           T (&vx)[NV], T (&vy)[NV], T (&h)[NV]) {
+  const T mch = -a.ch;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    h[v] = hz[v];
+    if (!row || j + v >= ny - 1) continue;
+    const T nA = sub_rn(eyn[v], ey[v]);
+    const T nB = sub_rn(v + 1 < NV ? ex[v + 1 < NV ? v + 1 : 0] : exr, ex[v]);
+    T dA, dB;
+    if (a.fast && qdiv_ok(absmax(nA, nB))) {
+      dA = qdiv_fast(nA, a.dx, a.rdx);
+      dB = qdiv_fast(nB, a.dy, a.rdy);
+    } else {
+      dA = div_cold(nA, a.dx);
+      dB = div_cold(nB, a.dy);
+    }
+    h[v] = add_rn(hz[v], mul_rn(sub_rn(dA, dB), mch));
+    if (rp.m >= 0) {
+      vx[v] = add_rn(mul_rn(rp.b, vx[v]), mul_rn(rp.c, dA));
+      h[v] = add_rn(h[v], mul_rn(mch, vx[v]));
+    }
+    if (cp.c[v] != T(0)) {
+      vy[v] = add_rn(mul_rn(cp.b[v], vy[v]), mul_rn(cp.c[v], dB));
+      h[v] = add_rn(h[v], mul_rn(a.ch, vy[v]));
+    }
+  }
+}
+
+// The step of one thread's V columns of row r. Everything it needs is loaded
+// at once; Hz of the row above and of the column to the left are recomputed
+// (the left one by the first thread of a tile row, the others take their
+// neighbour's by shuffle). EDGE: tiles with grid edges or CPML state.
+template <typename T, bool EDGE>
+__device__ __forceinline__ void tile_step(const BArgs<T>& a, const StepPost<T>& post,
+                                          const TileRec& tr, long long n, int step_t) {
+  constexpr int V = kTileV<T>, X = tile_x<T>(EDGE);
   const int L = (int)(n & 1);
-  const T* Ex = a.Ex2[L];
-  const T* Ey = a.Ey2[L];
-  const T* Hz = a.Hz2[L];
-  T* Exo = a.Ex2[L ^ 1];
-  T* Eyo = a.Ey2[L ^ 1];
-  T* Hzo = a.Hz2[L ^ 1];
-  const T* pzx = a.pHzx2[L];
-  const T* pzy = a.pHzy2[L];
-  T* pzxo = a.pHzx2[L ^ 1];
-  T* pzyo = a.pHzy2[L ^ 1];
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x;
-  const int nx = I.nx, ny = I.ny;
-  const long long pitch = I.pitch;
-  const int j = sg.j0 - 1 + lane;
-  const bool jv = j >= 0 && j < ny;
-  const bool own = lane >= 1 && jv;
-  const bool hcol = jv && j < ny - 1;       // Hz is updated in this column
-  const bool xr = lane == 31 && j + 1 < ny;  // lane 31 loads Ex one column right
-  const long long c0 = I.off + j;           // pooled index of (0, j)
-  const int myh = jv ? a.mhy[I.oy + j] : -1;
-  const int mye = jv ? a.mey[I.oy + j] : -1;
-  const int slot = (int)(n % a.ring_len);
-  const int r_first = sg.i0 > 0 ? sg.i0 - 1 : 0;
-  // row r_first
-  T ex = T(0), hz = T(0), ey = T(0), eyn = T(0), K = T(0), ex31 = T(0);
-  {
-    const long long id = c0 + r_first * pitch;
-    if (jv) {
-      ex = Ex[id];
-      hz = Hz[id];
-      ey = Ey[id];
-      if (r_first + 1 < nx) eyn = Ey[id + pitch];
-      if (r_first >= sg.i0) K = a.ce[id];
-    }
-    if (xr) ex31 = Ex[id + 1];
+  const int r = tr.i0 + threadIdx.y, j = tr.j0 + threadIdx.x * V;
+  const bool live = !EDGE || (r < tr.nx_end && j < tr.ny);
+  const int nv = EDGE ? (live ? min(V, tr.ny - j) : 0) : V;
+  const int pitch = tr.pitch;
+  const long long id = tr.base + (long long)threadIdx.y * pitch + threadIdx.x * V;
+  const T* Ex = a.Ex2[L] + id;
+  const T* Ey = a.Ey2[L] + id;
+  const T* Hz = a.Hz2[L] + id;
+  const bool top = !EDGE || (live && r >= 1);              // the row above exists
+  const bool low = !EDGE || (live && r + 1 < tr.nx);       // the row below
+  const bool right = !EDGE || (live && j + V < tr.ny);
+  const bool left = threadIdx.x == 0 && (!EDGE || (live && j >= 1));
+  T ey0[V], ey1[V], ey2[V], ex0[V], ex1[V], hz0[V], hz1[V], K[V];
+  tld_if<T>(Ey - pitch, top, ey0);
+  tld_if<T>(Ey, live, ey1);
+  tld_if<T>(Ey + pitch, low, ey2);
+  tld_if<T>(Ex - pitch, top, ex0);
+  tld_if<T>(Ex, live, ex1);
+  tld_if<T>(Hz - pitch, top, hz0);
+  tld_if<T>(Hz, live, hz1);
+  tld_if<T>(a.ce + id, live, K);
+  const T exr0 = top && right ? Ex[V - pitch] : T(0), exr1 = right ? Ex[V] : T(0);
+  T eyl[1] = {T(0)}, eyln[1] = {T(0)}, exl[1] = {T(0)}, hzl[1] = {T(0)};
+  if (left) {
+    eyl[0] = Ey[-1];
+    if (low) eyln[0] = Ey[pitch - 1];
+    exl[0] = Ex[-1];
+    hzl[0] = Hz[-1];
   }
-  T hz_prev = T(0);  // Hz^{n+1/2} of the row above
-  for (int r = r_first; r < sg.i1; ++r) {
-    // the next row's loads first
-    const int r1 = r + 1;
-    T ex_n = T(0), hz_n = T(0), eyn_n = T(0), K_n = T(0), ex31_n = T(0);
-    if (r1 < sg.i1) {
-      const long long id = c0 + r1 * pitch;
-      if (jv) {
-        ex_n = Ex[id];
-        hz_n = Hz[id];
-        if (r1 + 1 < nx) eyn_n = Ey[id + pitch];
-        K_n = a.ce[id];
+  T hp[V], h[V], hl[1] = {T(0)};
+  ColPml<T, V> ce;
+  RowPml<T> re;
+  T wx[V], wy[V];  // E psi
+  long long qex = 0, qey = 0;
+  bool ecol = false;
+  if constexpr (EDGE) {
+    const int cy = tr.oy + (j - tr.j0), cx = tr.ox + (r - tr.i0);
+    const int gh = live ? __ldg(a.ghy + (cy >> 2)) : -1, ge = live ? __ldg(a.gey + (cy >> 2)) : -1;
+    const int gl = left ? __ldg(a.ghy + ((cy - 1) >> 2)) : -1;
+    const RowPml<T> r1 = load_row<T>(a.mhx, a.bhx, a.chx, cx, live);
+    const RowPml<T> r0 = load_row<T>(a.mhx, a.bhx, a.chx, cx - 1, top);
+    re = load_row<T>(a.mex, a.bex, a.cex, cx, live);
+    const long long qhx = tr.p_hzx + (long long)r1.m * pitch + j;
+    const long long qhy = tr.p_hzy + (long long)r * tr.nphy + 4 * gh + (cy & 3);
+    qex = tr.p_eyx + (long long)re.m * pitch + j;
+    qey = tr.p_exy + (long long)r * tr.npey + 4 * ge + (cy & 3);
+    ecol = ge >= 0;
+    ColPml<T, V> cp;
+    ColPml<T, 1> cl = {{T(0)}, {T(0)}};
+    load_cols<T>(a.bhy, a.chy, cy, gh >= 0, cp);
+    load_cols<T>(a.bey, a.cey, cy, ge >= 0, ce);
+    T x1[V], y1[V], x0[V], y0[V], xl[1] = {T(0)}, yl[1] = {T(0)};
+    tld_if<T>(a.pHzx2[L] + qhx, r1.m >= 0, x1);
+    tld_if<T>(a.pHzy2[L] + qhy, gh >= 0, y1);
+    tld_if<T>(a.pHzx2[L] + tr.p_hzx + (long long)r0.m * pitch + j, r0.m >= 0, x0);
+    tld_if<T>(a.pHzy2[L] + qhy - tr.nphy, top && gh >= 0, y0);
+    tld_if<T>(a.pEyx + qex, re.m >= 0, wx);
+    tld_if<T>(a.pExy + qey, ge >= 0, wy);
+    if (left && r1.m >= 0) xl[0] = a.pHzx2[L][qhx - 1];
+    if (gl >= 0) {
+      cl.b[0] = a.bhy[cy - 1];
+      cl.c[0] = a.chy[cy - 1];
+      yl[0] = a.pHzy2[L][tr.p_hzy + (long long)r * tr.nphy + 4 * gl + ((cy - 1) & 3)];
+    }
+    h_cols_pml<T, V>(a, j, tr.ny, top && r - 1 < tr.nx - 1, r0, cp, ey0, ey1, ex0, exr0, hz0, x0, y0,
+                     hp);
+    h_cols_pml<T, V>(a, j, tr.ny, live && r < tr.nx - 1, r1, cp, ey1, ey2, ex1, exr1, hz1, x1, y1,
+                     h);
+    h_cols_pml<T, 1>(a, j - 1, tr.ny, left && r < tr.nx - 1, r1, cl, eyl, eyln, exl, ex1[0], hzl, xl,
+                     yl, hl);
+    if (r1.m >= 0) tst(a.pHzx2[L ^ 1] + qhx, x1, V);
+    if (gh >= 0) tst(a.pHzy2[L ^ 1] + qhy, y1, V);
+  } else {
+    h_cols<T, V>(a, ey0, ey1, ex0, exr0, hz0, hp);
+    h_cols<T, V>(a, ey1, ey2, ex1, exr1, hz1, h);
+    if (left) h_cols<T, 1>(a, eyl, eyln, exl, ex1[0], hzl, hl);
+  }
+  const T hs = __shfl_up_sync(0xffffffffu, h[V - 1], 1, X);
+  const T hl0 = threadIdx.x == 0 ? hl[0] : hs;
+  if (EDGE && !live) return;
+  tst(a.Hz2[L ^ 1] + id, h, nv);
+  // ---- Ex, Ey: kb_e's arithmetic (both quotients formed; each is used only
+  // where its difference exists)
+  const T up = QScale<T>::up, down = QScale<T>::down;
+  T e[V], f[V], cx[V], cy[V], nA[V], nB[V], m = T(0);
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    const T s = mul_rn(h[v], up);
+    nA[v] = fma_rn(-(v > 0 ? h[v > 0 ? v - 1 : 0] : hl0), up, s);
+    nB[v] = fma_rn(-hp[v], up, s);
+    m = absmax(m, absmax(nA[v], nB[v]));
+  }
+  const bool fast = a.fast && m < QScale<T>::limit * up;
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    T dA, dB;
+    if (fast) {
+      dA = mul_rn(qscaled(nA[v], a.dy, a.rdy), down);
+      dB = mul_rn(qscaled(nB[v], a.dx, a.rdx), down);
+    } else {
+      dA = div_cold(sub_rn(h[v], v > 0 ? h[v > 0 ? v - 1 : 0] : hl0), a.dy);
+      dB = div_cold(sub_rn(h[v], hp[v]), a.dx);
+    }
+    e[v] = ex1[v];
+    f[v] = ey1[v];
+    cx[v] = cy[v] = T(0);
+    if (!EDGE || j + v >= 1) {
+      e[v] = add_rn(ex1[v], mul_rn(dA, K[v]));
+      cx[v] = dA;
+    }
+    if (!EDGE || r >= 1) {
+      f[v] = add_rn(ey1[v], mul_rn(-dB, K[v]));
+      cy[v] = -dB;
+    }
+    if constexpr (EDGE) {
+      if (ce.c[v] != T(0) && j + v >= 1) {
+        wy[v] = add_rn(mul_rn(ce.b[v], wy[v]), mul_rn(ce.c[v], dA));
+        e[v] = add_rn(e[v], mul_rn(K[v], wy[v]));
+        cx[v] = add_rn(dA, wy[v]);
       }
-      if (xr) ex31_n = Ex[id + 1];
+      if (re.m >= 0 && r >= 1 && v < nv) {
+        wx[v] = add_rn(mul_rn(re.b, wx[v]), mul_rn(re.c, dB));
+        f[v] = add_rn(f[v], mul_rn(-K[v], wx[v]));
+        cy[v] = sub_rn(cy[v], wx[v]);
+      }
     }
-    const long long id = c0 + r * pitch;
-    const bool body = r >= sg.i0;  // uniform: a row this segment owns
-    // Hz of row r (every lane: the halo lane and the prologue row too)
-    T exr = __shfl_down_sync(full, ex, 1);
-    if (lane == 31) exr = ex31;
-    T h = hz;
-    if (hcol && r < nx - 1) {
-      const bool st = own && body;
-      h = hz_value<T>(a, I, r, j, ny, I.ox + r, I.oy + j, a.mhx[I.ox + r], myh, hz, eyn, ey,
-                      exr, ex, pzx, st ? pzxo : nullptr, pzy, st ? pzyo : nullptr);
+  }
+  if constexpr (EDGE) {
+    if (ecol) tst(a.pExy + qey, wy, V);
+    if (re.m >= 0) tst(a.pEyx + qex, wx, V);
+  }
+  if (tr.flags & kTileWindow) {
+    const int di = (int)threadIdx.y - tr.wdi;
+    if (di >= 0 && di < tr.wdn) {
+      T* ring = a.ring + ((n % a.ring_len) * a.n_design + a.inst[tr.k].goff + (long long)di * tr.wdn) * 2;
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const int dj = (int)threadIdx.x * V + v - tr.wdj;
+        if (dj < 0 || dj >= tr.wdn) continue;
+        ring[2 * dj] = cx[v];
+        ring[2 * dj + 1] = cy[v];
+      }
     }
-    const T hl = __shfl_up_sync(full, h, 1);  // Hz^{n+1/2} of column j - 1
-    if (body && own) {
-      Hzo[id] = h;
-      // Ex, Ey of (r, j): kb_e's arithmetic (both quotients formed; each is
-      // used only where its difference exists)
-      T cx = T(0), cy = T(0);
-      T e = ex;
-      T dA, dBq;
-      qdiv2(sub_rn(h, hl), a.dy, a.rdy, a.fdy, sub_rn(h, hz_prev), a.dx, a.rdx, a.fdx, dA, dBq);
-      if (j >= 1) {
-        e = add_rn(ex, mul_rn(dA, K));
-        cx = dA;
-        if (mye >= 0) {
-          const long long q = I.p_exy + (long long)r * I.npey + mye;
-          const int c = I.oy + j;
-          const T psi = add_rn(mul_rn(a.bey[c], a.pExy[q]), mul_rn(a.cey[c], dA));
-          a.pExy[q] = psi;
-          e = add_rn(e, mul_rn(K, psi));
-          cx = add_rn(dA, psi);
+  }
+  if (tr.flags & kTilePost) {
+    const int srow = post.srow ? post.srow[tr.ox + threadIdx.y] : -1;
+    if (srow >= 0) {
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        if (v >= nv) continue;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int g = post.scol[srow + c * tr.ny + j + v];
+          if (g < 0) continue;
+          T x = c == 0 ? e[v] : f[v];
+          for (int q = post.start[g]; q < post.start[g + 1]; ++q)
+            x = add_double<T>(x, __dmul_rn(post.amp[q],
+                                           post.wave[(long long)post.wave_row[q] * post.n_steps + n]));
+          if (c == 0) e[v] = x;
+          else f[v] = x;
         }
       }
-      Exo[id] = e;
-      e = ey;
-      if (r >= 1) {
-        const T dB = dBq;
-        e = add_rn(ey, mul_rn(-dB, K));
-        cy = -dB;
-        const int mx = a.mex[I.ox + r];
-        if (mx >= 0) {
-          const long long q = I.p_eyx + (long long)mx * ny + j;
-          const int c = I.ox + r;
-          const T psi = add_rn(mul_rn(a.bex[c], a.pEyx[q]), mul_rn(a.cex[c], dB));
-          a.pEyx[q] = psi;
-          e = add_rn(e, mul_rn(-K, psi));
-          cy = sub_rn(cy, psi);
-        }
-      }
-      Eyo[id] = e;
-      const int di = r - I.di0, dj = j - I.dj0;
-      if (di >= 0 && di < I.dn && dj >= 0 && dj < I.dn) {
-        T* rr = a.ring + ((long long)slot * a.n_design + I.goff + (long long)di * I.dn + dj) * 2;
-        rr[0] = cx;
-        rr[1] = cy;
-      }
     }
-    hz_prev = h;
-    ex = ex_n;
-    hz = hz_n;
-    ey = eyn;
-    eyn = eyn_n;
-    K = K_n;
-    ex31 = ex31_n;
+    const Inst& I = a.inst[tr.k];
+    if (r == I.line_i && post.dring) {
+      T* ring = post.dring + (long long)(step_t % kDftRing) * post.nline + I.loff + j;
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        if (v < nv) ring[v] = f[v];
+    }
   }
+  tst(a.Ex2[L ^ 1] + id, e, nv);
+  tst(a.Ey2[L ^ 1] + id, f, nv);
+}
+
+// One thread per 16-byte vector of a tile row, one tile per block; level n & 1
+// is read and level (n & 1) ^ 1 written, as in kb_step, with kb_h's and kb_e's
+// arithmetic, so the same bits. Edge and bulk tiles run as two kernels side
+// by side: the edge code needs twice the registers, and mixed in one kernel
+// the two kept missing the instruction cache (a third of all stalls).
+//
+// A step is bound by how many loads are in flight. Marching down the rows
+// (one warp per 31-column strip, the form before this one) kept one row of
+// 16 bytes per lane in flight, 25 KB per SM, and reached 2.9 TB/s; two columns
+// per lane cut its instructions but also its warps and was slower (457 us).
+// Here every thread issues eight vectors at once and has no loop; the Hz it
+// recomputes costs 13 operations per cell. us per step, marching -> this: 256
+// instances (36.1M cells) forward 373 -> 321, reverse 424 -> 379, 8 instances
+// (1.5M cells) 37 -> 14 and 31 -> 14. The bulk tiles alone (about four fifths)
+// take 180 us of the 321; scalar CPML code in 32-column edge tiles cost 70 more.
+template <typename T, bool EDGE>
+__global__ void __launch_bounds__(32 * tile_x<T>(false), sizeof(T) == 4 ? (EDGE ? PFB_MINB_EDGE : PFB_MINB_TILE) : 1) kb_tile(const __grid_constant__ BArgs<T> a,
+                                                             const __grid_constant__ StepPost<T> post,
+                                                             int step_t) {
+  const TileRec tr = a.tiles[EDGE ? blockIdx.x : a.nedge + blockIdx.x];
+  tile_step<T, EDGE>(a, post, tr, *a.base + step_t, step_t);
 }
 
 // Field pointers kb_post writes through: level 0 for the in-place split
@@ -699,7 +927,7 @@ __global__ void __launch_bounds__(32 * kWarps) kb_adj_h(const __grid_constant__ 
         if (mx[r] >= 0 || my >= 0) {
           const Inst& I = a.inst[tr.k];
           if (mx[r] >= 0) {
-            const long long q = I.p_hzx + (long long)mx[r] * tr.ny + j;
+            const long long q = I.p_hzx + (long long)mx[r] * tr.pitch + j;
             const int c = tr.ox + r0 + r;
             const T ap = fma_rn(-a.ch, h, d.aHzx[q]);
             ha = fma_rn(a.chx[c], ap, ha);
@@ -799,7 +1027,7 @@ __global__ void __launch_bounds__(32 * kWarps) kb_adj_cell(const __grid_constant
         if (i + r >= 1) {
           gb = mul_rn(-K[r], y);
           if (mx[r] >= 0) {
-            const long long q = I.p_eyx + (long long)mx[r] * tr.ny + j;
+            const long long q = I.p_eyx + (long long)mx[r] * tr.pitch + j;
             const int c = tr.ox + r0 + r;
             const T ap = fma_rn(-K[r], y, d.aEyx[q]);
             gb = fma_rn(a.cex[c], ap, gb);
@@ -841,7 +1069,7 @@ __device__ __forceinline__ void adj_h_value(const BArgs<T>& a, const Inst& I, in
     ha = mul_rn(-a.ch, h);
     hb = mul_rn(a.ch, h);
     if (mx >= 0) {
-      const long long q = I.p_hzx + (long long)mx * ny + j;
+      const long long q = I.p_hzx + (long long)mx * I.pitch + j;
       const T ap = fma_rn(-a.ch, h, pzx[q]);
       ha = fma_rn(a.chx[crow], ap, ha);
       if (pzxo) pzxo[q] = mul_rn(a.bhx[crow], ap);
@@ -1008,7 +1236,7 @@ __global__ void __launch_bounds__(32 * kWarps, PFB_MINB_ASTEP) kb_adj_step(
         if (i + r >= 1) {
           gbv = mul_rn(-K[r], y);
           if (mxe[r] >= 0) {
-            const long long q = I.p_eyx + (long long)mxe[r] * tr.ny + j;
+            const long long q = I.p_eyx + (long long)mxe[r] * tr.pitch + j;
             const int c = tr.ox + r0 + r;
             const T ap = fma_rn(-K[r], y, d.aEyx[q]);
             gbv = fma_rn(a.cex[c], ap, gbv);
@@ -1025,161 +1253,215 @@ __global__ void __launch_bounds__(32 * kWarps, PFB_MINB_ASTEP) kb_adj_step(
   }
 }
 
-// ---- marching reverse step ---------------------------------------------------
-// kb_adj_step's work on kb_march's segments: one warp marches down its rows;
-// gA of the column to the right comes from the lane above (lane 31 loads
-// it), gB of the next row is loaded one row ahead, hA of the row above stays
-// in a register, and hB of the column to the left comes from the lane below
-// (lane 0 recomputes the halo column's H transpose without storing it). A
-// segment that starts below row 0 first recomputes hA of row i0 - 1. Same
-// levels and arithmetic as kb_adj_step, so the same bits.
-template <typename T, bool HT, bool ET>
-__global__ void __launch_bounds__(32 * kMarchWarps, PFB_MINB_AMARCH) kb_adj_march(
-    const __grid_constant__ BArgs<T> a, const __grid_constant__ AArgs<T> d, int step_t) {
-  const int w = blockIdx.x * kMarchWarps + threadIdx.y;
-  if (w >= a.nsegs) return;  // uniform over the warp
-  const SegRec sg = a.segs[w];
-  const Inst& I = a.inst[sg.k];
-  const long long n = *a.base + step_t;
-  const long long m = HT ? n - 1 : n;  // the step of the E transpose
-  const int lg = (int)(n & 1);
-  const int lh = (int)((n + 1) & 1);
-  const T* gA = d.gA2[lg];
-  const T* gB = d.gB2[lg];
-  T* gAo = d.gA2[(int)(m & 1)];
-  T* gBo = d.gB2[(int)(m & 1)];
-  const T* aHz = d.aHz2[lh];
-  T* aHzo = d.aHz2[lh ^ 1];
-  const T* pzx = d.aHzx2[lh];
-  const T* pzy = d.aHzy2[lh];
-  T* pzxo = d.aHzx2[lh ^ 1];
-  T* pzyo = d.aHzy2[lh ^ 1];
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x;
-  const int nx = I.nx, ny = I.ny;
-  const long long pitch = I.pitch;
-  const int j = sg.j0 - 1 + lane;
-  const bool jv = j >= 0 && j < ny;
-  const bool own = lane >= 1 && jv;
-  const bool xr = HT && lane == 31 && j + 1 < ny;
-  const long long c0 = I.off + j;
-  const int myh = (HT && jv) ? a.mhy[I.oy + j] : -1;
-  const int mye = (ET && jv) ? a.mey[I.oy + j] : -1;
-  const int r_first = (HT && sg.i0 > 0) ? sg.i0 - 1 : sg.i0;
-  // row r_first
-  T ah = T(0), ga = T(0), ga31 = T(0), gb = T(0), gbn = T(0), lx = T(0), ly = T(0), K = T(0);
-  {
-    const long long id = c0 + r_first * pitch;
-    if (jv) {
-      if (HT) {
-        ah = aHz[id];
-        ga = gA[id];
-        gb = gB[id];
-        if (r_first + 1 < nx) gbn = gB[id + pitch];
+// ---- vector reverse step -------------------------------------------------------
+// H transpose of NV columns (adj_h_value's arithmetic). EDGE: row / col say
+// whether the forward update exists, vx / vy are the psi adjoints before and
+// after.
+template <typename T, int NV, bool EDGE>
+__device__ __forceinline__ void adj_h_cols(const BArgs<T>& a, int j, int ny, bool row,
+                                           const RowPml<T>& rp, const ColPml<T, NV>& cp,
+                                           const T (&ah)[NV], const T (&ga)[NV], T gar,
+                                           const T (&gb)[NV], const T (&gbn)[NV], T (&vx)[NV],
+                                           T (&vy)[NV], T (&h)[NV], T (&ha)[NV], T (&hb)[NV]) {
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const T gr = v + 1 < NV ? ga[v + 1 < NV ? v + 1 : 0] : gar;
+    h[v] = fma_rn(sub_rn(gb[v], gbn[v]), a.idx, fma_rn(sub_rn(ga[v], gr), a.idy, ah[v]));
+    ha[v] = hb[v] = T(0);
+    if (EDGE && (!row || j + v >= ny - 1)) continue;
+    ha[v] = mul_rn(-a.ch, h[v]);
+    hb[v] = mul_rn(a.ch, h[v]);
+    if constexpr (EDGE) {
+      if (rp.m >= 0) {
+        const T ap = fma_rn(-a.ch, h[v], vx[v]);
+        ha[v] = fma_rn(rp.c, ap, ha[v]);
+        vx[v] = mul_rn(rp.b, ap);
       }
-      if (r_first >= sg.i0) {
-        lx = d.aEx[id];
-        ly = d.aEy[id];
-        if (ET) K = a.ce[id];
+      if (cp.c[v] != T(0)) {
+        const T ap = fma_rn(a.ch, h[v], vy[v]);
+        hb[v] = fma_rn(cp.c[v], ap, hb[v]);
+        vy[v] = mul_rn(cp.b[v], ap);
       }
     }
-    if (xr) ga31 = gA[id + 1];
   }
-  T ha_prev = T(0);  // hA of the row above
-  for (int r = r_first; r < sg.i1; ++r) {
-    const int r1 = r + 1;
-    T ah_n = T(0), ga_n = T(0), ga31_n = T(0), gbn_n = T(0), lx_n = T(0), ly_n = T(0), K_n = T(0);
-    if (r1 < sg.i1) {
-      const long long id = c0 + r1 * pitch;
-      if (jv) {
-        if (HT) {
-          ah_n = aHz[id];
-          ga_n = gA[id];
-          if (r1 + 1 < nx) gbn_n = gB[id + pitch];
-        }
-        lx_n = d.aEx[id];
-        ly_n = d.aEy[id];
-        if (ET) K_n = a.ce[id];
-      }
-      if (xr) ga31_n = gA[id + 1];
+}
+
+// The reverse step of one thread's V columns of row r: the H transpose of
+// step n (its own cells, the row above for hA, the column to the left for
+// hB), then step n's E adjoints and the E transpose of step m = n - 1 (or of
+// step n alone when HT is false), as kb_adj_step.
+template <typename T, bool HT, bool ET, bool EDGE>
+__device__ __forceinline__ void adj_tile_step(const BArgs<T>& a, const AArgs<T>& d,
+                                              const TileRec& tr, long long n) {
+  constexpr int V = kTileV<T>, X = tile_x<T>(EDGE);
+  const long long m = HT ? n - 1 : n;  // the step of the E transpose
+  const int lg = (int)(n & 1), lh = (int)((n + 1) & 1), lm = (int)(m & 1);
+  const int r = tr.i0 + threadIdx.y, j = tr.j0 + threadIdx.x * V;
+  const bool live = !EDGE || (r < tr.nx_end && j < tr.ny);
+  const int nv = EDGE ? (live ? min(V, tr.ny - j) : 0) : V;
+  const int pitch = tr.pitch;
+  const long long id = tr.base + (long long)threadIdx.y * pitch + threadIdx.x * V;
+  T x[V], y[V], K[V];
+  tld_if<T>(d.aEx + id, live, x);
+  tld_if<T>(d.aEy + id, live, y);
+  if (ET) tld_if<T>(a.ce + id, live, K);
+  ColPml<T, V> ce;
+  RowPml<T> re;
+  T wx[V], wy[V];  // E psi adjoints
+  long long qex = 0, qey = 0;
+  bool ecol = false;
+  const int cy = tr.oy + (j - tr.j0), cx = tr.ox + (r - tr.i0);
+  if constexpr (EDGE && ET) {
+    const int ge = live ? __ldg(a.gey + (cy >> 2)) : -1;
+    re = load_row<T>(a.mex, a.bex, a.cex, cx, live);
+    ecol = ge >= 0;
+    qex = tr.p_eyx + (long long)re.m * pitch + j;
+    qey = tr.p_exy + (long long)r * tr.npey + 4 * ge + (cy & 3);
+    load_cols<T>(a.bey, a.cey, cy, ecol, ce);
+    tld_if<T>(d.aEyx + qex, re.m >= 0, wx);
+    tld_if<T>(d.aExy + qey, ecol, wy);
+  }
+  if (HT) {
+    const T* gA = d.gA2[lg] + id;
+    const T* gB = d.gB2[lg] + id;
+    const T* aH = d.aHz2[lh] + id;
+    const bool top = !EDGE || (live && r >= 1);
+    const bool low = !EDGE || (live && r + 1 < tr.nx);
+    const bool right = !EDGE || (live && j + V < tr.ny);
+    const bool left = threadIdx.x == 0 && (!EDGE || (live && j >= 1));
+    T ah0[V], ah1[V], ga0[V], ga1[V], gb0[V], gb1[V], gb2[V];
+    tld_if<T>(aH - pitch, top, ah0);
+    tld_if<T>(aH, live, ah1);
+    tld_if<T>(gA - pitch, top, ga0);
+    tld_if<T>(gA, live, ga1);
+    tld_if<T>(gB - pitch, top, gb0);
+    tld_if<T>(gB, live, gb1);
+    tld_if<T>(gB + pitch, low, gb2);
+    const T gar0 = top && right ? gA[V - pitch] : T(0), gar1 = right ? gA[V] : T(0);
+    T ahl[1] = {T(0)}, gal[1] = {T(0)}, gbl[1] = {T(0)}, gbln[1] = {T(0)};
+    if (left) {
+      ahl[0] = aH[-1];
+      gal[0] = gA[-1];
+      gbl[0] = gB[-1];
+      if (low) gbln[0] = gB[pitch - 1];
     }
-    const long long id = c0 + r * pitch;
-    const bool body = r >= sg.i0;  // uniform
-    T ha = T(0), hb = T(0);
-    if (HT) {
-      T ga1 = __shfl_down_sync(full, ga, 1);
-      if (lane == 31) ga1 = ga31;
-      T h = T(0);
-      if (jv) {
-        const bool st = own && body;
-        adj_h_value<T>(a, I, r, j, nx, ny, I.ox + r, I.oy + j, a.mhx[I.ox + r], myh, ah, ga,
-                       ga1, gb, gbn, pzx, st ? pzxo : nullptr, pzy, st ? pzyo : nullptr, h, ha,
-                       hb);
-        if (st) aHzo[id] = h;
+    T h[V], ha[V], hb[V], hap[V], t0[V], t1[V], hl[1], hal[1], hbl[1] = {T(0)};
+    ColPml<T, V> cp;
+    ColPml<T, 1> cl = {{T(0)}, {T(0)}};
+    RowPml<T> r0, r1;
+    T x1[V], y1[V], x0[V], y0[V], xl[1] = {T(0)}, yl[1] = {T(0)};
+    long long qhx = 0, qhy = 0;
+    int gh = -1;
+    if constexpr (EDGE) {
+      gh = live ? __ldg(a.ghy + (cy >> 2)) : -1;
+      const int gl = left ? __ldg(a.ghy + ((cy - 1) >> 2)) : -1;
+      r1 = load_row<T>(a.mhx, a.bhx, a.chx, cx, live);
+      r0 = load_row<T>(a.mhx, a.bhx, a.chx, cx - 1, top);
+      qhx = tr.p_hzx + (long long)r1.m * pitch + j;
+      qhy = tr.p_hzy + (long long)r * tr.nphy + 4 * gh + (cy & 3);
+      load_cols<T>(a.bhy, a.chy, cy, gh >= 0, cp);
+      tld_if<T>(d.aHzx2[lh] + qhx, r1.m >= 0, x1);
+      tld_if<T>(d.aHzy2[lh] + qhy, gh >= 0, y1);
+      tld_if<T>(d.aHzx2[lh] + tr.p_hzx + (long long)r0.m * pitch + j, r0.m >= 0, x0);
+      tld_if<T>(d.aHzy2[lh] + qhy - tr.nphy, top && gh >= 0, y0);
+      if (left && r1.m >= 0) xl[0] = d.aHzx2[lh][qhx - 1];
+      if (gl >= 0) {
+        cl.b[0] = a.bhy[cy - 1];
+        cl.c[0] = a.chy[cy - 1];
+        yl[0] = d.aHzy2[lh][tr.p_hzy + (long long)r * tr.nphy + 4 * gl + ((cy - 1) & 3)];
       }
     }
-    const T hbl = HT ? __shfl_up_sync(full, hb, 1) : T(0);  // hB of column j - 1
-    if (body && own) {
-      T x = lx, y = ly;
-      if (HT) {
-        y = fma_rn(sub_rn(ha_prev, ha), a.idx, y);
-        x = fma_rn(sub_rn(hbl, hb), a.idy, x);
-      }
-      if (ET) {
-        if (r == I.line_i) {
-          const double* ph = d.phase + m * d.n_freq * 2;
-          const double* g = d.cot + (I.loff + j) * d.n_freq * 2;
+    adj_h_cols<T, V, EDGE>(a, j, tr.ny, top && r - 1 < tr.nx - 1, r0, cp, ah0, ga0, gar0, gb0, gb1,
+                           x0, y0, t0, hap, t1);
+    adj_h_cols<T, V, EDGE>(a, j, tr.ny, live && r < tr.nx - 1, r1, cp, ah1, ga1, gar1, gb1, gb2, x1,
+                           y1, h, ha, hb);
+    if (left)
+      adj_h_cols<T, 1, EDGE>(a, j - 1, tr.ny, r < tr.nx - 1, r1, cl, ahl, gal, ga1[0], gbl, gbln,
+                             xl, yl, hl, hal, hbl);
+    if constexpr (EDGE) {
+      if (r1.m >= 0) tst(d.aHzx2[lh ^ 1] + qhx, x1, V);
+      if (gh >= 0) tst(d.aHzy2[lh ^ 1] + qhy, y1, V);
+    }
+    const T hs = __shfl_up_sync(0xffffffffu, hb[V - 1], 1, X);
+    const T hb0 = threadIdx.x == 0 ? hbl[0] : hs;
+    if (EDGE && !live) return;
+    tst(d.aHz2[lh ^ 1] + id, h, nv);
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      y[v] = fma_rn(sub_rn(hap[v], ha[v]), a.idx, y[v]);
+      x[v] = fma_rn(sub_rn(v > 0 ? hb[v > 0 ? v - 1 : 0] : hb0, hb[v]), a.idy, x[v]);
+    }
+  } else if (EDGE && !live) {
+    return;
+  }
+  if (ET) {
+    if (tr.flags & kTilePost) {
+      const Inst& I = a.inst[tr.k];
+      if (r == I.line_i) {
+        const double* ph = d.phase + m * d.n_freq * 2;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          if (v >= nv) continue;
+          const double* g = d.cot + (I.loff + j + v) * d.n_freq * 2;
           double sum = 0.0;
           for (int f = 0; f < d.n_freq; ++f)
             sum = __dadd_rn(sum, __dadd_rn(__dmul_rn(g[2 * f], ph[2 * f]),
                                            __dmul_rn(g[2 * f + 1], ph[2 * f + 1])));
-          y = (T)__dadd_rn((double)y, __dmul_rn(d.dt, sum));
+          y[v] = (T)__dadd_rn((double)y[v], __dmul_rn(d.dt, sum));
         }
-        const int di = r - I.di0, dj = j - I.dj0;
-        if (di >= 0 && di < I.dn && dj >= 0 && dj < I.dn) {
-          const long long dc = I.goff + (long long)di * I.dn + dj;
-          const T* rr = a.ring + ((m % a.ring_len) * a.n_design + dc) * 2;
-          d.grad[dc] = __dadd_rn(d.grad[dc], __dadd_rn(__dmul_rn((double)x, (double)rr[0]),
-                                                       __dmul_rn((double)y, (double)rr[1])));
-        }
-        T gav = T(0), gbv = T(0);
-        if (j >= 1) {
-          gav = mul_rn(K, x);
-          if (mye >= 0) {
-            const long long q = I.p_exy + (long long)r * I.npey + mye;
-            const int c = I.oy + j;
-            const T ap = fma_rn(K, x, d.aExy[q]);
-            gav = fma_rn(a.cey[c], ap, gav);
-            d.aExy[q] = mul_rn(a.bey[c], ap);
-          }
-        }
-        if (r >= 1) {
-          gbv = mul_rn(-K, y);
-          const int mx = a.mex[I.ox + r];
-          if (mx >= 0) {
-            const long long q = I.p_eyx + (long long)mx * ny + j;
-            const int c = I.ox + r;
-            const T ap = fma_rn(-K, y, d.aEyx[q]);
-            gbv = fma_rn(a.cex[c], ap, gbv);
-            d.aEyx[q] = mul_rn(a.bex[c], ap);
-          }
-        }
-        gAo[id] = gav;
-        gBo[id] = gbv;
       }
-      d.aEx[id] = x;
-      d.aEy[id] = y;
     }
-    ha_prev = ha;
-    ah = ah_n;
-    ga = ga_n;
-    ga31 = ga31_n;
-    gb = gbn;
-    gbn = gbn_n;
-    lx = lx_n;
-    ly = ly_n;
-    K = K_n;
+    if (tr.flags & kTileWindow) {
+      const int di = (int)threadIdx.y - tr.wdi;
+      if (di >= 0 && di < tr.wdn) {
+        const long long row = a.inst[tr.k].goff + (long long)di * tr.wdn;
+        const T* ring = a.ring + ((m % a.ring_len) * a.n_design + row) * 2;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const int dj = (int)threadIdx.x * V + v - tr.wdj;
+          if (dj < 0 || dj >= tr.wdn) continue;
+          d.grad[row + dj] =
+              __dadd_rn(d.grad[row + dj], __dadd_rn(__dmul_rn((double)x[v], (double)ring[2 * dj]),
+                                                    __dmul_rn((double)y[v], (double)ring[2 * dj + 1])));
+        }
+      }
+    }
+    T gav[V], gbv[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      gav[v] = !EDGE || j + v >= 1 ? mul_rn(K[v], x[v]) : T(0);
+      gbv[v] = !EDGE || r >= 1 ? mul_rn(-K[v], y[v]) : T(0);
+      if constexpr (EDGE && ET) {
+        if (ce.c[v] != T(0) && j + v >= 1) {
+          const T ap = fma_rn(K[v], x[v], wy[v]);
+          gav[v] = fma_rn(ce.c[v], ap, gav[v]);
+          wy[v] = mul_rn(ce.b[v], ap);
+        }
+        if (re.m >= 0 && r >= 1 && v < nv) {
+          const T ap = fma_rn(-K[v], y[v], wx[v]);
+          gbv[v] = fma_rn(re.c, ap, gbv[v]);
+          wx[v] = mul_rn(re.b, ap);
+        }
+      }
+    }
+    if constexpr (EDGE && ET) {
+      if (ecol) tst(d.aExy + qey, wy, V);
+      if (re.m >= 0) tst(d.aEyx + qex, wx, V);
+    }
+    tst(d.gA2[lm] + id, gav, nv);
+    tst(d.gB2[lm] + id, gbv, nv);
   }
+  tst(d.aEx + id, x, nv);
+  tst(d.aEy + id, y, nv);
+}
+
+// kb_adj_step's work in the shape of kb_tile; same levels and arithmetic, so
+// the same bits.
+template <typename T, bool HT, bool ET, bool EDGE>
+__global__ void __launch_bounds__(32 * tile_x<T>(false), sizeof(T) == 4 ? (EDGE ? PFB_MINB_AEDGE : PFB_MINB_ATILE) : 1) kb_adj_tile(
+    const __grid_constant__ BArgs<T> a, const __grid_constant__ AArgs<T> d, int step_t) {
+  const TileRec tr = a.tiles[EDGE ? blockIdx.x : a.nedge + blockIdx.x];
+  adj_tile_step<T, HT, ET, EDGE>(a, d, tr, *a.base + step_t);
 }
 
 }  // namespace b2d

@@ -73,6 +73,10 @@ __device__ __forceinline__ double absmax(double a, double b) { return fmax(fabs(
 // Whether every numerator of a cell may take qdiv_fast.
 template <typename T>
 __device__ __forceinline__ bool qdiv_ok(T m) { return m < QScale<T>::limit; }
+// IEEE division, out of line: the rare numerators beyond the reciprocal
+// path's range would otherwise put a division routine at every quotient.
+static __device__ __noinline__ float div_cold(float a, float d) { return __fdiv_rn(a, d); }
+static __device__ __noinline__ double div_cold(double a, double d) { return __ddiv_rn(a, d); }
 template <typename T>
 __device__ __forceinline__ T qdiv(T a, T d, T r, bool fast) {
   if (fast && qdiv_ok(absmax(a, a))) return qdiv_fast(a, d, r);
