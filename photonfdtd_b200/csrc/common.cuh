@@ -177,6 +177,8 @@ struct StepArgs {
   const T* cph[3];
   const int* mape[3];
   const int* maph[3];
+  const int* gze;  // vector passes: z-layer group of each vector of a row, or -1
+  const int* gzh;
   int npe[3], nph[3];
   // Bulk boxes: cells [b0, b1) per axis where the H (hb) or E (eb) update has
   // both difference terms and no CPML state; they take the straight-line path.

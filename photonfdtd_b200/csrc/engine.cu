@@ -132,6 +132,11 @@ struct pf_engine {
   int* map_e[3] = {};
   int* map_h[3] = {};
   int npe[3] = {}, nph[3] = {};
+  int* gze = nullptr;     // vector passes: z-layer group per vector of a row
+  int* gzh = nullptr;
+  int ncz_e = 0, ncz_h = 0;  // z cells with CPML state, and their places in a psi row
+  int* zpos_e = nullptr;
+  int* zpos_h = nullptr;
   int hb0[3] = {}, hb1[3] = {}, eb0[3] = {}, eb1[3] = {};
   void* psiE[6] = {};
   void* psiH[2][6] = {};
@@ -459,15 +464,50 @@ int finalize_typed(pf_engine* e) {
     const int na = dims[ax];
     std::vector<T> arr[4];
     for (int q = 0; q < 4; ++q) {
-      arr[q].assign(na, T(0));
+      arr[q].assign(ax == 2 ? e->pz : na, T(0));  // z: vectors past the row's end read zeros
       if (!e->h_cpml[ax][q].empty()) memcpy(arr[q].data(), e->h_cpml[ax][q].data(), na * S);
-      if ((rc = upload(e, &e->cp[ax][q], arr[q].data(), na * S))) return rc;
+      if ((rc = upload(e, &e->cp[ax][q], arr[q].data(), arr[q].size() * S))) return rc;
     }
     std::vector<int> me(na, -1), mh(na, -1);
     int ce_n = 0, ch_n = 0;
-    for (int t = 0; t < na; ++t) {
-      if (arr[1][t] != T(0)) me[t] = ce_n++;
-      if (arr[3][t] != T(0)) mh[t] = ch_n++;
+    if (e->vec && ax == 2) {
+      // the vector passes keep the z layers' psi in whole groups of V entries
+      const int V = 16 / (int)S;
+      auto groups = [&](const std::vector<T>& c, std::vector<int>& map, std::vector<int>& pos,
+                        int** gdev, int** pdev) {
+        std::vector<int> g;
+        int n = 0;
+        for (int t = 0; t < na; t += V) {
+          bool any = false;
+          for (int u = t; u < std::min(na, t + V); ++u)
+            if (c[u] != T(0)) {
+              any = true;
+              map[u] = n + (u - t);
+              pos.push_back(map[u]);
+            }
+          g.push_back(any ? n / V : -1);
+          if (any) n += V;
+        }
+        int r = upload(e, (void**)gdev, g.data(), g.size() * 4);
+        if (!r) r = upload(e, (void**)pdev, pos.data(), pos.size() * 4);
+        if (!r && cudaStreamSynchronize(e->stream) != cudaSuccess) r = PF_ERR_CUDA;
+        return r ? -1 : n;
+      };
+      std::vector<int> pe, ph;
+      ce_n = groups(arr[1], me, pe, &e->gze, &e->zpos_e);
+      ch_n = groups(arr[3], mh, ph, &e->gzh, &e->zpos_h);
+      if (ce_n < 0 || ch_n < 0) return fail(e, PF_ERR_CUDA, "uploading the z-layer groups failed");
+      e->ncz_e = (int)pe.size();
+      e->ncz_h = (int)ph.size();
+    } else {
+      for (int t = 0; t < na; ++t) {
+        if (arr[1][t] != T(0)) me[t] = ce_n++;
+        if (arr[3][t] != T(0)) mh[t] = ch_n++;
+      }
+      if (ax == 2) {
+        e->ncz_e = ce_n;
+        e->ncz_h = ch_n;
+      }
     }
     e->npe[ax] = ce_n;
     e->nph[ax] = ch_n;
@@ -626,6 +666,8 @@ StepArgs<T> step_args(pf_engine* e) {
     a.cph[ax] = (const T*)e->cp[ax][3];
     a.mape[ax] = e->map_e[ax];
     a.maph[ax] = e->map_h[ax];
+    a.gze = e->gze;
+    a.gzh = e->gzh;
     a.npe[ax] = e->npe[ax];
     a.nph[ax] = e->nph[ax];
   }
@@ -662,9 +704,8 @@ int scan_finite(pf_engine* e) {
 
 // Vectors along z per block of the vector passes: 8 (128 bytes of a row) or,
 // where that wastes more of the last block, 4; fewer on short rows. 256^3
-// without CPML: 243 us at 8, 255 at 4; at 32 a warp that touches a layer at
-// the end of a row drags 128 cells along the general path (with CPML 314 us
-// at 8, 461 at 32).
+// plain: 287 us at 8, 288 at 16, 330 at 32 (a warp that touches a layer at
+// the end of a row takes 128 cells along); 301x287x263 406 at 8, 449 at 16.
 int vec_lanes(int nzv) {
   if (nzv <= 2) return nzv;
   if (nzv <= 4) return 4;
@@ -1643,17 +1684,22 @@ namespace {
 struct StatePiece {
   char* p;
   size_t rows, bytes;  // bytes in the blob
+  const int* zpos = nullptr;  // z layers kept in groups: places of the nc entries of a psi row
+  int np = 0, nc = 0;
 };
 std::vector<StatePiece> state_pieces(pf_engine* e, long long step) {
   std::vector<StatePiece> v;
   const size_t S = e->rb, rows = (size_t)e->nx * e->ny, w = (size_t)e->nz * S;
-  auto psi = [&](void* p, long long r, long long n) {
-    v.push_back({(char*)p, (size_t)r, r ? (size_t)r * w : (size_t)n * S});
+  auto psi = [&](void* p, int q, long long r, long long n, const int* zpos, int np, int nc) {
+    if ((q == 1 || q == 2) && np != nc)
+      v.push_back({(char*)p, 0, rows * nc * S, zpos, np, nc});
+    else
+      v.push_back({(char*)p, (size_t)r, r ? (size_t)r * w : (size_t)n * S});
   };
   for (int c = 0; c < 3; ++c) v.push_back({(char*)e->E[e->cur][c], rows, rows * w});
   for (int c = 0; c < 3; ++c) v.push_back({(char*)e->H[e->cur][c], rows, rows * w});
-  for (int q = 0; q < 6; ++q) psi(e->psiE[q], e->rpsiE[q], e->npsiE[q]);
-  for (int q = 0; q < 6; ++q) psi(e->psiH[e->cur][q], e->rpsiH[q], e->npsiH[q]);
+  for (int q = 0; q < 6; ++q) psi(e->psiE[q], q, e->rpsiE[q], e->npsiE[q], e->zpos_e, e->npe[2], e->ncz_e);
+  for (int q = 0; q < 6; ++q) psi(e->psiH[e->cur][q], q, e->rpsiH[q], e->npsiH[q], e->zpos_h, e->nph[2], e->ncz_h);
   if (e->n_media > 0) {
     const size_t lev = (size_t)e->plev * S;
     const int ln = (int)(step & 1);
@@ -1682,6 +1728,25 @@ int copy_state(pf_engine* e, long long step, void* buf, int64_t bytes, int on_de
     if (p.rows) {
       int rc = copy_rows(e, p.p, b, p.rows, e->rb, kind, !get);
       if (rc) return rc;
+    } else if (p.zpos && p.bytes) {
+      // psi rows in groups <-> compact rows
+      const long long n = (long long)e->nx * e->ny * p.nc;
+      void* dense = b;
+      if (!on_device) {
+        int rc = stage(e, p.bytes);
+        if (rc) return rc;
+        dense = e->region;
+        if (!get) PF_CUDA(e, cudaMemcpyAsync(dense, b, p.bytes, kind, e->stream));
+      }
+      const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 148LL * 16);
+      if (e->rb == 4)
+        k_pack_rows<float><<<blocks, 256, 0, e->stream>>>((float*)p.p, (float*)dense, p.zpos, n,
+                                                          p.np, p.nc, get);
+      else
+        k_pack_rows<double><<<blocks, 256, 0, e->stream>>>((double*)p.p, (double*)dense, p.zpos, n,
+                                                           p.np, p.nc, get);
+      PF_CUDA(e, cudaGetLastError());
+      if (!on_device && get) PF_CUDA(e, cudaMemcpyAsync(b, dense, p.bytes, kind, e->stream));
     } else if (p.bytes) {
       PF_CUDA(e, cudaMemcpyAsync(get ? b : p.p, get ? p.p : b, p.bytes, kind, e->stream));
     }

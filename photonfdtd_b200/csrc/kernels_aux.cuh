@@ -229,6 +229,19 @@ __global__ void k_gather_region(const T* f, int ny, int pz, int3 start, int3 str
   }
 }
 
+// Rows of np entries <-> compact rows of their entries pos[0 .. nc).
+template <typename T>
+__global__ void k_pack_rows(T* rows, T* compact, const int* pos, long long n, int np, int nc,
+                            bool get) {
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
+       t += (long long)gridDim.x * blockDim.x) {
+    const long long r = t / nc;
+    T* at = rows + r * np + pos[(int)(t - r * nc)];
+    if (get) compact[t] = *at;
+    else *at = compact[t];
+  }
+}
+
 // Non-finite scan over a field: sets *flag when any value is inf or nan.
 template <typename T>
 __global__ void k_nonfinite(const T* f, long long n, int* flag) {

@@ -9,8 +9,8 @@
 // (StepArgs::pz), so every row's vectors are aligned. At 256^3 without CPML
 // the H pass now runs 88 instructions per cell at 5.5 TB/s of DRAM traffic
 // (84% of a plain copy), the E pass with ADE 181 at 5.05 TB/s. Step kernels
-// before and after, in us: 384^3 with ADE 1453, 1354; 301x287x263 with three
-// coefficients 517, 473; 160x152x144 double 165, 145.
+// of the scalar passes and now, in us: 384^3 with ADE 1453, 1278; 301x287x263
+// with three coefficients 517, 409; 160x152x144 double 165, 145.
 //
 // A warp covers a patch of rows (blockDim.x vectors along z); when every cell
 // of it lies in the bulk box (both differences, no CPML state) the warp takes
@@ -19,11 +19,12 @@
 
 #include "cell_update.cuh"
 
-// Minimum resident 128-thread blocks per SM the passes are compiled for
-// (float H, float E, float E with ADE, double H, double E). Measured step
-// kernels in us at 4/4/3/4/3, 5/5/4/5/4, 6/6/4/8/6 and 8/6/5/6/5: 384^3 with
-// ADE 1526, 1354, 1375, 1457; 301x287x263 tensor 507, 473, 504, 505;
-// 160x152x144 double 155, 152, 153, 145.
+// Minimum resident 128-thread blocks per SM the passes are compiled for:
+// float H, float E, float E with ADE or three coefficients, double H, double
+// E. Step kernels in us at 5/5/4, 4/4/4 and 5/4/3: 256^3 plain 287, 311, 301;
+// 384^3 with ADE 1278, 1309, 1370; 301x287x263 with three coefficients (at
+// 5, 4, 4 blocks) 441, 424, 409. Double 6/5 145 us, 4/3 155, 8/6 153
+// (160x152x144).
 #ifndef PFB_MINB_HV
 #define PFB_MINB_HV 5
 #endif
@@ -89,19 +90,6 @@ __device__ __forceinline__ constexpr int term_axis(int t) {
   return t == 0 || t == 5 ? 1 : (t == 1 || t == 2 ? 2 : 0);
 }
 
-// The six exact quotients of one cell, IEEE division where a numerator is
-// out of the reciprocal path's range.
-template <typename T, int SGN>
-__device__ __forceinline__ void quotients_ieee(const StepArgs<T>& a, const T own[3], const T nb[6],
-                                               T d[6]) {
-  const T dl[3] = {a.dx, a.dy, a.dz};
-#pragma unroll
-  for (int t = 0; t < 6; ++t) {
-    const T o = own[term_comp(t)];
-    d[t] = div_rn(SGN > 0 ? sub_rn(nb[t], o) : sub_rn(o, nb[t]), dl[term_axis(t)]);
-  }
-}
-
 // out[c] = f[c] + K[c] (d_A - d_B) for V bulk cells. SGN 1: forward
 // differences d = (nb - own) / dl (H), -1: backward d = (own - nb) / dl (E).
 // Own values are prescaled once; a prescaled difference is then one FMA, and
@@ -137,12 +125,12 @@ __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][
   if (!(a.fdall && m < QScale<T>::limit * up)) {
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-      T o[3], n[6], d[6];
+      T d[6];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) o[c] = own[c][q];
-#pragma unroll
-      for (int t = 0; t < 6; ++t) n[t] = nb[t][q];
-      quotients_ieee<T, SGN>(a, o, n, d);
+      for (int t = 0; t < 6; ++t) {
+        const T o = own[term_comp(t)][q];
+        d[t] = div_cold(SGN > 0 ? sub_rn(nb[t][q], o) : sub_rn(o, nb[t][q]), dl[term_axis(t)]);
+      }
 #pragma unroll
       for (int c = 0; c < 3; ++c) out[c][q] = bulk(f[c][q], K[c % NC][q], d[2 * c], d[2 * c + 1]);
     }
@@ -152,7 +140,8 @@ __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][
 // CPML tables of one field family as curl_general reads them.
 template <typename T>
 struct Cpml {
-  const int* map[3];
+  const int* map[2];  // x, y
+  const int* gz;      // per vector of a row: its group of V z-layer entries, or -1
   const int* np;
   const T* b[3];
   const T* c[3];
@@ -169,8 +158,12 @@ __device__ __forceinline__ T cpml_term(T f, T k, T d, T b, T c, T& psi) {
 
 // The curl update of V cells anywhere in a 3D grid: components outside the
 // reference's loop extents keep their value (and row padding stays zero),
-// psi state is touched only where the compact map of its axis is >= 0. The x
-// and y layers' psi rows have the fields' pitch, so they are vectors too.
+// psi state is touched only in the layers. psi rows of the x and y layers have
+// the fields' pitch, those of the z layers whole groups of V entries, so all
+// of it is loaded as vectors, and all before the first use: cell by cell,
+// each psi load waited behind the stores of the cell before it (256^3 with a
+// 12-cell layer on every face: the layers cost 70 us of 314, now 41 of 287; 29
+// of these are their bytes).
 template <typename T, int SGN, int NC>
 __device__ __forceinline__ void curl_general(const StepArgs<T>& a, const Cpml<T>& p, int i, int j,
                                              int k, const T (&f)[3][kVec<T>],
@@ -180,76 +173,63 @@ __device__ __forceinline__ void curl_general(const StepArgs<T>& a, const Cpml<T>
   constexpr int V = kVec<T>;
   const bool okx = SGN > 0 ? i < a.nx - 1 : i >= 1;
   const bool oky = SGN > 0 ? j < a.ny - 1 : j >= 1;
-  const int mx = p.map[0][i], my = p.map[1][j];
-  T y0[V], y5[V], x3[V], x4[V];
-  T by = T(0), cy = T(0), bx = T(0), cx = T(0);
+  const int mx = p.map[0][i], my = p.map[1][j], gz = p.gz[k / V];
+  const T by = p.b[1][j], cy = p.c[1][j], bx = p.b[0][i], cx = p.c[0][i];
   const long long qy = ((long long)i * p.np[1] + my) * a.pz + k;
   const long long qx = ((long long)mx * a.ny + j) * a.pz + k;
-  if (my >= 0) {
-    by = p.b[1][j];
-    cy = p.c[1][j];
-    vld(p.in[0] + qy, y0);
-    vld(p.in[5] + qy, y5);
-  }
-  if (mx >= 0) {
-    bx = p.b[0][i];
-    cx = p.c[0][i];
-    vld(p.in[3] + qx, x3);
-    vld(p.in[4] + qx, x4);
-  }
+  const long long qz = ((long long)i * a.ny + j) * p.np[2] + (long long)gz * V;
+  T y0[V], y5[V], x3[V], x4[V], z1[V], z2[V], bz[V], cz[V];
+  vld_if(p.in[0] + qy, my >= 0, y0);
+  vld_if(p.in[5] + qy, my >= 0, y5);
+  vld_if(p.in[3] + qx, mx >= 0, x3);
+  vld_if(p.in[4] + qx, mx >= 0, x4);
+  vld_if(p.in[1] + qz, gz >= 0, z1);
+  vld_if(p.in[2] + qz, gz >= 0, z2);
+  vld_if(p.b[2] + k, gz >= 0, bz);
+  vld_if(p.c[2] + k, gz >= 0, cz);
   const T dl[3] = {a.dx, a.dy, a.dz};
   const T rl[3] = {a.rdx, a.rdy, a.rdz};
+  T d[6][V], m = T(0);
+#pragma unroll
+  for (int q = 0; q < V; ++q)
+#pragma unroll
+    for (int t = 0; t < 6; ++t) {
+      const T o = own[term_comp(t)][q];
+      d[t][q] = SGN > 0 ? sub_rn(nb[t][q], o) : sub_rn(o, nb[t][q]);
+      m = absmax(m, d[t][q]);
+    }
+  if (a.fdall && qdiv_ok(m)) {
+#pragma unroll
+    for (int q = 0; q < V; ++q)
+#pragma unroll
+      for (int t = 0; t < 6; ++t) d[t][q] = qdiv_fast(d[t][q], dl[term_axis(t)], rl[term_axis(t)]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < V; ++q)
+#pragma unroll
+      for (int t = 0; t < 6; ++t) d[t][q] = div_cold(d[t][q], dl[term_axis(t)]);
+  }
 #pragma unroll
   for (int q = 0; q < V; ++q) {
     const int kk = k + q;
     const bool okz = SGN > 0 ? kk < a.nz - 1 : (kk >= 1 && kk < a.nz);
-    T o[3], n[6], d[6];
-    T m = T(0);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) o[c] = own[c][q];
-#pragma unroll
-    for (int t = 0; t < 6; ++t) {
-      n[t] = nb[t][q];
-      d[t] = SGN > 0 ? sub_rn(n[t], o[term_comp(t)]) : sub_rn(o[term_comp(t)], n[t]);
-      m = absmax(m, d[t]);
-    }
-    if (a.fdall && qdiv_ok(m)) {
-#pragma unroll
-      for (int t = 0; t < 6; ++t) d[t] = qdiv_fast(d[t], dl[term_axis(t)], rl[term_axis(t)]);
-    } else {
-      quotients_ieee<T, SGN>(a, o, n, d);
-    }
-    const int mz = kk < a.nz ? p.map[2][kk] : -1;
-    T bz = T(0), cz = T(0), z1 = T(0), z2 = T(0);
-    const long long qz = ((long long)i * a.ny + j) * p.np[2] + mz;
-    if (mz >= 0) {
-      bz = p.b[2][kk];
-      cz = p.c[2][kk];
-      z1 = p.in[1][qz];
-      z2 = p.in[2][qz];
-    }
+    const bool inz = cz[q] != T(0);
     const T k0 = K[0][q], k1 = K[1 % NC][q], k2 = K[2 % NC][q];
     T r0 = f[0][q], r1 = f[1][q], r2 = f[2][q];
     if (oky && okz) {
-      r0 = bulk(r0, k0, d[0], d[1]);
-      if (my >= 0) r0 = cpml_term(r0, k0, d[0], by, cy, y0[q]);
-      if (mz >= 0) {
-        r0 = cpml_term(r0, -k0, d[1], bz, cz, z1);
-        p.out[1][qz] = z1;
-      }
+      r0 = bulk(r0, k0, d[0][q], d[1][q]);
+      if (my >= 0) r0 = cpml_term(r0, k0, d[0][q], by, cy, y0[q]);
+      if (inz) r0 = cpml_term(r0, -k0, d[1][q], bz[q], cz[q], z1[q]);
     }
     if (okz && okx) {
-      r1 = bulk(r1, k1, d[2], d[3]);
-      if (mz >= 0) {
-        r1 = cpml_term(r1, k1, d[2], bz, cz, z2);
-        p.out[2][qz] = z2;
-      }
-      if (mx >= 0) r1 = cpml_term(r1, -k1, d[3], bx, cx, x3[q]);
+      r1 = bulk(r1, k1, d[2][q], d[3][q]);
+      if (inz) r1 = cpml_term(r1, k1, d[2][q], bz[q], cz[q], z2[q]);
+      if (mx >= 0) r1 = cpml_term(r1, -k1, d[3][q], bx, cx, x3[q]);
     }
     if (okx && oky) {
-      r2 = bulk(r2, k2, d[4], d[5]);
-      if (mx >= 0) r2 = cpml_term(r2, k2, d[4], bx, cx, x4[q]);
-      if (my >= 0) r2 = cpml_term(r2, -k2, d[5], by, cy, y5[q]);
+      r2 = bulk(r2, k2, d[4][q], d[5][q]);
+      if (mx >= 0) r2 = cpml_term(r2, k2, d[4][q], bx, cx, x4[q]);
+      if (my >= 0) r2 = cpml_term(r2, -k2, d[5][q], by, cy, y5[q]);
     }
     out[0][q] = r0;
     out[1][q] = r1;
@@ -262,6 +242,10 @@ __device__ __forceinline__ void curl_general(const StepArgs<T>& a, const Cpml<T>
   if (mx >= 0) {
     vst(p.out[3] + qx, x3);
     vst(p.out[4] + qx, x4);
+  }
+  if (gz >= 0) {
+    vst(p.out[1] + qz, z1);
+    vst(p.out[2] + qz, z2);
   }
 }
 
@@ -313,11 +297,12 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? PFB_MINB_HV : PF
     Cpml<T> p;
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
-      p.map[x] = a.maph[x];
+      if (x < 2) p.map[x] = a.maph[x];
       p.b[x] = a.bh[x];
       p.c[x] = a.cph[x];
     }
     p.np = a.nph;
+    p.gz = a.gzh;
 #pragma unroll
     for (int t = 0; t < 6; ++t) {
       p.in[t] = a.psiHin[t];
@@ -405,7 +390,8 @@ __device__ __forceinline__ void ade_cell(const StepArgs<T>& a, uint32_t w, T en0
 // issued in dependency order: the words, every field vector, then what the
 // words select (coefficients, ADE records of a run).
 template <typename T, int CE, bool ADE>
-__global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? (ADE ? PFB_MINB_EVA : PFB_MINB_EV)
+__global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? (ADE || CE == kCeCell3 ? PFB_MINB_EVA
+                                                                                      : PFB_MINB_EV)
                                                               : PFB_MINB_EV64)
     k_e_vec(const __grid_constant__ StepArgs<T> a, int i0) {
   constexpr int V = kVec<T>;
@@ -488,11 +474,12 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? (ADE ? PFB_MINB_
     Cpml<T> p;
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
-      p.map[x] = a.mape[x];
+      if (x < 2) p.map[x] = a.mape[x];
       p.b[x] = a.be[x];
       p.c[x] = a.cpe[x];
     }
     p.np = a.npe;
+    p.gz = a.gze;
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
       p.in[s] = a.psiE[s];
