@@ -108,6 +108,16 @@ __device__ __forceinline__ T add_double(T f, double v) {
   return to_real(__dadd_rn((double)f, v), T());
 }
 
+// First statement of a kernel that launch_pdl launches: lets the next kernel
+// of the stream be scheduled as soon as every block of this one has started
+// (its blocks then wait here in what the last wave leaves free), and waits
+// until everything before this kernel is complete and visible. Without the
+// attribute both are no-ops.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 constexpr int kMaxPoles = 8;
 constexpr int kMaxMedia = 16;
 constexpr uint32_t kDispersiveBit = 0x80000000u;

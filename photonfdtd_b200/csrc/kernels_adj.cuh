@@ -76,6 +76,7 @@ __device__ __forceinline__ void curl_transpose(T x, T K, bool rA, bool rB, long 
 template <typename T, int CE>
 __global__ void __launch_bounds__(256) k_adj_e(const __grid_constant__ StepArgs<T> a,
                                                const __grid_constant__ AdjState<T> s) {
+  pdl_enter();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int i = blockIdx.z;
@@ -136,6 +137,7 @@ __global__ void __launch_bounds__(256) k_adj_e(const __grid_constant__ StepArgs<
 template <typename T>
 __global__ void __launch_bounds__(256) k_adj_h(const __grid_constant__ StepArgs<T> a,
                                                const __grid_constant__ AdjState<T> s) {
+  pdl_enter();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int i = blockIdx.z;
@@ -187,6 +189,7 @@ __global__ void __launch_bounds__(256) k_adj_h(const __grid_constant__ StepArgs<
 template <typename T>
 __global__ void k_adj_dft_src(DftRegion r, const double* cot, const double* ph, int n_freq,
                               double dt, int fam, T* l0, T* l1, T* l2, int ny, int pz) {
+  pdl_enter();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= r.ncell * r.ncomp) return;
   const long long cell = t % r.ncell;
@@ -214,6 +217,7 @@ __global__ void k_adj_dft_src(DftRegion r, const double* cot, const double* ph, 
 // vals[cell] = dJ / d f(cell) over the region, added to the adjoint field.
 template <typename T>
 __global__ void k_adj_region_src(DftRegion r, const double* vals, T* l, int ny, int pz) {
+  pdl_enter();
   const long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (cell >= r.ncell) return;
   const long long ck = cell % r.count[2];
@@ -243,6 +247,7 @@ __device__ __forceinline__ long long flux_cell(const FluxPlane& p, long long t, 
 template <typename T>
 __global__ void k_flux_plane_record(FluxPlane p, const T* E0, const T* E1, const T* E2, T* dst,
                                     int ny, int pz) {
+  pdl_enter();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long np = (long long)p.n0 * p.n1;
   if (t >= np) return;
@@ -257,6 +262,7 @@ __global__ void k_flux_plane_record(FluxPlane p, const T* E0, const T* E1, const
 template <typename T>
 __global__ void k_adj_flux_src(FluxPlane p, double c, int fam, const T* H0, const T* H1,
                                const T* H2, const T* erec, T* l0, T* l1, T* l2, int ny, int pz) {
+  pdl_enter();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long np = (long long)p.n0 * p.n1;
   if (t >= np) return;

@@ -13,6 +13,7 @@ namespace pfb {
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void k_inject(SourceGroups s, T* f0, T* f1, T* f2, long long step) {
+  pdl_enter();
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= s.n_groups) return;
   T* F = s.comp[g] == 0 ? f0 : (s.comp[g] == 1 ? f1 : f2);
@@ -57,6 +58,7 @@ __device__ __forceinline__ void dft_sample_cell(const DftRegion& r, T* ring, int
 template <typename T>
 __global__ void k_dft_sample(DftRegion r, T* ring, int slot, Fields6<T> fields, int ny,
                              int pz) {
+  pdl_enter();
   const long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (cell < r.ncell) dft_sample_cell<T>(r, ring, slot, fields, cell, ny, pz);
 }
@@ -65,6 +67,7 @@ template <typename T>
 __global__ void k_dft_flush(DftRegion r, const T* ring, int n_pending, double* acc,
                             const double* ph_e, const double* ph_h, long long q0, int n_freq,
                             double dt) {
+  pdl_enter();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= r.ncell * r.ncomp) return;
   const long long cell = t % r.ncell;
@@ -170,6 +173,7 @@ struct FluxBatch {
 template <typename T>
 __global__ void __launch_bounds__(256) k_flux_sample_batch(FluxBatch b, Fields6<T> fields, int ny,
                                                            int pz) {
+  pdl_enter();
   __shared__ double sh[8];
   const FluxPlane& p = b.p[blockIdx.y];
   if ((int)blockIdx.x >= p.nblk) return;  // uniform over the block
@@ -191,6 +195,7 @@ struct FluxFold {
 };
 template <typename T>
 __global__ void __launch_bounds__(1024) k_flux_flush(FluxFold f) {
+  pdl_enter();
   __shared__ double sh[4][8];
   __shared__ double sum[kFluxRing];
   const int m = blockIdx.x, grp = threadIdx.x >> 8, t = threadIdx.x & 255;

@@ -436,6 +436,7 @@ struct FluxKept {
 };
 template <typename T>
 __global__ void __launch_bounds__(256) k_flux_groups(FluxKept<T> f) {
+  pdl_enter();
   __shared__ double sh[8];
   const int m = blockIdx.z;
   if ((int)blockIdx.x >= f.nblk[m] || (int)blockIdx.y >= f.pending[m]) return;  // whole block

@@ -25,6 +25,7 @@ __device__ __forceinline__ T ld_if(const T* f, long long id, long long off, bool
 // H pass: H^{n+1/2} = H^{n-1/2} - ch (curl E^n + psi).
 template <typename T>
 __global__ void __launch_bounds__(256) k_h_split(const __grid_constant__ StepArgs<T> a) {
+  pdl_enter();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int i = blockIdx.z;
@@ -44,6 +45,7 @@ __global__ void __launch_bounds__(256) k_h_split(const __grid_constant__ StepArg
 // E pass: E^{n+1} = E^n + ce (curl H^{n+1/2} + psi), then ADE.
 template <typename T, int CE, bool ADE>
 __global__ void __launch_bounds__(256) k_e_split(const __grid_constant__ StepArgs<T> a) {
+  pdl_enter();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int i = blockIdx.z;

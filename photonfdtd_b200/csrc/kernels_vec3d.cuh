@@ -262,6 +262,7 @@ __device__ __forceinline__ bool warp_bulk(bool live, int i, int j, int k, const 
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? PFB_MINB_HV : PFB_MINB_HV64)
     k_h_vec(const __grid_constant__ StepArgs<T> a, int i0) {
+  pdl_enter();
   constexpr int V = kVec<T>;
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) * V;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -394,6 +395,7 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? (ADE || CE == kC
                                                                                       : PFB_MINB_EV)
                                                               : PFB_MINB_EV64)
     k_e_vec(const __grid_constant__ StepArgs<T> a, int i0) {
+  pdl_enter();
   constexpr int V = kVec<T>;
   constexpr int NC = CE == kCeCell3 ? 3 : 1;
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) * V;
