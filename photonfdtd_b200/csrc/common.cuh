@@ -196,6 +196,7 @@ struct StepArgs {
   // psi: E terms Ex_y, Ex_z, Ey_z, Ey_x, Ez_x, Ez_y; H terms Hx_y, Hx_z,
   // Hy_z, Hy_x, Hz_x, Hz_y (rustbackend.py:200-207 order)
   T* psiE[6];
+  const T* psiEin[6];  // vector E pass: psi before the step (psiE, or the last record's)
   const T* psiHin[6];
   T* psiHout[6];
   // ADE

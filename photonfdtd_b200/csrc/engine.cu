@@ -28,6 +28,7 @@
 #include "common.cuh"
 #include "devmem.cuh"
 #include "kernels_adj.cuh"
+#include "kernels_adj_vec.cuh"
 #include "kernels_aux.cuh"
 #include "kernels_fused.cuh"
 #include "kernels_resident.cuh"
@@ -673,6 +674,7 @@ StepArgs<T> step_args(pf_engine* e) {
   }
   for (int q = 0; q < 6; ++q) {
     a.psiE[q] = (T*)e->psiE[q];
+    a.psiEin[q] = (const T*)e->psiE[q];
     a.psiHin[q] = (const T*)e->psiH[c0][q];
     a.psiHout[q] = (T*)e->psiH[c1][q];
   }
@@ -880,13 +882,46 @@ int sample_monitors(pf_engine* e, long long s, int lvl) {
 }
 
 template <typename T>
-int inject(pf_engine* e, int fam, int lvl, long long s) {
+int inject(pf_engine* e, int fam, T* const F[3], long long s) {
   SourceGroups& d = e->src[fam].dev;
   if (d.n_groups == 0) return PF_OK;
-  void** F = fam == 0 ? e->E[lvl] : e->H[lvl];
   LaunchScope ls(e, 1);
-  launch_pdl(e->stream, (d.n_groups + 127) / 128, 128, k_inject<T>, d, (T*)F[0], (T*)F[1],
-             (T*)F[2], s);
+  launch_pdl(e->stream, (d.n_groups + 127) / 128, 128, k_inject<T>, d, F[0], F[1], F[2], s);
+  return PF_OK;
+}
+
+// A replay with the vector passes writes its record in place of the state: the
+// H pass reads H from the last step's slot and writes this step's, the E pass
+// psi_E likewise (the copies into the slot took as long as the H pass).
+// Points the step's arguments at slots t - 1 (the engine's own state for t =
+// 0) and t.
+template <typename T>
+void record_into(pf_engine* e, long long t, StepArgs<T>& a, T* Hout[3]) {
+  char* at = e->rec + (size_t)t * e->rec_slot;
+  const char* last = at - e->rec_slot;
+  const size_t S = sizeof(T), n = (size_t)e->ncellp * S;
+  size_t off = 0;
+  for (int c = 0; c < 3; ++c, off += n) {
+    if (t > 0) a.Hin[c] = (const T*)(last + off);
+    a.Hout[c] = Hout[c] = (T*)(at + off);
+  }
+  for (int q = 0; q < 6; ++q) {
+    if (t > 0) a.psiEin[q] = (const T*)(last + off);
+    a.psiE[q] = (T*)(at + off);
+    off += (size_t)e->npsiE[q] * S;
+  }
+}
+// The engine's own state from the last slot of a replay.
+int record_out(pf_engine* e, long long t) {
+  const char* at = e->rec + (size_t)t * e->rec_slot;
+  const size_t n = (size_t)e->ncellp * e->rb;
+  for (int c = 0; c < 3; ++c, at += n)
+    PF_CUDA(e, cudaMemcpyAsync(e->H[e->cur][c], at, n, cudaMemcpyDeviceToDevice, e->stream));
+  for (int q = 0; q < 6; ++q) {
+    const size_t b = (size_t)e->npsiE[q] * e->rb;
+    if (b) PF_CUDA(e, cudaMemcpyAsync(e->psiE[q], at, b, cudaMemcpyDeviceToDevice, e->stream));
+    at += b;
+  }
   return PF_OK;
 }
 
@@ -894,14 +929,14 @@ int inject(pf_engine* e, int fam, int lvl, long long s) {
 // what the reverse step needs to recompute the gradient's g = curl + psi.
 template <typename T>
 int record_step(pf_engine* e, long long t) {
-  if (t < 0 || t >= e->ring_steps) return fail(e, PF_ERR_STATE, "record slot out of range");
   char* base = e->rec + (size_t)t * e->rec_slot;
+  const bool direct = e->vec && !e->fused;  // record_into wrote them
   const size_t S = sizeof(T), n = (size_t)e->ncellp * S;
   size_t off = 0;
-  for (int c = 0; c < 3; ++c, off += n)
+  for (int c = 0; c < 3 && !direct; ++c, off += n)
     PF_CUDA(e, cudaMemcpyAsync(base + off, e->H[e->cur][c], n, cudaMemcpyDeviceToDevice,
                                e->stream));
-  for (int q = 0; q < 6; ++q) {
+  for (int q = 0; q < 6 && !direct; ++q) {
     const size_t b = (size_t)e->npsiE[q] * S;
     if (b) PF_CUDA(e, cudaMemcpyAsync(base + off, e->psiE[q], b, cudaMemcpyDeviceToDevice, e->stream));
     off += b;
@@ -1132,13 +1167,21 @@ int advance_separate(pf_engine* e, long long n_sub) {
       // sources of the fused path are injected after its single pass: an H
       // source must reach the E update, so the fused path is only chosen
       // when there are no H-family sources.
-      inject<T>(e, 0, nxt, s);
+      T* Eout[3] = {a.Eout[0], a.Eout[1], a.Eout[2]};
+      inject<T>(e, 0, Eout, s);
     } else {
+      T* Hout[3] = {a.Hout[0], a.Hout[1], a.Hout[2]};
+      if (e->recording) {
+        const long long slot = s - e->rec_step0;
+        if (slot < 0 || slot >= e->ring_steps)
+          return fail(e, PF_ERR_STATE, "record slot out of range");
+        if (e->vec) record_into<T>(e, slot, a, Hout);
+      }
       {
         LaunchScope ls(e, 0);
         launch_h<T>(e, a, 0, e->nx);
       }
-      inject<T>(e, 1, nxt, s);
+      inject<T>(e, 1, Hout, s);
       a.Hin[0] = a.Hout[0];
       a.Hin[1] = a.Hout[1];
       a.Hin[2] = a.Hout[2];
@@ -1146,7 +1189,8 @@ int advance_separate(pf_engine* e, long long n_sub) {
         LaunchScope ls(e, 0);
         launch_e<T>(e, a, 0, e->nx);
       }
-      inject<T>(e, 0, nxt, s);
+      T* Eout[3] = {a.Eout[0], a.Eout[1], a.Eout[2]};
+      inject<T>(e, 0, Eout, s);
     }
     int rc = e->recording ? PF_OK : sample_monitors<T>(e, s, nxt);
     if (rc) return rc;
@@ -1941,6 +1985,9 @@ int adj_sources(pf_engine* e, long long m, int fam, const AdjState<T>& st, long 
   for (size_t k = 0; k < e->dfts.size(); ++k) {
     const DftMon& dm = e->dfts[k];
     if (!e->dft_cot[k] || m % dm.interval) continue;
+    bool any = false;  // a component of this family
+    for (int q = 0; q < dm.r.ncomp; ++q) any = any || (dm.r.comps[q] >= 3) == (fam == 1);
+    if (!any) continue;
     const long long q = m / dm.interval;
     const double* ph = (fam == 0 ? dm.ph_e : dm.ph_h) + q * dm.n_freq * 2;
     const long long nt = dm.r.ncell * dm.r.ncomp;
@@ -1970,21 +2017,31 @@ int adj_segment_typed(pf_engine* e, long long step0, long long n) {
   int rc = advance_typed<T>(e, n);
   e->recording = false;
   if (rc) return rc;
+  if (e->vec && !e->fused && (rc = record_out(e, n - 1))) return rc;
   const int nz = e->nz, ny = e->ny, nx = e->nx;
-  const dim3 blk = nz > 1 ? dim3(32, 8) : dim3(1, 256);
-  const dim3 grd((nz + blk.x - 1) / blk.x, (ny + blk.y - 1) / blk.y, nx);
+  const int nzv = (nz + kVec<T> - 1) / kVec<T>;
+  const dim3 blk = e->vec ? dim3(vec_lanes(nzv), kVecThreads / vec_lanes(nzv))
+                          : (nz > 1 ? dim3(32, 8) : dim3(1, 256));
+  const dim3 grd(((e->vec ? nzv : nz) + blk.x - 1) / blk.x, (ny + blk.y - 1) / blk.y, nx);
   const StepArgs<T> a = step_args<T>(e);
   for (long long m = step0 + n - 1; m >= step0; --m) {
     const AdjState<T> s = adj_state<T>(e, m - step0);
     if ((rc = adj_sources<T>(e, m, 0, s, m - step0))) return rc;
-    if (e->ce_mode == PF_CE_CELL1)
+    if (e->vec && e->ce_mode == PF_CE_CELL1)
+      launch_pdl(e->stream, grd, blk, k_adj_e_vec<T, kCeCell1>, a, s);
+    else if (e->vec && e->ce_mode == PF_CE_CELL3)
+      launch_pdl(e->stream, grd, blk, k_adj_e_vec<T, kCeCell3>, a, s);
+    else if (e->vec)
+      launch_pdl(e->stream, grd, blk, k_adj_e_vec<T, kCeTable>, a, s);
+    else if (e->ce_mode == PF_CE_CELL1)
       launch_pdl(e->stream, grd, blk, k_adj_e<T, kCeCell1>, a, s);
     else if (e->ce_mode == PF_CE_CELL3)
       launch_pdl(e->stream, grd, blk, k_adj_e<T, kCeCell3>, a, s);
     else
       launch_pdl(e->stream, grd, blk, k_adj_e<T, kCeTable>, a, s);
     if ((rc = adj_sources<T>(e, m, 1, s, m - step0))) return rc;
-    launch_pdl(e->stream, grd, blk, k_adj_h<T>, a, s);
+    if (e->vec) launch_pdl(e->stream, grd, blk, k_adj_h_vec<T>, a, s);
+    else launch_pdl(e->stream, grd, blk, k_adj_h<T>, a, s);
   }
   PF_CUDA(e, cudaGetLastError());
   PF_CUDA(e, cudaStreamSynchronize(e->stream));

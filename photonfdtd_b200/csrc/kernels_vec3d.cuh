@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? (ADE || CE == kC
     p.gz = a.gze;
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
-      p.in[s] = a.psiE[s];
+      p.in[s] = a.psiEin[s];
       p.out[s] = a.psiE[s];
     }
     curl_general<T, -1, NC>(a, p, i, j, k, en, K, own, nb, e);
