@@ -552,6 +552,18 @@ int pfs_mse(int64_t rows, int used, int ld, const float *y, const float *t, floa
  * w, refreshing the BF16 copy w16 if given. */
 int pfs_adam(int64_t n, float *w, const float *g, float *m, float *v, float lr, float b1,
              float b2, float eps, int step, float wd, void *w16, void *stream);
+/* The same step for all tensors of a network in one launch (one per 32
+ * tensors). The table is read before the call returns. */
+typedef struct pfs_adam_tensor {
+  int64_t n;
+  float *w;
+  const float *g;
+  float *m, *v;
+  void *w16; /* BF16 copy, or NULL */
+  float wd;
+} pfs_adam_tensor;
+int pfs_adam_many(int count, const pfs_adam_tensor *tensors, float lr, float b1, float b2,
+                  float eps, int step, void *stream);
 
 /* ------------------------------------------------------------------------
  * Waveguide mode operator (pfm_*), for the GPU mode solver

@@ -39,6 +39,13 @@ _pi64 = C.POINTER(C.c_int64)
 _pu32 = C.POINTER(C.c_uint32)
 _pdbl = C.POINTER(C.c_double)
 
+
+class AdamTensor(C.Structure):
+    """pfs_adam_tensor: one tensor of pfs_adam_many."""
+    _fields_ = [("n", _i64), ("w", _vp), ("g", _vp), ("m", _vp), ("v", _vp), ("w16", _vp),
+                ("wd", C.c_float)]
+
+
 # name -> (restype, argtypes); every symbol include/pfb200.h declares.
 SIGNATURES = {
     "pf_version": (C.c_char_p, []),
@@ -144,6 +151,8 @@ SIGNATURES = {
     "pfs_mse": (C.c_int, [_i64, C.c_int, C.c_int, _vp, _vp, _vp, _vp, C.c_int, _vp]),
     "pfs_adam": (C.c_int, [_i64, _vp, _vp, _vp, _vp, C.c_float, C.c_float, C.c_float, C.c_float,
                            C.c_int, C.c_float, _vp, _vp]),
+    "pfs_adam_many": (C.c_int, [C.c_int, C.POINTER(AdamTensor), C.c_float, C.c_float, C.c_float,
+                                C.c_float, C.c_int, _vp]),
 }
 
 

@@ -46,6 +46,39 @@ int cuda_status(const char* what) {
   return PF_ERR_CUDA;
 }
 
+// Programmatic dependent launch: a training step is 91 launches of 3 to 80 us
+// in one chain, and a plain launch starts only after the last block of the
+// one before has drained. With the attribute the next kernel's blocks are
+// placed while that tail runs and wait in pdl_enter (first statement of every
+// kernel here but the tensor-core GEMM, which waits after its set-up) until
+// everything before them is complete and visible.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_release() {
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+__device__ __forceinline__ void pdl_enter() {
+  pdl_release();
+  pdl_wait();
+}
+
+template <typename... P, typename... A>
+void launch_pdl(cudaStream_t st, dim3 grid, dim3 block, size_t smem, void (*kernel)(P...),
+                A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---- GEMM ------------------------------------------------------------------
 constexpr int BM = 64, BN = 64, BK = 32, PADK = BK + 8;  // padded rows: fewer bank conflicts
 
@@ -73,6 +106,7 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(int M, int N, int K, const __
                                                    int lda, const __nv_bfloat16* B, int ldb,
                                                    float* C, int ldc, float alpha, float beta,
                                                    int kc, float* work) {
+  pdl_enter();
   const int kbeg = blockIdx.z * kc;
   const int kend = min(K, kbeg + kc);
   if (gridDim.z > 1) {
@@ -190,6 +224,7 @@ __host__ __device__ constexpr int tc_stage_bytes(int bn) { return (TBM + bn) * T
 __host__ __device__ constexpr int tc_smem_bytes(int bn, int stages = TC_STAGES) {
   return stages * tc_stage_bytes(bn) + 1024;  // + alignment of the ring to 1024 bytes
 }
+constexpr int kTcSmemSm = 227 * 1024;  // shared memory of an SM's blocks
 // Ring depth of a launch: no more stages than K tiles in a block's slice, so
 // a short-K GEMM (a layer's input gradient: K = 32..256) takes less shared
 // memory and several blocks share an SM (one block's epilogue overlapping
@@ -260,6 +295,13 @@ __device__ __forceinline__ void tc_tma_2d(uint32_t dst, const CUtensorMap* map, 
       : "memory");
 }
 
+// Leading dimension of a warp's 32 x 32 epilogue chunk in shared memory: rows
+// 16-byte aligned, and eight lanes writing four floats each of eight rows (or
+// reading 32 floats of one) touch all 32 banks. Four chunks fit the smallest
+// ring (one stage of the 32-wide tile).
+constexpr int kStageLd = 36;
+static_assert(4 * 32 * kStageLd * 4 <= tc_stage_bytes(32), "the epilogue reuses the ring");
+
 // Epilogue of a layer's forward GEMM (EPI): y = act(C + bias) written as
 // FP32 (to C) and BF16 (y16, same leading dimension), k_bias_act's
 // arithmetic on the value C would have held; beta is 0 and K unsplit.
@@ -300,12 +342,6 @@ __global__ void __launch_bounds__(128, 1)
   }
   const int nk = (kend - kbeg + TBK - 1) / TBK;  // >= 1 (host guarantees non-empty slices)
   const uint32_t s0 = (smem_u32(tc_smem) + 1023u) & ~1023u;
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(&tmem_slot)),
-                 "r"(BN));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
   if (tid == 32) {
     for (int i = 0; i < TC_STAGES; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full[i])));
@@ -318,10 +354,21 @@ __global__ void __launch_bounds__(128, 1)
     n_loaded = 0;
     n_seen = 0;
   }
+  // The tensor memory is taken after the wait and the next kernel let in only
+  // once every block holds its own: no block ever waits for columns that a
+  // block of a later launch holds.
+  pdl_wait();
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&tmem_slot)),
+                 "r"(BN));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_slot;
+  pdl_release();
   if (warp == 0) {  // producer
     int kt = 0;
     for (; kt < nk; ++kt) {
@@ -409,8 +456,17 @@ __global__ void __launch_bounds__(128, 1)
     }
   } else {
     asm volatile("tcgen05.fence::after_thread_sync;");
-    float* stage = reinterpret_cast<float*>(tc_smem + (s0 - smem_u32(tc_smem))) + warp * 32 * 33;
+    float* stage =
+        reinterpret_cast<float*>(tc_smem + (s0 - smem_u32(tc_smem))) + warp * 32 * kStageLd;
     const int rbase = m0 + warp * 32;
+    // Short-K products are bound by these stores (K = 64: 128 x 256 results
+    // per block against one TMA stage). A warp turns its 32 x 32 chunk in
+    // shared memory and each lane then stores four columns of every fourth
+    // row as one vector: 8 stores where a float per lane takes 32. 131072 x
+    // 288 at K = 64: 86.0 -> 49.2 us. Rows that are not 16-byte aligned (ldc or
+    // C) keep the scalar stores; a column group cut by N falls back by itself.
+    const bool cvec = (ldc & 3) == 0 && ((uintptr_t)C & 15) == 0 &&
+                      (!EPI || ((uintptr_t)ep.y16 & 7) == 0);
 #pragma unroll 1
     for (int cb = 0; cb < BN / 32; ++cb) {
       if (n0 + cb * 32 >= N) break;  // uniform
@@ -429,21 +485,65 @@ __global__ void __launch_bounds__(128, 1)
           : "r"(taddr));
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int j = 0; j < 32; ++j) stage[lane * 33 + j] = __uint_as_float(v[j]);
+      for (int j = 0; j < 32; j += 4)
+        *reinterpret_cast<uint4*>(stage + lane * kStageLd + j) =
+            make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
       __syncwarp();
-      const int n = n0 + cb * 32 + lane;
-      for (int rr = 0; rr < 32; ++rr) {
-        const int r = rbase + rr;
-        if (r < M && n < N) {
-          float* o = C + (long long)r * ldc + n;
-          const float val = alpha * stage[rr * 33 + lane];
-          if constexpr (EPI) {
-            float v = val + (ep.bias ? ep.bias[n] : 0.f);
-            if (ep.relu) v = fmaxf(v, 0.f);
-            *o = v;
-            if (ep.y16) ep.y16[(long long)r * ldc + n] = __float2bfloat16(v);
-          } else {
-            *o = beta == 0.f ? val : val + beta * *o;
+      const int nq = n0 + cb * 32 + (lane & 7) * 4, rq = lane >> 3;
+      if (cvec && n0 + cb * 32 + 32 <= N) {  // uniform
+        float bq[4] = {0.f, 0.f, 0.f, 0.f};
+        if constexpr (EPI) {
+          if (ep.bias) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) bq[q] = ep.bias[nq + q];
+          }
+        }
+#pragma unroll
+        for (int rr = 0; rr < 32; rr += 4) {
+          const int r = rbase + rr + rq;
+          const float4 s4 =
+              *reinterpret_cast<const float4*>(stage + (rr + rq) * kStageLd + (lane & 7) * 4);
+          if (r < M) {
+            float* o = C + (long long)r * ldc + nq;
+            float x[4] = {alpha * s4.x, alpha * s4.y, alpha * s4.z, alpha * s4.w};
+            if constexpr (EPI) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                x[q] = x[q] + bq[q];
+                if (ep.relu) x[q] = fmaxf(x[q], 0.f);
+              }
+              if (ep.y16) {
+                __nv_bfloat16 h[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) h[q] = __float2bfloat16(x[q]);
+                *reinterpret_cast<uint2*>(ep.y16 + (long long)r * ldc + nq) =
+                    *reinterpret_cast<const uint2*>(h);
+              }
+            } else if (beta != 0.f) {
+              const float4 c = *reinterpret_cast<const float4*>(o);
+              x[0] = x[0] + beta * c.x;
+              x[1] = x[1] + beta * c.y;
+              x[2] = x[2] + beta * c.z;
+              x[3] = x[3] + beta * c.w;
+            }
+            *reinterpret_cast<float4*>(o) = make_float4(x[0], x[1], x[2], x[3]);
+          }
+        }
+      } else {
+        const int n = n0 + cb * 32 + lane;
+        for (int rr = 0; rr < 32; ++rr) {
+          const int r = rbase + rr;
+          if (r < M && n < N) {
+            float* o = C + (long long)r * ldc + n;
+            const float val = alpha * stage[rr * kStageLd + lane];
+            if constexpr (EPI) {
+              float v = val + (ep.bias ? ep.bias[n] : 0.f);
+              if (ep.relu) v = fmaxf(v, 0.f);
+              *o = v;
+              if (ep.y16) ep.y16[(long long)r * ldc + n] = __float2bfloat16(v);
+            } else {
+              *o = beta == 0.f ? val : val + beta * *o;
+            }
           }
         }
       }
@@ -456,14 +556,29 @@ __global__ void __launch_bounds__(128, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN));
 }
 
-// C = sum over the split slabs, in order, + beta * C.
+// C = sum over the split slabs, in order, + beta * C: one serial sum per
+// result. Bound by the latency of the slab loads, so a thread has sixteen in
+// flight before it adds them (a weight gradient of 32 x 32 from 293 slabs,
+// product and sum: 48.1 us a load at a time, 41.9 so; 39.7 with a kernel whose
+// warps fetched the slabs through shared memory, which cost 2 us at 17 slabs
+// and 12 at 5).
+constexpr int kReduceAhead = 16;
 __global__ void k_splitk_reduce(int M, int N, int splits, const float* work, float* C, int ldc,
                                 float beta) {
+  pdl_enter();
   const long long total = (long long)M * N;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
     float s = 0.f;
-    for (int z = 0; z < splits; ++z) s += work[(long long)z * total + t];
+    int z = 0;
+    for (; z + kReduceAhead <= splits; z += kReduceAhead) {
+      float v[kReduceAhead];
+#pragma unroll
+      for (int q = 0; q < kReduceAhead; ++q) v[q] = work[(long long)(z + q) * total + t];
+#pragma unroll
+      for (int q = 0; q < kReduceAhead; ++q) s += v[q];
+    }
+    for (; z < splits; ++z) s += work[(long long)z * total + t];
     const long long m = t / N, n = t % N;
     float* o = C + m * ldc + n;
     *o = beta == 0.f ? s : s + beta * *o;
@@ -474,6 +589,7 @@ __global__ void k_splitk_reduce(int M, int N, int splits, const float* work, flo
 // col[(b, oy, ox)][k], k = (ky * kw + kx) * C + c for k < kh*kw*C, zero above.
 __global__ void k_im2col(int nb, int H, int W, int C, int kh, int kw, int stride, int ph, int pw,
                          int Ho, int Wo, const __nv_bfloat16* x, __nv_bfloat16* col, int Kp) {
+  pdl_enter();
   const long long total = (long long)nb * Ho * Wo * Kp;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -495,6 +611,7 @@ __global__ void k_im2col(int nb, int H, int W, int C, int kh, int kw, int stride
 // and in range of dcol[(b, oy, ox)][(ky * kw + kx) * C + c].
 __global__ void k_col2im(int nb, int H, int W, int C, int kh, int kw, int stride, int ph, int pw,
                          int Ho, int Wo, const float* dcol, int Kp, float* dx) {
+  pdl_enter();
   const long long total = (long long)nb * H * W * C;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -502,19 +619,11 @@ __global__ void k_col2im(int nb, int H, int W, int C, int kh, int kw, int stride
     const int ix = (int)((t / C) % W), iy = (int)((t / ((long long)C * W)) % H);
     const int b = (int)(t / ((long long)C * W * H));
     float s = 0.f;
-    for (int ky = 0; ky < kh; ++ky) {
-      const int ny = iy + ph - ky;
-      if (ny < 0 || ny % stride) continue;
-      const int oy = ny / stride;
-      if (oy >= Ho) continue;
-      for (int kx = 0; kx < kw; ++kx) {
-        const int nx = ix + pw - kx;
-        if (nx < 0 || nx % stride) continue;
-        const int ox = nx / stride;
-        if (ox >= Wo) continue;
-        s += dcol[(((long long)b * Ho + oy) * Wo + ox) * Kp + (ky * kw + kx) * C + c];
-      }
-    }
+    const int oyt = (iy + ph) / stride, oxt = (ix + pw) / stride;
+    for (int oy = min(oyt, Ho - 1); oy >= 0 && iy + ph - oy * stride < kh; --oy)
+      for (int ox = min(oxt, Wo - 1); ox >= 0 && ix + pw - ox * stride < kw; --ox)
+        s += dcol[(((long long)b * Ho + oy) * Wo + ox) * Kp +
+                  ((iy + ph - oy * stride) * kw + ix + pw - ox * stride) * C + c];
     dx[t] = s;
   }
 }
@@ -525,68 +634,135 @@ __global__ void k_col2im(int nb, int H, int W, int C, int kh, int kw, int stride
 // tap, read with one 16-byte load. col2im: one thread per 8 channels of an
 // input position (C % 8 == 0), the taps summed in the same order as k_col2im,
 // so both forms give identical results.
+//
+// Both were bound by the index divisions (five by run-time integers for 16
+// bytes): the divisors are launch constants, so the host passes multipliers.
+struct Div {  // n / d for 0 <= n < 2^31: (n * m) >> sh
+  uint32_t m;
+  int sh, d;
+  __device__ __forceinline__ int quot(int n) const {
+    return (int)(((uint64_t)(uint32_t)n * m) >> sh);
+  }
+};
+
+// m = floor(2^(31 + s) / d) + 1 with 2^s >= d exceeds 2^(31 + s) / d by at
+// most 1: for n < 2^31 the product's error stays below 1 / d of the shift.
+Div make_div(int d) {
+  int s = 0;
+  while ((1LL << s) < d) ++s;
+  return Div{(uint32_t)((1ull << (31 + s)) / (unsigned)d + 1), 31 + s, d};
+}
+
+struct ConvDivs {
+  Div q, wo, ho, c, kw;
+};
+
+// cpt: chunks of a col row per thread. The element path (!VEC) takes whole
+// rows up to kRowChunks chunks: a row's position is resolved once and adjacent
+// threads read adjacent inputs (64 x 64 x 1, 3 x 3, batch 128: 63.5 us with a
+// division per element, 34.8 with one per chunk, 26.6 by rows). Longer rows keep
+// a chunk per thread, whose stores are contiguous. Vector path, batch 128, 64
+// x 64 x 32 from 3 x 3 taps at stride 2: 36.9 -> 26.7 us (109 MB).
+constexpr int kRowChunks = 8;
 template <bool VEC>
 __global__ void k_im2col8(int rows, int H, int W, int C, int kh, int kw, int stride, int ph,
                           int pw, int Ho, int Wo, const __nv_bfloat16* x, __nv_bfloat16* col,
-                          int Kp) {
-  const int qn = Kp >> 3, K = kh * kw * C;
+                          int Kp, ConvDivs dv, int cpt) {
+  pdl_enter();
+  const int qn = VEC ? Kp >> 3 : (Kp >> 3) / cpt, K = kh * kw * C;
   const int total = rows * qn;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int q = t % qn, m = t / qn;
-    const int ox = m % Wo, r = m / Wo, oy = r % Ho, b = r / Ho;
-    const int k0 = q * 8;
+    const int m = dv.q.quot(t), q = t - m * qn;
+    const int r = dv.wo.quot(m), ox = m - r * Wo, b = dv.ho.quot(r), oy = r - b * Ho;
+    int k0 = (VEC ? q : q * cpt) * 8;
     uint4 out = make_uint4(0, 0, 0, 0);
     if (VEC) {
       if (k0 < K) {
-        const int tap = k0 / C, c = k0 - tap * C, kx = tap % kw, ky = tap / kw;
+        const int tap = dv.c.quot(k0), c = k0 - tap * C, ky = dv.kw.quot(tap), kx = tap - ky * kw;
         const int iy = oy * stride - ph + ky, ix = ox * stride - pw + kx;
         if (iy >= 0 && iy < H && ix >= 0 && ix < W)
           out = *reinterpret_cast<const uint4*>(x + ((long long)(b * H + iy) * W + ix) * C + c);
       }
+      *reinterpret_cast<uint4*>(col + (long long)m * Kp + k0) = out;
     } else {
-      __nv_bfloat16 v[8];
+      const int tap = dv.c.quot(k0);
+      int c = k0 - tap * C, ky = dv.kw.quot(tap), kx = tap - ky * kw;
+      for (int g = 0; g < cpt; ++g, k0 += 8) {
+        __nv_bfloat16 v[8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        v[e] = __float2bfloat16(0.f);
-        const int k = k0 + e;
-        if (k < K) {
-          const int c = k % C, tap = k / C, kx = tap % kw, ky = tap / kw;
+        for (int e = 0; e < 8; ++e) {
+          v[e] = __float2bfloat16(0.f);
           const int iy = oy * stride - ph + ky, ix = ox * stride - pw + kx;
-          if (iy >= 0 && iy < H && ix >= 0 && ix < W)
+          if (k0 + e < K && iy >= 0 && iy < H && ix >= 0 && ix < W)
             v[e] = x[((long long)(b * H + iy) * W + ix) * C + c];
+          if (++c == C) {
+            c = 0;
+            if (++kx == kw) {
+              kx = 0;
+              ++ky;
+            }
+          }
         }
+        out = *reinterpret_cast<const uint4*>(v);
+        *reinterpret_cast<uint4*>(col + (long long)m * Kp + k0) = out;
       }
-      out = *reinterpret_cast<const uint4*>(v);
     }
-    *reinterpret_cast<uint4*>(col + (long long)m * Kp + k0) = out;
   }
 }
 
+// The taps of a position are walked by output row and column, descending
+// (ascending taps), so only those that exist are visited; SMALL (at most two
+// output rows and columns reach a position, ceil(k / stride) <= 2 both ways)
+// has all of their loads in flight before the first sum. Batch 128, 64 x 64 x
+// 32 from 3 x 3 taps at stride 2: 65.6 -> 41.0 us (167 MB).
+struct ColDivs {
+  Div cg, w, h, stride;
+};
+template <bool SMALL>
 __global__ void k_col2im8(int nb, int H, int W, int C, int kh, int kw, int stride, int ph, int pw,
-                          int Ho, int Wo, const float* dcol, int Kp, float* dx) {
+                          int Ho, int Wo, const float* dcol, int Kp, float* dx, ColDivs dv) {
+  pdl_enter();
   const int cg = C >> 3;
   const int total = nb * H * W * cg;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int g = t % cg, p = t / cg;
-    const int ix = p % W, r = p / W, iy = r % H, b = r / H;
+    const int p = dv.cg.quot(t), g = t - p * cg;
+    const int r = dv.w.quot(p), ix = p - r * W, b = dv.h.quot(r), iy = r - b * H;
     const int c0 = g * 8;
     float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
-    for (int ky = 0; ky < kh; ++ky) {
-      const int ny = iy + ph - ky;
-      if (ny < 0 || ny % stride) continue;
-      const int oy = ny / stride;
-      if (oy >= Ho) continue;
-      for (int kx = 0; kx < kw; ++kx) {
-        const int nx = ix + pw - kx;
-        if (nx < 0 || nx % stride) continue;
-        const int ox = nx / stride;
-        if (ox >= Wo) continue;
-        const float4* src = reinterpret_cast<const float4*>(
-            dcol + (long long)((b * Ho + oy) * Wo + ox) * Kp + (ky * kw + kx) * C + c0);
-        const float4 u = src[0], v = src[1];
-        s0.x += u.x; s0.y += u.y; s0.z += u.z; s0.w += u.w;
-        s1.x += v.x; s1.y += v.y; s1.z += v.z; s1.w += v.w;
+    const int oyt = dv.stride.quot(iy + ph), oxt = dv.stride.quot(ix + pw);
+    auto tap = [&](int oy, int ox) {
+      const int ky = iy + ph - oy * stride, kx = ix + pw - ox * stride;
+      return reinterpret_cast<const float4*>(
+          dcol + (long long)((b * Ho + oy) * Wo + ox) * Kp + (ky * kw + kx) * C + c0);
+    };
+    auto have = [&](int oy, int ox) {
+      return oy >= 0 && oy < Ho && iy + ph - oy * stride < kh && ox >= 0 && ox < Wo &&
+             ix + pw - ox * stride < kw;
+    };
+    auto add = [&](const float4& u, const float4& v) {
+      s0.x += u.x; s0.y += u.y; s0.z += u.z; s0.w += u.w;
+      s1.x += v.x; s1.y += v.y; s1.z += v.z; s1.w += v.w;
+    };
+    if (SMALL) {
+      float4 u[4], v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int oy = oyt - (q >> 1), ox = oxt - (q & 1);
+        if (have(oy, ox)) {
+          const float4* src = tap(oy, ox);
+          u[q] = src[0];
+          v[q] = src[1];
+        }
       }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (have(oyt - (q >> 1), oxt - (q & 1))) add(u[q], v[q]);
+    } else {
+      for (int oy = min(oyt, Ho - 1); oy >= 0 && iy + ph - oy * stride < kh; --oy)
+        for (int ox = min(oxt, Wo - 1); ox >= 0 && ix + pw - ox * stride < kw; --ox) {
+          const float4* src = tap(oy, ox);
+          add(src[0], src[1]);
+        }
     }
     float4* dst = reinterpret_cast<float4*>(dx + (long long)p * C + c0);
     dst[0] = s0;
@@ -598,6 +774,7 @@ __global__ void k_col2im8(int nb, int H, int W, int C, int kh, int kw, int strid
 // (either may be NULL).
 __global__ void k_bias_act(long long M, int N, const float* x, const float* bias, int relu,
                            float* y32, __nv_bfloat16* y16) {
+  pdl_enter();
   const long long total = M * N;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -613,6 +790,7 @@ __global__ void k_bias_act(long long M, int N, const float* x, const float* bias
 // lanes; each row block strides the rows, then a fixed-order reduction.
 __global__ void k_act_bwd(long long M, int N, const float* dy, const float* y, int relu,
                           float* d32, __nv_bfloat16* d16, float* part) {
+  pdl_enter();
   __shared__ float sh[8][33];
   const int n = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
@@ -635,26 +813,108 @@ __global__ void k_act_bwd(long long M, int N, const float* dy, const float* y, i
   }
 }
 
-// dbias[n] = sum over the row blocks of part[q][n]: one block per column,
-// strided partial sums and a fixed-order tree (independent of scheduling).
+// The same sums in the same order on 16-byte vectors (N % 4 == 0, aligned
+// rows): a thread takes four columns of a row, two of its rows ahead, and a
+// block four neighbouring row blocks, so what it reads is 32 rows together.
+// Bound by memory: 524288 x 32 (168 MB) 55.3 us with a float per thread, 36.9
+// so. (Eight scalar rows ahead took 95 registers, two blocks per SM, 145 us.)
+constexpr int kActBlocks = 4;
+__global__ void __launch_bounds__(64 * kActBlocks, 6)
+    k_act_bwd4(long long M, int N, const float* dy, const float* y, int relu, float* d32,
+               __nv_bfloat16* d16, float* part, int row_blocks) {
+  pdl_enter();
+  __shared__ float4 sh[kActBlocks][8][9];
+  const int n = blockIdx.x * 32 + threadIdx.x * 4;
+  const int rb = blockIdx.y * kActBlocks + threadIdx.z;
+  const long long step = (long long)row_blocks * 8;
+  const bool in = n < N && rb < row_blocks;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (in) {
+    for (long long m0 = (long long)rb * 8 + threadIdx.y; m0 < M; m0 += 2 * step) {
+      float4 dv[2], yv[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const long long t = (m0 + q * step) * N + n;
+        yv[q] = make_float4(1.f, 1.f, 1.f, 1.f);
+        if (m0 + q * step < M) {
+          dv[q] = *reinterpret_cast<const float4*>(dy + t);
+          if (relu) yv[q] = *reinterpret_cast<const float4*>(y + t);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const long long t = (m0 + q * step) * N + n;
+        if (m0 + q * step >= M) break;
+        float4 v = dv[q];
+        if (!(yv[q].x > 0.f)) v.x = 0.f;
+        if (!(yv[q].y > 0.f)) v.y = 0.f;
+        if (!(yv[q].z > 0.f)) v.z = 0.f;
+        if (!(yv[q].w > 0.f)) v.w = 0.f;
+        if (d32) *reinterpret_cast<float4*>(d32 + t) = v;
+        if (d16) {
+          const __nv_bfloat16 h[4] = {__float2bfloat16(v.x), __float2bfloat16(v.y),
+                                      __float2bfloat16(v.z), __float2bfloat16(v.w)};
+          *reinterpret_cast<uint2*>(d16 + t) = *reinterpret_cast<const uint2*>(h);
+        }
+        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+      }
+    }
+  }
+  sh[threadIdx.z][threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0 && in && part) {
+    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = 0; q < 8; ++q) {
+      const float4 u = sh[threadIdx.z][q][threadIdx.x];
+      r.x += u.x; r.y += u.y; r.z += u.z; r.w += u.w;
+    }
+    *reinterpret_cast<float4*>(part + (long long)rb * N + n) = r;
+  }
+}
+
+// dbias[n] = sum over the row blocks of part[q][n]: one block per column (or
+// per four, V = float4, where N % 4 == 0 and the rows are aligned), strided
+// partial sums and a fixed-order tree (independent of scheduling). Bound by
+// the latency of reads that take one column of each row: sixteen in flight
+// per thread (8192 x 32: 16 us a load at a time, 7 with vectors).
+__device__ __forceinline__ void add_to(float& a, float b) { a += b; }
+__device__ __forceinline__ void add_to(float4& a, const float4& b) {
+  a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+}
+
+template <typename V>
 __global__ void k_colsum(int R, int N, const float* part, float* out) {
-  __shared__ float sh[256];
-  const int n = blockIdx.x;
-  float r = 0.f;
-  for (int q = threadIdx.x; q < R; q += blockDim.x) r += part[(long long)q * N + n];
+  pdl_enter();
+  constexpr int kAhead = 16;
+  __shared__ V sh[256];
+  const V* src = reinterpret_cast<const V*>(part);
+  const int n = blockIdx.x, ld = N / (int)(sizeof(V) / sizeof(float));
+  V r = V{};
+  for (long long q0 = threadIdx.x; q0 < R; q0 += kAhead * blockDim.x) {
+    V v[kAhead];
+#pragma unroll
+    for (int e = 0; e < kAhead; ++e) {
+      const long long q = q0 + e * blockDim.x;
+      if (q < R) v[e] = src[q * ld + n];
+    }
+#pragma unroll
+    for (int e = 0; e < kAhead; ++e)
+      if (q0 + e * blockDim.x < R) add_to(r, v[e]);
+  }
   sh[threadIdx.x] = r;
   __syncthreads();
   for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+    if ((int)threadIdx.x < o) add_to(sh[threadIdx.x], sh[threadIdx.x + o]);
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[n] = sh[0];
+  if (threadIdx.x == 0) reinterpret_cast<V*>(out)[n] = sh[0];
 }
 
 // out[c][r] = in[r][c] for an R x Cc row-major BF16 matrix; out has leading
 // dimension ldo (>= R, extra columns zero-filled up to ldo).
 __global__ void k_transpose_bf16(int R, int Cc, const __nv_bfloat16* in, int ldi,
                                  __nv_bfloat16* out, int ldo) {
+  pdl_enter();
   __shared__ __nv_bfloat16 tile[32][33];
   const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
   for (int q = threadIdx.y; q < 32; q += blockDim.y) {
@@ -669,6 +929,7 @@ __global__ void k_transpose_bf16(int R, int Cc, const __nv_bfloat16* in, int ldi
 }
 
 __global__ void k_to_bf16(long long n, const float* x, __nv_bfloat16* y) {
+  pdl_enter();
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x)
     y[t] = __float2bfloat16(x[t]);
@@ -677,6 +938,7 @@ __global__ void k_to_bf16(long long n, const float* x, __nv_bfloat16* y) {
 // Nearest 2x upsampling along the width of an (nb, W, C) tensor (H = 1):
 // y[b, 2w + s, c] = x[b, w, c]; the backward sums the two copies.
 __global__ void k_upsample2(long long nb, int W, int C, const __nv_bfloat16* x, __nv_bfloat16* y) {
+  pdl_enter();
   const long long total = nb * 2 * W * C;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -687,6 +949,7 @@ __global__ void k_upsample2(long long nb, int W, int C, const __nv_bfloat16* x, 
 }
 
 __global__ void k_upsample2_bwd(long long nb, int W, int C, const float* dy, float* dx) {
+  pdl_enter();
   const long long total = nb * W * C;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -702,6 +965,7 @@ __global__ void k_upsample2_bwd(long long nb, int W, int C, const float* dy, flo
 // the other columns; per-block partial losses in fixed order.
 __global__ void k_mse(long long rows, int used, int ld, const float* y, const float* t,
                       float* grad, float* loss) {
+  pdl_enter();
   __shared__ float sh[256];
   const long long n = rows * ld;
   const float inv = 1.f / (float)(rows * used);
@@ -728,19 +992,80 @@ __global__ void k_mse(long long rows, int used, int ld, const float* y, const fl
 
 // Adam on FP32 master weights (bias-corrected, weight decay decoupled from
 // the gradient statistics), then the BF16 copy.
-__global__ void k_adam(long long n, float* w, const float* g, float* m, float* v, float lr,
-                       float b1, float b2, float eps, float c1, float c2, float wd,
-                       __nv_bfloat16* w16) {
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const float gt = g[t];
-    const float mt = b1 * m[t] + (1.f - b1) * gt;
-    const float vt = b2 * v[t] + (1.f - b2) * gt * gt;
-    m[t] = mt;
-    v[t] = vt;
-    const float wn = w[t] - lr * ((mt / c1) / (sqrtf(vt / c2) + eps) + wd * w[t]);
-    w[t] = wn;
-    if (w16) w16[t] = __float2bfloat16(wn);
+struct AdamCoef {
+  float lr, b1, b2, eps, c1, c2;
+};
+
+__device__ __forceinline__ float adam_one(const AdamCoef& a, float wd, float w, float gt, float& m,
+                                          float& v) {
+  const float mt = a.b1 * m + (1.f - a.b1) * gt;
+  const float vt = a.b2 * v + (1.f - a.b2) * gt * gt;
+  m = mt;
+  v = vt;
+  return w - a.lr * ((mt / a.c1) / (sqrtf(vt / a.c2) + a.eps) + wd * w);
+}
+
+// All tensors of a network in one launch: block b works on kAdamChunk
+// elements of the tensor whose block range holds b, four per thread as 16-byte
+// vectors where the tensor's arrays are aligned. Bound by memory (30 bytes an
+// element); a launch per tensor left 16 of 18 launches with a handful of
+// blocks: the 18 tensors of the network (1.8 million elements) 97 -> 19.5 us.
+constexpr int kAdamMax = 32, kAdamThreads = 256, kAdamChunk = 4 * kAdamThreads;
+struct AdamTable {
+  int count;
+  unsigned first[kAdamMax + 1];  // first block of each tensor
+  unsigned vec;                  // bit i: tensor i takes 16-byte vectors
+  pfs_adam_tensor t[kAdamMax];
+};
+
+__global__ void __launch_bounds__(kAdamThreads) k_adam(const __grid_constant__ AdamTable tab,
+                                                       AdamCoef a) {
+  pdl_enter();
+  int i = 0;
+  while (i + 1 < tab.count && blockIdx.x >= tab.first[i + 1]) ++i;
+  const pfs_adam_tensor& p = tab.t[i];
+  const long long base = (long long)(blockIdx.x - tab.first[i]) * kAdamChunk;
+  __nv_bfloat16* w16 = (__nv_bfloat16*)p.w16;
+  if ((tab.vec >> i) & 1) {
+    const long long t = base + 4 * threadIdx.x;
+    if (t + 4 <= p.n) {
+      float4 w = *reinterpret_cast<const float4*>(p.w + t);
+      const float4 g = *reinterpret_cast<const float4*>(p.g + t);
+      float4 m = *reinterpret_cast<const float4*>(p.m + t);
+      float4 v = *reinterpret_cast<const float4*>(p.v + t);
+      w.x = adam_one(a, p.wd, w.x, g.x, m.x, v.x);
+      w.y = adam_one(a, p.wd, w.y, g.y, m.y, v.y);
+      w.z = adam_one(a, p.wd, w.z, g.z, m.z, v.z);
+      w.w = adam_one(a, p.wd, w.w, g.w, m.w, v.w);
+      *reinterpret_cast<float4*>(p.m + t) = m;
+      *reinterpret_cast<float4*>(p.v + t) = v;
+      *reinterpret_cast<float4*>(p.w + t) = w;
+      if (w16) {
+        const __nv_bfloat16 h[4] = {__float2bfloat16(w.x), __float2bfloat16(w.y),
+                                    __float2bfloat16(w.z), __float2bfloat16(w.w)};
+        *reinterpret_cast<uint2*>(w16 + t) = *reinterpret_cast<const uint2*>(h);
+      }
+      return;
+    }
+    for (long long q = t; q < p.n; ++q) {  // the last, partial vector
+      float m = p.m[q], v = p.v[q];
+      const float w = adam_one(a, p.wd, p.w[q], p.g[q], m, v);
+      p.m[q] = m;
+      p.v[q] = v;
+      p.w[q] = w;
+      if (w16) w16[q] = __float2bfloat16(w);
+    }
+    return;
+  }
+  for (int e = 0; e < 4; ++e) {
+    const long long q = base + e * kAdamThreads + threadIdx.x;
+    if (q >= p.n) return;
+    float m = p.m[q], v = p.v[q];
+    const float w = adam_one(a, p.wd, p.w[q], p.g[q], m, v);
+    p.m[q] = m;
+    p.v[q] = v;
+    p.w[q] = w;
+    if (w16) w16[q] = __float2bfloat16(w);
   }
 }
 
@@ -791,20 +1116,20 @@ void tc_launch(int bn, dim3 grid, cudaStream_t st, const CUtensorMap& ta, const 
   switch (bn) {
     case 32:
       if constexpr (!BMN)
-        k_gemm_tc<32, AMN, BMN, EPI><<<grid, 128, tc_smem_bytes(32, ns), st>>>(
-            ta, tb, M, N, K, C, ldc, alpha, beta, kc, work, err, wt, ep, ns);
+        launch_pdl(st, grid, 128, tc_smem_bytes(32, ns), k_gemm_tc<32, AMN, BMN, EPI>, ta, tb, M,
+                   N, K, C, ldc, alpha, beta, kc, work, err, wt, ep, ns);
       break;
     case 64:
-      k_gemm_tc<64, AMN, BMN, EPI><<<grid, 128, tc_smem_bytes(64, ns), st>>>(
-          ta, tb, M, N, K, C, ldc, alpha, beta, kc, work, err, wt, ep, ns);
+      launch_pdl(st, grid, 128, tc_smem_bytes(64, ns), k_gemm_tc<64, AMN, BMN, EPI>, ta, tb, M, N,
+                 K, C, ldc, alpha, beta, kc, work, err, wt, ep, ns);
       break;
     case 128:
-      k_gemm_tc<128, AMN, BMN, EPI><<<grid, 128, tc_smem_bytes(128, ns), st>>>(
-          ta, tb, M, N, K, C, ldc, alpha, beta, kc, work, err, wt, ep, ns);
+      launch_pdl(st, grid, 128, tc_smem_bytes(128, ns), k_gemm_tc<128, AMN, BMN, EPI>, ta, tb, M,
+                 N, K, C, ldc, alpha, beta, kc, work, err, wt, ep, ns);
       break;
     default:
-      k_gemm_tc<256, AMN, BMN, EPI><<<grid, 128, tc_smem_bytes(256, ns), st>>>(
-          ta, tb, M, N, K, C, ldc, alpha, beta, kc, work, err, wt, ep, ns);
+      launch_pdl(st, grid, 128, tc_smem_bytes(256, ns), k_gemm_tc<256, AMN, BMN, EPI>, ta, tb, M,
+                 N, K, C, ldc, alpha, beta, kc, work, err, wt, ep, ns);
   }
 }
 
@@ -823,7 +1148,8 @@ int launch_gemm(int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv
   if (g_gemm_engine == 0) {
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, sz);
     if (grid.y > 65535) return sfail(PF_ERR_INVALID, "pfs_gemm: M too large");
-    k_gemm_bf16<<<grid, 128, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, kc, work);
+    launch_pdl(st, grid, 128, 0, k_gemm_bf16, M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, kc,
+               work);
     return PF_OK;
   }
   static int* err = nullptr;
@@ -847,10 +1173,23 @@ int launch_gemm(int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv
   if (kc % TBK) return sfail(PF_ERR_INVALID, "pfs_gemm: K slice not a multiple of 64");
   const long long gy = (M + TBM - 1) / TBM;
   if (gy > 65535) return sfail(PF_ERR_INVALID, "pfs_gemm: M too large");
-  // the narrowest tile that covers N, narrowed further (down to 32 columns)
-  // while the grid has fewer blocks than SMs
+  // The narrowest tile that covers N, narrowed further (down to 32 columns)
+  // while the grid has fewer blocks than SMs. A short K (two TMA stages or
+  // fewer) leaves the stores as the work: 128 columns let four blocks of
+  // tensor memory share an SM instead of two (131072 x 288, K = 64: 49.2 us
+  // at 256, 38.9 at 128, 41.0 at 64; K = 256, 8192 x 1152: 28.7 against 30.7
+  // with the line there). And where the grid runs over into a second wave of
+  // a few blocks that the next narrower tile would not need, that tile (64 x
+  // 288, 59 slices of K: 177 blocks of 128 columns on 148 SMs 53.3 us, 295
+  // of 64 columns, two per SM, 35.8).
   int bn = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256;
-  while (bn > 32 && gy * ((N + bn - 1) / bn) * sz < 148) bn /= 2;
+  auto blocks = [&](int w) { return gy * ((N + w - 1) / w) * sz; };
+  auto slots = [&](int w) {
+    return 148LL * std::min(512 / w, kTcSmemSm / tc_smem_bytes(w, tc_ring_stages(kc)));
+  };
+  while (bn > 32 && blocks(bn) < 148) bn /= 2;
+  if (kc <= 2 * TBK && bn > 128) bn = 128;
+  if (bn > 64 && blocks(bn) > slots(bn) && blocks(bn / 2) <= slots(bn / 2)) bn /= 2;
   if (b_mn && bn < 64) bn = 64;  // an MN-major B is loaded in 64-wide strips
   CUtensorMap ta, tb;
   // K-major: rows of K elements, box 64 (K) x tile rows; MN-major: rows of
@@ -956,8 +1295,8 @@ int pfs_gemm_bf16_splitk(int M, int N, int K, const void* A, int lda, const void
     rc = launch_gemm(M, N, K, (const __nv_bfloat16*)A, lda, (const __nv_bfloat16*)B, ldb, C, ldc,
                      alpha, beta, kc, sz, work, st);
     if (!rc)
-      k_splitk_reduce<<<grid_for((long long)M * N, 256), 256, 0, st>>>(M, N, sz, work, C, ldc,
-                                                                        beta);
+      launch_pdl(st, grid_for((long long)M * N, 256), 256, 0, k_splitk_reduce, M, N, sz, work, C,
+                 ldc, beta);
   }
   if (rc) return rc;
   return cuda_status("pfs_gemm_bf16_splitk");
@@ -988,7 +1327,8 @@ int pfs_gemm_bf16_ex(int M, int N, int K, const void* A, int lda, int a_mn, cons
                        ldc, alpha, beta, sz == 1 ? K : kc, sz, sz == 1 ? nullptr : work, st,
                        a_mn != 0, b_mn != 0);
   if (!rc && sz > 1)
-    k_splitk_reduce<<<grid_for((long long)M * N, 256), 256, 0, st>>>(M, N, sz, work, C, ldc, beta);
+    launch_pdl(st, grid_for((long long)M * N, 256), 256, 0, k_splitk_reduce, M, N, sz, work, C,
+                 ldc, beta);
   if (rc) return rc;
   return cuda_status("pfs_gemm_bf16_ex");
 }
@@ -1023,18 +1363,16 @@ int pfs_im2col(int nb, int H, int W, int C, int kh, int kw, int stride, int ph, 
   const long long n = (long long)nb * Ho * Wo * Kp;
   cudaStream_t st = (cudaStream_t)stream;
   if (Kp % 8 == 0 && n / 8 < (1LL << 31) && aligned16(col)) {
-    const int rows = nb * Ho * Wo;
-    if (C % 8 == 0 && aligned16(x))
-      k_im2col8<true><<<grid_for(n / 8, 256), 256, 0, st>>>(rows, H, W, C, kh, kw, stride, ph, pw,
-                                                           Ho, Wo, (const __nv_bfloat16*)x,
-                                                           (__nv_bfloat16*)col, Kp);
-    else
-      k_im2col8<false><<<grid_for(n / 8, 256), 256, 0, st>>>(rows, H, W, C, kh, kw, stride, ph,
-                                                            pw, Ho, Wo, (const __nv_bfloat16*)x,
-                                                            (__nv_bfloat16*)col, Kp);
+    const int rows = nb * Ho * Wo, qn = Kp / 8;
+    const bool vec = C % 8 == 0 && aligned16(x);
+    const int cpt = !vec && qn <= kRowChunks ? qn : 1;
+    const ConvDivs dv{make_div(qn / cpt), make_div(Wo), make_div(Ho), make_div(C), make_div(kw)};
+    launch_pdl(st, grid_for(n / 8 / cpt, 256), 256, 0, vec ? k_im2col8<true> : k_im2col8<false>,
+               rows, H, W, C, kh, kw, stride, ph, pw, Ho, Wo, (const __nv_bfloat16*)x,
+               (__nv_bfloat16*)col, Kp, dv, cpt);
   } else {
-    k_im2col<<<grid_for(n, 256), 256, 0, st>>>(nb, H, W, C, kh, kw, stride, ph, pw, Ho, Wo,
-                                               (const __nv_bfloat16*)x, (__nv_bfloat16*)col, Kp);
+    launch_pdl(st, grid_for(n, 256), 256, 0, k_im2col, nb, H, W, C, kh, kw, stride, ph, pw, Ho, Wo,
+               (const __nv_bfloat16*)x, (__nv_bfloat16*)col, Kp);
   }
   return cuda_status("pfs_im2col");
 }
@@ -1050,19 +1388,23 @@ int pfs_col2im(int nb, int H, int W, int C, int kh, int kw, int stride, int ph, 
   cudaStream_t st = (cudaStream_t)stream;
   if (C % 8 == 0 && Kp % 4 == 0 && n < (1LL << 31) && (long long)nb * Ho * Wo * Kp < (1LL << 31) &&
       aligned16(dcol) && aligned16(dx))
-    k_col2im8<<<grid_for(n / 8, 256), 256, 0, st>>>(nb, H, W, C, kh, kw, stride, ph, pw, Ho, Wo,
-                                                    dcol, Kp, dx);
+    launch_pdl(st, grid_for(n / 8, 256), 256, 0,
+               (kh + stride - 1) / stride <= 2 && (kw + stride - 1) / stride <= 2
+                   ? k_col2im8<true>
+                   : k_col2im8<false>,
+               nb, H, W, C, kh, kw, stride, ph, pw, Ho, Wo, dcol, Kp, dx,
+               ColDivs{make_div(C / 8), make_div(W), make_div(H), make_div(stride)});
   else
-    k_col2im<<<grid_for(n, 256), 256, 0, st>>>(nb, H, W, C, kh, kw, stride, ph, pw, Ho, Wo, dcol,
-                                               Kp, dx);
+    launch_pdl(st, grid_for(n, 256), 256, 0, k_col2im, nb, H, W, C, kh, kw, stride, ph, pw, Ho, Wo,
+               dcol, Kp, dx);
   return cuda_status("pfs_col2im");
 }
 
 int pfs_bias_act(int64_t M, int N, const float* x, const float* bias, int relu, float* y32,
                  void* y16, void* stream) {
   if (M < 0 || N < 1 || !x || (!y32 && !y16)) return sfail(PF_ERR_INVALID, "pfs_bias_act: bad arguments");
-  k_bias_act<<<grid_for(M * N, 256), 256, 0, (cudaStream_t)stream>>>(M, N, x, bias, relu, y32,
-                                                                     (__nv_bfloat16*)y16);
+  launch_pdl((cudaStream_t)stream, grid_for(M * N, 256), 256, 0, k_bias_act, M, N, x, bias, relu,
+             y32, (__nv_bfloat16*)y16);
   return cuda_status("pfs_bias_act");
 }
 
@@ -1071,9 +1413,22 @@ int pfs_act_bwd(int64_t M, int N, const float* dy, const float* y, int relu, flo
   if (M < 1 || N < 1 || !dy || (relu && !y) || row_blocks < 1 || row_blocks > 65535 ||
       (dbias && !part))
     return sfail(PF_ERR_INVALID, "pfs_act_bwd: bad arguments");
-  k_act_bwd<<<dim3((N + 31) / 32, row_blocks), dim3(32, 8), 0, (cudaStream_t)stream>>>(
-      M, N, dy, y, relu, d32, (__nv_bfloat16*)d16, dbias ? part : nullptr);
-  if (dbias) k_colsum<<<N, 256, 0, (cudaStream_t)stream>>>(row_blocks, N, part, dbias);
+  const bool vec = N % 4 == 0 && aligned16(dy) && (!relu || aligned16(y)) && aligned16(d32) &&
+                   ((uintptr_t)d16 & 7) == 0 && (!dbias || aligned16(part));
+  cudaStream_t st = (cudaStream_t)stream;
+  if (vec)
+    launch_pdl(st, dim3((N + 31) / 32, (row_blocks + kActBlocks - 1) / kActBlocks),
+               dim3(8, 8, kActBlocks), 0, k_act_bwd4, M, N, dy, y, relu, d32, (__nv_bfloat16*)d16,
+               dbias ? part : nullptr, row_blocks);
+  else
+    launch_pdl(st, dim3((N + 31) / 32, row_blocks), dim3(32, 8), 0, k_act_bwd, M, N, dy, y, relu,
+               d32, (__nv_bfloat16*)d16, dbias ? part : nullptr);
+  if (dbias) {
+    if (N % 4 == 0 && aligned16(part) && aligned16(dbias))
+      launch_pdl(st, N / 4, 256, 0, k_colsum<float4>, row_blocks, N, part, dbias);
+    else
+      launch_pdl(st, N, 256, 0, k_colsum<float>, row_blocks, N, part, dbias);
+  }
   return cuda_status("pfs_act_bwd");
 }
 
@@ -1081,28 +1436,29 @@ int pfs_transpose_bf16(int R, int Cc, const void* in, int ldi, void* out, int ld
   if (R < 1 || Cc < 1 || !in || !out || ldi < Cc || ldo < R)
     return sfail(PF_ERR_INVALID, "pfs_transpose_bf16: bad arguments");
   const int rows = (ldo + 31) / 32;  // cover the zero fill up to ldo
-  k_transpose_bf16<<<dim3((Cc + 31) / 32, rows), dim3(32, 8), 0, (cudaStream_t)stream>>>(
-      R, Cc, (const __nv_bfloat16*)in, ldi, (__nv_bfloat16*)out, ldo);
+  launch_pdl((cudaStream_t)stream, dim3((Cc + 31) / 32, rows), dim3(32, 8), 0, k_transpose_bf16, R,
+             Cc, (const __nv_bfloat16*)in, ldi, (__nv_bfloat16*)out, ldo);
   return cuda_status("pfs_transpose_bf16");
 }
 
 int pfs_to_bf16(int64_t n, const float* x, void* y, void* stream) {
   if (n < 0 || (n && (!x || !y))) return sfail(PF_ERR_INVALID, "pfs_to_bf16: bad arguments");
   if (!n) return PF_OK;
-  k_to_bf16<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(n, x, (__nv_bfloat16*)y);
+  launch_pdl((cudaStream_t)stream, grid_for(n, 256), 256, 0, k_to_bf16, n, x, (__nv_bfloat16*)y);
   return cuda_status("pfs_to_bf16");
 }
 
 int pfs_upsample2(int64_t nb, int W, int C, const void* x, void* y, void* stream) {
   if (nb < 1 || W < 1 || C < 1 || !x || !y) return sfail(PF_ERR_INVALID, "pfs_upsample2: bad arguments");
-  k_upsample2<<<grid_for(nb * 2 * W * C, 256), 256, 0, (cudaStream_t)stream>>>(
-      nb, W, C, (const __nv_bfloat16*)x, (__nv_bfloat16*)y);
+  launch_pdl((cudaStream_t)stream, grid_for(nb * 2 * W * C, 256), 256, 0, k_upsample2, nb, W, C,
+             (const __nv_bfloat16*)x, (__nv_bfloat16*)y);
   return cuda_status("pfs_upsample2");
 }
 
 int pfs_upsample2_bwd(int64_t nb, int W, int C, const float* dy, float* dx, void* stream) {
   if (nb < 1 || W < 1 || C < 1 || !dy || !dx) return sfail(PF_ERR_INVALID, "pfs_upsample2_bwd: bad arguments");
-  k_upsample2_bwd<<<grid_for(nb * W * C, 256), 256, 0, (cudaStream_t)stream>>>(nb, W, C, dy, dx);
+  launch_pdl((cudaStream_t)stream, grid_for(nb * W * C, 256), 256, 0, k_upsample2_bwd, nb, W, C,
+             dy, dx);
   return cuda_status("pfs_upsample2_bwd");
 }
 
@@ -1110,17 +1466,45 @@ int pfs_mse(int64_t rows, int used, int ld, const float* y, const float* t, floa
             float* loss_parts, int nparts, void* stream) {
   if (rows < 1 || used < 1 || ld < used || !y || !t || !grad || !loss_parts || nparts < 1)
     return sfail(PF_ERR_INVALID, "pfs_mse: bad arguments");
-  k_mse<<<nparts, 256, 0, (cudaStream_t)stream>>>(rows, used, ld, y, t, grad, loss_parts);
+  launch_pdl((cudaStream_t)stream, nparts, 256, 0, k_mse, rows, used, ld, y, t, grad, loss_parts);
   return cuda_status("pfs_mse");
+}
+
+int pfs_adam_many(int count, const pfs_adam_tensor* tensors, float lr, float b1, float b2,
+                  float eps, int step, void* stream) {
+  if (count < 1 || !tensors || step < 1) return sfail(PF_ERR_INVALID, "pfs_adam: bad arguments");
+  for (int i = 0; i < count; ++i) {
+    const pfs_adam_tensor& t = tensors[i];
+    if (t.n < 1 || !t.w || !t.g || !t.m || !t.v)
+      return sfail(PF_ERR_INVALID, "pfs_adam: bad arguments");
+    if ((t.n + kAdamChunk - 1) / kAdamChunk > 0x7fffffffLL / kAdamMax)
+      return sfail(PF_ERR_INVALID, "pfs_adam: tensor too large");
+  }
+  const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
+  const AdamCoef a{lr, b1, b2, eps, c1, c2};
+  for (int i0 = 0; i0 < count; i0 += kAdamMax) {
+    AdamTable tab = {};
+    tab.count = count - i0 < kAdamMax ? count - i0 : kAdamMax;
+    unsigned blocks = 0;
+    for (int i = 0; i < tab.count; ++i) {
+      const pfs_adam_tensor& t = tensors[i0 + i];
+      tab.t[i] = t;
+      tab.first[i] = blocks;
+      blocks += (unsigned)((t.n + kAdamChunk - 1) / kAdamChunk);
+      if (aligned16(t.w) && aligned16(t.g) && aligned16(t.m) && aligned16(t.v) &&
+          ((uintptr_t)t.w16 & 7) == 0)
+        tab.vec |= 1u << i;
+    }
+    tab.first[tab.count] = blocks;
+    launch_pdl((cudaStream_t)stream, blocks, kAdamThreads, 0, k_adam, tab, a);
+  }
+  return cuda_status("pfs_adam");
 }
 
 int pfs_adam(int64_t n, float* w, const float* g, float* m, float* v, float lr, float b1, float b2,
              float eps, int step, float wd, void* w16, void* stream) {
-  if (n < 1 || !w || !g || !m || !v || step < 1) return sfail(PF_ERR_INVALID, "pfs_adam: bad arguments");
-  const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-  k_adam<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(n, w, g, m, v, lr, b1, b2, eps, c1,
-                                                             c2, wd, (__nv_bfloat16*)w16);
-  return cuda_status("pfs_adam");
+  const pfs_adam_tensor t{n, w, g, m, v, w16, wd};
+  return pfs_adam_many(1, &t, lr, b1, b2, eps, step, stream);
 }
 
 }  // extern "C"

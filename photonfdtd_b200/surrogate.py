@@ -364,15 +364,17 @@ class SurrogateNet:
                   wd: float = 0.0) -> None:
         self.step_count += 1
         L_, s = self.L, self._s()
+        tensors = []
         for li, L in enumerate(self.layers):
             if L.kind == "up":
                 continue
-            self._chk(L_.pfs_adam(self.w32[li].numel(), self._p(self.w32[li]), self._p(self.gw[li]),
-                                  self._p(self.m_w[li]), self._p(self.v_w[li]), lr, b1, b2, eps,
-                                  self.step_count, wd, self._p(self.w16[li]), s))
-            self._chk(L_.pfs_adam(self.b32[li].numel(), self._p(self.b32[li]), self._p(self.gb[li]),
-                                  self._p(self.m_b[li]), self._p(self.v_b[li]), lr, b1, b2, eps,
-                                  self.step_count, 0.0, 0, s))
+            tensors.append((self.w32[li].numel(), self._p(self.w32[li]), self._p(self.gw[li]),
+                            self._p(self.m_w[li]), self._p(self.v_w[li]), self._p(self.w16[li]),
+                            wd))
+            tensors.append((self.b32[li].numel(), self._p(self.b32[li]), self._p(self.gb[li]),
+                            self._p(self.m_b[li]), self._p(self.v_b[li]), 0, 0.0))
+        self._chk(L_.pfs_adam_many(len(tensors), (N.AdamTensor * len(tensors))(*tensors), lr, b1,
+                                   b2, eps, self.step_count, s))
 
     # ---- parameters ---------------------------------------------------- #
     def params(self) -> List[Tuple[np.ndarray, np.ndarray]]:
