@@ -47,8 +47,8 @@ extern "C" {
 #define PF_CE_TABLE 2 /* per-cell uint32 word indexing a coefficient table */
 
 /* Stepping kernels (pf_set_kernel). */
-#define PF_KERNEL_AUTO 0  /* the faster path for the grid (split on B200) */
-#define PF_KERNEL_SPLIT 1 /* separate H and E passes, one thread per cell  */
+#define PF_KERNEL_AUTO 0  /* the faster path for the grid (H, E passes)    */
+#define PF_KERNEL_SPLIT 1 /* separate H and E passes (small grids: in one launch) */
 #define PF_KERNEL_FUSED 2 /* require the fused H+E pass (3D only)          */
 
 typedef struct pf_engine pf_engine;
