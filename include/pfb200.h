@@ -193,9 +193,11 @@ int pf_write_field(pf_engine *eng, int comp, const void *host_src);
  * size; pf_get_state copies it out (dst_on_device != 0: dst is a device
  * pointer); pf_set_state copies it in and sets the step counter to `step`
  * (the state is taken to be the one reached after `step` steps; pending
- * monitor samples are folded first). This is the checkpoint pair of a
- * time-reversed pass: the reference's gradient path keeps the same quantities
- * between remat segments (src/photonfdtd/jaxbackend.py:511-570). */
+ * monitor samples are folded first, and the accumulators keep what they hold:
+ * steps taken again are added again, with their own phases). This is the
+ * checkpoint pair of a time-reversed pass: the reference's gradient path keeps
+ * the same quantities between remat segments
+ * (src/photonfdtd/jaxbackend.py:511-570). */
 int pf_state_bytes(const pf_engine *eng, int64_t *bytes);
 int pf_get_state(pf_engine *eng, void *dst, int64_t bytes, int dst_on_device);
 int pf_set_state(pf_engine *eng, int64_t step, const void *src, int64_t bytes,

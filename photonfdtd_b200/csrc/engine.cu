@@ -1844,6 +1844,8 @@ int pf_set_state(pf_engine* e, int64_t step, const void* src, int64_t bytes, int
   rc = copy_state(e, step, const_cast<void*>(src), bytes, src_on_device, false);
   if (rc) return rc;
   e->step = step;
+  // the phase rows follow the step, not the count of samples taken so far
+  for (DftMon& m : e->dfts) m.q_done = (step + m.interval - 1) / m.interval;
   return PF_OK;
 }
 
