@@ -149,7 +149,7 @@ struct pf_engine {
   double* wave = nullptr;
   int* flag = nullptr;
   unsigned* res_bar = nullptr;  // resident launches: grid barrier, error (mapped host memory)
-  int* res_err = nullptr;
+  ErrWord res_err;
   bool flux_kept = false;  // the pending flux samples are kept values, not partials
   int sms = 0;
   void* region = nullptr;     // pf_read_region staging buffer (grown on demand)
@@ -960,29 +960,6 @@ int record_step(pf_engine* e, long long t) {
 // 96^3 33 / 33, float64 88^3 32 / 40, 96^3 43 / 41.
 constexpr long long kResN2 = 3000000, kResN3 = 700000;
 
-// Error words of resident launches: mapped host memory, so that reading one
-// costs no copy. One page serves 1024 engines (pinning memory per engine took
-// longer than a small run); pages are kept for the process.
-std::mutex g_err_mu;
-std::vector<int*> g_err_free;
-int* err_word() {
-  std::lock_guard<std::mutex> lk(g_err_mu);
-  if (g_err_free.empty()) {
-    int* page = nullptr;
-    if (cudaHostAlloc((void**)&page, 4096, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess)
-      return nullptr;
-    for (int q = 0; q < 1024; ++q) g_err_free.push_back(page + q);
-  }
-  int* w = g_err_free.back();
-  g_err_free.pop_back();
-  *w = 0;
-  return w;
-}
-void err_word_release(int* w) {
-  std::lock_guard<std::mutex> lk(g_err_mu);
-  g_err_free.push_back(w);
-}
-
 // Engines of this process inside pf_advance now. A cooperative grid takes the
 // whole chip, so engines stepped concurrently (24 scenes of 40^3 to 96^3:
 // 0.46 s with separate launches, 1.44 s with grids waiting for one another)
@@ -1096,11 +1073,11 @@ int launch_resident(pf_engine* e, long long n, long long* took) {
   if (!e->res_bar) {
     int rc = dalloc(e, (void**)&e->res_bar, sizeof(unsigned));
     if (rc) return rc;
-    e->res_err = err_word();
-    if (!e->res_err) return fail(e, PF_ERR_OOM, "no pinned host memory for an error word");
+    e->res_err = err_word(e->device, e->stream);
+    if (!e->res_err.p) return fail(e, PF_ERR_OOM, "no pinned host memory for an error word");
   }
   g.bar = e->res_bar;
-  PF_CUDA(e, cudaHostGetDevicePointer((void**)&g.err, e->res_err, 0));
+  PF_CUDA(e, cudaHostGetDevicePointer((void**)&g.err, e->res_err.p, 0));
   const bool ade = e->n_media > 0;
   int rc;
   switch (e->ce_mode) {
@@ -1243,7 +1220,7 @@ int advance_typed(pf_engine* e, long long n_sub) {
     if (h == 2) return fail(e, PF_ERR_CUDA, "TMA staging buffer misaligned; results are invalid");
     if (h) return fail(e, PF_ERR_TIMEOUT, "a TMA stage wait timed out; results are invalid");
   }
-  if (e->res_err && *(volatile int*)e->res_err)
+  if (e->res_err.p && *(volatile int*)e->res_err.p)
     return fail(e, PF_ERR_TIMEOUT, "a grid barrier timed out; results are invalid");
   return PF_OK;
 }
@@ -1254,17 +1231,52 @@ bool valid_comp(int c) { return c >= 0 && c < 6; }
 
 namespace pfb {
 namespace {
-std::mutex g_pool_mu;
-std::map<int, cudaMemPool_t> g_pools;  // per device, kept for the process
-}  // namespace
+struct DeviceKeep {
+  unsigned long long ctx = 0;  // id of the context that the rest belongs to
+  cudaMemPool_t pool = nullptr;
+  std::vector<int*> err_free;
+};
+std::mutex g_keep_mu;
+std::map<int, DeviceKeep> g_keep;  // per device
 
-namespace {
-// The pool of a device, made on first use; fresh: replace the one there (a
-// device reset took it).
-cudaMemPool_t device_pool(int dev, bool fresh) {
-  std::lock_guard<std::mutex> lk(g_pool_mu);
-  auto it = g_pools.find(dev);
-  if (it != g_pools.end() && !fresh) return it->second;
+// Id of a live stream's context, 0 if the driver does not tell.
+unsigned long long context_id(cudaStream_t st) {
+  typedef CUresult (*StreamCtxFn)(CUstream, CUcontext*);
+  typedef CUresult (*CtxIdFn)(CUcontext, unsigned long long*);
+  static const auto entry = [](const char* name) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    // by version: later forms of cuStreamGetCtx take another argument
+    const bool ok = cudaGetDriverEntryPointByVersion(name, &p, 12000, cudaEnableDefault, &q) ==
+                        cudaSuccess && q == cudaDriverEntryPointSuccess;
+    return ok ? p : nullptr;
+  };
+  static const auto stream_ctx = (StreamCtxFn)entry("cuStreamGetCtx");
+  static const auto ctx_id = (CtxIdFn)entry("cuCtxGetId");
+  CUcontext c = nullptr;
+  unsigned long long id = 0;
+  if (!stream_ctx || !ctx_id || stream_ctx((CUstream)st, &c) != CUDA_SUCCESS ||
+      ctx_id(c, &id) != CUDA_SUCCESS)
+    return 0;
+  return id;
+}
+
+// What is kept for the context (g_keep_mu held); that of an earlier context
+// of the device is dropped.
+DeviceKeep* keep_of(int dev, unsigned long long ctx) {
+  if (!ctx) return nullptr;
+  DeviceKeep& k = g_keep[dev];
+  if (k.ctx != ctx) {
+    k = DeviceKeep{};
+    k.ctx = ctx;
+  }
+  return &k;
+}
+
+cudaMemPool_t device_pool(int dev, cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(g_keep_mu);
+  DeviceKeep* k = keep_of(dev, context_id(st));
+  if (!k || k->pool) return k ? k->pool : nullptr;
   cudaMemPoolProps props = {};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
@@ -1276,14 +1288,39 @@ cudaMemPool_t device_pool(int dev, bool fresh) {
   }
   unsigned long long keep = kPoolKeep;
   cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-  g_pools[dev] = pool;
+  k->pool = pool;
   return pool;
 }
 }  // namespace
 
+ErrWord err_word(int dev, cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(g_keep_mu);
+  DeviceKeep* k = keep_of(dev, context_id(st));
+  if (!k) return {};
+  if (k->err_free.empty()) {
+    int* page = nullptr;
+    if (cudaHostAlloc((void**)&page, 4096, cudaHostAllocMapped | cudaHostAllocPortable) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return {};
+    }
+    for (int q = 0; q < 1024; ++q) k->err_free.push_back(page + q);
+  }
+  ErrWord w{k->err_free.back(), k->ctx};
+  k->err_free.pop_back();
+  *w.p = 0;
+  return w;
+}
+
+void err_word_release(int dev, const ErrWord& w) {
+  std::lock_guard<std::mutex> lk(g_keep_mu);
+  const auto it = g_keep.find(dev);
+  if (w.p && it != g_keep.end() && it->second.ctx == w.ctx) it->second.err_free.push_back(w.p);
+}
+
 cudaError_t pool_alloc(void** p, size_t bytes, int dev, cudaStream_t st) {
   *p = nullptr;
-  cudaMemPool_t pool = device_pool(dev, false);
+  cudaMemPool_t pool = device_pool(dev, st);
   cudaError_t rc = pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaErrorMemoryAllocation;
   if (rc == cudaErrorMemoryAllocation && pool) {
     cudaGetLastError();
@@ -1291,10 +1328,6 @@ cudaError_t pool_alloc(void** p, size_t bytes, int dev, cudaStream_t st) {
     cudaStreamSynchronize(st);
     cudaMemPoolTrimTo(pool, 0);
     rc = cudaMallocFromPoolAsync(p, bytes, pool, st);
-  } else if (rc == cudaErrorInvalidValue) {
-    cudaGetLastError();
-    pool = device_pool(dev, true);
-    rc = pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaErrorMemoryAllocation;
   }
   if (rc != cudaSuccess) {
     cudaGetLastError();
@@ -1926,7 +1959,7 @@ void pf_destroy(pf_engine* e) {
   for (void* p : e->allocs) pool_free(p, e->stream);
   if (e->region) pool_free(e->region, e->stream);
   if (e->stream) cudaStreamSynchronize(e->stream);
-  if (e->res_err) err_word_release(e->res_err);
+  err_word_release(e->device, e->res_err);
   for (cudaEvent_t ev : e->ev_pool) cudaEventDestroy(ev);
   if (e->stream) cudaStreamDestroy(e->stream);
   delete e;
