@@ -275,7 +275,10 @@ int pf_set_check_every(pf_engine *eng, int64_t k);
  * barrier that nothing arrives on, with a short limit, so the wait runs out
  * and the block takes its timeout path (it lets its issued copies land, sets
  * the error flag and leaves); pf_advance then returns PF_ERR_TIMEOUT and the
- * fields are invalid. No counterpart in the reference. */
+ * fields are invalid. on == 2: the engine finds that its context has no room
+ * for resident launches (many steps per launch of a small grid) and launches
+ * every pass by itself; results are the same. No counterpart in the
+ * reference. */
 int pf_set_wait_test(pf_engine *eng, int on);
 
 /* The CUDA stream (a cudaStream_t) the engine launches on, so a caller can

@@ -150,6 +150,8 @@ struct pf_engine {
   int* flag = nullptr;
   unsigned* res_bar = nullptr;  // resident launches: grid barrier, error (mapped host memory)
   ErrWord res_err;
+  bool res_asked = false;       // resident launches fit this context
+  bool res_off = false;         // they do not
   bool flux_kept = false;  // the pending flux samples are kept values, not partials
   int sms = 0;
   void* region = nullptr;     // pf_read_region staging buffer (grown on demand)
@@ -160,7 +162,7 @@ struct pf_engine {
   bool tma = false;      // fused path stages planes with TMA
   TmaMaps maps;
   int* tma_err = nullptr;
-  int wait_test = 0;     // pf_set_wait_test: one TMA stage wait runs out
+  int wait_test = 0;     // pf_set_wait_test: 1 one TMA stage wait runs out, 2 no resident launches
   long long check_every = 0;  // pf_set_check_every: non-finite scan period
   int fused_ty = 8;      // fused tile height (8 or 16), env PFB200_FUSED_TY
   int fused_chunks = 0;  // x chunks per column (0 = auto), env PFB200_XCHUNKS
@@ -683,7 +685,7 @@ StepArgs<T> step_args(pf_engine* e) {
   a.P = (T*)e->P;
   a.plev = e->plev;
   a.lvl = (int)(e->step & 1);
-  a.wait_test = e->wait_test;
+  a.wait_test = e->wait_test == 1;
   return a;
 }
 
@@ -973,6 +975,12 @@ struct Advancing {
 };
 constexpr long long kResChunk = 512;
 
+// Not a status of the ABI: this engine cannot have resident launches (a context
+// with fewer SMs than the grid or cluster needs, or no memory for what they
+// take besides). Nothing was launched or counted; its steps go on as separate
+// launches.
+constexpr int kResRefused = -1;
+
 template <typename T, int CE, bool ADE, int MODE>
 int launch_resident_as(pf_engine* e, const ResidentArgs<T>& g) {
   const auto fn = k_resident<T, CE, ADE, MODE>;
@@ -996,10 +1004,31 @@ int launch_resident_as(pf_engine* e, const ResidentArgs<T>& g) {
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
     cfg.gridDim = dim3(std::min(want, e->sms * res_blocks<T>(MODE)));
-    PF_CUDA(e, cudaMemsetAsync(g.bar, 0, sizeof(unsigned), e->stream));
   }
-  LaunchScope ls(e, 0);
-  PF_CUDA(e, cudaLaunchKernelEx(&cfg, fn, g));
+  if (!e->res_asked) {  // once per engine: the launches of a run differ in nothing that counts
+    int fit = 0;
+    cudaError_t rc;
+    if (MODE == kResCell1) {
+      rc = cudaOccupancyMaxActiveClusters(&fit, fn, &cfg);
+    } else {
+      rc = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, thr, 0);
+      fit = fit * e->sms >= (int)cfg.gridDim.x;
+    }
+    if (rc != cudaSuccess || fit < 1 || e->wait_test == 2) {
+      cudaGetLastError();
+      return kResRefused;
+    }
+    e->res_asked = true;
+  }
+  if (MODE != kResCell1) PF_CUDA(e, cudaMemsetAsync(g.bar, 0, sizeof(unsigned), e->stream));
+  const cudaError_t rc = cudaLaunchKernelEx(&cfg, fn, g);
+  if (rc == cudaErrorCooperativeLaunchTooLarge || rc == cudaErrorInvalidClusterSize ||
+      rc == cudaErrorLaunchOutOfResources) {
+    cudaGetLastError();
+    return kResRefused;
+  }
+  PF_CUDA(e, rc);
+  e->launches[0]++;
   return PF_OK;
 }
 
@@ -1030,7 +1059,7 @@ bool resident_small(const pf_engine* e) {
 }
 template <typename T>
 bool resident_ok(const pf_engine* e) {
-  return resident_small<T>(e) && !e->recording && !e->profiling &&
+  return resident_small<T>(e) && !e->recording && !e->profiling && !e->res_off &&
          (g_advancing.load() == 1 || resident_mode<T>(e) == kResCell1);
 }
 
@@ -1056,26 +1085,18 @@ int launch_resident(pf_engine* e, long long n, long long* took) {
     g.dft_ring[q] = (T*)m.ring;
     g.dft_slot[q] = m.pending;
     g.dft_interval[q] = m.interval;
-    if (due(m) < s + n) m.pending += (int)((s + n - 1 - due(m)) / m.interval + 1);
   }
-  e->flux_kept = !e->fluxes.empty();
   for (FluxMon& f : e->fluxes) {
     const int q = g.n_flux++;
-    if (!f.val) {
-      int rc = dalloc(e, &f.val, (size_t)f.ring_cap * f.p.n0 * f.p.n1 * sizeof(T));
-      if (rc) return rc;
-    }
+    if (!f.val && dalloc(e, &f.val, (size_t)f.ring_cap * f.p.n0 * f.p.n1 * sizeof(T)))
+      return kResRefused;
     g.flux[q] = f.p;
     g.flux_val[q] = (T*)f.val;
     g.flux_slot[q] = f.pending;
-    f.pending += (int)n;
   }
-  if (!e->res_bar) {
-    int rc = dalloc(e, (void**)&e->res_bar, sizeof(unsigned));
-    if (rc) return rc;
-    e->res_err = err_word(e->device, e->stream);
-    if (!e->res_err.p) return fail(e, PF_ERR_OOM, "no pinned host memory for an error word");
-  }
+  if (!e->res_bar && dalloc(e, (void**)&e->res_bar, sizeof(unsigned))) return kResRefused;
+  if (!e->res_err.p) e->res_err = err_word(e->device, e->stream);
+  if (!e->res_err.p) return kResRefused;
   g.bar = e->res_bar;
   PF_CUDA(e, cudaHostGetDevicePointer((void**)&g.err, e->res_err.p, 0));
   const bool ade = e->n_media > 0;
@@ -1092,12 +1113,18 @@ int launch_resident(pf_engine* e, long long n, long long* took) {
       rc = ade ? launch_resident_mode<T, kCeTable, true>(e, g)
                : launch_resident_mode<T, kCeTable, false>(e, g);
   }
+  if (rc) return rc;
+  for (DftMon& m : e->dfts)
+    if (due(m) < s + n) m.pending += (int)((s + n - 1 - due(m)) / m.interval + 1);
+  for (FluxMon& f : e->fluxes) f.pending += (int)n;
+  e->flux_kept = !e->fluxes.empty();
   *took = n;
   e->step += n;
-  return rc;
+  return PF_OK;
 }
 
-// Resident launches for up to n steps (at most kResChunk); *took: steps taken.
+// Resident launches for up to n steps (at most kResChunk); *took: steps taken,
+// fewer if a launch was refused.
 template <typename T>
 int advance_resident(pf_engine* e, long long n, long long* took) {
   *took = 0;
@@ -1110,7 +1137,12 @@ int advance_resident(pf_engine* e, long long n, long long* took) {
     if (full && (rc = flush_monitors<T>(e))) return rc;
     long long k = n - *took;
     if (e->check_every > 0) k = std::min(k, e->check_every - e->step % e->check_every);
-    if ((rc = launch_resident<T>(e, k, &k))) return rc;
+    rc = launch_resident<T>(e, k, &k);
+    if (rc == kResRefused) {
+      e->res_off = true;
+      return PF_OK;
+    }
+    if (rc) return rc;
     *took += k;
     if (e->check_every > 0 && e->step % e->check_every == 0) {
       PF_CUDA(e, cudaGetLastError());
@@ -1904,7 +1936,8 @@ int pf_set_check_every(pf_engine* e, int64_t k) {
 
 int pf_set_wait_test(pf_engine* e, int on) {
   if (!e) return PF_ERR_INVALID;
-  e->wait_test = on ? 1 : 0;
+  e->wait_test = on == 2 ? 2 : (on ? 1 : 0);
+  e->res_asked = e->res_off = false;
   return PF_OK;
 }
 
