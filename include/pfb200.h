@@ -270,15 +270,17 @@ int pf_check_finite(pf_engine *eng);
  * reference has no such check. */
 int pf_set_check_every(pf_engine *eng, int64_t k);
 
-/* Test hook of the TMA-staged fused step (PF_KERNEL_FUSED where the grid
- * allows TMA): with on != 0, block (0, 0, 0) of every step waits once on a
- * barrier that nothing arrives on, with a short limit, so the wait runs out
- * and the block takes its timeout path (it lets its issued copies land, sets
- * the error flag and leaves); pf_advance then returns PF_ERR_TIMEOUT and the
- * fields are invalid. on == 2: the engine finds that its context has no room
- * for resident launches (many steps per launch of a small grid) and launches
- * every pass by itself; results are the same. No counterpart in the
- * reference. */
+/* Test hooks of the failure paths; 0 turns them off.
+ * on == 1: one bounded wait runs out with a short limit. In the TMA-staged
+ * fused step (PF_KERNEL_FUSED where the grid allows TMA) block (0, 0, 0) of
+ * every step waits once on a barrier that nothing arrives on, lets its issued
+ * copies land, sets the error flag and leaves. In a resident launch of a small
+ * grid (the cooperative forms; a cluster's hardware barrier cannot run out)
+ * block 0 waits for arrivals that never come, and every block gives up.
+ * pf_advance then returns PF_ERR_TIMEOUT and the fields are invalid.
+ * on == 2: the engine finds that its context has no room for resident launches
+ * (many steps per launch of a small grid) and launches every pass by itself;
+ * results are the same. No counterpart in the reference. */
 int pf_set_wait_test(pf_engine *eng, int on);
 
 /* The CUDA stream (a cudaStream_t) the engine launches on, so a caller can

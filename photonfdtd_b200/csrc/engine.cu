@@ -162,7 +162,7 @@ struct pf_engine {
   bool tma = false;      // fused path stages planes with TMA
   TmaMaps maps;
   int* tma_err = nullptr;
-  int wait_test = 0;     // pf_set_wait_test: 1 one TMA stage wait runs out, 2 no resident launches
+  int wait_test = 0;     // pf_set_wait_test: 1 a bounded wait runs out, 2 no resident launches
   long long check_every = 0;  // pf_set_check_every: non-finite scan period
   int fused_ty = 8;      // fused tile height (8 or 16), env PFB200_FUSED_TY
   int fused_chunks = 0;  // x chunks per column (0 = auto), env PFB200_XCHUNKS

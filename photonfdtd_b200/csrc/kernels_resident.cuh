@@ -43,6 +43,7 @@ __host__ __device__ constexpr int res_blocks(int mode) {
 constexpr int kResDft = 4;        // DFT monitors one launch samples
 constexpr int kResOwned = 32;     // source groups injected by their cells' threads
 constexpr int kResSpin = 1 << 22; // polls before a grid barrier gives up (seconds)
+constexpr int kResSpinTest = 1 << 12;  // with the test hook (milliseconds)
 
 template <typename T>
 struct ResidentArgs {
@@ -62,9 +63,12 @@ struct ResidentArgs {
   int* err;                 // set when a barrier gave up
 };
 
-// Barrier over the launch; false when the grid barrier gave up.
+// Barrier over the launch; false when the grid barrier gave up. Test hook
+// (wait_test): block 0 waits for a count that is never reached, gives up and
+// leaves, and every other block gives up at the barrier after.
 template <int MODE>
-__device__ __forceinline__ bool res_barrier(unsigned* bar, unsigned& phase, int* err) {
+__device__ __forceinline__ bool res_barrier(unsigned* bar, unsigned& phase, int* err,
+                                            int wait_test) {
   if (MODE == kResCell1) {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
     return true;
@@ -75,12 +79,13 @@ __device__ __forceinline__ bool res_barrier(unsigned* bar, unsigned& phase, int*
   if (threadIdx.x == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
     unsigned v;
-    int spin = 0;
+    int left = wait_test ? kResSpinTest : kResSpin;
+    const unsigned want = wait_test && blockIdx.x == 0 ? ~0u : phase;
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-    } while (v < phase && ++spin < kResSpin);
-    if (v < phase) {
-      atomicExch(err, 1);
+    } while (v < want && --left > 0);
+    if (v < want) {
+      *(volatile int*)err = 1;
       bad = 1;
     }
   }
@@ -298,7 +303,7 @@ __global__ void __launch_bounds__(res_threads<T>(MODE), res_blocks<T>(MODE))
       }
     }
     if (shared_h) {
-      if (!res_barrier<MODE>(g.bar, phase, g.err)) return;
+      if (!res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
       for (int q = (int)me; q < g.src[1].n_groups; q += (int)nthr)
         inject_group<T>(g.src[1], q, a.Hout, step);
     } else {
@@ -307,7 +312,7 @@ __global__ void __launch_bounds__(res_threads<T>(MODE), res_blocks<T>(MODE))
     }
     AdeRec<T> rec;
     if (ADE && ONE && live && w) ade_load<T>(a, a.media, w, rec);  // its own: no barrier needed
-    if (!res_barrier<MODE>(g.bar, phase, g.err)) return;
+    if (!res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
     // ---- E pass
     if (ONE) {
       if (live) {
@@ -350,10 +355,10 @@ __global__ void __launch_bounds__(res_threads<T>(MODE), res_blocks<T>(MODE))
       }
     }
     if (shared_e) {
-      if (!res_barrier<MODE>(g.bar, phase, g.err)) return;
+      if (!res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
       for (int q = (int)me; q < g.src[0].n_groups; q += (int)nthr)
         inject_group<T>(g.src[0], q, a.Eout, step);
-      if (ONE && !res_barrier<MODE>(g.bar, phase, g.err)) return;
+      if (ONE && !res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
     } else {
       for (unsigned left = mine[0]; left; left &= left - 1u)
         inject_group<T>(g.src[0], __ffs(left) - 1, a.Eout, step);
@@ -391,9 +396,9 @@ __global__ void __launch_bounds__(res_threads<T>(MODE), res_blocks<T>(MODE))
               p.axis == 0 ? v0 : (p.axis == 1 ? v1 : v2);
         }
       }
-      if (!shared_e && !res_barrier<MODE>(g.bar, phase, g.err)) return;
+      if (!shared_e && !res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
     } else {
-      if (!res_barrier<MODE>(g.bar, phase, g.err)) return;
+      if (!res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
       bool due = g.n_flux > 0;
       Fields6<T> F;
 #pragma unroll
@@ -417,7 +422,7 @@ __global__ void __launch_bounds__(res_threads<T>(MODE), res_blocks<T>(MODE))
           g.flux_val[m][(g.flux_slot[m] + s) * np + t] =
               flux_cell_value<T>(p, t, F, a.ny, a.pz);
       }
-      if (due && !res_barrier<MODE>(g.bar, phase, g.err)) return;
+      if (due && !res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
     }
   }
   if (live) {
