@@ -517,14 +517,16 @@ __device__ __forceinline__ void h_cols(const BArgs<T>& a, const T (&ey)[NV], con
                                        const T (&ex)[NV], T exr, const T (&hz)[NV], T (&h)[NV]) {
   const T up = QScale<T>::up;
   const T mch = -a.ch, mchs = mul_rn(mch, QScale<T>::down);
-  T nA[NV], nB[NV], m = T(0);
+  T nA[NV], nB[NV];
+  QCheck<T> range;
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     nA[v] = fma_rn(eyn[v], up, -mul_rn(ey[v], up));
     nB[v] = fma_rn(v + 1 < NV ? ex[v + 1 < NV ? v + 1 : 0] : exr, up, -mul_rn(ex[v], up));
-    m = absmax(m, absmax(nA[v], nB[v]));
+    range.take(nA[v]);
+    range.take(nB[v]);
   }
-  if (a.fast && m < QScale<T>::limit * up) {
+  if (a.fast && range.ok()) {
 #pragma unroll
     for (int v = 0; v < NV; ++v)
       h[v] = add_rn(hz[v], mul_rn(sub_rn(qscaled(nA[v], a.dx, a.rdx), qscaled(nB[v], a.dy, a.rdy)),
@@ -665,15 +667,17 @@ __device__ __forceinline__ void tile_step(const BArgs<T>& a, const StepPost<T>& 
   // ---- Ex, Ey: kb_e's arithmetic (both quotients formed; each is used only
   // where its difference exists)
   const T up = QScale<T>::up, down = QScale<T>::down;
-  T e[V], f[V], cx[V], cy[V], nA[V], nB[V], m = T(0);
+  T e[V], f[V], cx[V], cy[V], nA[V], nB[V];
+  QCheck<T> range;
 #pragma unroll
   for (int v = 0; v < V; ++v) {
     const T s = mul_rn(h[v], up);
     nA[v] = fma_rn(-(v > 0 ? h[v > 0 ? v - 1 : 0] : hl0), up, s);
     nB[v] = fma_rn(-hp[v], up, s);
-    m = absmax(m, absmax(nA[v], nB[v]));
+    range.take(nA[v]);
+    range.take(nB[v]);
   }
-  const bool fast = a.fast && m < QScale<T>::limit * up;
+  const bool fast = a.fast && range.ok();
 #pragma unroll
   for (int v = 0; v < V; ++v) {
     T dA, dB;

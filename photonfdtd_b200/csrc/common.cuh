@@ -73,6 +73,30 @@ __device__ __forceinline__ double absmax(double a, double b) { return fmax(fabs(
 // Whether every numerator of a cell may take qdiv_fast.
 template <typename T>
 __device__ __forceinline__ bool qdiv_ok(T m) { return m < QScale<T>::limit; }
+// The same over prescaled numerators. A NaN must fail it: prescaling takes a
+// finite field of 2^64 (2^824) or more to infinity, and beside an infinite
+// neighbour the prescaled difference is NaN where the difference is infinite.
+template <typename T>
+struct QCheck;
+template <>
+struct QCheck<float> {
+  float m = 0.f;
+  __device__ __forceinline__ void take(float n) {
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(m), "f"(fabsf(n)));
+  }
+  __device__ __forceinline__ bool ok() const {
+    return m < QScale<float>::limit * QScale<float>::up;
+  }
+};
+template <>
+struct QCheck<double> {  // by the exponent: infinities and NaN have the largest
+  unsigned m = 0u;
+  __device__ __forceinline__ void take(double n) {
+    m = max(m, (unsigned)__double2hiint(n) & 0x7fffffffu);
+  }
+  __device__ __forceinline__ bool ok() const { return m < (1023u + 900u) << 20; }
+};
+static_assert(QScale<double>::limit * QScale<double>::up == 0x1p900, "QCheck's limit");
 // IEEE division, out of line: the rare numerators beyond the reciprocal
 // path's range would otherwise put a division routine at every quotient.
 static __device__ __noinline__ float div_cold(float a, float d) { return __fdiv_rn(a, d); }

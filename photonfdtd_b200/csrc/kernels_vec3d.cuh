@@ -103,7 +103,7 @@ __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][
   const T dl[3] = {a.dx, a.dy, a.dz};
   const T rl[3] = {a.rdx, a.rdy, a.rdz};
   const T up = QScale<T>::up;
-  T m = T(0);
+  QCheck<T> range;
 #pragma unroll
   for (int q = 0; q < V; ++q) {
     T os[3], n[6];
@@ -113,7 +113,7 @@ __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][
     for (int t = 0; t < 6; ++t) {
       n[t] = SGN > 0 ? fma_rn(nb[t][q], up, -os[term_comp(t)])
                      : fma_rn(-nb[t][q], up, os[term_comp(t)]);
-      m = absmax(m, n[t]);
+      range.take(n[t]);
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -122,7 +122,7 @@ __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][
       out[c][q] = add_rn(f[c][q], mul_rn(mul_rn(sub_rn(dA, dB), QScale<T>::down), K[c % NC][q]));
     }
   }
-  if (!(a.fdall && m < QScale<T>::limit * up)) {
+  if (!(a.fdall && range.ok())) {
 #pragma unroll
     for (int q = 0; q < V; ++q) {
       T d[6];
