@@ -518,7 +518,7 @@ __device__ __forceinline__ void h_cols(const BArgs<T>& a, const T (&ey)[NV], con
   const T up = QScale<T>::up;
   const T mch = -a.ch, mchs = mul_rn(mch, QScale<T>::down);
   T nA[NV], nB[NV];
-  QCheck<T> range;
+  QCheck<T, true> range;
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     nA[v] = fma_rn(eyn[v], up, -mul_rn(ey[v], up));
@@ -526,7 +526,13 @@ __device__ __forceinline__ void h_cols(const BArgs<T>& a, const T (&ey)[NV], con
     range.take(nA[v]);
     range.take(nB[v]);
   }
-  if (a.fast && range.ok()) {
+  bool fast = range.ok();
+  if (range.kAgain && !fast) {
+    fast = true;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) fast = fast && range.sure(nA[v]) && range.sure(nB[v]);
+  }
+  if (a.fast && fast) {
 #pragma unroll
     for (int v = 0; v < NV; ++v)
       h[v] = add_rn(hz[v], mul_rn(sub_rn(qscaled(nA[v], a.dx, a.rdx), qscaled(nB[v], a.dy, a.rdy)),
@@ -555,7 +561,7 @@ __device__ __forceinline__ void h_cols_pml(const BArgs<T>& a, int j, int ny, boo
     const T nA = sub_rn(eyn[v], ey[v]);
     const T nB = sub_rn(v + 1 < NV ? ex[v + 1 < NV ? v + 1 : 0] : exr, ex[v]);
     T dA, dB;
-    if (a.fast && qdiv_ok(absmax(nA, nB))) {
+    if (a.fast && qdiv_ok<T>(nA, nB)) {
       dA = qdiv_fast(nA, a.dx, a.rdx);
       dB = qdiv_fast(nB, a.dy, a.rdy);
     } else {
@@ -668,7 +674,7 @@ __device__ __forceinline__ void tile_step(const BArgs<T>& a, const StepPost<T>& 
   // where its difference exists)
   const T up = QScale<T>::up, down = QScale<T>::down;
   T e[V], f[V], cx[V], cy[V], nA[V], nB[V];
-  QCheck<T> range;
+  QCheck<T, true> range;
 #pragma unroll
   for (int v = 0; v < V; ++v) {
     const T s = mul_rn(h[v], up);
@@ -677,7 +683,13 @@ __device__ __forceinline__ void tile_step(const BArgs<T>& a, const StepPost<T>& 
     range.take(nA[v]);
     range.take(nB[v]);
   }
-  const bool fast = a.fast && range.ok();
+  bool fast = range.ok();
+  if (range.kAgain && !fast) {
+    fast = true;
+#pragma unroll
+    for (int v = 0; v < V; ++v) fast = fast && range.sure(nA[v]) && range.sure(nB[v]);
+  }
+  fast = fast && a.fast;
 #pragma unroll
   for (int v = 0; v < V; ++v) {
     T dA, dB;

@@ -20,8 +20,7 @@ __device__ __forceinline__ void divide6(const StepArgs<T>& a, const T n[6], cons
   const T dl[3] = {a.dx, a.dy, a.dz};
   const T rl[3] = {a.rdx, a.rdy, a.rdz};
   const bool fl[3] = {a.fdx, a.fdy, a.fdz};
-  const T m = absmax(absmax(n[0], n[1]), absmax(absmax(n[2], n[3]), absmax(n[4], n[5])));
-  if (a.fdall && qdiv_ok(m)) {
+  if (a.fdall && qdiv_ok<T>(n[0], n[1], n[2], n[3], n[4], n[5])) {
 #pragma unroll
     for (int t = 0; t < 6; ++t) q[t] = qdiv_fast(n[t], dl[ax[t]], rl[ax[t]]);
   } else {

@@ -38,9 +38,8 @@ __device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(
 //    q1 = RN(q0 - rem r) is one of the two neighbours of a / d, and from such
 //    a q1 Markstein's theorem makes the second correction the rounded
 //    quotient for every d whose significand is not all ones and r = RN(1/d)
-//    (the host checks that, and d in [2^-30, 2^-23]). |a| < 2^700. Quotients
-//    below 2^-1022, where scaling back rounds, may differ from IEEE division
-//    by one unit of 2^-1074.
+//    (the host checks that, and d in [2^-30, 2^-23]). a is 0 or 2^-1042 <=
+//    |a| < 2^700, so that a quotient is normal and scaling it back exact.
 // Four FP32 (six FP64) operations per quotient and one to scale it back;
 // sums and differences of scaled quotients are the scaled sums and
 // differences, so a curl scales back once (kUnscale) instead of per term.
@@ -48,11 +47,11 @@ template <typename T>
 struct QScale;
 template <>
 struct QScale<float> {
-  static constexpr float up = 0x1p64f, down = 0x1p-64f, limit = 0x1p26f;
+  static constexpr float up = 0x1p64f, down = 0x1p-64f;
 };
 template <>
 struct QScale<double> {
-  static constexpr double up = 0x1p200, down = 0x1p-200, limit = 0x1p700;
+  static constexpr double up = 0x1p200, down = 0x1p-200;
 };
 // Quotient of a prescaled numerator, still scaled.
 __device__ __forceinline__ float qscaled(float as, float d, float r) {
@@ -68,42 +67,57 @@ template <typename T>
 __device__ __forceinline__ T qdiv_fast(T a, T d, T r) {
   return mul_rn(qscaled(mul_rn(a, QScale<T>::up), d, r), QScale<T>::down);
 }
-__device__ __forceinline__ float absmax(float a, float b) { return fmaxf(fabsf(a), fabsf(b)); }
-__device__ __forceinline__ double absmax(double a, double b) { return fmax(fabs(a), fabs(b)); }
-// Whether every numerator of a cell may take qdiv_fast.
-template <typename T>
-__device__ __forceinline__ bool qdiv_ok(T m) { return m < QScale<T>::limit; }
-// The same over prescaled numerators. A NaN must fail it: prescaling takes a
-// finite field of 2^64 (2^824) or more to infinity, and beside an infinite
-// neighbour the prescaled difference is NaN where the difference is infinite.
-template <typename T>
+// Whether numerators may take the reciprocal path, tested over all of a cell's
+// (or vector's) at once. SCALED: they are prescaled.
+//  float: |a| < 2^26. A NaN must fail when prescaled: prescaling takes a finite
+//    field of 2^64 or more to infinity, and beside an infinite neighbour the
+//    prescaled difference is NaN where the difference is infinite.
+//  double: 2^-1042 <= |a| < 2^700, by the exponent (infinities and NaN have the
+//    largest): one shift-and-add and one maximum per numerator. 0 fails that
+//    too, so what fails is asked again one by one (sure; kAgain).
+template <typename T, bool SCALED>
 struct QCheck;
-template <>
-struct QCheck<float> {
+template <bool SCALED>
+struct QCheck<float, SCALED> {
+  static constexpr bool kAgain = false;
   float m = 0.f;
   __device__ __forceinline__ void take(float n) {
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(m), "f"(fabsf(n)));
+    if (SCALED) asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(m), "f"(fabsf(n)));
+    else m = fmaxf(m, fabsf(n));
   }
-  __device__ __forceinline__ bool ok() const {
-    return m < QScale<float>::limit * QScale<float>::up;
-  }
+  __device__ __forceinline__ bool ok() const { return m < (SCALED ? 0x1p90f : 0x1p26f); }
+  __device__ static __forceinline__ bool sure(float) { return false; }
 };
-template <>
-struct QCheck<double> {  // by the exponent: infinities and NaN have the largest
+template <bool SCALED>
+struct QCheck<double, SCALED> {
+  static constexpr bool kAgain = true;
+  // high words: of 2^-1042 (a subnormal) and 2^700, or these times 2^200
+  static constexpr unsigned lo = SCALED ? (1023u - 842u) << 20 : 1u;
+  static constexpr unsigned hi = (1023u + (SCALED ? 900u : 700u)) << 20;
   unsigned m = 0u;
-  __device__ __forceinline__ void take(double n) {
-    m = max(m, (unsigned)__double2hiint(n) & 0x7fffffffu);
+  __device__ static __forceinline__ unsigned key(double n) {
+    return 2u * (unsigned)__double2hiint(n) - 2u * lo;
   }
-  __device__ __forceinline__ bool ok() const { return m < (1023u + 900u) << 20; }
+  __device__ __forceinline__ void take(double n) { m = max(m, key(n)); }
+  __device__ __forceinline__ bool ok() const { return m < 2u * (hi - lo); }
+  __device__ static __forceinline__ bool sure(double n) {
+    return n == 0.0 || key(n) < 2u * (hi - lo);
+  }
 };
-static_assert(QScale<double>::limit * QScale<double>::up == 0x1p900, "QCheck's limit");
+// The same for single numerators that are not prescaled.
+template <typename T, typename... N>
+__device__ __forceinline__ bool qdiv_ok(N... n) {
+  QCheck<T, false> c;
+  (c.take(n), ...);
+  return c.ok() || (c.kAgain && (c.sure(n) && ...));
+}
 // IEEE division, out of line: the rare numerators beyond the reciprocal
 // path's range would otherwise put a division routine at every quotient.
 static __device__ __noinline__ float div_cold(float a, float d) { return __fdiv_rn(a, d); }
 static __device__ __noinline__ double div_cold(double a, double d) { return __ddiv_rn(a, d); }
 template <typename T>
 __device__ __forceinline__ T qdiv(T a, T d, T r, bool fast) {
-  if (fast && qdiv_ok(absmax(a, a))) return qdiv_fast(a, d, r);
+  if (fast && qdiv_ok<T>(a)) return qdiv_fast(a, d, r);
   return div_rn(a, d);
 }
 // Two exact quotients sharing one range check and one branch: both by the
@@ -111,7 +125,7 @@ __device__ __forceinline__ T qdiv(T a, T d, T r, bool fast) {
 template <typename T>
 __device__ __forceinline__ void qdiv2(T a0, T d0, T r0, bool f0, T a1, T d1, T r1, bool f1,
                                       T& q0, T& q1) {
-  if (f0 && f1 && qdiv_ok(absmax(a0, a1))) {
+  if (f0 && f1 && qdiv_ok<T>(a0, a1)) {
     q0 = qdiv_fast(a0, d0, r0);
     q1 = qdiv_fast(a1, d1, r1);
   } else {

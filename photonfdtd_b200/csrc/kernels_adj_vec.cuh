@@ -143,15 +143,15 @@ __global__ void __launch_bounds__(kVecThreads, 2) k_adj_e_vec(const __grid_const
   // the quotients of the recorded H
   const T dl[3] = {a.dx, a.dy, a.dz};
   const T rl[3] = {a.rdx, a.rdy, a.rdz};
-  T m = T(0);
+  QCheck<T, false> range;
 #pragma unroll
   for (int t = 0; t < 6; ++t)
 #pragma unroll
     for (int q = 0; q < V; ++q) {
       nb[t][q] = sub_rn(own[term_comp(t)][q], nb[t][q]);
-      m = absmax(m, nb[t][q]);
+      range.take(nb[t][q]);
     }
-  if (a.fdall && qdiv_ok(m)) {
+  if (a.fdall && in_range(range, nb)) {
 #pragma unroll
     for (int t = 0; t < 6; ++t)
 #pragma unroll

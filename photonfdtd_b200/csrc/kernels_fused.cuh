@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(32 * TY, 1024 / (32 * TY)) k_fused(
       const T n0 = sub_rn(E0[2][jj + 1][kk], ezc), n1 = sub_rn(E0[1][jj][kk + 1], eyc);
       const T n2 = sub_rn(E0[0][jj][kk + 1], exc), n3 = sub_rn(E1[2][jj][kk], ezc);
       const T n4 = sub_rn(E1[1][jj][kk], eyc), n5 = sub_rn(E0[0][jj + 1][kk], exc);
-      if (qfast && qdiv_ok(absmax(absmax(n0, n1), absmax(absmax(n2, n3), absmax(n4, n5))))) {
+      if (qfast && qdiv_ok<T>(n0, n1, n2, n3, n4, n5)) {
         hx = bulk(h_old[0], mch, qdiv_fast(n0, a.dy, a.rdy), qdiv_fast(n1, a.dz, a.rdz));
         hy = bulk(h_old[1], mch, qdiv_fast(n2, a.dz, a.rdz), qdiv_fast(n3, a.dx, a.rdx));
         hz = bulk(h_old[2], mch, qdiv_fast(n4, a.dx, a.rdx), qdiv_fast(n5, a.dy, a.rdy));
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(32 * TY, 1024 / (32 * TY)) k_fused(
         const T n0 = sub_rn(hz, sm.h[2][jj - 1][kk]), n1 = sub_rn(hy, sm.h[1][jj][kk - 1]);
         const T n2 = sub_rn(hx, sm.h[0][jj][kk - 1]), n3 = sub_rn(hz, hz_prev);
         const T n4 = sub_rn(hy, hy_prev), n5 = sub_rn(hx, sm.h[0][jj - 1][kk]);
-        if (qfast && qdiv_ok(absmax(absmax(n0, n1), absmax(absmax(n2, n3), absmax(n4, n5))))) {
+        if (qfast && qdiv_ok<T>(n0, n1, n2, n3, n4, n5)) {
           e[0] = bulk(en[0], K[0], qdiv_fast(n0, a.dy, a.rdy), qdiv_fast(n1, a.dz, a.rdz));
           e[1] = bulk(en[1], K[1], qdiv_fast(n2, a.dz, a.rdz), qdiv_fast(n3, a.dx, a.rdx));
           e[2] = bulk(en[2], K[2], qdiv_fast(n4, a.dx, a.rdx), qdiv_fast(n5, a.dy, a.rdy));

@@ -21,10 +21,11 @@
 
 // Minimum resident 128-thread blocks per SM the passes are compiled for:
 // float H, float E, float E with ADE or three coefficients, double H, double
-// E. Step kernels in us at 5/5/4, 4/4/4 and 5/4/3: 256^3 plain 287, 311, 301;
-// 384^3 with ADE 1278, 1309, 1370; 301x287x263 with three coefficients (at
-// 5, 4, 4 blocks) 441, 424, 409. Double 6/5 145 us, 4/3 155, 8/6 153
-// (160x152x144).
+// E, double E with ADE or three coefficients. Step kernels in us at 5/5/4,
+// 4/4/4 and 5/4/3: 256^3 plain 287, 311, 301; 384^3 with ADE 1278, 1309, 1370;
+// 301x287x263 with three coefficients (at 5, 4, 4 blocks) 441, 424, 409.
+// Double at 5/5, 6/5, 6/4 and 5/4 (H/E): 144^3 plain 106.8, 109.0, 112.4,
+// 109.9; 160x160x147 with ADE 237, 243, 217, 211.
 #ifndef PFB_MINB_HV
 #define PFB_MINB_HV 5
 #endif
@@ -35,10 +36,13 @@
 #define PFB_MINB_EVA 4
 #endif
 #ifndef PFB_MINB_HV64
-#define PFB_MINB_HV64 6
+#define PFB_MINB_HV64 5
 #endif
 #ifndef PFB_MINB_EV64
 #define PFB_MINB_EV64 5
+#endif
+#ifndef PFB_MINB_EVA64
+#define PFB_MINB_EVA64 4
 #endif
 
 namespace pfb {
@@ -90,6 +94,20 @@ __device__ __forceinline__ constexpr int term_axis(int t) {
   return t == 0 || t == 5 ? 1 : (t == 1 || t == 2 ? 2 : 0);
 }
 
+// Whether the differences d may take the reciprocal path; range: over all of them.
+template <typename T>
+__device__ __forceinline__ bool in_range(const QCheck<T, false>& range, const T (&d)[6][kVec<T>]) {
+  bool fast = range.ok();
+  if (range.kAgain && !fast) {
+    fast = true;
+#pragma unroll
+    for (int t = 0; t < 6; ++t)
+#pragma unroll
+      for (int q = 0; q < kVec<T>; ++q) fast = fast && range.sure(d[t][q]);
+  }
+  return fast;
+}
+
 // out[c] = f[c] + K[c] (d_A - d_B) for V bulk cells. SGN 1: forward
 // differences d = (nb - own) / dl (H), -1: backward d = (own - nb) / dl (E).
 // Own values are prescaled once; a prescaled difference is then one FMA, and
@@ -103,16 +121,17 @@ __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][
   const T dl[3] = {a.dx, a.dy, a.dz};
   const T rl[3] = {a.rdx, a.rdy, a.rdz};
   const T up = QScale<T>::up;
-  QCheck<T> range;
+  QCheck<T, true> range;
+  auto diff = [&](int t, int q) {
+    const T os = mul_rn(own[term_comp(t)][q], up);
+    return SGN > 0 ? fma_rn(nb[t][q], up, -os) : fma_rn(-nb[t][q], up, os);
+  };
 #pragma unroll
   for (int q = 0; q < V; ++q) {
-    T os[3], n[6];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) os[c] = mul_rn(own[c][q], up);
+    T n[6];
 #pragma unroll
     for (int t = 0; t < 6; ++t) {
-      n[t] = SGN > 0 ? fma_rn(nb[t][q], up, -os[term_comp(t)])
-                     : fma_rn(-nb[t][q], up, os[term_comp(t)]);
+      n[t] = diff(t, q);
       range.take(n[t]);
     }
 #pragma unroll
@@ -122,7 +141,15 @@ __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][
       out[c][q] = add_rn(f[c][q], mul_rn(mul_rn(sub_rn(dA, dB), QScale<T>::down), K[c % NC][q]));
     }
   }
-  if (!(a.fdall && range.ok())) {
+  bool fast = range.ok();
+  if (range.kAgain && !fast) {
+    fast = true;
+#pragma unroll
+    for (int q = 0; q < V; ++q)
+#pragma unroll
+      for (int t = 0; t < 6; ++t) fast = fast && range.sure(diff(t, q));
+  }
+  if (!(a.fdall && fast)) {
 #pragma unroll
     for (int q = 0; q < V; ++q) {
       T d[6];
@@ -189,16 +216,17 @@ __device__ __forceinline__ void curl_general(const StepArgs<T>& a, const Cpml<T>
   vld_if(p.c[2] + k, gz >= 0, cz);
   const T dl[3] = {a.dx, a.dy, a.dz};
   const T rl[3] = {a.rdx, a.rdy, a.rdz};
-  T d[6][V], m = T(0);
+  T d[6][V];
+  QCheck<T, false> range;
 #pragma unroll
   for (int q = 0; q < V; ++q)
 #pragma unroll
     for (int t = 0; t < 6; ++t) {
       const T o = own[term_comp(t)][q];
       d[t][q] = SGN > 0 ? sub_rn(nb[t][q], o) : sub_rn(o, nb[t][q]);
-      m = absmax(m, d[t][q]);
+      range.take(d[t][q]);
     }
-  if (a.fdall && qdiv_ok(m)) {
+  if (a.fdall && in_range(range, d)) {
 #pragma unroll
     for (int q = 0; q < V; ++q)
 #pragma unroll
@@ -391,9 +419,10 @@ __device__ __forceinline__ void ade_cell(const StepArgs<T>& a, uint32_t w, T en0
 // issued in dependency order: the words, every field vector, then what the
 // words select (coefficients, ADE records of a run).
 template <typename T, int CE, bool ADE>
-__global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? (ADE || CE == kCeCell3 ? PFB_MINB_EVA
-                                                                                      : PFB_MINB_EV)
-                                                              : PFB_MINB_EV64)
+constexpr int kMinBlocksE = ADE || CE == kCeCell3 ? (sizeof(T) == 4 ? PFB_MINB_EVA : PFB_MINB_EVA64)
+                                                  : (sizeof(T) == 4 ? PFB_MINB_EV : PFB_MINB_EV64);
+template <typename T, int CE, bool ADE>
+__global__ void __launch_bounds__(kVecThreads, kMinBlocksE<T, CE, ADE>)
     k_e_vec(const __grid_constant__ StepArgs<T> a, int i0) {
   pdl_enter();
   constexpr int V = kVec<T>;

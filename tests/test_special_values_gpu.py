@@ -1,6 +1,7 @@
 """Quotients of special fields: the reciprocal division against IEEE division.
 
-A diverging run reaches fields near the type's limits and infinities. Every
+A diverging run reaches fields near the type's limits and infinities, a decayed
+one subnormals, whose quotients may be subnormal themselves (float64). Every
 quotient of the stepping is defined as the IEEE quotient of the difference, so
 a run with the reciprocal division and one with IEEE division
 (PFB200_IEEE_DIV) must hold the same state: same values, infinities and NaN in
@@ -18,8 +19,7 @@ pytestmark = pytest.mark.gpu
 ALL6 = ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
 
 
-def _tables(shape, pml, precision):
-    d = 20e-9
+def _tables(shape, pml, precision, d=20e-9):
     size = tuple(n * d if n > 1 else 0.0 for n in shape)
     grid = pf.Grid(size=size, cell_size=tuple(d if n > 1 else 0.0 for n in shape),
                    pml_layers=tuple(pml if n > 1 else 0 for n in shape))
@@ -67,6 +67,26 @@ def test_large_and_infinite_fields(shape, pml, comp, precision, monkeypatch):
         got = _state(t, fields, separate, False, 1, monkeypatch)
         want = _state(t, fields, separate, True, 1, monkeypatch)
         assert np.isinf(want).any() and np.isnan(want).any() and np.isfinite(want).any()
+        np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("precision", ["float32", "float64"])
+@pytest.mark.parametrize("shape,pml", [((24, 22, 37), 5), ((31, 26, 24), 6), ((70, 61, 1), 8)])
+def test_subnormal_fields(shape, pml, precision, monkeypatch):
+    """The CPML state holds the quotients nearly as they are, down to the last
+    subnormal bit. Float64 differences of some 2^25 units of 2^-1074 give
+    subnormal quotients with one bit less than a normal one, on a cell size
+    that does not divide them."""
+    t = _tables(shape, pml, precision, 13e-9)
+    rng = np.random.default_rng(4)
+    lo, hi = (-45.0, -36.0) if precision == "float32" else (-318.0, -315.0)
+    fields = {c: (rng.choice([-1.0, 0.0, 1.0], size=shape)
+                  * 10.0 ** rng.uniform(lo, hi, size=shape)).astype(precision) for c in ALL6}
+    for separate in (False, True):
+        got = _state(t, fields, separate, False, 2, monkeypatch)
+        want = _state(t, fields, separate, True, 2, monkeypatch)
+        tiny = np.finfo(precision).tiny
+        assert ((want != 0) & (np.abs(want) < tiny)).any()
         np.testing.assert_array_equal(got, want)
 
 
