@@ -1882,6 +1882,12 @@ int copy_state(pf_engine* e, long long step, void* buf, int64_t bytes, int on_de
   PF_CUDA(e, cudaStreamSynchronize(e->stream));
   return PF_OK;
 }
+// The engine is at `step` with no sample pending: the monitors' phase rows follow
+// the step, not the count of samples taken so far.
+void set_step(pf_engine* e, long long step) {
+  e->step = step;
+  for (DftMon& m : e->dfts) m.q_done = (step + m.interval - 1) / m.interval;
+}
 }  // namespace
 
 int pf_state_bytes(const pf_engine* e, int64_t* bytes) {
@@ -1908,9 +1914,7 @@ int pf_set_state(pf_engine* e, int64_t step, const void* src, int64_t bytes, int
   if (rc) return rc;
   rc = copy_state(e, step, const_cast<void*>(src), bytes, src_on_device, false);
   if (rc) return rc;
-  e->step = step;
-  // the phase rows follow the step, not the count of samples taken so far
-  for (DftMon& m : e->dfts) m.q_done = (step + m.interval - 1) / m.interval;
+  set_step(e, step);
   return PF_OK;
 }
 
@@ -2252,7 +2256,9 @@ int pf_adj_segment(pf_engine* e, int64_t step0, int64_t n, const void* state, in
   if ((rc = copy_state(e, step0, const_cast<void*>(state), bytes, state_on_device, false)))
     return rc;
   e->step = step0;
-  return e->rb == 4 ? adj_segment_typed<float>(e, step0, n) : adj_segment_typed<double>(e, step0, n);
+  rc = e->rb == 4 ? adj_segment_typed<float>(e, step0, n) : adj_segment_typed<double>(e, step0, n);
+  set_step(e, e->step);  // a replay samples nothing
+  return rc;
 }
 
 int pf_adj_read_grad_components(pf_engine* e, double* dst) {

@@ -67,3 +67,35 @@ def test_phases_follow_the_step(shape, separate, k):
         assert tol > 0
         assert np.abs(f + r - w).max() <= tol
         assert np.abs(w + r - s).max() <= tol
+
+
+@pytest.mark.parametrize("shape", [(40, 36, 1), (24, 22, 20)])
+def test_phases_after_a_reverse_segment(shape):
+    """A reverse segment leaves the engine at the segment's end; steps taken from
+    there carry their own phases."""
+    steps, n = 90, 20
+    t = _tables(shape, steps)
+    a, b = B200Engine(t), B200Engine(t)
+    try:
+        a.advance(0, steps - 2 * n)
+        mid = a.get_state()
+        a.advance(steps - 2 * n, n)
+        last = a.get_state()
+        a.advance(steps - n, n)
+        a._chk(a._L.pf_adj_init(a.h, n))
+        before = _sums(a, t)
+        for s0, st in ((steps - n, last), (steps - 2 * n, mid)):
+            a._chk(a._L.pf_adj_segment(a.h, s0, n, st.ctypes.data, st.size, 0))
+        assert a.step() == steps - n
+        a.advance(steps - n, n)
+        after = _sums(a, t)
+        b.set_state(steps - n, last)
+        b.advance(steps - n, n)
+        rest = _sums(b, t)
+    finally:
+        a.close()
+        b.close()
+    for x, y, r in zip(before, after, rest):
+        tol = 1e-11 * np.abs(x).max()
+        assert tol > 0
+        assert np.abs(x + r - y).max() <= tol
