@@ -689,12 +689,13 @@ StepArgs<T> step_args(pf_engine* e) {
   return a;
 }
 
-// Scans the six current fields for inf / nan (synchronous).
-int scan_finite(pf_engine* e) {
+// Scans the six current fields for inf / nan (synchronous). H: where the H of
+// a recorded step lies instead of the engine's own arrays.
+int scan_finite(pf_engine* e, void* const H[3] = nullptr) {
   int* flag = e->flag;
   PF_CUDA(e, cudaMemsetAsync(flag, 0, sizeof(int), e->stream));
   for (int c = 0; c < 6; ++c) {
-    const void* f = c < 3 ? e->E[e->cur][c] : e->H[e->cur][c - 3];
+    const void* f = c < 3 ? e->E[e->cur][c] : (H ? H : e->H[e->cur])[c - 3];
     if (e->rb == 4)
       k_nonfinite<float><<<592, 256, 0, e->stream>>>((const float*)f, e->ncellp, flag);
     else
@@ -1161,6 +1162,7 @@ int advance_separate(pf_engine* e, long long n_sub) {
     // value and the other family's fields
     const int nxt = e->fused ? e->cur ^ 1 : e->cur;
     StepArgs<T> a = step_args<T>(e);
+    void* H[3] = {a.Hout[0], a.Hout[1], a.Hout[2]};
     if (e->fused) {
       int rc;
       {
@@ -1185,6 +1187,7 @@ int advance_separate(pf_engine* e, long long n_sub) {
         if (slot < 0 || slot >= e->ring_steps)
           return fail(e, PF_ERR_STATE, "record slot out of range");
         if (e->vec) record_into<T>(e, slot, a, Hout);
+        for (int c = 0; c < 3; ++c) H[c] = Hout[c];
       }
       {
         LaunchScope ls(e, 0);
@@ -1208,7 +1211,7 @@ int advance_separate(pf_engine* e, long long n_sub) {
     if (e->recording && (rc = record_step<T>(e, s - e->rec_step0))) return rc;
     if (e->check_every > 0 && e->step % e->check_every == 0) {
       PF_CUDA(e, cudaGetLastError());
-      if ((rc = scan_finite(e))) {
+      if ((rc = scan_finite(e, H))) {
         collect_profile(e);
         return rc;
       }
@@ -2088,8 +2091,12 @@ int adj_segment_typed(pf_engine* e, long long step0, long long n) {
   e->rec_step0 = step0;
   int rc = advance_typed<T>(e, n);
   e->recording = false;
+  // the engine's own H and psi_E, also where the periodic scan stopped it
+  if ((!rc || rc == PF_ERR_NONFINITE) && e->vec && !e->fused && e->step > step0) {
+    const int rc2 = record_out(e, e->step - 1 - step0);
+    if (!rc) rc = rc2;
+  }
   if (rc) return rc;
-  if (e->vec && !e->fused && (rc = record_out(e, n - 1))) return rc;
   const int nz = e->nz, ny = e->ny, nx = e->nx;
   const int nzv = (nz + kVec<T> - 1) / kVec<T>;
   const dim3 blk = e->vec ? dim3(vec_lanes(nzv), kVecThreads / vec_lanes(nzv))
