@@ -19,7 +19,7 @@ import ctypes
 import numpy as np
 
 from . import _native as N
-from .scene import EPS_0, MU_0
+from .scene import EPS_0, MU_0, GaussianPulse
 
 _COMP = {"Ex": 0, "Ey": 1, "Ez": 2, "Hx": 3, "Hy": 4, "Hz": 5}
 _FIELD_KEYS = ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
@@ -307,12 +307,20 @@ def build_tables(sim, dtype=None, ce3=None) -> dict:
     return t
 
 
+def _elementwise(waveform) -> bool:
+    """Whether a waveform is this package's pulse or the reference's
+    (photonfdtd.sources), not a subclass or a user's class of that name."""
+    t = type(waveform)
+    return t is GaussianPulse or (t.__module__, t.__qualname__) == ("photonfdtd.sources",
+                                                                    "GaussianPulse")
+
+
 def source_tables(sim, n_steps: int, dt: float) -> dict:
     """Per-source component, flat cell, waveform row and amplitude, plus the
     waveform rows: value of each distinct waveform at its family's Yee times
     ((s+1/2)dt for H, (s+1)dt for E; simulation.py:1322-1323), evaluated one
     time at a time as the reference's loop calls it, except for the package's
-    own pulse, whose elementwise formula takes all times at once."""
+    own pulse and the reference's, whose formula takes all times at once."""
     grid = sim.grid
     ny, nz = grid.shape[1], grid.shape[2]
     rows: Dict[tuple, int] = {}
@@ -324,8 +332,8 @@ def source_tables(sim, n_steps: int, dt: float) -> dict:
         key = (id(src.waveform), fam)
         if key not in rows:
             off = 0.5 if fam == "H" else 1.0
-            if type(src.waveform).__name__ == "GaussianPulse":
-                # elementwise NumPy on the times: the same values in one call
+            if _elementwise(src.waveform):
+                # NumPy operations on the times: the same values in one call
                 vals = np.asarray(src.waveform((np.arange(n_steps) + off) * dt), np.float64)
             else:
                 vals = np.empty(n_steps, dtype=np.float64)
