@@ -304,6 +304,11 @@ int pf_info(const pf_engine *eng, char *buf, int len);
 /* Device bytes held by the engine. */
 int pf_device_bytes(const pf_engine *eng, int64_t *bytes);
 
+/* Up to 2 GiB of the memory of destroyed engines stays mapped for the next one.
+ * This gives it back to the driver (the current device's); allocations of this
+ * library that find no memory do so by themselves. */
+int pf_release_memory(void);
+
 /* Release everything. NULL is a no-op. */
 void pf_destroy(pf_engine *eng);
 

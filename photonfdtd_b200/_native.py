@@ -88,6 +88,7 @@ SIGNATURES = {
     "pf_set_profiling": (C.c_int, [_vp, C.c_int]),
     "pf_read_profile": (C.c_int, [_vp, _pi64, _pdbl, C.c_int]),
     "pf_info": (C.c_int, [_vp, C.c_char_p, C.c_int]),
+    "pf_release_memory": (C.c_int, []),
     "pf_destroy": (None, [_vp]),
     "pf_flux_plane_noalloc": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(_vp),
                                         C.c_int, C.c_int, _dbl, _dbl, _vp, _vp]),

@@ -167,10 +167,12 @@ def choose_checkpoint(n_steps: int, state_reals: int, design_cells: int, real_by
 
 
 def default_memory_budget() -> float:
-    """Half of the device memory free now (0 without a CUDA device)."""
+    """Half of the device memory free now (0 without a CUDA device), once the
+    memory kept from earlier engines is given back."""
     try:
         import torch
         if torch.cuda.is_available():
+            N.check(N.lib().pf_release_memory())
             return 0.5 * float(torch.cuda.mem_get_info()[0])
     except Exception:  # noqa: BLE001 - no usable CUDA runtime: no budget
         pass

@@ -44,6 +44,7 @@
 #include "../../include/pfb200.h"
 #include "batch2d_kernels.cuh"
 #include "common.cuh"
+#include "devmem.cuh"
 
 using namespace pfb;
 using namespace pfb::b2d;
@@ -141,7 +142,7 @@ int bfail(pf_batch* b, int code, const char* fmt, ...) {
 
 int balloc(pf_batch* b, void** p, size_t bytes) {
   if (!bytes) bytes = 16;
-  cudaError_t rc = cudaMalloc(p, bytes);
+  cudaError_t rc = malloc_trim(p, bytes);
   if (rc != cudaSuccess) {
     *p = nullptr;
     return bfail(b, PF_ERR_OOM, "cudaMalloc of %zu bytes failed", bytes);

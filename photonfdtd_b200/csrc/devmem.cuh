@@ -5,7 +5,8 @@
 // as long as a small scene's stepping. A stream-ordered pool keeps up to
 // kPoolKeep bytes of freed memory mapped for the next engine; what is above
 // that goes back to the driver at the next synchronisation, and everything
-// when an allocation fails. The pool belongs to no engine and is
+// when an allocation of this library fails (pool_trim), a batch sizes itself,
+// or the user asks (pf_release_memory). The pool belongs to no engine and is
 // never handed pointers of another allocator. Its calls are thread safe, and
 // its ordering is per stream: memory freed on one engine's stream reaches
 // another only behind the work queued before the free.
@@ -28,6 +29,10 @@ constexpr unsigned long long kPoolKeep = 2ull << 30;
 // bytes of device memory in `st`'s order (a stream of device `dev`).
 cudaError_t pool_alloc(void** p, size_t bytes, int dev, cudaStream_t st);
 void pool_free(void* p, cudaStream_t st);
+// Gives back what the pool of the thread's current context holds unused.
+void pool_trim();
+// cudaMalloc, and once more after pool_trim if there was no memory.
+cudaError_t malloc_trim(void** p, size_t bytes);
 
 // An error word (zero) of the context of `st`, or p == nullptr.
 struct ErrWord {

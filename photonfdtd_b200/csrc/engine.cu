@@ -1353,6 +1353,24 @@ void err_word_release(int dev, const ErrWord& w) {
   if (w.p && it != g_keep.end() && it->second.ctx == w.ctx) it->second.err_free.push_back(w.p);
 }
 
+void pool_trim() {
+  int dev = 0;
+  std::lock_guard<std::mutex> lk(g_keep_mu);
+  if (g_keep.empty() || cudaGetDevice(&dev) != cudaSuccess) return;
+  const auto it = g_keep.find(dev);
+  // the null stream's context is the current one
+  if (it != g_keep.end() && it->second.pool && it->second.ctx == context_id(nullptr))
+    cudaMemPoolTrimTo(it->second.pool, 0);
+}
+
+cudaError_t malloc_trim(void** p, size_t bytes) {
+  cudaError_t rc = cudaMalloc(p, bytes);
+  if (rc != cudaErrorMemoryAllocation) return rc;
+  cudaGetLastError();
+  pool_trim();
+  return cudaMalloc(p, bytes);
+}
+
 cudaError_t pool_alloc(void** p, size_t bytes, int dev, cudaStream_t st) {
   *p = nullptr;
   cudaMemPool_t pool = device_pool(dev, st);
@@ -1991,6 +2009,14 @@ int pf_info(const pf_engine* e, char* buf, int len) {
 int pf_device_bytes(const pf_engine* e, int64_t* bytes) {
   if (!e || !bytes) return PF_ERR_INVALID;
   *bytes = (int64_t)e->dev_bytes;
+  return PF_OK;
+}
+
+int pf_release_memory(void) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess)
+    return fail(nullptr, PF_ERR_CUDA, "no CUDA device");
+  pool_trim();
   return PF_OK;
 }
 

@@ -29,6 +29,7 @@
 #include <string>
 
 #include "../../include/pfb200.h"
+#include "devmem.cuh"
 
 namespace {
 
@@ -217,15 +218,15 @@ int pf_smooth_boxes(int nx, int ny, int nz, int factor, double background, int n
   do {
     if (!cuda_ok(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream")) break;
     const size_t nb = (size_t)(n_box ? n_box : 1);
-    if (!cuda_ok(cudaMalloc((void**)&dspan, nb * 6 * sizeof(int)), "cudaMalloc")) break;
-    if (!cuda_ok(cudaMalloc((void**)&deps, nb * sizeof(double)), "cudaMalloc")) break;
-    if (!cuda_ok(cudaMalloc((void**)&ea, (size_t)n * 8), "cudaMalloc")) break;
-    if (!cuda_ok(cudaMalloc((void**)&eh, (size_t)n * 8), "cudaMalloc")) break;
-    if (!cuda_ok(cudaMalloc((void**)&gm, (size_t)n * 8), "cudaMalloc")) break;
-    if (!cuda_ok(cudaMalloc((void**)&gmax, 8), "cudaMalloc")) break;
+    if (!cuda_ok(pfb::malloc_trim((void**)&dspan, nb * 6 * sizeof(int)), "cudaMalloc")) break;
+    if (!cuda_ok(pfb::malloc_trim((void**)&deps, nb * sizeof(double)), "cudaMalloc")) break;
+    if (!cuda_ok(pfb::malloc_trim((void**)&ea, (size_t)n * 8), "cudaMalloc")) break;
+    if (!cuda_ok(pfb::malloc_trim((void**)&eh, (size_t)n * 8), "cudaMalloc")) break;
+    if (!cuda_ok(pfb::malloc_trim((void**)&gm, (size_t)n * 8), "cudaMalloc")) break;
+    if (!cuda_ok(pfb::malloc_trim((void**)&gmax, 8), "cudaMalloc")) break;
     bool ok = true;
     for (int c = 0; c < 3 && ok; ++c)
-      ok = cuda_ok(cudaMalloc(&dout[c], (size_t)n * out_bytes), "cudaMalloc");
+      ok = cuda_ok(pfb::malloc_trim(&dout[c], (size_t)n * out_bytes), "cudaMalloc");
     if (!ok) break;
     if (n_box) {
       if (!cuda_ok(cudaMemcpyAsync(dspan, spans, (size_t)n_box * 6 * sizeof(int),
