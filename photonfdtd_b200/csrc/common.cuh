@@ -38,7 +38,7 @@ __device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(
 //    q1 = RN(q0 - rem r) is one of the two neighbours of a / d, and from such
 //    a q1 Markstein's theorem makes the second correction the rounded
 //    quotient for every d whose significand is not all ones and r = RN(1/d)
-//    (the host checks that, and d in [2^-30, 2^-23]). a is 0 or 2^-1042 <=
+//    (the host checks that, and d in [2^-30, 2^-23]). a is 0 or 2^-1022 <=
 //    |a| < 2^700, so that a quotient is normal and scaling it back exact.
 // Four FP32 (six FP64) operations per quotient and one to scale it back;
 // sums and differences of scaled quotients are the scaled sums and
@@ -72,9 +72,11 @@ __device__ __forceinline__ T qdiv_fast(T a, T d, T r) {
 //  float: |a| < 2^26. A NaN must fail when prescaled: prescaling takes a finite
 //    field of 2^64 or more to infinity, and beside an infinite neighbour the
 //    prescaled difference is NaN where the difference is infinite.
-//  double: 2^-1042 <= |a| < 2^700, by the exponent (infinities and NaN have the
+//  double: 2^-1022 <= |a| < 2^700, by the exponent (infinities and NaN have the
 //    largest): one shift-and-add and one maximum per numerator. 0 fails that
 //    too, so what fails is asked again one by one (sure; kAgain).
+// These limits hold for divisors in [2^-30, 2^-23] (double: [2^-60, 1]); ok(top)
+// takes another prescaled upper limit, lowkey() serves a lower one (float).
 template <typename T, bool SCALED>
 struct QCheck;
 template <bool SCALED>
@@ -85,14 +87,21 @@ struct QCheck<float, SCALED> {
     if (SCALED) asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(m), "f"(fabsf(n)));
     else m = fmaxf(m, fabsf(n));
   }
-  __device__ __forceinline__ bool ok() const { return m < (SCALED ? 0x1p90f : 0x1p26f); }
+  __device__ __forceinline__ bool ok() const { return ok(0x1p90f); }
+  __device__ __forceinline__ bool ok(float top) const {
+    return m < (SCALED ? top : mul_rn(top, QScale<float>::down));
+  }
   __device__ static __forceinline__ bool sure(float) { return false; }
+  // Orders prescaled magnitudes; 0 comes last.
+  __device__ static __forceinline__ unsigned lowkey(float n) {
+    return 2u * __float_as_uint(SCALED ? n : mul_rn(n, QScale<float>::up)) - 1u;
+  }
 };
 template <bool SCALED>
 struct QCheck<double, SCALED> {
   static constexpr bool kAgain = true;
-  // high words: of 2^-1042 (a subnormal) and 2^700, or these times 2^200
-  static constexpr unsigned lo = SCALED ? (1023u - 842u) << 20 : 1u;
+  // high words of 2^-1022 and 2^700, or of these times 2^200
+  static constexpr unsigned lo = SCALED ? (1023u - 822u) << 20 : 1u << 20;
   static constexpr unsigned hi = (1023u + (SCALED ? 900u : 700u)) << 20;
   unsigned m = 0u;
   __device__ static __forceinline__ unsigned key(double n) {
@@ -208,6 +217,12 @@ struct StepArgs {
   T rdx, rdy, rdz;      // RN(1/d) per axis
   bool fdx, fdy, fdz;   // reciprocal division verified exact for that axis
   bool fdall;           // and for all three
+  // the same for the vector passes, which take divisors in [2^-60, 1]. Prescaled
+  // limits of the numerators (float): below qtop, and with a QCheck::lowkey of
+  // qlow or more (0: no lower limit)
+  bool fdvec;
+  T qtop;
+  unsigned qlow;
   T ch;          // dt / mu0 rounded to T; the H coefficient is -ch
   const T* Ein[3];
   const T* Hin[3];

@@ -159,6 +159,9 @@ struct pf_engine {
   bool fused = false;
   double rdl[3] = {1, 1, 1};     // RN(1/d) in the real type, per axis
   bool fdiv[3] = {false, false, false};  // reciprocal division verified
+  bool vdiv = false;             // the same for the vector passes, all axes
+  float qtop = 0;                // and its limits (StepArgs)
+  uint32_t qlow = 0;
   bool tma = false;      // fused path stages planes with TMA
   TmaMaps maps;
   int* tma_err = nullptr;
@@ -302,11 +305,11 @@ int upload_cells(pf_engine* e, void** p, const void* src, size_t elem) {
 // q = fma(rem, r, q0), r = RN(1/d)) equals IEEE a / d for every float
 // significand a in [1, 2). Sign and binade of a do not change the outcome
 // while nothing over- or underflows; the device's 2^64 prescaling and the
-// range check on d below keep every input of the fast path in that regime.
-// About 8.4M fmaf evaluations (~50 ms); the answer per divisor is kept for
-// the process, so engines on the same grid spacing check it once.
-bool recip_division_exact_scan(float d);
-bool recip_division_exact(float d) {
+// range checks keep every input of the fast path in that regime. The answer per
+// divisor is kept for the process, so engines on the same grid spacing check
+// it once. scan(d): the check itself.
+template <typename Scan>
+bool recip_division_known(float d, Scan scan) {
   static std::mutex mu;
   static std::map<uint32_t, bool> known;
   uint32_t key;
@@ -316,13 +319,13 @@ bool recip_division_exact(float d) {
     auto it = known.find(key);
     if (it != known.end()) return it->second;
   }
-  const bool ok = recip_division_exact_scan(d);
+  const bool ok = scan(d);
   std::lock_guard<std::mutex> lk(mu);
   known[key] = ok;
   return ok;
 }
-bool recip_division_exact_scan(float d) {
-  if (!(d >= 0x1p-30f && d <= 0x1p-23f)) return false;
+// On the host: about 8.4M fmaf evaluations (~50 ms).
+bool recip_division_scan(float d) {
   const float r = 1.0f / d;
   for (uint32_t m = 0; m < (1u << 23); ++m) {
     const uint32_t bits = 0x3f800000u | m;
@@ -336,15 +339,64 @@ bool recip_division_exact_scan(float d) {
   }
   return true;
 }
+bool recip_division_exact(float d) {
+  return d >= 0x1p-30f && d <= 0x1p-23f && recip_division_known(d, recip_division_scan);
+}
 
 // The double reciprocal division of qdiv (two corrections): r = 1 / d is
 // correctly rounded here, so Markstein's theorem needs only a divisor whose
 // significand is not all ones, and a range where nothing over- or underflows.
-bool recip_division_exact(double d) {
+bool recip_division_provable(double d) {
   uint64_t bits;
   memcpy(&bits, &d, 8);
   const uint64_t frac = (1ull << 52) - 1;
-  return d >= 0x1p-30 && d <= 0x1p-23 && (bits & frac) != frac;
+  return (bits & frac) != frac;
+}
+bool recip_division_exact(double d) {
+  return d >= 0x1p-30 && d <= 0x1p-23 && recip_division_provable(d);
+}
+
+// What the vector passes need of the grid's divisors: every one in [2^-60, 1]
+// and exact. Divisors outside the scalar passes' window (2^-30 .. 2^-23) are
+// checked on the device, some 30 us, since such grids had nothing to check.
+int vector_division(pf_engine* e) {
+  e->vdiv = false;
+  if (!e->vec || e->fused || getenv("PFB200_IEEE_DIV")) return PF_OK;
+  const double dmin = std::min({e->dl[0], e->dl[1], e->dl[2]});
+  const double dmax = std::max({e->dl[0], e->dl[1], e->dl[2]});
+  if (!(dmin >= 0x1p-60 && dmax <= 1.0)) return PF_OK;
+  int rc = PF_OK;
+  auto scan = [&](float d) {
+    int bad = 1;
+    cudaMemsetAsync(e->flag, 0, sizeof(int), e->stream);
+    k_recip_exact<<<592, 256, 0, e->stream>>>(d, 1.0f / d, e->flag);
+    cudaMemcpyAsync(&bad, e->flag, sizeof(int), cudaMemcpyDeviceToHost, e->stream);
+    if (cudaStreamSynchronize(e->stream) != cudaSuccess) {
+      rc = PF_ERR_CUDA;
+      return false;
+    }
+    return bad == 0;
+  };
+  bool ok = true;
+  for (int ax = 0; ax < 3 && ok; ++ax)
+    ok = e->rb == 8 ? recip_division_provable(e->dl[ax])
+                    : recip_division_exact((float)e->dl[ax]) ||
+                          recip_division_known((float)e->dl[ax], scan);
+  if (rc) return fail(e, rc, "CUDA error: checking the grid spacing's reciprocal failed");
+  e->vdiv = ok;
+  // prescaled numerators: quotients from 2^-62 (normal once scaled back; below
+  // 2^-23 every numerator gives one) to 2^121
+  int lo, hi;
+  std::frexp((float)dmin, &lo);  // dmin >= 2^(lo - 1)
+  std::frexp((float)dmax, &hi);  // dmax < 2^hi
+  e->qtop = std::min(0x1p90f, std::ldexp(1.0f, 121 + lo - 1));
+  e->qlow = 0;
+  if (dmax > 0x1p-23) {
+    const float low = std::ldexp(1.0f, -62 + hi);
+    memcpy(&e->qlow, &low, 4);
+    e->qlow = 2 * e->qlow - 1;
+  }
+  return PF_OK;
 }
 
 // Bracket one launch of `kind` (0 step, 1 sources, 2 sampling, 3 flush).
@@ -644,6 +696,9 @@ StepArgs<T> step_args(pf_engine* e) {
   a.fdy = e->fdiv[1];
   a.fdz = e->fdiv[2];
   a.fdall = a.fdx && a.fdy && a.fdz;
+  a.fdvec = e->vdiv;
+  a.qtop = e->vdiv ? (T)e->qtop : T(0);
+  a.qlow = e->vdiv ? e->qlow : 0u;
   a.ch = (T)e->ch;
   for (int ax = 0; ax < 3; ++ax) {
     a.hb0[ax] = e->hb0[ax];
@@ -742,7 +797,7 @@ void launch_h(pf_engine* e, const StepArgs<T>& a, int i0, int i1) {
     const int nzv = (e->nz + kVec<T> - 1) / kVec<T>;
     const dim3 b(vec_lanes(nzv), kVecThreads / vec_lanes(nzv));
     launch_pdl(e->stream, dim3((nzv + b.x - 1) / b.x, (e->ny + b.y - 1) / b.y, i1 - i0), b,
-               k_h_vec<T>, a, i0);
+               sizeof(T) == 4 && a.qlow ? k_h_vec<T, sizeof(T) == 4> : k_h_vec<T, false>, a, i0);
     return;
   }
   const dim3 b = e->nz > 1 ? dim3(32, 8) : dim3(1, 256);
@@ -756,7 +811,8 @@ void launch_e_mode(pf_engine* e, const StepArgs<T>& a, int i0, int i1) {
     const int nzv = (e->nz + kVec<T> - 1) / kVec<T>;
     const dim3 b(vec_lanes(nzv), kVecThreads / vec_lanes(nzv));
     launch_pdl(e->stream, dim3((nzv + b.x - 1) / b.x, (e->ny + b.y - 1) / b.y, i1 - i0), b,
-               k_e_vec<T, CE, ADE>, a, i0);
+               sizeof(T) == 4 && a.qlow ? k_e_vec<T, CE, ADE, sizeof(T) == 4>
+                                        : k_e_vec<T, CE, ADE, false>, a, i0);
     return;
   }
   const dim3 b = e->nz > 1 ? dim3(32, 8) : dim3(1, 256);
@@ -1711,6 +1767,7 @@ int pf_finalize(pf_engine* e) {
     }
   }
   int rc = e->rb == 4 ? finalize_typed<float>(e) : finalize_typed<double>(e);
+  if (!rc) rc = vector_division(e);
   if (rc) return rc;
   // host staging no longer needed
   for (int c = 0; c < 3; ++c) std::vector<char>().swap(e->h_ce[c]);

@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kVecThreads, 2) k_adj_e_vec(const __grid_const
       nb[t][q] = sub_rn(own[term_comp(t)][q], nb[t][q]);
       range.take(nb[t][q]);
     }
-  if (a.fdall && in_range(range, nb)) {
+  if (in_range<true>(a, range, [&](int t, int q) { return nb[t][q]; })) {
 #pragma unroll
     for (int t = 0; t < 6; ++t)
 #pragma unroll

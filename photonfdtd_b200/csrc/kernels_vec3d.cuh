@@ -94,18 +94,51 @@ __device__ __forceinline__ constexpr int term_axis(int t) {
   return t == 0 || t == 5 ? 1 : (t == 1 || t == 2 ? 2 : 0);
 }
 
-// Whether the differences d may take the reciprocal path; range: over all of them.
-template <typename T>
-__device__ __forceinline__ bool in_range(const QCheck<T, false>& range, const T (&d)[6][kVec<T>]) {
-  bool fast = range.ok();
-  if (range.kAgain && !fast) {
-    fast = true;
-#pragma unroll
-    for (int t = 0; t < 6; ++t)
-#pragma unroll
-      for (int q = 0; q < kVec<T>; ++q) fast = fast && range.sure(d[t][q]);
+// *bad = 1 when the reciprocal division by d (r = RN(1/d)) misses the IEEE
+// quotient of some float significand.
+static __global__ void k_recip_exact(float d, float r, int* bad) {
+  for (unsigned m = blockIdx.x * blockDim.x + threadIdx.x; m < 1u << 23;
+       m += gridDim.x * blockDim.x) {
+    const float a = __uint_as_float(0x3f800000u | m);
+    if (qscaled(a, d, r) != __fdiv_rn(a, d)) *bad = 1;
   }
-  return fast;
+}
+
+// Whether a vector's differences n(term, cell) may take the reciprocal path;
+// range: over all of them. LOW: a float grid with cells above 2^-23 m (119 nm),
+// whose small numerators give subnormal quotients, has a lower limit too (its
+// own kernels: tested at run time, the skipped loop cost the others 1%). The
+// scalar passes divide such grids by IEEE division; 24 of these bound a
+// vector's step. us at 200 nm, IEEE in line by the scalar passes, out of line by
+// the vector passes, and so: 192^3 float 179, 184, 124, with ADE 221, 239, 175;
+// 144^3 double 120, 168, 109.
+template <bool LOW, typename T, bool SCALED, typename N>
+__device__ __forceinline__ bool in_range(const StepArgs<T>& a, const QCheck<T, SCALED>& range,
+                                         const N& n) {
+  constexpr int V = kVec<T>;
+  if constexpr (sizeof(T) == 4) {
+    bool fast = range.ok(a.qtop);
+    if (LOW && fast && a.qlow) {
+      unsigned low = ~0u;
+#pragma unroll
+      for (int t = 0; t < 6; ++t)
+#pragma unroll
+        for (int q = 0; q < V; ++q) low = min(low, range.lowkey(n(t, q)));
+      fast = low >= a.qlow;
+    }
+    return fast;
+  } else {
+    if (!a.fdvec) return false;
+    bool fast = range.ok();
+    if (!fast) {
+      fast = true;
+#pragma unroll
+      for (int t = 0; t < 6; ++t)
+#pragma unroll
+        for (int q = 0; q < V; ++q) fast = fast && range.sure(n(t, q));
+    }
+    return fast;
+  }
 }
 
 // out[c] = f[c] + K[c] (d_A - d_B) for V bulk cells. SGN 1: forward
@@ -113,7 +146,7 @@ __device__ __forceinline__ bool in_range(const QCheck<T, false>& range, const T 
 // Own values are prescaled once; a prescaled difference is then one FMA, and
 // the curl is scaled back once per component (QScale in common.cuh): 6.5
 // operations per term instead of 11. One range check covers the V cells.
-template <typename T, int SGN, int NC>
+template <typename T, int SGN, int NC, bool LOW>
 __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][kVec<T>],
                                           const T (&K)[NC][kVec<T>], const T (&own)[3][kVec<T>],
                                           const T (&nb)[6][kVec<T>], T (&out)[3][kVec<T>]) {
@@ -141,15 +174,7 @@ __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][
       out[c][q] = add_rn(f[c][q], mul_rn(mul_rn(sub_rn(dA, dB), QScale<T>::down), K[c % NC][q]));
     }
   }
-  bool fast = range.ok();
-  if (range.kAgain && !fast) {
-    fast = true;
-#pragma unroll
-    for (int q = 0; q < V; ++q)
-#pragma unroll
-      for (int t = 0; t < 6; ++t) fast = fast && range.sure(diff(t, q));
-  }
-  if (!(a.fdall && fast)) {
+  if (!in_range<LOW>(a, range, diff)) {
 #pragma unroll
     for (int q = 0; q < V; ++q) {
       T d[6];
@@ -191,7 +216,7 @@ __device__ __forceinline__ T cpml_term(T f, T k, T d, T b, T c, T& psi) {
 // each psi load waited behind the stores of the cell before it (256^3 with a
 // 12-cell layer on every face: the layers cost 70 us of 314, now 41 of 287; 29
 // of these are their bytes).
-template <typename T, int SGN, int NC>
+template <typename T, int SGN, int NC, bool LOW>
 __device__ __forceinline__ void curl_general(const StepArgs<T>& a, const Cpml<T>& p, int i, int j,
                                              int k, const T (&f)[3][kVec<T>],
                                              const T (&K)[NC][kVec<T>],
@@ -226,7 +251,7 @@ __device__ __forceinline__ void curl_general(const StepArgs<T>& a, const Cpml<T>
       d[t][q] = SGN > 0 ? sub_rn(nb[t][q], o) : sub_rn(o, nb[t][q]);
       range.take(d[t][q]);
     }
-  if (a.fdall && in_range(range, d)) {
+  if (in_range<LOW>(a, range, [&](int t, int q) { return d[t][q]; })) {
 #pragma unroll
     for (int q = 0; q < V; ++q)
 #pragma unroll
@@ -287,7 +312,7 @@ __device__ __forceinline__ bool warp_bulk(bool live, int i, int j, int k, const 
 }
 
 // H pass: H^{n+1/2} = H^{n-1/2} - ch (curl E^n + psi), planes i0 + blockIdx.z.
-template <typename T>
+template <typename T, bool LOW>
 __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? PFB_MINB_HV : PFB_MINB_HV64)
     k_h_vec(const __grid_constant__ StepArgs<T> a, int i0) {
   pdl_enter();
@@ -321,7 +346,7 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? PFB_MINB_HV : PF
 #pragma unroll
   for (int q = 0; q < V; ++q) K[0][q] = -a.ch;
   if (box) {
-    curl_bulk<T, 1, 1>(a, f, K, own, nb, out);
+    curl_bulk<T, 1, 1, LOW>(a, f, K, own, nb, out);
   } else {
     Cpml<T> p;
 #pragma unroll
@@ -337,7 +362,7 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? PFB_MINB_HV : PF
       p.in[t] = a.psiHin[t];
       p.out[t] = a.psiHout[t];
     }
-    curl_general<T, 1, 1>(a, p, i, j, k, f, K, own, nb, out);
+    curl_general<T, 1, 1, LOW>(a, p, i, j, k, f, K, own, nb, out);
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c) vst(a.Hout[c] + id, out[c]);
@@ -421,7 +446,7 @@ __device__ __forceinline__ void ade_cell(const StepArgs<T>& a, uint32_t w, T en0
 template <typename T, int CE, bool ADE>
 constexpr int kMinBlocksE = ADE || CE == kCeCell3 ? (sizeof(T) == 4 ? PFB_MINB_EVA : PFB_MINB_EVA64)
                                                   : (sizeof(T) == 4 ? PFB_MINB_EV : PFB_MINB_EV64);
-template <typename T, int CE, bool ADE>
+template <typename T, int CE, bool ADE, bool LOW>
 __global__ void __launch_bounds__(kVecThreads, kMinBlocksE<T, CE, ADE>)
     k_e_vec(const __grid_constant__ StepArgs<T> a, int i0) {
   pdl_enter();
@@ -500,7 +525,7 @@ __global__ void __launch_bounds__(kVecThreads, kMinBlocksE<T, CE, ADE>)
     nb[2][q] = q > 0 ? own[0][q > 0 ? q - 1 : 0] : h0;
   }
   if (box) {
-    curl_bulk<T, -1, NC>(a, en, K, own, nb, e);
+    curl_bulk<T, -1, NC, LOW>(a, en, K, own, nb, e);
   } else {
     Cpml<T> p;
 #pragma unroll
@@ -516,7 +541,7 @@ __global__ void __launch_bounds__(kVecThreads, kMinBlocksE<T, CE, ADE>)
       p.in[s] = a.psiEin[s];
       p.out[s] = a.psiE[s];
     }
-    curl_general<T, -1, NC>(a, p, i, j, k, en, K, own, nb, e);
+    curl_general<T, -1, NC, LOW>(a, p, i, j, k, en, K, own, nb, e);
   }
   if (ADE) {
     if (vec) {
