@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kVecThreads, 2) k_adj_e_vec(const __grid_const
   // the quotients of the recorded H
   const T dl[3] = {a.dx, a.dy, a.dz};
   const T rl[3] = {a.rdx, a.rdy, a.rdz};
-  QCheck<T, false> range;
+  QCheck<T, false> range(a.qtop);
 #pragma unroll
   for (int t = 0; t < 6; ++t)
 #pragma unroll

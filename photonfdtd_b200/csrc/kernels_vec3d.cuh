@@ -117,7 +117,7 @@ __device__ __forceinline__ bool in_range(const StepArgs<T>& a, const QCheck<T, S
                                          const N& n) {
   constexpr int V = kVec<T>;
   if constexpr (sizeof(T) == 4) {
-    bool fast = range.ok(a.qtop);
+    bool fast = range.ok();
     if (LOW && fast && a.qlow) {
       unsigned low = ~0u;
 #pragma unroll
@@ -154,7 +154,7 @@ __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][
   const T dl[3] = {a.dx, a.dy, a.dz};
   const T rl[3] = {a.rdx, a.rdy, a.rdz};
   const T up = QScale<T>::up;
-  QCheck<T, true> range;
+  QCheck<T, true> range(a.qtop);
   auto diff = [&](int t, int q) {
     const T os = mul_rn(own[term_comp(t)][q], up);
     return SGN > 0 ? fma_rn(nb[t][q], up, -os) : fma_rn(-nb[t][q], up, os);
@@ -242,7 +242,7 @@ __device__ __forceinline__ void curl_general(const StepArgs<T>& a, const Cpml<T>
   const T dl[3] = {a.dx, a.dy, a.dz};
   const T rl[3] = {a.rdx, a.rdy, a.rdz};
   T d[6][V];
-  QCheck<T, false> range;
+  QCheck<T, false> range(a.qtop);
 #pragma unroll
   for (int q = 0; q < V; ++q)
 #pragma unroll
