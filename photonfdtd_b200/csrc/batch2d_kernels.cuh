@@ -518,7 +518,7 @@ __device__ __forceinline__ void h_cols(const BArgs<T>& a, const T (&ey)[NV], con
   const T up = QScale<T>::up;
   const T mch = -a.ch, mchs = mul_rn(mch, QScale<T>::down);
   T nA[NV], nB[NV];
-  QCheck<T, true> range;
+  QCheck<T, true, true> range;
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     nA[v] = fma_rn(eyn[v], up, -mul_rn(ey[v], up));
@@ -674,7 +674,7 @@ __device__ __forceinline__ void tile_step(const BArgs<T>& a, const StepPost<T>& 
   // where its difference exists)
   const T up = QScale<T>::up, down = QScale<T>::down;
   T e[V], f[V], cx[V], cy[V], nA[V], nB[V];
-  QCheck<T, true> range;
+  QCheck<T, true, true> range;
 #pragma unroll
   for (int v = 0; v < V; ++v) {
     const T s = mul_rn(h[v], up);

@@ -77,28 +77,34 @@ __device__ __forceinline__ T qdiv_fast(T a, T d, T r) {
 //    too, so what fails is asked again one by one (sure; kAgain).
 // These limits hold for divisors in [2^-30, 2^-23] (double: [2^-60, 1]); the
 // constructor takes another upper limit, lowkey() serves a lower one (float).
-template <typename T, bool SCALED>
+// CHAIN (float): a chain of compares instead of a maximum and one compare. The
+// batch's tile step is faster so (64 instances 59.0 against 62.8 us), the 3D
+// passes with ADE, whose registers spill, without (192^3 170 against 173 us).
+template <typename T, bool SCALED, bool CHAIN = false>
 struct QCheck;
-template <bool SCALED>
-struct QCheck<float, SCALED> {
+template <bool SCALED, bool CHAIN>
+struct QCheck<float, SCALED, CHAIN> {
   static constexpr bool kAgain = false;
   float top;
+  float m = 0.f;
   bool in = true;
   // top: prescaled
   __device__ __forceinline__ explicit QCheck(float t = 0x1p90f)
       : top(SCALED ? t : mul_rn(t, QScale<float>::down)) {}
-  // A chain of compares: the tile step of a batch of 64 runs 59.0 us so, 62.8
-  // with a maximum and one compare (NaN kept or not).
-  __device__ __forceinline__ void take(float n) { in = in & (fabsf(n) < top); }
-  __device__ __forceinline__ bool ok() const { return in; }
+  __device__ __forceinline__ void take(float n) {
+    if (CHAIN) in = in & (fabsf(n) < top);
+    else if (SCALED) asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(m), "f"(fabsf(n)));
+    else m = fmaxf(m, fabsf(n));
+  }
+  __device__ __forceinline__ bool ok() const { return CHAIN ? in : m < top; }
   __device__ static __forceinline__ bool sure(float) { return false; }
   // Orders prescaled magnitudes; 0 comes last.
   __device__ static __forceinline__ unsigned lowkey(float n) {
     return 2u * __float_as_uint(SCALED ? n : mul_rn(n, QScale<float>::up)) - 1u;
   }
 };
-template <bool SCALED>
-struct QCheck<double, SCALED> {
+template <bool SCALED, bool CHAIN>
+struct QCheck<double, SCALED, CHAIN> {
   static constexpr bool kAgain = true;
   // high words of 2^-1022 and 2^700, or of these times 2^200
   static constexpr unsigned lo = SCALED ? (1023u - 822u) << 20 : 1u << 20;
