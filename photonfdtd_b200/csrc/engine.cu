@@ -159,6 +159,7 @@ struct pf_engine {
   bool fused = false;
   double rdl[3] = {1, 1, 1};     // RN(1/d) in the real type, per axis
   bool fdiv[3] = {false, false, false};  // reciprocal division verified
+  bool ade_cells = false;        // E pass of a dispersive scene: one cell per thread
   bool vdiv = false;             // the same for the vector passes, all axes
   float qtop = 0;                // and its limits (StepArgs)
   uint32_t qlow = 0;
@@ -790,6 +791,38 @@ int vec_lanes(int nzv) {
   return (nzv + 7) / 8 * 8 > (nzv + 3) / 4 * 4 ? 4 : 8;
 }
 
+// Whether a dispersive 3D scene's E pass runs one cell per thread. The vector
+// pass reads polarisation records as vectors where V cells of one medium have
+// consecutive ranks from an aligned one on; other records it takes cell by
+// cell, each cell's loads behind the stores of the one before, and a warp
+// waits for its slowest lane. So the share of warps with such one-pole records
+// (w1) and with such records of more poles (w2; in double all of these, whose
+// two chunks spill) decides: w1 + 2.5 w2 > 1 (double: 0.75). us per step, vectors /
+// cells, at that sum: float 160^2 x 163 of 12-cell blocks 130 / 135 at 0.94,
+// 160^2 x 147 of 8-cell blocks 132 / 116 at 1.06, one-pole sphere in 192^3 157 /
+// 171 at 0.62, two-pole sphere 190 / 182 at 1.5, single cells in 160^3 171 / 121
+// at 3.5, aligned blocks in 192^3 170 / 192 at 0; double 144^3: box 138 / 135 at 0.70,
+// spheres 128 / 136 at 0.55, 176 / 150 at 1.54, aligned blocks 162 / 150 at 1.38.
+template <typename T>
+int ade_by_cell(pf_engine* e) {
+  e->ade_cells = false;
+  if (!e->vec || e->fused || e->n_media == 0) return PF_OK;
+  const uint32_t* word = e->ce_mode == PF_CE_TABLE ? e->word : e->adeword;
+  unsigned long long* dev = nullptr;
+  int rc = dalloc(e, (void**)&dev, 3 * sizeof *dev);
+  if (rc) return rc;
+  const int nzv = (e->nz + kVec<T> - 1) / kVec<T>;
+  const dim3 b(vec_lanes(nzv), kVecThreads / vec_lanes(nzv));
+  k_ade_runs<T><<<dim3((nzv + b.x - 1) / b.x, (e->ny + b.y - 1) / b.y, e->nx), b, 0, e->stream>>>(
+      word, (const MediumT<T>*)e->media, e->ny, e->nz, e->pz, dev);
+  PF_CUDA(e, cudaGetLastError());
+  unsigned long long n[3];  // warps, w1, w2
+  PF_CUDA(e, cudaMemcpyAsync(n, dev, sizeof n, cudaMemcpyDeviceToHost, e->stream));
+  PF_CUDA(e, cudaStreamSynchronize(e->stream));
+  e->ade_cells = 4 * n[1] + 10 * n[2] > (sizeof(T) == 4 ? 4 : 3) * n[0];
+  return PF_OK;
+}
+
 // H and E passes over planes [i0, i1).
 template <typename T>
 void launch_h(pf_engine* e, const StepArgs<T>& a, int i0, int i1) {
@@ -807,6 +840,13 @@ void launch_h(pf_engine* e, const StepArgs<T>& a, int i0, int i1) {
 
 template <typename T, int CE, bool ADE>
 void launch_e_mode(pf_engine* e, const StepArgs<T>& a, int i0, int i1) {
+  if constexpr (ADE) {
+    if (e->ade_cells) {
+      launch_pdl(e->stream, dim3((e->nz + 31) / 32, (e->ny + 7) / 8, e->nx), dim3(32, 8),
+                 k_e_cell<T, CE>, a);
+      return;
+    }
+  }
   if (e->vec) {
     const int nzv = (e->nz + kVec<T> - 1) / kVec<T>;
     const dim3 b(vec_lanes(nzv), kVecThreads / vec_lanes(nzv));
@@ -1768,6 +1808,7 @@ int pf_finalize(pf_engine* e) {
   }
   int rc = e->rb == 4 ? finalize_typed<float>(e) : finalize_typed<double>(e);
   if (!rc) rc = vector_division(e);
+  if (!rc) rc = e->rb == 4 ? ade_by_cell<float>(e) : ade_by_cell<double>(e);
   if (rc) return rc;
   // host staging no longer needed
   for (int c = 0; c < 3; ++c) std::vector<char>().swap(e->h_ce[c]);
@@ -2054,10 +2095,11 @@ int pf_info(const pf_engine* e, char* buf, int len) {
   if (!e || !buf || len < 1) return PF_ERR_INVALID;
   snprintf(buf, (size_t)len,
            "kernel=%s fused_ty=%d x_chunks=%d qdiv=%d%d%d ce_mode=%d media=%d real_bytes=%d "
-           "tma=%d "
+           "tma=%d e_pass=%s "
            "shape=%dx%dx%d dft=%zu flux=%zu",
            e->fused ? "fused" : "split", e->fused_ty, e->fused_chunks, (int)e->fdiv[0],
-           (int)e->fdiv[1], (int)e->fdiv[2], e->ce_mode, e->n_media, e->rb, (int)e->tma, e->nx,
+           (int)e->fdiv[1], (int)e->fdiv[2], e->ce_mode, e->n_media, e->rb, (int)e->tma,
+           !e->vec || e->ade_cells ? "cell" : "vector", e->nx,
            e->ny, e->nz,
            e->dfts.size(), e->fluxes.size());
   return PF_OK;

@@ -411,6 +411,61 @@ __device__ __forceinline__ void ade_vec(const MediumT<T>& M, const T* Rc, T* Rp,
   }
 }
 
+// Whether a vector of words takes k_e_vec's vector path for its records; their
+// pole count and place (reals from the level's start).
+template <typename T>
+__device__ __forceinline__ bool ade_run(const MediumT<T>* media, const uint32_t (&t)[kVec<T>],
+                                        int& np, long long& rec) {
+  bool run = (t[0] & kDispersiveBit) && (t[kVec<T> - 1] >> kMediumShift) == (t[0] >> kMediumShift);
+#pragma unroll
+  for (int q = 1; q < kVec<T>; ++q) run = run && t[q] == t[0] + (uint32_t)q;
+  if (!run) return false;
+  const MediumT<T>& M = media[(t[0] >> kMediumShift) & 15u];
+  np = M.npole;
+  rec = M.poff + (long long)(t[0] & kLocMask) * (3 * np);
+  return (np == 1 || np == 2) && rec % kVec<T> == 0;
+}
+
+// Warps of k_e_vec's grid, those with one-pole records outside aligned runs, and
+// those with such records of more poles (double: with any).
+template <typename T>
+__global__ void __launch_bounds__(kVecThreads) k_ade_runs(const uint32_t* word,
+                                                          const MediumT<T>* media, int ny, int nz,
+                                                          int pz, unsigned long long* count) {
+  constexpr int V = kVec<T>;
+  const int k = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  __shared__ unsigned n[3];
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+  if (tid < 3) n[tid] = 0u;
+  __syncthreads();
+  const bool live = k < nz && j < ny;
+  bool one = false, more = false;
+  if (live) {
+    uint32_t t[V];
+    wld(word + ((long long)blockIdx.z * ny + j) * pz + k, t);
+    int np = 0;
+    long long rec = 0;
+    const bool run = ade_run<T>(media, t, np, rec);
+#pragma unroll
+    for (int q = 0; q < V; ++q)
+      if (t[q] & kDispersiveBit) {
+        const int p = media[(t[q] >> kMediumShift) & 15u].npole;
+        one = one || (p == 1 && !run);
+        more = more || (p > 1 && (sizeof(T) == 8 || !run));
+      }
+  }
+  const unsigned all = __ballot_sync(0xffffffffu, live), w1 = __ballot_sync(0xffffffffu, one),
+                 w2 = __ballot_sync(0xffffffffu, more);
+  if ((tid & 31) == 0) {
+    if (all) atomicAdd(&n[0], 1u);
+    if (w1) atomicAdd(&n[1], 1u);
+    if (w2) atomicAdd(&n[2], 1u);
+  }
+  __syncthreads();
+  if (tid < 3 && n[tid]) atomicAdd(&count[tid], (unsigned long long)n[tid]);
+}
+
 // One dispersive cell, any pole count, state read and written in place.
 template <typename T>
 __device__ __forceinline__ void ade_cell(const StepArgs<T>& a, uint32_t w, T en0, T en1, T en2,
