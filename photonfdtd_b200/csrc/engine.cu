@@ -265,32 +265,46 @@ int stage(pf_engine* e, size_t bytes) {
   return PF_OK;
 }
 
-// Copies `rows` rows of nz elements between a compact array and a device
-// array with the engine's row pitch. `kind` says where the compact side lies;
-// host arrays go through the staging buffer in one contiguous copy.
-int copy_rows(pf_engine* e, void* padded, void* compact, size_t rows, size_t elem,
-              cudaMemcpyKind kind, bool to_padded) {
+RowCopy row_copy(void* padded, void* compact, size_t rows, int w, int p, const int* pos) {
+  // m exceeds 2^(31 + s) / w by at most 1 with 2^s >= w, so the product's
+  // error stays below 1 / w of the shift for every n < 2^31
+  int s = 0;
+  while ((1LL << s) < w) ++s;
+  return RowCopy{padded, compact, pos, (unsigned)(rows * w), (unsigned)w, (unsigned)p,
+                 (unsigned)((1ull << (31 + s)) / (unsigned)w + 1), 31 + s};
+}
+void launch_copy_rows(pf_engine* e, const RowCopies& c, int n, size_t elem, bool get) {
+  unsigned most = 1;
+  for (int q = 0; q < n; ++q) most = std::max(most, c.r[q].total);
+  const dim3 g(std::min<unsigned>((most + 1023) / 1024, 148 * 8), n);
+  if (elem == 4) k_copy_rows<uint32_t><<<g, 256, 0, e->stream>>>(c, get);
+  else k_copy_rows<uint64_t><<<g, 256, 0, e->stream>>>(c, get);
+}
+
+// Copies `rows` rows of nz elements between a host array and a device array with
+// the engine's row pitch, through the staging buffer (free for the next copy only
+// in stream order).
+int copy_rows(pf_engine* e, void* padded, void* compact, size_t rows, size_t elem, bool to_padded) {
   const size_t w = (size_t)e->nz * elem, p = (size_t)e->pz * elem, bytes = rows * w;
+  const cudaMemcpyKind kind = to_padded ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
   if (bytes == 0) return PF_OK;
   if (w == p) {
     PF_CUDA(e, cudaMemcpyAsync(to_padded ? padded : compact, to_padded ? compact : padded, bytes,
                                kind, e->stream));
     return PF_OK;
   }
-  void* dense = compact;
-  if (kind != cudaMemcpyDeviceToDevice) {
-    int rc = stage(e, bytes);
-    if (rc) return rc;
-    dense = e->region;
-    if (to_padded) PF_CUDA(e, cudaMemcpyAsync(dense, compact, bytes, kind, e->stream));
+  int rc = stage(e, bytes);
+  if (rc) return rc;
+  if (to_padded) PF_CUDA(e, cudaMemcpyAsync(e->region, compact, bytes, kind, e->stream));
+  const size_t most = 0x7fffffffu / (unsigned)e->nz;  // rows of one launch
+  for (size_t r = 0; r < rows; r += most) {
+    RowCopies c = {};
+    c.r[0] = row_copy((char*)padded + r * p, (char*)e->region + r * w, std::min(most, rows - r),
+                      e->nz, e->pz, nullptr);
+    launch_copy_rows(e, c, 1, elem, !to_padded);
   }
-  if (to_padded) {
-    PF_CUDA(e, cudaMemcpy2DAsync(padded, p, dense, w, w, rows, cudaMemcpyDeviceToDevice, e->stream));
-    // the staging buffer is free for the next copy only in stream order
-  } else {
-    PF_CUDA(e, cudaMemcpy2DAsync(dense, w, padded, p, w, rows, cudaMemcpyDeviceToDevice, e->stream));
-    if (dense != compact) PF_CUDA(e, cudaMemcpyAsync(compact, dense, bytes, kind, e->stream));
-  }
+  PF_CUDA(e, cudaGetLastError());
+  if (!to_padded) PF_CUDA(e, cudaMemcpyAsync(compact, e->region, bytes, kind, e->stream));
   return PF_OK;
 }
 
@@ -299,7 +313,7 @@ int upload_cells(pf_engine* e, void** p, const void* src, size_t elem) {
   int rc = dalloc(e, p, (size_t)e->ncellp * elem);
   if (rc) return rc;
   return copy_rows(e, *p, const_cast<void*>(src), (size_t)e->nx * e->ny, elem,
-                   cudaMemcpyHostToDevice, true);
+                   true);
 }
 
 // Whether qdiv's reciprocal division (q0 = a*r, rem = fma(-q0, d, a),
@@ -1579,8 +1593,7 @@ int pf_set_ce(pf_engine* e, int mode, const void* ce0, const void* ce1, const vo
     PF_CUDA(e, cudaSetDevice(e->device));
     int rc;
     if (!e->word && (rc = dalloc(e, (void**)&e->word, (size_t)e->ncellp * 4))) return rc;
-    if ((rc = copy_rows(e, e->word, const_cast<uint32_t*>(word), (size_t)e->nx * e->ny, 4,
-                        cudaMemcpyHostToDevice, true)))
+    if ((rc = copy_rows(e, e->word, const_cast<uint32_t*>(word), (size_t)e->nx * e->ny, 4, true)))
       return rc;
     PF_CUDA(e, cudaStreamSynchronize(e->stream));
     memcpy(e->word_need, need, sizeof need);
@@ -1834,7 +1847,7 @@ int pf_read_field(pf_engine* e, int comp, void* dst) {
   if (!e->finalized) return fail(e, PF_ERR_STATE, "pf_read_field before pf_finalize");
   if (!valid_comp(comp)) return fail(e, PF_ERR_INVALID, "bad component %d", comp);
   void* src = comp < 3 ? e->E[e->cur][comp] : e->H[e->cur][comp - 3];
-  int rc = copy_rows(e, src, dst, (size_t)e->nx * e->ny, e->rb, cudaMemcpyDeviceToHost, false);
+  int rc = copy_rows(e, src, dst, (size_t)e->nx * e->ny, e->rb, false);
   if (rc) return rc;
   PF_CUDA(e, cudaStreamSynchronize(e->stream));
   return PF_OK;
@@ -1886,8 +1899,7 @@ int pf_read_region(pf_engine* e, int comp, const int32_t start[3], const int32_t
   const void* src = comp < 3 ? e->E[e->cur][comp] : e->H[e->cur][comp - 3];
   int rc;
   if (n == e->ncell) {  // the whole field: no gather
-    if ((rc = copy_rows(e, const_cast<void*>(src), dst, (size_t)e->nx * e->ny, e->rb,
-                        cudaMemcpyDeviceToHost, false)))
+    if ((rc = copy_rows(e, const_cast<void*>(src), dst, (size_t)e->nx * e->ny, e->rb, false)))
       return rc;
     PF_CUDA(e, cudaStreamSynchronize(e->stream));
     return PF_OK;
@@ -1915,8 +1927,7 @@ int pf_write_field(pf_engine* e, int comp, const void* src) {
   if (!valid_comp(comp)) return fail(e, PF_ERR_INVALID, "bad component %d", comp);
   PF_CUDA(e, cudaSetDevice(e->device));
   void* dst = comp < 3 ? e->E[e->cur][comp] : e->H[e->cur][comp - 3];
-  int rc = copy_rows(e, dst, const_cast<void*>(src), (size_t)e->nx * e->ny, e->rb,
-                     cudaMemcpyHostToDevice, true);
+  int rc = copy_rows(e, dst, const_cast<void*>(src), (size_t)e->nx * e->ny, e->rb, true);
   if (rc) return rc;
   PF_CUDA(e, cudaStreamSynchronize(e->stream));
   return PF_OK;
@@ -1969,35 +1980,34 @@ int copy_state(pf_engine* e, long long step, void* buf, int64_t bytes, int on_de
   const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice
                                         : (get ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice);
   size_t off = 0;
+  RowCopies c = {};
+  int n = 0;
   for (const auto& p : pieces) {
     char* b = (char*)buf + off;
     off += p.bytes;
-    if (p.rows) {
-      int rc = copy_rows(e, p.p, b, p.rows, e->rb, kind, !get);
-      if (rc) return rc;
-    } else if (p.zpos && p.bytes) {
-      // psi rows in groups <-> compact rows
-      const long long n = (long long)e->nx * e->ny * p.nc;
-      void* dense = b;
-      if (!on_device) {
-        int rc = stage(e, p.bytes);
-        if (rc) return rc;
-        dense = e->region;
-        if (!get) PF_CUDA(e, cudaMemcpyAsync(dense, b, p.bytes, kind, e->stream));
-      }
-      const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 148LL * 16);
-      if (e->rb == 4)
-        k_pack_rows<float><<<blocks, 256, 0, e->stream>>>((float*)p.p, (float*)dense, p.zpos, n,
-                                                          p.np, p.nc, get);
-      else
-        k_pack_rows<double><<<blocks, 256, 0, e->stream>>>((double*)p.p, (double*)dense, p.zpos, n,
-                                                           p.np, p.nc, get);
-      PF_CUDA(e, cudaGetLastError());
-      if (!on_device && get) PF_CUDA(e, cudaMemcpyAsync(b, dense, p.bytes, kind, e->stream));
-    } else if (p.bytes) {
+    if (p.bytes == 0) continue;
+    const bool same = p.rows ? e->nz == e->pz : !p.zpos;  // the same bytes in both
+    if (same) {
       PF_CUDA(e, cudaMemcpyAsync(get ? b : p.p, get ? p.p : b, p.bytes, kind, e->stream));
+      continue;
     }
+    void* dense = b;
+    const bool direct = on_device && (uintptr_t)b % e->rb == 0;
+    if (!direct) {
+      int rc = stage(e, p.bytes);
+      if (rc) return rc;
+      dense = e->region;
+      if (!get) PF_CUDA(e, cudaMemcpyAsync(dense, b, p.bytes, kind, e->stream));
+    }
+    c.r[n++] = p.rows ? row_copy(p.p, dense, p.rows, e->nz, e->pz, nullptr)
+                      : row_copy(p.p, dense, (size_t)e->nx * e->ny, p.nc, p.np, p.zpos);
+    if (direct) continue;  // all of them in one launch below
+    launch_copy_rows(e, c, 1, e->rb, get);
+    n = 0;
+    if (get) PF_CUDA(e, cudaMemcpyAsync(b, dense, p.bytes, kind, e->stream));
   }
+  if (n) launch_copy_rows(e, c, n, e->rb, get);
+  PF_CUDA(e, cudaGetLastError());
   PF_CUDA(e, cudaStreamSynchronize(e->stream));
   return PF_OK;
 }
@@ -2401,7 +2411,7 @@ int pf_adj_read_grad_components(pf_engine* e, double* dst) {
                 "per-component gradient kept only for per-component coefficients "
                 "(PF_CE_CELL3); use pf_adj_read_grad");
   PF_CUDA(e, cudaSetDevice(e->device));
-  int rc = copy_rows(e, e->grad, dst, (size_t)e->nx * e->ny * 3, 8, cudaMemcpyDeviceToHost, false);
+  int rc = copy_rows(e, e->grad, dst, (size_t)e->nx * e->ny * 3, 8, false);
   if (rc) return rc;
   PF_CUDA(e, cudaStreamSynchronize(e->stream));
   return PF_OK;
@@ -2413,7 +2423,7 @@ int pf_adj_read_grad(pf_engine* e, double* dst) {
   const size_t n = (size_t)e->ncell;
   if (e->ce_mode != PF_CE_CELL3) {  // accumulated summed over the components
     PF_CUDA(e, cudaSetDevice(e->device));
-    int rc = copy_rows(e, e->grad, dst, (size_t)e->nx * e->ny, 8, cudaMemcpyDeviceToHost, false);
+    int rc = copy_rows(e, e->grad, dst, (size_t)e->nx * e->ny, 8, false);
     if (rc) return rc;
     PF_CUDA(e, cudaStreamSynchronize(e->stream));
     return PF_OK;

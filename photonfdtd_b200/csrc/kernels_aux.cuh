@@ -234,16 +234,49 @@ __global__ void k_gather_region(const T* f, int ny, int pz, int3 start, int3 str
   }
 }
 
-// Rows of np entries <-> compact rows of their entries pos[0 .. nc).
-template <typename T>
-__global__ void k_pack_rows(T* rows, T* compact, const int* pos, long long n, int np, int nc,
-                            bool get) {
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long r = t / nc;
-    T* at = rows + r * np + pos[(int)(t - r * nc)];
-    if (get) compact[t] = *at;
-    else *at = compact[t];
+// Rows of a padded array <-> a compact array: w entries of every p, the first
+// ones or (pos) those at given places. Several arrays in one launch
+// (blockIdx.y). Bound by memory: each lane moves four entries a warp apart, all
+// loads before the stores, the row by a multiplication. A checkpoint of 160 x
+// 160 x 147 float32 took 300 us with cudaMemcpy2DAsync per array, 88 so; 1100 x
+// 1100 x 4 871, 66.
+struct RowCopy {
+  void* padded;
+  void* compact;
+  const int* pos;
+  unsigned total;      // entries of the compact array, below 2^31
+  unsigned w, p;
+  unsigned m;          // n / w == (n m) >> sh for n < 2^31
+  int sh;
+};
+constexpr int kRowCopies = 18;
+struct RowCopies {
+  RowCopy r[kRowCopies];
+};
+template <typename U>
+__global__ void __launch_bounds__(256) k_copy_rows(const __grid_constant__ RowCopies c, bool get) {
+  const RowCopy& r = c.r[blockIdx.y];
+  U* pad = (U*)r.padded;
+  U* dense = (U*)r.compact;
+  const unsigned first = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 128 + (threadIdx.x & 31);
+  for (unsigned t = first; t < r.total; t += gridDim.x * 1024) {
+    size_t at[4];
+    U v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const unsigned n = t + 32 * q;
+      const unsigned row = (unsigned)(((uint64_t)n * r.m) >> r.sh), col = n - row * r.w;
+      const bool ok = n < r.total;
+      at[q] = (size_t)row * r.p + (r.pos && ok ? (unsigned)r.pos[col] : col);
+      if (ok) v[q] = get ? pad[at[q]] : dense[n];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const unsigned n = t + 32 * q;
+      if (n >= r.total) continue;
+      if (get) dense[n] = v[q];
+      else pad[at[q]] = v[q];
+    }
   }
 }
 
