@@ -808,32 +808,36 @@ int vec_lanes(int nzv) {
 // Whether a dispersive 3D scene's E pass runs one cell per thread. The vector
 // pass reads polarisation records as vectors where V cells of one medium have
 // consecutive ranks from an aligned one on; other records it takes cell by
-// cell, each cell's loads behind the stores of the one before, and a warp
-// waits for its slowest lane. So the share of warps with such one-pole records
-// (w1) and with such records of more poles (w2; in double all of these, whose
-// two chunks spill) decides: w1 + 2.5 w2 > 1 (double: 0.75). us per step, vectors /
-// cells, at that sum: float 160^2 x 163 of 12-cell blocks 130 / 135 at 0.94,
-// 160^2 x 147 of 8-cell blocks 132 / 116 at 1.06, one-pole sphere in 192^3 157 /
-// 171 at 0.62, two-pole sphere 190 / 182 at 1.5, single cells in 160^3 171 / 121
-// at 3.5, aligned blocks in 192^3 170 / 192 at 0; double 144^3: box 138 / 135 at 0.70,
-// spheres 128 / 136 at 0.55, 176 / 150 at 1.54, aligned blocks 162 / 150 at 1.38.
+// cell, each cell's loads behind the stores of the one before, and a warp runs
+// every kind that one of its lanes has. So the shares of warps with aligned
+// runs of one pole (a1) and two (a2), other one-pole records (i1) and others of
+// more poles (i2) decide, with weights fitted to the difference of the two
+// forms' times over 36 scenes in float and 12 in double (blocks of 1 to 40 cells
+// on rows of every remainder, boxes, spheres). us per step, vectors / cells:
+// float aligned 8-cell blocks in 192^3 170 / 192, the same on 160 x 160 x 147 132 /
+// 116, 246 x 257 x 269 570 / 474, 12-cell blocks on 160 x 160 x 163 130 / 135,
+// one-pole sphere in 192^3 157 / 171, two-pole 190 / 182, single cells in 160^3
+// 171 / 121; double 144^3 aligned blocks 160 / 150, one-pole sphere 128 / 136. Where the
+// rule takes the slower form it loses 4% at most.
 template <typename T>
 int ade_by_cell(pf_engine* e) {
   e->ade_cells = false;
   if (!e->vec || e->fused || e->n_media == 0) return PF_OK;
   const uint32_t* word = e->ce_mode == PF_CE_TABLE ? e->word : e->adeword;
   unsigned long long* dev = nullptr;
-  int rc = dalloc(e, (void**)&dev, 3 * sizeof *dev);
+  int rc = dalloc(e, (void**)&dev, 5 * sizeof *dev);
   if (rc) return rc;
   const int nzv = (e->nz + kVec<T> - 1) / kVec<T>;
   const dim3 b(vec_lanes(nzv), kVecThreads / vec_lanes(nzv));
   k_ade_runs<T><<<dim3((nzv + b.x - 1) / b.x, (e->ny + b.y - 1) / b.y, e->nx), b, 0, e->stream>>>(
       word, (const MediumT<T>*)e->media, e->ny, e->nz, e->pz, dev);
   PF_CUDA(e, cudaGetLastError());
-  unsigned long long n[3];  // warps, w1, w2
+  unsigned long long n[5];  // warps, a1, a2, i1, i2
   PF_CUDA(e, cudaMemcpyAsync(n, dev, sizeof n, cudaMemcpyDeviceToHost, e->stream));
   PF_CUDA(e, cudaStreamSynchronize(e->stream));
-  e->ade_cells = 4 * n[1] + 10 * n[2] > (sizeof(T) == 4 ? 4 : 3) * n[0];
+  const double a1 = (double)n[1], a2 = (double)n[2], i1 = (double)n[3], i2 = (double)n[4];
+  e->ade_cells = sizeof(T) == 4 ? 2.25 * (a1 + a2) + 4.25 * i1 + 11.5 * i2 > 5.0 * (double)n[0]
+                                : 1.4 * a1 + 21.0 * a2 + 8.0 * i1 + 12.0 * i2 > 5.6 * (double)n[0];
   return PF_OK;
 }
 

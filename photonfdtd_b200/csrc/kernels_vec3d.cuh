@@ -426,8 +426,8 @@ __device__ __forceinline__ bool ade_run(const MediumT<T>* media, const uint32_t 
   return (np == 1 || np == 2) && rec % kVec<T> == 0;
 }
 
-// Warps of k_e_vec's grid, those with one-pole records outside aligned runs, and
-// those with such records of more poles (double: with any).
+// Warps of k_e_vec's grid, and those with aligned runs of one pole, of two, with
+// other one-pole records, with other records of more poles.
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_ade_runs(const uint32_t* word,
                                                           const MediumT<T>* media, int ny, int nz,
@@ -435,35 +435,34 @@ __global__ void __launch_bounds__(kVecThreads) k_ade_runs(const uint32_t* word,
   constexpr int V = kVec<T>;
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) * V;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  __shared__ unsigned n[3];
+  __shared__ unsigned n[5];
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-  if (tid < 3) n[tid] = 0u;
+  if (tid < 5) n[tid] = 0u;
   __syncthreads();
-  const bool live = k < nz && j < ny;
-  bool one = false, more = false;
-  if (live) {
+  bool has[5] = {k < nz && j < ny, false, false, false, false};
+  if (has[0]) {
     uint32_t t[V];
     wld(word + ((long long)blockIdx.z * ny + j) * pz + k, t);
     int np = 0;
     long long rec = 0;
-    const bool run = ade_run<T>(media, t, np, rec);
+    if (ade_run<T>(media, t, np, rec)) {
+      has[1] = np == 1;
+      has[2] = np == 2;
+    } else {
 #pragma unroll
-    for (int q = 0; q < V; ++q)
-      if (t[q] & kDispersiveBit) {
-        const int p = media[(t[q] >> kMediumShift) & 15u].npole;
-        one = one || (p == 1 && !run);
-        more = more || (p > 1 && (sizeof(T) == 8 || !run));
-      }
+      for (int q = 0; q < V; ++q)
+        if (t[q] & kDispersiveBit) {
+          const int p = media[(t[q] >> kMediumShift) & 15u].npole;
+          has[3] = has[3] || p == 1;
+          has[4] = has[4] || p > 1;
+        }
+    }
   }
-  const unsigned all = __ballot_sync(0xffffffffu, live), w1 = __ballot_sync(0xffffffffu, one),
-                 w2 = __ballot_sync(0xffffffffu, more);
-  if ((tid & 31) == 0) {
-    if (all) atomicAdd(&n[0], 1u);
-    if (w1) atomicAdd(&n[1], 1u);
-    if (w2) atomicAdd(&n[2], 1u);
-  }
+#pragma unroll
+  for (int q = 0; q < 5; ++q)
+    if (__ballot_sync(0xffffffffu, has[q]) && (tid & 31) == 0) atomicAdd(&n[q], 1u);
   __syncthreads();
-  if (tid < 3 && n[tid]) atomicAdd(&count[tid], (unsigned long long)n[tid]);
+  if (tid < 5 && n[tid]) atomicAdd(&count[tid], (unsigned long long)n[tid]);
 }
 
 // One dispersive cell, any pole count, state read and written in place.
