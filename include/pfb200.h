@@ -276,7 +276,7 @@ int pf_set_check_every(pf_engine *eng, int64_t k);
  * every step waits once on a barrier that nothing arrives on, lets its issued
  * copies land, sets the error flag and leaves. In a resident launch of a small
  * grid (the cooperative forms; a cluster's hardware barrier cannot run out)
- * block 0 waits for arrivals that never come, and every block gives up.
+ * every block waits for arrivals that never come and gives up.
  * pf_advance then returns PF_ERR_TIMEOUT and the fields are invalid.
  * on == 2: the engine finds that its context has no room for resident launches
  * (many steps per launch of a small grid) and launches every pass by itself;

@@ -121,7 +121,7 @@ struct QCheck<double, SCALED, CHAIN> {
 // The same for single numerators that are not prescaled.
 template <typename T, typename... N>
 __device__ __forceinline__ bool qdiv_ok(N... n) {
-  QCheck<T, false> c;
+  QCheck<T, false, true> c;
   (c.take(n), ...);
   return c.ok() || (c.kAgain && (c.sure(n) && ...));
 }
@@ -263,7 +263,7 @@ struct StepArgs {
   T* P;
   long long plev;  // reals per polarisation level
   int lvl;         // polarisation level holding P^n (n & 1)
-  int wait_test;   // test hook: a bounded wait runs out (pf_set_wait_test)
+  int wait_test;   // test hook of the TMA-staged step (pf_set_wait_test)
 };
 
 enum CeMode { kCeCell1 = 0, kCeCell3 = 1, kCeTable = 2 };

@@ -1213,6 +1213,8 @@ int launch_resident(pf_engine* e, long long n, long long* took) {
   if (!e->res_err.p) e->res_err = err_word(e->device, e->stream);
   if (!e->res_err.p) return kResRefused;
   g.bar = e->res_bar;
+  g.spin = e->wait_test == 1 ? kResSpinTest : kResSpin;
+  g.phase0 = e->wait_test == 1 ? 1u << 30 : 0u;
   PF_CUDA(e, cudaHostGetDevicePointer((void**)&g.err, e->res_err.p, 0));
   const bool ade = e->n_media > 0;
   int rc;

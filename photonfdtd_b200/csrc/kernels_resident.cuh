@@ -60,15 +60,17 @@ struct ResidentArgs {
   T* flux_val[kFluxBatch];  // [slot][plane cell]
   int flux_slot[kFluxBatch];
   unsigned* bar;            // grid barrier: arrivals (zero at launch)
+  // polls before a barrier gives up, arrivals counted as missing before the first
+  // one. The test hook gives few polls and arrivals that never come; as data they
+  // cost nothing (a test of the hook in the barrier cost 1 to 2% of a step).
+  int spin;
+  unsigned phase0;
   int* err;                 // set when a barrier gave up
 };
 
-// Barrier over the launch; false when the grid barrier gave up. Test hook
-// (wait_test): block 0 waits for a count that is never reached, gives up and
-// leaves, and every other block gives up at the barrier after.
+// Barrier over the launch; false when the grid barrier gave up.
 template <int MODE>
-__device__ __forceinline__ bool res_barrier(unsigned* bar, unsigned& phase, int* err,
-                                            int wait_test) {
+__device__ __forceinline__ bool res_barrier(unsigned* bar, unsigned& phase, int* err, int limit) {
   if (MODE == kResCell1) {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
     return true;
@@ -79,12 +81,11 @@ __device__ __forceinline__ bool res_barrier(unsigned* bar, unsigned& phase, int*
   if (threadIdx.x == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
     unsigned v;
-    int left = wait_test ? kResSpinTest : kResSpin;
-    const unsigned want = wait_test && blockIdx.x == 0 ? ~0u : phase;
+    int spin = 0;
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-    } while (v < want && --left > 0);
-    if (v < want) {
+    } while (v < phase && ++spin < limit);
+    if (v < phase) {
       *(volatile int*)err = 1;
       bad = 1;
     }
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(res_threads<T>(MODE), res_blocks<T>(MODE))
   const int n[3] = {a.nx, a.ny, a.nz};
   const long long st[3] = {(long long)a.ny * a.pz, a.pz, 1};
   const T Kh[3] = {-a.ch, -a.ch, -a.ch};
-  unsigned phase = 0;
+  unsigned phase = g.phase0;
   // source groups on this thread's cells (few groups), else a barrier and
   // one thread per group
   unsigned mine[2] = {0u, 0u};
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(res_threads<T>(MODE), res_blocks<T>(MODE))
       }
     }
     if (shared_h) {
-      if (!res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
+      if (!res_barrier<MODE>(g.bar, phase, g.err, g.spin)) return;
       for (int q = (int)me; q < g.src[1].n_groups; q += (int)nthr)
         inject_group<T>(g.src[1], q, a.Hout, step);
     } else {
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(res_threads<T>(MODE), res_blocks<T>(MODE))
     }
     AdeRec<T> rec;
     if (ADE && ONE && live && w) ade_load<T>(a, a.media, w, rec);  // its own: no barrier needed
-    if (!res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
+    if (!res_barrier<MODE>(g.bar, phase, g.err, g.spin)) return;
     // ---- E pass
     if (ONE) {
       if (live) {
@@ -355,10 +356,10 @@ __global__ void __launch_bounds__(res_threads<T>(MODE), res_blocks<T>(MODE))
       }
     }
     if (shared_e) {
-      if (!res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
+      if (!res_barrier<MODE>(g.bar, phase, g.err, g.spin)) return;
       for (int q = (int)me; q < g.src[0].n_groups; q += (int)nthr)
         inject_group<T>(g.src[0], q, a.Eout, step);
-      if (ONE && !res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
+      if (ONE && !res_barrier<MODE>(g.bar, phase, g.err, g.spin)) return;
     } else {
       for (unsigned left = mine[0]; left; left &= left - 1u)
         inject_group<T>(g.src[0], __ffs(left) - 1, a.Eout, step);
@@ -396,9 +397,9 @@ __global__ void __launch_bounds__(res_threads<T>(MODE), res_blocks<T>(MODE))
               p.axis == 0 ? v0 : (p.axis == 1 ? v1 : v2);
         }
       }
-      if (!shared_e && !res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
+      if (!shared_e && !res_barrier<MODE>(g.bar, phase, g.err, g.spin)) return;
     } else {
-      if (!res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
+      if (!res_barrier<MODE>(g.bar, phase, g.err, g.spin)) return;
       bool due = g.n_flux > 0;
       Fields6<T> F;
 #pragma unroll
@@ -422,7 +423,7 @@ __global__ void __launch_bounds__(res_threads<T>(MODE), res_blocks<T>(MODE))
           g.flux_val[m][(g.flux_slot[m] + s) * np + t] =
               flux_cell_value<T>(p, t, F, a.ny, a.pz);
       }
-      if (due && !res_barrier<MODE>(g.bar, phase, g.err, a.wait_test)) return;
+      if (due && !res_barrier<MODE>(g.bar, phase, g.err, g.spin)) return;
     }
   }
   if (live) {

@@ -1,9 +1,8 @@
 """The grid barrier of resident launches is bounded.
 
-With the test hook one block waits for arrivals that never come: it gives up
-after a few milliseconds, the other blocks give up at their next barrier, the
-kernel ends, and pf_advance reports PF_ERR_TIMEOUT. The next engine is right:
-the context survived.
+With the test hook every block waits for arrivals that never come and gives up
+after a few milliseconds, the kernel ends, and pf_advance reports
+PF_ERR_TIMEOUT. The next engine is right: the context survived.
 """
 import numpy as np
 import pytest
