@@ -784,9 +784,10 @@ __device__ __forceinline__ void tile_step(const BArgs<T>& a, const StepPost<T>& 
 // per lane cut its instructions but also its warps and was slower (457 us).
 // Here every thread issues eight vectors at once and has no loop; the Hz it
 // recomputes costs 13 operations per cell. us per step, marching -> this: 256
-// instances (36.1M cells) forward 373 -> 321, reverse 424 -> 379, 8 instances
+// instances (36.1M cells) forward 376 -> 307, reverse 428 -> 381, 8 instances
 // (1.5M cells) 37 -> 14 and 31 -> 14. The bulk tiles alone (about four fifths)
-// take 180 us of the 321; scalar CPML code in 32-column edge tiles cost 70 more.
+// took 180 us of 321 (before the range test became a chain of compares); scalar
+// CPML code in 32-column edge tiles cost 70 more.
 template <typename T, bool EDGE>
 __global__ void __launch_bounds__(32 * tile_x<T>(false), sizeof(T) == 4 ? (EDGE ? PFB_MINB_EDGE : PFB_MINB_TILE) : 1) kb_tile(const __grid_constant__ BArgs<T> a,
                                                              const __grid_constant__ StepPost<T> post,

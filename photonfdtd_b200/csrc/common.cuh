@@ -30,19 +30,20 @@ __device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(
 // prescaled by a power of two (exact), so that rem cannot underflow for any
 // a down to the smallest subnormal, and the quotient is scaled back at the
 // end; rem is formed as q0 d - a, which keeps the sign of a zero quotient.
-//  float: prescale 2^64. The host enables it for a divisor d in [2^-30,
-//    2^-23] only after checking all 2^23 significands of a against IEEE
-//    division. |a| < 2^26 keeps every intermediate below 2^121, and a
-//    quotient is 0 or at least 2^-126, so scaling it back is exact.
+//  float: prescale 2^64. Enabled for a divisor d only after checking all 2^23
+//    significands of a against IEEE division. For d in [2^-30, 2^-23], |a| <
+//    2^26 keeps every intermediate below 2^121, and a quotient is 0 or at least
+//    2^-126, so scaling it back is exact; the 3D vector passes take other d with
+//    limits of their own (StepArgs::qtop, qlow).
 //  double: prescale 2^200, and one more correction: q0 can be two units off,
 //    q1 = RN(q0 - rem r) is one of the two neighbours of a / d, and from such
 //    a q1 Markstein's theorem makes the second correction the rounded
 //    quotient for every d whose significand is not all ones and r = RN(1/d)
-//    (the host checks that, and d in [2^-30, 2^-23]). a is 0 or 2^-1022 <=
+//    (the host checks that, and d in [2^-60, 1]). a is 0 or 2^-1022 <=
 //    |a| < 2^700, so that a quotient is normal and scaling it back exact.
 // Four FP32 (six FP64) operations per quotient and one to scale it back;
 // sums and differences of scaled quotients are the scaled sums and
-// differences, so a curl scales back once (kUnscale) instead of per term.
+// differences, so a curl scales back once instead of per term.
 template <typename T>
 struct QScale;
 template <>

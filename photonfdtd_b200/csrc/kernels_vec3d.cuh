@@ -8,9 +8,10 @@
 // tests that V cells of one row share. Rows are padded to 32 bytes
 // (StepArgs::pz), so every row's vectors are aligned. At 256^3 without CPML
 // the H pass now runs 88 instructions per cell at 5.5 TB/s of DRAM traffic
-// (84% of a plain copy), the E pass with ADE 181 at 5.05 TB/s. Step kernels
-// of the scalar passes and now, in us: 384^3 with ADE 1453, 1278; 301x287x263
-// with three coefficients 517, 409; 160x152x144 double 165, 145.
+// (84% of a plain copy), the E pass with ADE 181 at 5.05 TB/s. us per step with
+// the scalar passes and now: 384^3 with ADE (media aligned to vectors; others
+// take k_e_cell for the E half, see ade_by_cell) 1453, 1269; 301x287x263 with
+// three coefficients 480, 390; 160x152x144 double 146, 134.
 //
 // A warp covers a patch of rows (blockDim.x vectors along z); when every cell
 // of it lies in the bulk box (both differences, no CPML state) the warp takes
