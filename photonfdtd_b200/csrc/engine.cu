@@ -159,10 +159,10 @@ struct pf_engine {
   bool fused = false;
   double rdl[3] = {1, 1, 1};     // RN(1/d) in the real type, per axis
   bool fdiv[3] = {false, false, false};  // reciprocal division verified
-  bool ade_cells = false;        // E pass of a dispersive scene: one cell per thread
   bool vdiv = false;             // the same for the vector passes, all axes
   float qtop = 0;                // and its limits (StepArgs)
   uint32_t qlow = 0;
+  bool ade_cells = false;        // E pass of a dispersive scene: one cell per thread
   bool tma = false;      // fused path stages planes with TMA
   TmaMaps maps;
   int* tma_err = nullptr;
@@ -281,30 +281,39 @@ void launch_copy_rows(pf_engine* e, const RowCopies& c, int n, size_t elem, bool
   else k_copy_rows<uint64_t><<<g, 256, 0, e->stream>>>(c, get);
 }
 
-// Copies `rows` rows of nz elements between a host array and a device array with
-// the engine's row pitch, through the staging buffer (free for the next copy only
-// in stream order).
-int copy_rows(pf_engine* e, void* padded, void* compact, size_t rows, size_t elem, bool to_padded) {
-  const size_t w = (size_t)e->nz * elem, p = (size_t)e->pz * elem, bytes = rows * w;
-  const cudaMemcpyKind kind = to_padded ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
-  if (bytes == 0) return PF_OK;
-  if (w == p) {
-    PF_CUDA(e, cudaMemcpyAsync(to_padded ? padded : compact, to_padded ? compact : padded, bytes,
-                               kind, e->stream));
-    return PF_OK;
-  }
-  int rc = stage(e, bytes);
+// Copies between a compact array (kind says where it lies) and `rows` rows of w
+// elements, p apart, through the staging buffer, kStage bytes at a time: the
+// buffer is free for the next piece in stream order.
+constexpr size_t kStage = 256u << 20;
+int copy_staged(pf_engine* e, void* padded, void* compact, size_t rows, int w, int p,
+                const int* pos, size_t elem, cudaMemcpyKind kind, bool to_padded) {
+  const size_t row = (size_t)w * elem;
+  const size_t most = std::max<size_t>(1, kStage / row);  // rows of one piece
+  int rc = stage(e, std::min(most, rows) * row);
   if (rc) return rc;
-  if (to_padded) PF_CUDA(e, cudaMemcpyAsync(e->region, compact, bytes, kind, e->stream));
-  const size_t most = 0x7fffffffu / (unsigned)e->nz;  // rows of one launch
   for (size_t r = 0; r < rows; r += most) {
+    const size_t n = std::min(most, rows - r);
+    char* at = (char*)compact + r * row;
+    if (to_padded) PF_CUDA(e, cudaMemcpyAsync(e->region, at, n * row, kind, e->stream));
     RowCopies c = {};
-    c.r[0] = row_copy((char*)padded + r * p, (char*)e->region + r * w, std::min(most, rows - r),
-                      e->nz, e->pz, nullptr);
+    c.r[0] = row_copy((char*)padded + r * p * elem, e->region, n, w, p, pos);
     launch_copy_rows(e, c, 1, elem, !to_padded);
+    PF_CUDA(e, cudaGetLastError());
+    if (!to_padded) PF_CUDA(e, cudaMemcpyAsync(at, e->region, n * row, kind, e->stream));
   }
-  PF_CUDA(e, cudaGetLastError());
-  if (!to_padded) PF_CUDA(e, cudaMemcpyAsync(compact, e->region, bytes, kind, e->stream));
+  return PF_OK;
+}
+
+// Copies `rows` rows of nz elements between a host array and a device array with
+// the engine's row pitch.
+int copy_rows(pf_engine* e, void* padded, void* compact, size_t rows, size_t elem, bool to_padded) {
+  const cudaMemcpyKind kind = to_padded ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+  const size_t bytes = rows * e->nz * elem;
+  if (bytes == 0) return PF_OK;
+  if (e->nz != e->pz)
+    return copy_staged(e, padded, compact, rows, e->nz, e->pz, nullptr, elem, kind, to_padded);
+  PF_CUDA(e, cudaMemcpyAsync(to_padded ? padded : compact, to_padded ? compact : padded, bytes,
+                             kind, e->stream));
   return PF_OK;
 }
 
@@ -1090,11 +1099,11 @@ struct Advancing {
 };
 constexpr long long kResChunk = 512;
 
-// Not a status of the ABI: this engine cannot have resident launches (a context
+// Not a status of the ABI (those are 0 and below): this engine cannot have resident launches (a context
 // with fewer SMs than the grid or cluster needs, or no memory for what they
 // take besides). Nothing was launched or counted; its steps go on as separate
 // launches.
-constexpr int kResRefused = -1;
+constexpr int kResRefused = 1;
 
 template <typename T, int CE, bool ADE, int MODE>
 int launch_resident_as(pf_engine* e, const ResidentArgs<T>& g) {
@@ -1138,7 +1147,7 @@ int launch_resident_as(pf_engine* e, const ResidentArgs<T>& g) {
   if (MODE != kResCell1) PF_CUDA(e, cudaMemsetAsync(g.bar, 0, sizeof(unsigned), e->stream));
   const cudaError_t rc = cudaLaunchKernelEx(&cfg, fn, g);
   if (rc == cudaErrorCooperativeLaunchTooLarge || rc == cudaErrorInvalidClusterSize ||
-      rc == cudaErrorLaunchOutOfResources) {
+      rc == cudaErrorLaunchOutOfResources || rc == cudaErrorNotSupported) {
     cudaGetLastError();
     return kResRefused;
   }
@@ -1852,6 +1861,7 @@ int pf_read_field(pf_engine* e, int comp, void* dst) {
   if (!e || !dst) return PF_ERR_INVALID;
   if (!e->finalized) return fail(e, PF_ERR_STATE, "pf_read_field before pf_finalize");
   if (!valid_comp(comp)) return fail(e, PF_ERR_INVALID, "bad component %d", comp);
+  PF_CUDA(e, cudaSetDevice(e->device));
   void* src = comp < 3 ? e->E[e->cur][comp] : e->H[e->cur][comp - 3];
   int rc = copy_rows(e, src, dst, (size_t)e->nx * e->ny, e->rb, false);
   if (rc) return rc;
@@ -1985,6 +1995,9 @@ int copy_state(pf_engine* e, long long step, void* buf, int64_t bytes, int on_de
   PF_CUDA(e, cudaSetDevice(e->device));
   const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice
                                         : (get ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice);
+  // device blobs aligned to their type are read and written as they lie, all
+  // arrays in one launch; others go through the staging buffer
+  const bool direct = on_device && (uintptr_t)buf % e->rb == 0;
   size_t off = 0;
   RowCopies c = {};
   int n = 0;
@@ -1997,20 +2010,14 @@ int copy_state(pf_engine* e, long long step, void* buf, int64_t bytes, int on_de
       PF_CUDA(e, cudaMemcpyAsync(get ? b : p.p, get ? p.p : b, p.bytes, kind, e->stream));
       continue;
     }
-    void* dense = b;
-    const bool direct = on_device && (uintptr_t)b % e->rb == 0;
-    if (!direct) {
-      int rc = stage(e, p.bytes);
+    const size_t rows = p.rows ? p.rows : (size_t)e->nx * e->ny;
+    const int w = p.rows ? e->nz : p.nc, pitch = p.rows ? e->pz : p.np;
+    if (direct) {
+      c.r[n++] = row_copy(p.p, b, rows, w, pitch, p.zpos);
+    } else {
+      int rc = copy_staged(e, p.p, b, rows, w, pitch, p.zpos, e->rb, kind, !get);
       if (rc) return rc;
-      dense = e->region;
-      if (!get) PF_CUDA(e, cudaMemcpyAsync(dense, b, p.bytes, kind, e->stream));
     }
-    c.r[n++] = p.rows ? row_copy(p.p, dense, p.rows, e->nz, e->pz, nullptr)
-                      : row_copy(p.p, dense, (size_t)e->nx * e->ny, p.nc, p.np, p.zpos);
-    if (direct) continue;  // all of them in one launch below
-    launch_copy_rows(e, c, 1, e->rb, get);
-    n = 0;
-    if (get) PF_CUDA(e, cudaMemcpyAsync(b, dense, p.bytes, kind, e->stream));
   }
   if (n) launch_copy_rows(e, c, n, e->rb, get);
   PF_CUDA(e, cudaGetLastError());

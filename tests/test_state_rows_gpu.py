@@ -75,3 +75,20 @@ def test_blob_rows(shape, pml, precision):
     finally:
         a.close()
         b.close()
+
+
+def test_fields_larger_than_the_staging_buffer():
+    """72 million cells, 289 MB a field: two pieces of the staging buffer."""
+    shape = (300, 600, 401)
+    d = 20e-9
+    grid = pf.Grid(size=tuple(n * d for n in shape), cell_size=d, pml_layers=0)
+    t = build_tables(pf.Simulation(grid, run_time=1e-16, precision="float32"))
+    f = np.random.default_rng(1).standard_normal(shape, dtype=np.float32)
+    eng = B200Engine(t)
+    try:
+        eng.set_field("Ey", f)
+        eng._cache.clear()
+        np.testing.assert_array_equal(eng.get("Ey"), f)
+        assert not eng.get("Ex").any() and not eng.get("Ez").any()
+    finally:
+        eng.close()
