@@ -298,7 +298,8 @@ int pf_read_profile(pf_engine *eng, int64_t launches[4], double ms[4], int reset
 
 /* Engine configuration as "key=value" pairs separated by spaces (kernel
  * path, tile shape, x chunks, reciprocal-division axes, coefficient mode,
- * media), written NUL-terminated into buf (at most len bytes). */
+ * media, form of the E pass), written NUL-terminated into buf (at most len
+ * bytes). */
 int pf_info(const pf_engine *eng, char *buf, int len);
 
 /* Device bytes held by the engine. */
