@@ -218,7 +218,7 @@ struct DftRegion {
 template <typename T>
 struct StepArgs {
   int nx, ny, nz;
-  int pz;  // reals from one row to the next: nz padded to 32 bytes (1 when nz = 1)
+  int pz;  // reals from one row to the next: nz padded to 32 bytes, or 16 (1 when nz = 1)
   T dx, dy, dz;  // derivative divisors (1 on a collapsed axis)
   T rdx, rdy, rdz;      // RN(1/d) per axis
   bool fdx, fdy, fdz;   // reciprocal division verified exact for that axis

@@ -5,8 +5,8 @@
 // too. What bounds a step here is memory latency and issue slots, not FLOPs:
 // with one cell per thread the passes ran 222 (H) and 414 (E with ADE)
 // instructions per cell at 4.2 TB/s, most of them addresses, bounds and CPML
-// tests that V cells of one row share. Rows are padded to 32 bytes
-// (StepArgs::pz), so every row's vectors are aligned. At 256^3 without CPML
+// tests that V cells of one row share. Rows are padded to 32 bytes, short
+// ones to 16 (StepArgs::pz), so every row's vectors are aligned. At 256^3 without CPML
 // the H pass now runs 88 instructions per cell at 5.5 TB/s of DRAM traffic
 // (84% of a plain copy), the E pass with ADE 181 at 5.05 TB/s. us per step with
 // the scalar passes and now: 384^3 with ADE (media aligned to vectors; others
