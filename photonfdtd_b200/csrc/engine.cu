@@ -160,7 +160,8 @@ struct pf_engine {
   double rdl[3] = {1, 1, 1};     // RN(1/d) in the real type, per axis
   bool fdiv[3] = {false, false, false};  // reciprocal division verified
   bool vdiv = false;             // the same for the vector passes, all axes
-  float qtop = 0;                // and its limits (StepArgs)
+  bool vwide = false;            // with limits other than the scalar passes' window gives
+  float qtop = 0;                // which are these (StepArgs)
   uint32_t qlow = 0;
   bool ade_cells = false;        // E pass of a dispersive scene: one cell per thread
   bool tma = false;      // fused path stages planes with TMA
@@ -420,6 +421,7 @@ int vector_division(pf_engine* e) {
     memcpy(&e->qlow, &low, 4);
     e->qlow = 2 * e->qlow - 1;
   }
+  e->vwide = e->qlow || e->qtop != 0x1p90f;
   return PF_OK;
 }
 
@@ -721,8 +723,8 @@ StepArgs<T> step_args(pf_engine* e) {
   a.fdz = e->fdiv[2];
   a.fdall = a.fdx && a.fdy && a.fdz;
   a.fdvec = e->vdiv;
-  a.qtop = e->vdiv ? (T)e->qtop : T(0);
-  a.qlow = e->vdiv ? e->qlow : 0u;
+  a.qtop = (T)e->qtop;
+  a.qlow = e->qlow;
   a.ch = (T)e->ch;
   for (int ax = 0; ax < 3; ++ax) {
     a.hb0[ax] = e->hb0[ax];
@@ -857,7 +859,7 @@ void launch_h(pf_engine* e, const StepArgs<T>& a, int i0, int i1) {
     const int nzv = (e->nz + kVec<T> - 1) / kVec<T>;
     const dim3 b(vec_lanes(nzv), kVecThreads / vec_lanes(nzv));
     launch_pdl(e->stream, dim3((nzv + b.x - 1) / b.x, (e->ny + b.y - 1) / b.y, i1 - i0), b,
-               sizeof(T) == 4 && a.qlow ? k_h_vec<T, sizeof(T) == 4> : k_h_vec<T, false>, a, i0);
+               sizeof(T) == 4 && e->vwide ? k_h_vec<T, sizeof(T) == 4> : k_h_vec<T, false>, a, i0);
     return;
   }
   const dim3 b = e->nz > 1 ? dim3(32, 8) : dim3(1, 256);
@@ -878,7 +880,7 @@ void launch_e_mode(pf_engine* e, const StepArgs<T>& a, int i0, int i1) {
     const int nzv = (e->nz + kVec<T> - 1) / kVec<T>;
     const dim3 b(vec_lanes(nzv), kVecThreads / vec_lanes(nzv));
     launch_pdl(e->stream, dim3((nzv + b.x - 1) / b.x, (e->ny + b.y - 1) / b.y, i1 - i0), b,
-               sizeof(T) == 4 && a.qlow ? k_e_vec<T, CE, ADE, sizeof(T) == 4>
+               sizeof(T) == 4 && e->vwide ? k_e_vec<T, CE, ADE, sizeof(T) == 4>
                                         : k_e_vec<T, CE, ADE, false>, a, i0);
     return;
   }

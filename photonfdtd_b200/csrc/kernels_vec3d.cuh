@@ -106,20 +106,21 @@ static __global__ void k_recip_exact(float d, float r, int* bad) {
 }
 
 // Whether a vector's differences n(term, cell) may take the reciprocal path;
-// range: over all of them. LOW: a float grid with cells above 2^-23 m (119 nm),
-// whose small numerators give subnormal quotients, has a lower limit too (its
-// own kernels: tested at run time, the skipped loop cost the others 1%). The
+// range: over all of them. WIDE: a float grid with divisors outside [2^-30,
+// 2^-23] m, whose limits are its own (above 119 nm small numerators give
+// subnormal quotients, so there is a lower one too). It has its own kernels:
+// limits read at run time and a skipped loop cost the others 1%. The
 // scalar passes divide such grids by IEEE division; 24 of these bound a
 // vector's step. us at 200 nm, IEEE in line by the scalar passes, out of line by
-// the vector passes, and so: 192^3 float 179, 184, 124, with ADE 221, 239, 175;
+// the vector passes, and so: 192^3 float 179, 184, 123, with ADE 221, 239, 175;
 // 144^3 double 120, 168, 109.
-template <bool LOW, typename T, bool SCALED, typename N>
+template <bool WIDE, typename T, bool SCALED, typename N>
 __device__ __forceinline__ bool in_range(const StepArgs<T>& a, const QCheck<T, SCALED>& range,
                                          const N& n) {
   constexpr int V = kVec<T>;
   if constexpr (sizeof(T) == 4) {
-    bool fast = range.ok();
-    if (LOW && fast && a.qlow) {
+    bool fast = a.fdvec && range.ok();
+    if (WIDE && fast && a.qlow) {
       unsigned low = ~0u;
 #pragma unroll
       for (int t = 0; t < 6; ++t)
@@ -147,7 +148,7 @@ __device__ __forceinline__ bool in_range(const StepArgs<T>& a, const QCheck<T, S
 // Own values are prescaled once; a prescaled difference is then one FMA, and
 // the curl is scaled back once per component (QScale in common.cuh): 6.5
 // operations per term instead of 11. One range check covers the V cells.
-template <typename T, int SGN, int NC, bool LOW>
+template <typename T, int SGN, int NC, bool WIDE>
 __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][kVec<T>],
                                           const T (&K)[NC][kVec<T>], const T (&own)[3][kVec<T>],
                                           const T (&nb)[6][kVec<T>], T (&out)[3][kVec<T>]) {
@@ -155,7 +156,7 @@ __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][
   const T dl[3] = {a.dx, a.dy, a.dz};
   const T rl[3] = {a.rdx, a.rdy, a.rdz};
   const T up = QScale<T>::up;
-  QCheck<T, true> range(a.qtop);
+  QCheck<T, true> range(WIDE ? a.qtop : T(0x1p90));
   auto diff = [&](int t, int q) {
     const T os = mul_rn(own[term_comp(t)][q], up);
     return SGN > 0 ? fma_rn(nb[t][q], up, -os) : fma_rn(-nb[t][q], up, os);
@@ -175,7 +176,7 @@ __device__ __forceinline__ void curl_bulk(const StepArgs<T>& a, const T (&f)[3][
       out[c][q] = add_rn(f[c][q], mul_rn(mul_rn(sub_rn(dA, dB), QScale<T>::down), K[c % NC][q]));
     }
   }
-  if (!in_range<LOW>(a, range, diff)) {
+  if (!in_range<WIDE>(a, range, diff)) {
 #pragma unroll
     for (int q = 0; q < V; ++q) {
       T d[6];
@@ -217,7 +218,7 @@ __device__ __forceinline__ T cpml_term(T f, T k, T d, T b, T c, T& psi) {
 // each psi load waited behind the stores of the cell before it (256^3 with a
 // 12-cell layer on every face: the layers cost 70 us of 314, now 41 of 287; 29
 // of these are their bytes).
-template <typename T, int SGN, int NC, bool LOW>
+template <typename T, int SGN, int NC, bool WIDE>
 __device__ __forceinline__ void curl_general(const StepArgs<T>& a, const Cpml<T>& p, int i, int j,
                                              int k, const T (&f)[3][kVec<T>],
                                              const T (&K)[NC][kVec<T>],
@@ -243,7 +244,7 @@ __device__ __forceinline__ void curl_general(const StepArgs<T>& a, const Cpml<T>
   const T dl[3] = {a.dx, a.dy, a.dz};
   const T rl[3] = {a.rdx, a.rdy, a.rdz};
   T d[6][V];
-  QCheck<T, false> range(a.qtop);
+  QCheck<T, false> range(WIDE ? a.qtop : T(0x1p90));
 #pragma unroll
   for (int q = 0; q < V; ++q)
 #pragma unroll
@@ -252,7 +253,7 @@ __device__ __forceinline__ void curl_general(const StepArgs<T>& a, const Cpml<T>
       d[t][q] = SGN > 0 ? sub_rn(nb[t][q], o) : sub_rn(o, nb[t][q]);
       range.take(d[t][q]);
     }
-  if (in_range<LOW>(a, range, [&](int t, int q) { return d[t][q]; })) {
+  if (in_range<WIDE>(a, range, [&](int t, int q) { return d[t][q]; })) {
 #pragma unroll
     for (int q = 0; q < V; ++q)
 #pragma unroll
@@ -313,7 +314,7 @@ __device__ __forceinline__ bool warp_bulk(bool live, int i, int j, int k, const 
 }
 
 // H pass: H^{n+1/2} = H^{n-1/2} - ch (curl E^n + psi), planes i0 + blockIdx.z.
-template <typename T, bool LOW>
+template <typename T, bool WIDE>
 __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? PFB_MINB_HV : PFB_MINB_HV64)
     k_h_vec(const __grid_constant__ StepArgs<T> a, int i0) {
   pdl_enter();
@@ -347,7 +348,7 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? PFB_MINB_HV : PF
 #pragma unroll
   for (int q = 0; q < V; ++q) K[0][q] = -a.ch;
   if (box) {
-    curl_bulk<T, 1, 1, LOW>(a, f, K, own, nb, out);
+    curl_bulk<T, 1, 1, WIDE>(a, f, K, own, nb, out);
   } else {
     Cpml<T> p;
 #pragma unroll
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? PFB_MINB_HV : PF
       p.in[t] = a.psiHin[t];
       p.out[t] = a.psiHout[t];
     }
-    curl_general<T, 1, 1, LOW>(a, p, i, j, k, f, K, own, nb, out);
+    curl_general<T, 1, 1, WIDE>(a, p, i, j, k, f, K, own, nb, out);
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c) vst(a.Hout[c] + id, out[c]);
@@ -501,7 +502,7 @@ __device__ __forceinline__ void ade_cell(const StepArgs<T>& a, uint32_t w, T en0
 template <typename T, int CE, bool ADE>
 constexpr int kMinBlocksE = ADE || CE == kCeCell3 ? (sizeof(T) == 4 ? PFB_MINB_EVA : PFB_MINB_EVA64)
                                                   : (sizeof(T) == 4 ? PFB_MINB_EV : PFB_MINB_EV64);
-template <typename T, int CE, bool ADE, bool LOW>
+template <typename T, int CE, bool ADE, bool WIDE>
 __global__ void __launch_bounds__(kVecThreads, kMinBlocksE<T, CE, ADE>)
     k_e_vec(const __grid_constant__ StepArgs<T> a, int i0) {
   pdl_enter();
@@ -580,7 +581,7 @@ __global__ void __launch_bounds__(kVecThreads, kMinBlocksE<T, CE, ADE>)
     nb[2][q] = q > 0 ? own[0][q > 0 ? q - 1 : 0] : h0;
   }
   if (box) {
-    curl_bulk<T, -1, NC, LOW>(a, en, K, own, nb, e);
+    curl_bulk<T, -1, NC, WIDE>(a, en, K, own, nb, e);
   } else {
     Cpml<T> p;
 #pragma unroll
@@ -596,7 +597,7 @@ __global__ void __launch_bounds__(kVecThreads, kMinBlocksE<T, CE, ADE>)
       p.in[s] = a.psiEin[s];
       p.out[s] = a.psiE[s];
     }
-    curl_general<T, -1, NC, LOW>(a, p, i, j, k, en, K, own, nb, e);
+    curl_general<T, -1, NC, WIDE>(a, p, i, j, k, en, K, own, nb, e);
   }
   if (ADE) {
     if (vec) {
